@@ -21,10 +21,10 @@
 namespace qb {
 
 template <int N, bool ADJ>
-__global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchParams p) {
+__global__ void __launch_bounds__(Fft2<N>::T, 1) cluster_batch_kernel(const BatchParams p) {
   namespace cg = cooperative_groups;
   using F = Fft2<N>;
-  constexpr int E = F::E, D = F::D, G3 = F::G3, T = F::T, PITCH = F::PITCH;
+  constexpr int E = F::E, A = F::A, D = F::D, G3 = F::G3, T = F::T, PITCH = F::PITCH;
   cg::cluster_group cluster = cg::this_cluster();
   const int P = p.P;  // == cluster size
   const int m = (int)cluster.block_rank();
@@ -33,31 +33,22 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
   extern __shared__ float4 smem_raw[];
   float2* sm = reinterpret_cast<float2*>(smem_raw);
   float2* tw = sm + F::SM_FLOAT2;
-  float2* rowf = tw + N;
+  float2* rowf = tw + F::TW_FLOAT2;
   float2* colf = rowf + N;
   float* inten = reinterpret_cast<float*>(colf + N);
   int* rowmap = reinterpret_cast<int*>(inten + N * N);
   int* colmap = rowmap + N;
   float2* sKr = reinterpret_cast<float2*>(colmap + N);
   float2* sKc = sKr + (size_t)N * (p.S > 1 ? p.S - 1 : 0);
-  const bool sep = p.prop_r != nullptr;
+  const bool sep = p.prop_r != nullptr && p.sep_shared;
   __shared__ double red[32];
   __shared__ int nfred[32];  // per-warp non-finite counts
 
   const int tid = threadIdx.x;
   F f;
   f.init(tid);
-  for (int k = tid; k < N; k += T) {
-    double s, c;
-    sincospi(-2.0 * (double)k / (double)N, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
-  }
-  if (sep) {
-    for (int k = tid; k < (p.S - 1) * N; k += T) {
-      sKr[k] = p.prop_r[k];
-      sKc[k] = p.prop_c[k];
-    }
-  }
+  F::fill_twiddles(tw, tid, T);
+  if (sep) load_prop_factors<N>(p, sKr, sKc);
   const float inv_n = 1.0f / (float)N;
   const float inv_n2 = inv_n * inv_n;
   const size_t NN = (size_t)N * N;
@@ -104,7 +95,7 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
       }
     }
     __syncthreads();
-    const int orow = rowmap[f.s1_r];
+    const int cin = (c0 >= N / 2 && c0 + N / 2 <= p.Wo) ? c0 + f.s1_cB : -1;
 
     // One loop with a single inverse and a single forward transform site walks
     // the whole chain of mode m: probe shift, S slices, detector, loss and (ADJ)
@@ -126,7 +117,7 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
     while (true) {
       f.inverse(x, sm, tw);
       // ---------------- real space (S1 layout) ----------------
-      const float2* orow_ptr = p.obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
+      const float2* slice = p.obj + (size_t)s * HoWo;
       if (!bwd) {
 #pragma unroll
         for (int e = 0; e < E; ++e) x[e] = cscale(x[e], inv_n2);
@@ -136,15 +127,15 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
           for (int e = 0; e < E; ++e) wv[e * T + tid] = x[e];
         }
         if (p.out_waves) {
-          float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN + (size_t)f.s1_r * N;
+          float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) ow[f.s1_col(e)] = x[e];
+          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
         }
-        gather_mul<N, false>(f, x, orow_ptr, colmap, evict_last_policy());
+        gather_mul<N, false>(f, x, slice, p.Wo, rowmap, colmap, cin);
         if (s == S - 1 && p.out_exit) {
-          float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN + (size_t)f.s1_r * N;
+          float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) oe[f.s1_col(e)] = x[e];
+          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
         }
       } else {
         const float sc = first_bwd ? inv_n : inv_n2;  // adjoint of the orthonormal FFT, or of a propagation
@@ -158,7 +149,7 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
 #pragma unroll
           for (int j = 0; j < 8; ++j) ps[j] = wv[(e0 + j) * T + tid];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) sm[f.s1_r * PITCH + f.s1_col(e0 + j)] = cmulc(x[e0 + j], ps[j]);
+          for (int j = 0; j < 8; ++j) sm[f.s1_row((e0 + j) / A) * PITCH + f.s1_col((e0 + j) % A)] = cmulc(x[e0 + j], ps[j]);
         }
         cluster.sync();  // every mode's contribution tile is in place
         float2* grow_s = p.grad_obj + (size_t)s * HoWo;
@@ -170,7 +161,7 @@ __global__ void __launch_bounds__(4 * N, 1) cluster_batch_kernel(const BatchPara
           atomicAdd(grow_s + (size_t)rowmap[r] * p.Wo + colmap[c], a);
         }
         cluster.sync();  // all tiles read before any exchange buffer is reused
-        gather_mul<N, true>(f, x, orow_ptr, colmap, evict_last_policy());
+        gather_mul<N, true>(f, x, slice, p.Wo, rowmap, colmap, cin);
       }
       f.forward(x, sm, tw);
       // ---------------- Fourier space (S3 layout) ----------------

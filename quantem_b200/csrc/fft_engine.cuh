@@ -1,6 +1,6 @@
 // Register-resident 2-D FFT engine for one N x N complex64 wave per CTA (sm_100a).
 //
-// A CTA of T = 4N threads holds the wave in registers, E = N/4 complex values per
+// A CTA of T threads holds the wave in registers, E = N^2 / T complex values per
 // thread.  The 2-D transform is factored into three register stages that each
 // consume a subset of the 2*log2(N) index bits, with one shared-memory exchange
 // between consecutive stages:
@@ -19,11 +19,25 @@
 // an exchange.  One multislice step (FFT, propagator, IFFT, transmission) costs
 // four exchanges.
 //
-// Shared-memory layout: float2 sm[N][N+1] (one padding column).  With the lane
-// assignments below every stage's 32 lanes touch each bank pair at most twice,
-// i.e. two wavefronts per 256-byte warp access, the minimum for 8-byte words.
+// Exchanges.  The rows rD + D*rC of one residue rD form a class: S1 and S2 of a class
+// touch no other class, and one warp owns whole classes (A threads each), so the
+// exchange between S1 and S2 stays inside the warp (__syncwarp).  Only S2 <-> S3 crosses
+// warps, with each side reading and writing the same elements in place: one
+// __syncthreads per transform.  The class's transpose (A x (B C), padded) and its C rows
+// of N spectral values share the class's region of the buffer.  Every warp access is two
+// wavefronts per 256 bytes, the minimum for 8-byte words.
 //
-// Supported N: 64 (A=16,B=4,C=4,D=16, 256 threads) and 128 (A=32,B=4,C=8,D=16,
+// The load/store unit's data pipe is the busiest unit of the batch kernels (58 % at 128^2
+// against 47 % of the FP32 pipe and 37 % of the issue slots), so the factorisation is
+// chosen for the real-space accesses: B = 8 puts 8 consecutive columns x 4 rows in a warp
+// access of the object (B = 4: 4 columns x 8 rows took 3.7 L1 wavefronts per gather and
+// 4.6 per gradient scatter, B = 8 takes 1.7 and 2.3: 28.5 -> 26.4 ms per 4096-position
+// launch).  At 64^2 B = 4 keeps 16 registers per thread, half the code and three CTAs per
+// SM (256 threads of 80 registers); B = 8 with 32 registers and four CTAs of 128 threads
+// was 5-15 % slower on single-slice and forward-only launches, its code no longer fitting
+// the instruction caches (no-instruction stalls 1.4 per issue against 0.3).
+//
+// Supported N: 64 (A=16,B=4,C=4,D=16, 256 threads) and 128 (A=16,B=8,C=4,D=32,
 // 512 threads); 96 is a specialisation at the end of this file (192 threads,
 // mixed radix 3 x 2^k).
 #pragma once
@@ -41,9 +55,9 @@ namespace qb {
 //   a * b       = (fma(a.x, b.x, -(a.y b.y)), fma(a.x, b.y, a.y b.x))
 //   a * conj(b) = (fma(a.x, b.x, a.y b.y),    fma(a.y, b.x, -(a.x b.y)))
 // so results are bit-identical either way.  The packed operands live in aligned
-// register pairs, which costs registers: packed products pay in the 64^2, 96^2 and
-// 256^2 kernels but not in the 128^2 batch kernel, whose 512 threads already sit at
-// 128 registers (it packs only its additions).
+// register pairs, which costs registers: packed products pay everywhere but in the 128^2
+// kernels with extensions or the analytic update (they pack their additions and the
+// middle-stage twiddles).
 #ifndef QB_F32X2_ADD
 #define QB_F32X2_ADD 0
 #endif
@@ -175,115 +189,153 @@ __device__ __forceinline__ void dft_reg(float2 (&x)[LEN]) {
 // 2-D engine
 // ---------------------------------------------------------------------------
 template <int N> struct FftCfg;
-template <> struct FftCfg<64> { static constexpr int A = 16, B = 4, C = 4, D = 16; };
-template <> struct FftCfg<128> { static constexpr int A = 32, B = 4, C = 8, D = 16; };
+template <> struct FftCfg<64> { static constexpr int A = 16, B = 4, C = 4, D = 16, CTAS = 3; };
+template <> struct FftCfg<128> { static constexpr int A = 16, B = 8, C = 4, D = 32, CTAS = 1; };
 
 template <int N>
 struct Fft2 {
   static constexpr int A = FftCfg<N>::A, B = FftCfg<N>::B, C = FftCfg<N>::C, D = FftCfg<N>::D;
-  static constexpr int T = 4 * N;        // threads per CTA
-  static constexpr int E = N / 4;        // complex registers per thread
+  static constexpr int E = B * C;        // complex registers per thread
+  static constexpr int T = N * N / E;    // threads per CTA
+  static constexpr int CTAS = FftCfg<N>::CTAS;  // resident CTAs per SM of the batch kernels
+  static constexpr int G1 = E / A;       // S1 groups per thread
   static constexpr int G3 = E / D;       // S3 groups per thread
-  static constexpr int PITCH = N + 1;    // shared-memory row pitch (float2)
-  static constexpr int SM_FLOAT2 = N * PITCH;
+  static constexpr int PITCH = N + 1;    // row pitch of a plain N x N tile kept in this buffer
+  static constexpr int PP = B * C + 1;   // pitch of a class's A x (B C) transpose
+  static constexpr int CS = A * PP;      // class stride: its transpose, or its C rows of N
+  static constexpr int SM_FLOAT2 = D * CS;
   static_assert(A * B == N && C * D == N, "bad factorisation");
-  static_assert(B * C == E && G3 * D == E && A == E, "stage sizes must match");
+  static_assert(G3 * D == E && G1 * A == E, "stage sizes must match");
+  static_assert(CS >= C * N && SM_FLOAT2 >= N * PITCH, "buffer too small");
+  static_assert(D * A == T && 32 % A == 0 && A % B == 0, "a warp owns whole classes");
 
   // stage coordinates of this thread
-  int s1_r, s1_cB;       // S1: row, column residue
-  int s2_rD, s2_kA;      // S2
+  int s1_r0, s1_cB;      // S1: row of group 0, column residue
+  int s2_rD, s2_kA;      // S2 (s2_rD: the class this thread works on in S1 and S2)
   int s3_c, s3_kC0;      // S3: column, first kC (group g adds 4*g)
+  int pv_w, pv_r;        // class-private transpose: S1 side, S2 side
+  int mn_3;              // main exchange, S3 side (the S2 side starts at pv_w)
 
   __device__ __forceinline__ void init(int tid) {
     const int lane = tid & 31, w = tid >> 5;
-    s1_cB = lane & 3;
-    s1_r = (w & 3) + 4 * (lane >> 2) + 32 * (w >> 2);
-    s2_rD = lane & 15;
-    s2_kA = (lane >> 4) + 2 * w;
+    const int cl = tid & (A - 1);  // thread within its class (A threads)
+    s2_rD = tid / A;
+    s2_kA = cl;
+    s1_cB = cl & (B - 1);
+    s1_r0 = s2_rD + D * (cl / B);
     constexpr int CW = N / 32;  // warps per 32-column strip
     s3_c = lane + 32 * (w % CW);
     s3_kC0 = w / CW;
+    pv_w = s2_rD * CS + cl;
+    pv_r = s2_rD * CS + PP * cl;
+    mn_3 = s3_kC0 * N + s3_c;
   }
   __device__ __forceinline__ int s3_kC(int g) const { return s3_kC0 + (T / 32 / (N / 32)) * g; }
-  // natural (row, col) of S1 register e
+  // natural (row, col) of S1 register (g, e) = x[g A + e]
+  __device__ __forceinline__ int s1_row(int g) const { return s1_r0 + D * (A / B) * g; }
   __device__ __forceinline__ int s1_col(int e) const { return s1_cB + B * e; }
   // frequency row of S3 register (g, e)
   __device__ __forceinline__ int s3_row(int g, int e) const { return s3_kC(g) + C * e; }
 
-  // ---- exchanges (caller guarantees all prior reads of sm are complete) ----
+  // ---- class-private transpose between S1 and S2 (one warp, __syncwarp only) ----
+  // element (kA, line l = B rC + cB) of the class at kA PP + l; group g holds lines cl + A g
   __device__ __forceinline__ void write_s1(float2* sm, const float2 (&x)[E]) const {
 #pragma unroll
-    for (int e = 0; e < A; ++e) sm[s1_r * PITCH + s1_cB + B * e] = x[e];
+    for (int g = 0; g < G1; ++g)
+#pragma unroll
+      for (int e = 0; e < A; ++e) sm[pv_w + PP * e + A * g] = x[g * A + e];
   }
   __device__ __forceinline__ void read_s1(const float2* sm, float2 (&x)[E]) const {
 #pragma unroll
-    for (int e = 0; e < A; ++e) x[e] = sm[s1_r * PITCH + s1_cB + B * e];
+    for (int g = 0; g < G1; ++g)
+#pragma unroll
+      for (int e = 0; e < A; ++e) x[g * A + e] = sm[pv_w + PP * e + A * g];
   }
-  // S2 input layout (cB, rC): element (rD + D rC, cB + B kA)
+  // S2 input layout (cB, rC)
   __device__ __forceinline__ void read_s2_in(const float2* sm, float2 (&x)[E]) const {
 #pragma unroll
     for (int cB = 0; cB < B; ++cB)
 #pragma unroll
-      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = sm[(s2_rD + D * rC) * PITCH + cB + B * s2_kA];
+      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = sm[pv_r + B * rC + cB];
   }
   __device__ __forceinline__ void write_s2_in(float2* sm, const float2 (&x)[E]) const {
 #pragma unroll
     for (int cB = 0; cB < B; ++cB)
 #pragma unroll
-      for (int rC = 0; rC < C; ++rC) sm[(s2_rD + D * rC) * PITCH + cB + B * s2_kA] = x[cB * C + rC];
+      for (int rC = 0; rC < C; ++rC) sm[pv_r + B * rC + cB] = x[cB * C + rC];
   }
-  // S2 output layout (kB, kC): element (rD + D kC, kA + A kB)
+  // ---- main exchange between S2 and S3: element (rD, kC, column) at rD CS + kC N + column ----
+  // S2 output layout (kB, kC): column kA + A kB
   __device__ __forceinline__ void write_s2_out(float2* sm, const float2 (&x)[E]) const {
 #pragma unroll
     for (int kB = 0; kB < B; ++kB)
 #pragma unroll
-      for (int kC = 0; kC < C; ++kC) sm[(s2_rD + D * kC) * PITCH + s2_kA + A * kB] = x[kB * C + kC];
+      for (int kC = 0; kC < C; ++kC) sm[pv_w + N * kC + A * kB] = x[kB * C + kC];
   }
   __device__ __forceinline__ void read_s2_out(const float2* sm, float2 (&x)[E]) const {
 #pragma unroll
     for (int kB = 0; kB < B; ++kB)
 #pragma unroll
-      for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = sm[(s2_rD + D * kC) * PITCH + s2_kA + A * kB];
+      for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = sm[pv_w + N * kC + A * kB];
   }
-  // S3 layout (g, e): element (e + D kC_g, col)
+  // S3 layout (g, e): rD = e, kC = kC_g, column s3_c
   __device__ __forceinline__ void read_s3(const float2* sm, float2 (&x)[E]) const {
 #pragma unroll
     for (int g = 0; g < G3; ++g)
 #pragma unroll
-      for (int e = 0; e < D; ++e) x[g * D + e] = sm[(e + D * s3_kC(g)) * PITCH + s3_c];
+      for (int e = 0; e < D; ++e) x[g * D + e] = sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g];
   }
   __device__ __forceinline__ void write_s3(float2* sm, const float2 (&x)[E]) const {
 #pragma unroll
     for (int g = 0; g < G3; ++g)
 #pragma unroll
-      for (int e = 0; e < D; ++e) sm[(e + D * s3_kC(g)) * PITCH + s3_c] = x[g * D + e];
+      for (int e = 0; e < D; ++e) sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g] = x[g * D + e];
   }
 
   // ---- register stages ----
+  // G transforms of L consecutive registers each
+  template <int L, int G, bool INV, int K>
+  __device__ __forceinline__ void groups(float2 (&x)[E]) const {
+    if constexpr (K < G) {
+      dft_reg<L, INV, 1, K * L>(x);
+      groups<L, G, INV, K + 1>(x);
+    }
+  }
   template <bool INV>
-  __device__ __forceinline__ void s1(float2 (&x)[E]) const { dft_reg<A, INV, 1, 0>(x); }
+  __device__ __forceinline__ void s1(float2 (&x)[E]) const {
+    groups<A, G1, INV, 0>(x);
+  }
 
   template <bool INV>
   __device__ __forceinline__ void s3(float2 (&x)[E]) const {
-#pragma unroll
-    for (int g = 0; g < G3; ++g) {
-      if (g == 0) dft_reg<D, INV, 1, 0>(x);
-      else dft_reg<D, INV, 1, D>(x);  // G3 <= 2 for the supported sizes
-    }
+    groups<D, G3, INV, 0>(x);
   }
 
-  // S2 forward: x holds (cB, rC) on entry, (kB, kC) on exit.  tw = w_N^k table.
+  // S2 twiddles in the order the warps read them: w_N^(cB kA) at (cB - 1) A + kA (a
+  // class's lanes on consecutive words), then w_N^(rD kC) at TWC + (kC - 1) D + rD (one word
+  // per class).
+  static constexpr int TWC = (B - 1) * A;
+  static constexpr int TW_FLOAT2 = TWC + (C - 1) * D;
+  static __device__ __forceinline__ void fill_twiddles(float2* tw, int tid, int nthreads) {
+    for (int k = tid; k < TW_FLOAT2; k += nthreads) {
+      const int e = k < TWC ? (k / A + 1) * (k % A) : ((k - TWC) / D + 1) * ((k - TWC) % D);
+      double s, c;
+      sincospi(-2.0 * (double)e / (double)N, &s, &c);
+      tw[k] = make_float2((float)c, (float)s);
+    }
+  }
+  // S2 forward: x holds (cB, rC) on entry, (kB, kC) on exit.
   __device__ __forceinline__ void s2_fwd(float2 (&x)[E], const float2* tw) const {
 #pragma unroll
     for (int cB = 1; cB < B; ++cB) {
-      const float2 w = tw[(cB * s2_kA) & (N - 1)];
+      const float2 w = tw[(cB - 1) * A + s2_kA];
 #pragma unroll
       for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmul(x[cB * C + rC], w) : cmul(x[cB * C + rC], w);
     }
     s2_core<false>(x);
 #pragma unroll
     for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[(s2_rD * kC) & (N - 1)];
+      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
 #pragma unroll
       for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmul(x[kB * C + kC], w) : cmul(x[kB * C + kC], w);
     }
@@ -292,14 +344,14 @@ struct Fft2 {
   __device__ __forceinline__ void s2_inv(float2 (&x)[E], const float2* tw) const {
 #pragma unroll
     for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[(s2_rD * kC) & (N - 1)];
+      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
 #pragma unroll
       for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmulc(x[kB * C + kC], w) : cmulc(x[kB * C + kC], w);
     }
     s2_core<true>(x);
 #pragma unroll
     for (int cB = 1; cB < B; ++cB) {
-      const float2 w = tw[(cB * s2_kA) & (N - 1)];
+      const float2 w = tw[(cB - 1) * A + s2_kA];
 #pragma unroll
       for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmulc(x[cB * C + rC], w) : cmulc(x[cB * C + rC], w);
     }
@@ -325,16 +377,21 @@ struct Fft2 {
     }
   }
 
-  // ---- whole transforms between layouts (each exchange brackets with barriers) ----
+  // ---- whole transforms between layouts ----
+  // One CTA barrier each.  Between two barriers either every class is owned by its warp
+  // (S2 side: main exchange, private transpose, S1) or every (kC, column) pair by its
+  // thread (S3 side reads and writes the same elements), so no barrier is needed before
+  // a write.  A caller that leaves the S2 side (after inverse) without forward, or enters
+  // it (forward) without inverse, puts a __syncthreads between.
   // Forward: registers in S1 layout -> registers in S3 layout (unnormalised).
   __device__ __forceinline__ void forward(float2 (&x)[E], float2* sm, const float2* tw) const {
     s1<false>(x);
-    __syncthreads();
+    __syncwarp();  // the warp's reads of the inverse's transpose are complete
     write_s1(sm, x);
-    __syncthreads();
+    __syncwarp();
     read_s2_in(sm, x);
     s2_fwd(x, tw);
-    __syncthreads();
+    __syncwarp();
     write_s2_out(sm, x);
     __syncthreads();
     read_s3(sm, x);
@@ -343,14 +400,13 @@ struct Fft2 {
   // Inverse: registers in S3 layout -> registers in S1 layout (unnormalised).
   __device__ __forceinline__ void inverse(float2 (&x)[E], float2* sm, const float2* tw) const {
     s3<true>(x);
-    __syncthreads();
     write_s3(sm, x);
     __syncthreads();
     read_s2_out(sm, x);
     s2_inv(x, tw);
-    __syncthreads();
+    __syncwarp();
     write_s2_in(sm, x);
-    __syncthreads();
+    __syncwarp();
     read_s1(sm, x);
     s1<true>(x);
   }
@@ -465,8 +521,18 @@ struct Fft2<96> {
   static constexpr int N = 96, A = 48, B = 2, C = 24, D = 4;
   static constexpr int T = 192;
   static constexpr int E = 48;
+  static constexpr int G1 = 1;
+  static constexpr int CTAS = 1;
   static constexpr int G3 = 12;
   static constexpr int SM_FLOAT2 = 9976;
+  static constexpr int TW_FLOAT2 = N;
+  static __device__ __forceinline__ void fill_twiddles(float2* tw, int tid, int nthreads) {
+    for (int k = tid; k < N; k += nthreads) {
+      double s, c;
+      sincospi(-2.0 * (double)k / (double)N, &s, &c);
+      tw[k] = make_float2((float)c, (float)s);
+    }
+  }
 
   int s1_r, s1_cB;
   int s2_rD, s2_kA;
@@ -482,6 +548,7 @@ struct Fft2<96> {
     s3_kC0 = w / 3;
   }
   __device__ __forceinline__ int s3_kC(int g) const { return s3_kC0 + 2 * g; }
+  __device__ __forceinline__ int s1_row(int) const { return s1_r; }
   __device__ __forceinline__ int s1_col(int e) const { return s1_cB + B * e; }
   __device__ __forceinline__ int s3_row(int g, int e) const { return s3_kC(g) + C * e; }
 

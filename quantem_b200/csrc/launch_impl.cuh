@@ -43,12 +43,26 @@ inline BatchParams to_params(const ptycho_batch_args* a) {
   p.descan = a->descan;
   p.grad_descan = a->grad_descan;
   p.grad_prop = a->grad_prop;
+  p.sep_shared = 0;
   return p;
 }
 
+// dynamic shared memory of a launch with (tile) or without the intensity tile in it
 template <int N>
-size_t batch_smem(const ptycho_batch_args* a) {
-  return a->prop_r ? fused_smem_bytes_sep<N>(a->S) : fused_smem_bytes<N>();
+size_t batch_smem(const ptycho_batch_args* a, bool tile = true) {
+  return batch_smem_bytes<N>(tile, a->prop_r != nullptr && sep_in_smem<N>(tile, a->S), a->S);
+}
+// smallest shared-memory carve-out (percent) that holds the resident CTAs: the rest is L1
+template <int N>
+int carveout(size_t smem) {
+  const size_t pc = Fft2<N>::CTAS * (smem + 2048) * 100 / (228 * 1024) + 1;
+  return pc < 100 ? (int)pc : 100;
+}
+template <int N>
+BatchParams batch_params(const ptycho_batch_args* a, bool tile = true) {
+  BatchParams p = to_params(a);
+  p.sep_shared = sep_in_smem<N>(tile, a->S);
+  return p;
 }
 
 // the serial kernel with its optional extensions compiled in (descan, position / descan /
@@ -63,41 +77,54 @@ void launch_ext(const BatchParams& p, int grid, size_t smem, cudaStream_t st) {
                        (int)smem);
   if (ADJ)
     cudaFuncSetAttribute(fused_batch_kernel<N, ADJ, false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)((smem + 1024) * 100 / (228 * 1024) + 1));
+                         carveout<N>(smem));
   fused_batch_kernel<N, ADJ, false, true><<<grid, Fft2<N>::T, smem, st>>>(p);
 }
 
-// one CTA per position, modes in sequence
+// One CTA per position, modes in sequence.  The attributes are per device; setting them on
+// every launch keeps multi-device processes correct and costs far less than one launch.
+// The adjoint kernels take the smallest shared-memory carve-out that fits: the rest of the
+// 256 KB is L1.
 template <int N>
-int launch_serial(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const BatchParams p = to_params(a);
-  const size_t smem = adj ? batch_smem_bytes<N, true>(a->prop_r != nullptr, a->S)
-                          : batch_smem_bytes<N, false>(a->prop_r != nullptr, a->S);
-  if (wants_ext(a) && !a->analytic) {
-    if (adj)
-      launch_ext<N, true>(p, a->grid, smem, st);
-    else
-      launch_ext<N, false>(p, a->grid, smem, st);
-    return cudaPeekAtLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
-  }
-  // the attribute is per device; setting it on every launch keeps multi-device
-  // processes correct and costs far less than one launch
-  if (adj && a->analytic) {
-    cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)((smem + 1024) * 100 / (228 * 1024) + 1));
-    fused_batch_kernel<N, true, true><<<a->grid, Fft2<N>::T, smem, st>>>(p);
-  } else if (adj) {
+int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
+  const BatchParams p = batch_params<N>(a, !adj);
+  const size_t smem = batch_smem<N>(a, !adj);
+  if (adj) {
     cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // smallest shared-memory carve-out that fits: the rest of the 256 KB is L1 for spills
     cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)((smem + 1024) * 100 / (228 * 1024) + 1));
+                         carveout<N>(smem));
     fused_batch_kernel<N, true><<<a->grid, Fft2<N>::T, smem, st>>>(p);
   } else {
     cudaFuncSetAttribute(fused_batch_kernel<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     fused_batch_kernel<N, false><<<a->grid, Fft2<N>::T, smem, st>>>(p);
   }
   return cudaPeekAtLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
+}
+
+// the instances with the analytic update or with extensions
+template <int N>
+int launch_special(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
+  const BatchParams p = batch_params<N>(a, !adj);
+  const size_t smem = batch_smem<N>(a, !adj);
+  if (!a->analytic) {
+    if (adj)
+      launch_ext<N, true>(p, a->grid, smem, st);
+    else
+      launch_ext<N, false>(p, a->grid, smem, st);
+  } else {
+    cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         carveout<N>(smem));
+    fused_batch_kernel<N, true, true><<<a->grid, Fft2<N>::T, smem, st>>>(p);
+  }
+  return cudaPeekAtLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
+}
+
+inline bool wants_special(const ptycho_batch_args* a) { return a->analytic || wants_ext(a); }
+
+template <int N>
+int launch_serial(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
+  return wants_special(a) ? launch_special<N>(a, adj, st) : launch_plain<N>(a, adj, st);
 }
 
 // several datasets in one persistent launch (serial body, adjoint)
@@ -108,14 +135,14 @@ int launch_multi(const ptycho_batch_args* sets, int nsets, cudaStream_t st) {
   mp.begin[0] = 0;
   size_t smem = 0;
   for (int d = 0; d < nsets; ++d) {
-    mp.d[d] = to_params(&sets[d]);
+    mp.d[d] = batch_params<N>(&sets[d], false);
     mp.begin[d + 1] = mp.begin[d] + sets[d].grid;
-    const size_t sd = batch_smem_bytes<N, true>(sets[d].prop_r != nullptr, sets[d].S);
+    const size_t sd = batch_smem<N>(&sets[d], false);
     if (sd > smem) smem = sd;
   }
   cudaFuncSetAttribute(multi_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(multi_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                       (int)((smem + 1024) * 100 / (228 * 1024) + 1));
+                       carveout<N>(smem));
   multi_batch_kernel<N, true><<<mp.begin[nsets], Fft2<N>::T, smem, st>>>(mp);
   return cudaPeekAtLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
 }
@@ -124,7 +151,7 @@ template <int N, bool ADJ>
 cudaLaunchConfig_t cluster_config(const ptycho_batch_args* a, int grid, cudaStream_t st, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(4 * N, 1, 1);
+  cfg.blockDim = dim3(Fft2<N>::T, 1, 1);
   cfg.dynamicSmemBytes = batch_smem<N>(a);
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -162,7 +189,7 @@ int max_clusters(const ptycho_batch_args* a, bool adj) {
 
 template <int N>
 int launch_cluster(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const BatchParams p = to_params(a);
+  const BatchParams p = batch_params<N>(a);
   cudaLaunchAttribute attr[1];
   cudaError_t e;
   if (adj) {

@@ -1,8 +1,7 @@
 // Multi-dataset persistent batch kernel for a 128 x 128 probe window.
-// Complex additions and the middle-stage FFT twiddles on packed FP32 pairs; other
-// products stay scalar (fft_engine.cuh).
+// Complex arithmetic on packed FP32 pairs, as the plain adjoint kernel.
 #define QB_F32X2_ADD 1
-#define QB_F32X2_S2 1
+#define QB_F32X2_MUL 1
 #include "launch_impl.cuh"
 
 int qb_launch_multi_128(const ptycho_batch_args* sets, int nsets, cudaStream_t st) {

@@ -465,10 +465,7 @@ int validate_batch(const ptycho_batch_args* a, bool adj) {
   if ((a->prop_r == nullptr) != (a->prop_c == nullptr))
     return fail(PTYCHO_ERR_INVALID, "prop_r and prop_c must be given together");
   if (a->prop_r && a->n != 256) {  // n = 256 reads the factors through the L1 cache
-    const size_t need = (size_t)(a->n == 64 ? qb::fused_smem_bytes_sep<64>(a->S)
-                                            : (a->n == 96 ? qb::fused_smem_bytes_sep<96>(a->S)
-                                                          : qb::fused_smem_bytes_sep<128>(a->S)));
-    if (need + 1024 > 232448)
+    if (qb::sep_limit_bytes(a->n, a->S) > qb::kMaxSmem)
       return fail(PTYCHO_ERR_UNSUPPORTED, "separable propagators of %d slices do not fit in shared memory; pass prop",
                   a->S);
   }
@@ -603,7 +600,11 @@ int ptycho_batch_plan(const ptycho_batch_args* a, int adjoint, int* variant, int
     scr = (int64_t)g * a->S * nn;
     part = (int64_t)g * nn;
   } else {
-    g = B < sms ? B : sms;
+    // one CTA per resident slot: CTAS per SM for the small windows
+    const bool ext = a->analytic || qb::wants_ext(a);
+    const int slots = sms * (a->n == 64 ? qb::batch_ctas<64>(ext) : (a->n == 96 ? qb::batch_ctas<96>(ext)
+                                                                                 : qb::batch_ctas<128>(ext)));
+    g = B < slots ? B : slots;
     parts = g;
     // waves, far fields, intensity tile (+ the Fourier waves after each propagation)
     scr = (int64_t)g * (a->P * a->S + a->P + 1 + (a->grad_prop ? a->P * (a->S - 1) : 0)) * nn;
@@ -665,8 +666,8 @@ int ptycho_fft2(const void* in, void* out, int count, int n, int inverse, float 
   const int grid = count < 148 ? count : 148;
   if (n == 64) {
     const size_t smem = qb::fft2_smem_bytes<64>();
-    if (inverse) qb::fft2_batch_kernel<64, true><<<grid, 256, smem, st>>>(i2, o2, count, scale);
-    else qb::fft2_batch_kernel<64, false><<<grid, 256, smem, st>>>(i2, o2, count, scale);
+    if (inverse) qb::fft2_batch_kernel<64, true><<<grid, qb::Fft2<64>::T, smem, st>>>(i2, o2, count, scale);
+    else qb::fft2_batch_kernel<64, false><<<grid, qb::Fft2<64>::T, smem, st>>>(i2, o2, count, scale);
   } else if (n == 96) {
     const size_t smem = qb::fft2_smem_bytes<96>();
     cudaFuncSetAttribute(qb::fft2_batch_kernel<96, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -677,8 +678,8 @@ int ptycho_fft2(const void* in, void* out, int count, int n, int inverse, float 
     const size_t smem = qb::fft2_smem_bytes<128>();
     cudaFuncSetAttribute(qb::fft2_batch_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(qb::fft2_batch_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (inverse) qb::fft2_batch_kernel<128, true><<<grid, 512, smem, st>>>(i2, o2, count, scale);
-    else qb::fft2_batch_kernel<128, false><<<grid, 512, smem, st>>>(i2, o2, count, scale);
+    if (inverse) qb::fft2_batch_kernel<128, true><<<grid, qb::Fft2<128>::T, smem, st>>>(i2, o2, count, scale);
+    else qb::fft2_batch_kernel<128, false><<<grid, qb::Fft2<128>::T, smem, st>>>(i2, o2, count, scale);
   }
   return check_launch("fft2_batch_kernel");
 }

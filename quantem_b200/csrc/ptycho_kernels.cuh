@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "fft_engine.cuh"
 
 namespace qb {
@@ -64,6 +66,7 @@ struct BatchParams {
   float* grad_positions;      // optional (B, 2) dL/d(position), serial autograd adjoint only
   const float* descan;        // optional (npos, 2) descan shifts [px] applied to the exit wave
   float* grad_descan;         // optional (B, 2) dL/d(descan), serial autograd adjoint only
+  int sep_shared;             // the separable factors fit in shared memory (else read through L1)
   float* grad_prop;           // optional (S-1, 2) propagator sensitivities, serial autograd adjoint only
 };
 
@@ -145,23 +148,43 @@ __device__ __forceinline__ void load_pairs(const float2* src, int tid, float2 (&
   }
 }
 
-// shared-memory bytes used by fused_batch_kernel<N, *> (without the separable
-// propagator factors, which add 2 * N * (S-1) float2 when used)
+// Shared-memory bytes of the batch kernels: exchange buffer, twiddles, shift ramps and
+// wrap maps; the intensity tile of the forward kernel (the adjoint kernel keeps its
+// intensity / dL/dI tile in its global scratch slot, L2-resident, 64 KB per CTA at 128^2:
+// the shared memory it would take is left to the L1 cache); and the separable propagator
+// factors when they are kept here.
 template <int N>
-constexpr size_t fused_smem_bytes() {
-  return sizeof(float2) * (size_t)(Fft2<N>::SM_FLOAT2 + 3 * N) + sizeof(float) * (size_t)N * N +
-         sizeof(int) * (size_t)(2 * N);
+constexpr size_t batch_smem_bytes(bool tile, bool sep, int S) {
+  return sizeof(float2) * (size_t)(Fft2<N>::SM_FLOAT2 + Fft2<N>::TW_FLOAT2 + 2 * N) + sizeof(int) * (size_t)(2 * N) +
+         (tile ? sizeof(float) * (size_t)N * N : 0) +
+         (sep ? sizeof(float2) * (size_t)2 * N * (size_t)(S > 1 ? S - 1 : 0) : 0);
 }
+// Resident CTAs per SM of the batch kernels; the instances with extensions (EXT, AN) take
+// one less, since they spill at 128 registers.
 template <int N>
-constexpr size_t fused_smem_bytes_sep(int S) {
-  return fused_smem_bytes<N>() + sizeof(float2) * (size_t)2 * N * (size_t)(S > 1 ? S - 1 : 0);
+constexpr int batch_ctas(bool ext) {
+  return ext && Fft2<N>::CTAS > 1 ? Fft2<N>::CTAS - 1 : Fft2<N>::CTAS;
 }
-// The adjoint kernel keeps its intensity / dL/dI tile in its global scratch slot
-// (L2-resident, 64 KB per CTA at 128^2) instead of shared memory; the 64 KB left
-// to the L1 cache hold the register spills of the 512-thread CTA.
-template <int N, bool ADJ>
-constexpr size_t batch_smem_bytes(bool sep, int S) {
-  return (sep ? fused_smem_bytes_sep<N>(S) : fused_smem_bytes<N>()) - (ADJ ? sizeof(float) * (size_t)N * N : 0);
+// Largest dynamic shared memory of a CTA: 228 KB shared by the resident CTAs, less 1 KB of
+// the system's and 1 KB for the static arrays of each.
+constexpr size_t kMaxSmem = 232448 - 1024;
+template <int N>
+constexpr size_t max_smem(int ctas) {
+  return ctas == 1 ? kMaxSmem : (size_t)228 * 1024 / ctas - 2048;
+}
+// The separable factors go to shared memory while they fit beside the rest without
+// costing a resident CTA; beyond that the kernels read them through the L1 cache.
+template <int N>
+constexpr bool sep_in_smem(bool tile, int S) {
+  return batch_smem_bytes<N>(tile, true, S) <= max_smem<N>(Fft2<N>::CTAS);
+}
+// Slices accepted with separable propagators: the bound of the interface (a tile of
+// N (N + 1) complex values, 3 N more, the intensity tile, the maps and the factors of
+// every slice within one SM), whatever a kernel keeps in shared memory itself.
+constexpr size_t sep_limit_bytes(int n, int S) {
+  return sizeof(float2) * ((n == 96 ? (size_t)9976 : (size_t)n * (n + 1)) + 3 * (size_t)n) +
+         sizeof(float) * (size_t)n * n + sizeof(int) * 2 * (size_t)n +
+         sizeof(float2) * 2 * (size_t)n * (size_t)(S > 1 ? S - 1 : 0);
 }
 
 template <int N>
@@ -204,48 +227,107 @@ __device__ __forceinline__ void loss_elem(const BatchParams& p, float I, float t
   }
 }
 
+// Position of frequency row r in the shared row factors: the D rows of one S3 group
+// are consecutive, so a thread reads them two at a time.
+template <int N>
+__device__ __forceinline__ int prop_slot(int r) {
+  return (r % Fft2<N>::C) * Fft2<N>::D + r / Fft2<N>::C;
+}
+
+// Separable propagator factors into shared memory (rows in prop_slot order).
+template <int N>
+__device__ __forceinline__ void load_prop_factors(const BatchParams& p, float2* sKr, float2* sKc) {
+  for (int k = threadIdx.x; k < (p.S - 1) * N; k += Fft2<N>::T) {
+    sKr[k / N * N + prop_slot<N>(k % N)] = p.prop_r[k];
+    sKc[k] = p.prop_c[k];
+  }
+}
+
 // x (S3 layout, Fourier space) *= K_s (CONJ: conj(K_s)), separable factors from
-// shared memory or the full (S-1, N, N) array from global memory.
+// shared memory (sep), or the factors / the full (S-1, N, N) array from global memory.
 template <int N, bool CONJ>
 __device__ __forceinline__ void apply_prop(const Fft2<N>& f, float2 (&x)[Fft2<N>::E], const BatchParams& p, int s,
                                            bool sep, const float2* sKr, const float2* sKc) {
   constexpr int D = Fft2<N>::D, G3 = Fft2<N>::G3;
   if (sep) {
+    const float2 kc = sKc[s * N + f.s3_c];
 #pragma unroll
     for (int g = 0; g < G3; ++g) {
-      const float2 kc = sKc[s * N + f.s3_c];
+      const float4* kr = reinterpret_cast<const float4*>(sKr + s * N + f.s3_kC(g) * D);
 #pragma unroll
-      for (int e = 0; e < D; ++e) {
-        const float2 k = cmul(sKr[s * N + f.s3_row(g, e)], kc);
-        x[g * D + e] = CONJ ? cmulc(x[g * D + e], k) : cmul(x[g * D + e], k);
+      for (int e = 0; e < D; e += 2) {
+        const float4 v = kr[e / 2];
+        const float2 k0 = cmul(make_float2(v.x, v.y), kc), k1 = cmul(make_float2(v.z, v.w), kc);
+        const int i = g * D + e;
+        x[i] = CONJ ? cmulc(x[i], k0) : cmul(x[i], k0);
+        x[i + 1] = CONJ ? cmulc(x[i + 1], k1) : cmul(x[i + 1], k1);
       }
     }
   } else {
-    const float2* pr = p.prop + (size_t)s * N * N;
+    const bool fac = p.prop_r != nullptr;
+    const float2* pr = fac ? p.prop_r + (size_t)s * N : p.prop + (size_t)s * N * N + f.s3_c;
+    const size_t pitch = fac ? 1 : N;
+    const float2 kc = fac ? __ldg(p.prop_c + (size_t)s * N + f.s3_c) : make_float2(1.f, 0.f);
 #pragma unroll
     for (int g = 0; g < G3; ++g)
 #pragma unroll
       for (int e = 0; e < D; ++e) {
-        const float2 k = __ldg(pr + (size_t)f.s3_row(g, e) * N + f.s3_c);
+        float2 k = __ldg(pr + (size_t)f.s3_row(g, e) * pitch);
+        if (fac) k = cmul(k, kc);
         x[g * D + e] = CONJ ? cmulc(x[g * D + e], k) : cmul(x[g * D + e], k);
       }
   }
 }
 
-// x (S1 layout) *= o (CONJ: conj(o)) for the object row orow_ptr, columns through
-// colmap.  Loads go in batches of 8 so that a batch is in flight at once while
-// the wave occupies half of the register file.
+// Offset of S1 column register e from the window's centre column c0 when the window
+// does not wrap around the object's columns: compile-time apart from the thread's cB.
+template <int N>
+__device__ __forceinline__ constexpr int inside_off(int e) {
+  return Fft2<N>::B * e - (e >= Fft2<N>::A / 2 ? N : 0);
+}
+
+// x (S1 layout) *= o (CONJ: conj(o)) for the object slice, rows through rowmap, columns
+// through colmap or, when the window does not wrap (cin >= 0: its first column of this
+// thread), at compile-time offsets.  Loads go in batches so that a batch is in flight at
+// once while the wave occupies half of the register file.
 template <int N, bool CONJ>
-__device__ __forceinline__ void gather_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>::E], const float2* orow_ptr,
-                                           const int* colmap, uint64_t pol) {
-  constexpr int E = Fft2<N>::E;
+__device__ __forceinline__ void gather_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>::E], const float2* slice, int Wo,
+                                           const int* rowmap, const int* colmap, int cin) {
+  const uint64_t pol = evict_last_policy();
+  constexpr int A = Fft2<N>::A, G1 = Fft2<N>::G1;
+  constexpr int BT = 8;
+  if (cin >= 0) {
 #pragma unroll
-  for (int e0 = 0; e0 < E; e0 += 8) {
-    float2 ob[8];
+    for (int g = 0; g < G1; ++g) {
+      const float2* row = slice + (size_t)rowmap[f.s1_row(g)] * Wo + cin;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ob[j] = ld_obj(orow_ptr + colmap[f.s1_col(e0 + j)], pol);
+      for (int e0 = 0; e0 < A; e0 += BT) {
+        float2 ob[BT];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[e0 + j] = CONJ ? cmulc(x[e0 + j], ob[j]) : cmul(x[e0 + j], ob[j]);
+        for (int j = 0; j < BT; ++j) ob[j] = ld_obj(row + inside_off<N>(e0 + j), pol);
+#pragma unroll
+        for (int j = 0; j < BT; ++j) {
+          const int i = g * A + e0 + j;
+          x[i] = CONJ ? cmulc(x[i], ob[j]) : cmul(x[i], ob[j]);
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int g = 0; g < G1; ++g) {
+      const float2* row = slice + (size_t)rowmap[f.s1_row(g)] * Wo;
+#pragma unroll
+      for (int e0 = 0; e0 < A; e0 += 2) {
+        float2 ob[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) ob[j] = ld_obj(row + colmap[f.s1_col(e0 + j)], pol);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int i = g * A + e0 + j;
+          x[i] = CONJ ? cmulc(x[i], ob[j]) : cmul(x[i], ob[j]);
+        }
+      }
+    }
   }
 }
 
@@ -255,13 +337,17 @@ __device__ __forceinline__ void gather_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>
 // conjugate, for the adjoint.
 template <int N, bool CONJ>
 __device__ __forceinline__ void descan_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>::E], float dr, float dc) {
-  constexpr int E = Fft2<N>::E;
-  const float ar = (float)fsigned(f.s1_r, N) * dr;
+  constexpr int A = Fft2<N>::A, G1 = Fft2<N>::G1;
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    float sn, cs;
-    sincospif(-2.0f * (ar + (float)fsigned(f.s1_col(e), N) * dc) / (float)N, &sn, &cs);
-    x[e] = CONJ ? cmulc(x[e], make_float2(cs, sn)) : cmul(x[e], make_float2(cs, sn));
+  for (int g = 0; g < G1; ++g) {
+    const float ar = (float)fsigned(f.s1_row(g), N) * dr;
+#pragma unroll
+    for (int e = 0; e < A; ++e) {
+      float sn, cs;
+      sincospif(-2.0f * (ar + (float)fsigned(f.s1_col(e), N) * dc) / (float)N, &sn, &cs);
+      const int i = g * A + e;
+      x[i] = CONJ ? cmulc(x[i], make_float2(cs, sn)) : cmul(x[i], make_float2(cs, sn));
+    }
   }
 }
 
@@ -296,12 +382,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   // AN (compile time): analytic update directions instead of the autograd adjoint,
   // so the autograd kernel carries none of the analytic code or live values
   using F = Fft2<N>;
-  constexpr int E = F::E, D = F::D, G3 = F::G3, T = F::T;
-  static_assert(E % 8 == 0, "gathers and scatters go in batches of 8 registers");
+  constexpr int E = F::E, A = F::A, G1 = F::G1, D = F::D, G3 = F::G3, T = F::T;
+  static_assert(A % 8 == 0, "gathers and scatters go in batches of 8 registers");
   extern __shared__ float4 smem_raw[];
   float2* sm = reinterpret_cast<float2*>(smem_raw);
   float2* tw = sm + F::SM_FLOAT2;
-  float2* rowf = tw + N;
+  float2* rowf = tw + F::TW_FLOAT2;
   float2* colf = rowf + N;
   // intensity / dL/dI tile: shared memory (forward-only) or the CTA's scratch slot (ADJ)
   float* inten_sm = reinterpret_cast<float*>(colf + N);
@@ -311,9 +397,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   // builds exp(-i pi lambda dz (kr^2 + kc^2)) times per-axis tilt ramps)
   float2* sKr = reinterpret_cast<float2*>(colmap + N);
   float2* sKc = sKr + (size_t)N * (p.S > 1 ? p.S - 1 : 0);
-  const bool sep = p.prop_r != nullptr;
-  const uint64_t pol = evict_last_policy();
-  __shared__ double red[32];
+  const bool sep = p.prop_r != nullptr && p.sep_shared;
+  __shared__ double red[32];      // per-warp loss sums
   __shared__ int nfred[32];  // per-warp non-finite counts
   __shared__ float posred[32][2];  // per-warp position / descan gradient partials
   __shared__ float propred[2 * 16];  // EXT: this CTA's propagator sensitivities (S <= 17)
@@ -321,17 +406,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   const int tid = threadIdx.x;
   F f;
   f.init(tid);
-  for (int k = tid; k < N; k += T) {
-    double s, c;
-    sincospi(-2.0 * (double)k / (double)N, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
-  }
-  if (sep) {
-    for (int k = tid; k < (p.S - 1) * N; k += T) {
-      sKr[k] = p.prop_r[k];
-      sKc[k] = p.prop_c[k];
-    }
-  }
+  F::fill_twiddles(tw, tid, T);
+  if (sep) load_prop_factors<N>(p, sKr, sKc);
   const float inv_n = 1.0f / (float)N;
   const float inv_n2 = inv_n * inv_n;
   const size_t NN = (size_t)N * N;
@@ -361,8 +437,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         for (int e = 0; e < D; ++e)
           pgrad[(size_t)m * NN + (size_t)f.s3_row(g, e) * N + f.s3_c] = make_float2(0.f, 0.f);
   }
-  double loss_acc = 0.0;
-  int nonfinite = 0;
+  // loss and non-finite counts live in shared memory between positions (warp w owns
+  // entry w), so the transforms do not carry them in registers
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = 0.0;
+    nfred[tid >> 5] = 0;
+  }
 
   // each CTA takes a contiguous block of the batch: positions processed at the same
   // time are far apart in the batch order, so raster-ordered batches do not pile
@@ -370,12 +450,13 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   const int bchunk = (p.B + ncta - 1) / ncta;
   const int bend = min(p.B, (cta + 1) * bchunk);
   for (int b = cta * bchunk; b < bend; ++b) {
-    const int64_t gi = p.batch_idx[b];
-    if (gi < 0 || gi >= p.npos) {  // invalid index: skip the position and report it
+    const int64_t gi64 = p.batch_idx[b];
+    if (gi64 < 0 || gi64 >= p.npos) {  // invalid index: skip the position and report it
       if (tid == 0) status_add_invalid(p.status, 1);
       continue;
     }
-    const float py = p.positions[2 * gi], px = p.positions[2 * gi + 1];
+    const int gi = (int)gi64;
+    const float py = p.positions[2 * (size_t)gi], px = p.positions[2 * (size_t)gi + 1];
     const float ry = rintf(py), rx = rintf(px);  // round half to even
     const float fy = py - ry, fx = px - rx;
     const int r0 = wrap_index((int)ry, p.Ho), c0 = wrap_index((int)rx, p.Wo);
@@ -395,7 +476,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
       }
     }
     __syncthreads();
-    const int orow = rowmap[f.s1_r];
+    // first column of this thread when the window lies inside the object's columns, else -1
+    const int cin = (c0 >= N / 2 && c0 + N / 2 <= p.Wo) ? c0 + f.s1_cB : -1;
 
     // One loop with a single inverse and a single forward transform site walks
     // the forward chains of all modes, the loss, and (ADJ) the reverse chains.
@@ -444,7 +526,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
     while (true) {
       f.inverse(x, sm, tw);
       // ---------------- real space (S1 layout) ----------------
-      const float2* orow_ptr = p.obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
+      const float2* slice = p.obj + (size_t)s * HoWo;
       if (!bwd) {
 #pragma unroll
         for (int e = 0; e < E; ++e) x[e] = cscale(x[e], inv_n2);
@@ -453,51 +535,61 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
           store_pairs<E, T>(wv, tid, x);
         }
         if (p.out_waves) {
-          float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN + (size_t)f.s1_r * N;
+          float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) ow[f.s1_col(e)] = x[e];
+          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
         }
-        gather_mul<N, false>(f, x, orow_ptr, colmap, pol);
-        if (EXT && s == S - 1 && p.descan) descan_mul<N, false>(f, x, __ldg(p.descan + 2 * gi), __ldg(p.descan + 2 * gi + 1));
+        gather_mul<N, false>(f, x, slice, p.Wo, rowmap, colmap, cin);
+        if (EXT && s == S - 1 && p.descan) descan_mul<N, false>(f, x, __ldg(p.descan + 2 * (size_t)gi), __ldg(p.descan + 2 * (size_t)gi + 1));
         if (s == S - 1 && p.out_exit) {
-          float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN + (size_t)f.s1_r * N;
+          float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) oe[f.s1_col(e)] = x[e];
+          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
         }
       } else {
         const float sc = first_bwd ? inv_n : inv_n2;  // adjoint of the orthonormal FFT, or of a propagation
         const float2* wv = slot + (size_t)(m * S + s) * NN;
-        float2* grow = p.grad_obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
         // the exit wave carries the descan ramp: its gradient times conj(ramp) is the
         // gradient of the last slice's transmitted wave
         if (EXT && first_bwd && p.descan)
-          descan_mul<N, true>(f, x, __ldg(p.descan + 2 * gi), __ldg(p.descan + 2 * gi + 1));
+          descan_mul<N, true>(f, x, __ldg(p.descan + 2 * (size_t)gi), __ldg(p.descan + 2 * (size_t)gi + 1));
+        const uint64_t pol = evict_last_policy();
+        // BT registers (g, e0 ..) at a time: gradient contribution conj(psi) g scattered, x = conj(o) g
+        auto scatter = [&](auto batch, int i0, auto column) {
+          constexpr int BT = decltype(batch)::value;
+          const int g = i0 / A, e0 = i0 % A;
+          const size_t ro = (size_t)s * HoWo + (size_t)rowmap[f.s1_row(g)] * p.Wo;
+          const float2* orow = p.obj + ro;
+          float2* grow = p.grad_obj + ro;
+          float2 ps[BT], ob[BT];
 #pragma unroll
-        for (int e0 = 0; e0 < E; e0 += 8) {
-          float2 ps[8], ob[8];
-          int col[8];
-#pragma unroll
-          for (int j = 0; j < 8; j += 2) {
-            const float4 v = ld_stream4(reinterpret_cast<const float4*>(wv) + ((e0 + j) >> 1) * T + tid);
+          for (int j = 0; j < BT; j += 2) {
+            const float4 v = ld_stream4(reinterpret_cast<const float4*>(wv) + ((i0 + j) >> 1) * T + tid);
             ps[j] = make_float2(v.x, v.y);
             ps[j + 1] = make_float2(v.z, v.w);
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            col[j] = colmap[f.s1_col(e0 + j)];
-            ob[j] = ld_obj(orow_ptr + col[j], pol);
-          }
+          for (int j = 0; j < BT; ++j) ob[j] = ld_obj(orow + column(e0 + j), pol);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float2 g = cscale(x[e0 + j], sc);
-            atomicAdd(grow + col[j], cmulc(g, ps[j]));  // conj(psi) * g
-            x[e0 + j] = cmulc(g, ob[j]);                 // conj(o) * g
+          for (int j = 0; j < BT; ++j) {
+            const float2 gx = cscale(x[i0 + j], sc);
+            atomicAdd(grow + column(e0 + j), cmulc(gx, ps[j]));  // conj(psi) * g
+            x[i0 + j] = cmulc(gx, ob[j]);                        // conj(o) * g
           }
           if (AN) {  // sum_patches(|psi|^2) of this slice and mode (object_models.py:701-703)
-            float* nrow = p.an_norm + ((size_t)s * P + m) * HoWo + (size_t)orow * p.Wo;
+            float* nrow = p.an_norm + ((size_t)s * P + m) * HoWo + (size_t)rowmap[f.s1_row(g)] * p.Wo;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) atomicAdd(nrow + col[j], cabs2(ps[j]));
+            for (int j = 0; j < BT; ++j) atomicAdd(nrow + column(e0 + j), cabs2(ps[j]));
           }
+        };
+        if (cin >= 0) {
+#pragma unroll
+          for (int i = 0; i < E; i += 8)
+            scatter(std::integral_constant<int, 8>(), i, [&](int e) { return cin + inside_off<N>(e); });
+        } else {  // wrapping windows are few: small batches, so that this path costs no registers
+#pragma unroll
+          for (int i = 0; i < E; i += 2)
+            scatter(std::integral_constant<int, 2>(), i, [&](int e) { return colmap[f.s1_col(e)]; });
         }
         if (EXT && first_bwd && p.grad_descan) {
           // x = dL/dw of the last slice's incident wave w, so conj(x) w = conj(dL/dE) E for the
@@ -508,11 +600,10 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
             const float4 v = reinterpret_cast<const float4*>(wv)[(e >> 1) * T + tid];
             const float im0 = x[e].x * v.y - x[e].y * v.x;
             const float im1 = x[e + 1].x * v.w - x[e + 1].y * v.z;
-            gc = fmaf((float)fsigned(f.s1_col(e), N), im0, gc);
-            gc = fmaf((float)fsigned(f.s1_col(e + 1), N), im1, gc);
-            gr += im0 + im1;
+            gc = fmaf((float)fsigned(f.s1_col(e % A), N), im0, gc);
+            gc = fmaf((float)fsigned(f.s1_col(e % A + 1), N), im1, gc);
+            gr = fmaf((float)fsigned(f.s1_row(e / A), N), im0 + im1, gr);
           }
-          gr *= (float)fsigned(f.s1_r, N);
           for (int o = 16; o > 0; o >>= 1) {
             gr += __shfl_xor_sync(0xffffffffu, gr, o);
             gc += __shfl_xor_sync(0xffffffffu, gc, o);
@@ -539,20 +630,21 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         if (AN && s == 0) {
           // analytic probe update: sum over positions of the back-propagated
           // gradient at the probe plane, no inverse shift (probe_models.py:774-783)
-          float2* pg = pgrad + (size_t)m * NN + (size_t)f.s1_r * N;
 #pragma unroll
           for (int e0 = 0; e0 < E; e0 += 8) {
+            float2* pg = pgrad + (size_t)m * NN + (size_t)f.s1_row(e0 / A) * N;
             float2 old[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) old[j] = pg[f.s1_col(e0 + j)];
+            for (int j = 0; j < 8; ++j) old[j] = pg[f.s1_col(e0 % A + j)];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) pg[f.s1_col(e0 + j)] = cadd(old[j], x[e0 + j]);
+            for (int j = 0; j < 8; ++j) pg[f.s1_col(e0 % A + j)] = cadd(old[j], x[e0 + j]);
           }
           if (m > 0) {
             --m;
             s = S - 1;
             first_bwd = true;
             load_far_seed(m);
+            __syncthreads();  // inverse follows inverse: every warp is done with its classes
             continue;
           }
           break;
@@ -596,6 +688,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         // loss over the mode-summed intensity (each thread owns its S3 slots)
         {
           const float* tg = p.targets + (size_t)gi * NN;
+          double loss_acc = 0.0;
+          int nonfinite = 0;
 #pragma unroll
           for (int g = 0; g < G3; ++g)
 #pragma unroll
@@ -622,6 +716,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
               inten[li] = dldi;
               if (p.out_intensity) p.out_intensity[(size_t)b * NN + di] = I;
             }
+          for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
+          const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
+          if ((tid & 31) == 0) {
+            red[tid >> 5] += loss_acc;
+            nfred[tid >> 5] += nf_warp;
+          }
         }
         if (!ADJ) break;
         bwd = true;
@@ -717,13 +817,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   }
 
   // ------------------------------ loss reduction ------------------------------
-  for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
   // one status update per CTA: per-thread updates of a shared word contend and can drop counts
-  const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
-  if ((tid & 31) == 0) {
-    red[tid >> 5] = loss_acc;
-    nfred[tid >> 5] = nf_warp;
-  }
   __syncthreads();
   if (tid == 0) {
     int nf = 0;
@@ -738,7 +832,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
 }
 
 template <int N, bool ADJ, bool AN = false, bool EXT = false>
-__global__ void __launch_bounds__(Fft2<N>::T, 1) fused_batch_kernel(const BatchParams p) {
+__global__ void __launch_bounds__(Fft2<N>::T, batch_ctas<N>(AN || EXT)) fused_batch_kernel(const BatchParams p) {
   serial_body<N, ADJ, AN, EXT>(p, blockIdx.x, gridDim.x);
 }
 
@@ -754,7 +848,7 @@ struct MultiParams {
 };
 
 template <int N, bool ADJ>
-__global__ void __launch_bounds__(Fft2<N>::T, 1) multi_batch_kernel(const __grid_constant__ MultiParams mp) {
+__global__ void __launch_bounds__(Fft2<N>::T, Fft2<N>::CTAS) multi_batch_kernel(const __grid_constant__ MultiParams mp) {
   int d = 0;
   while (d + 1 < mp.nd && (int)blockIdx.x >= mp.begin[d + 1]) ++d;
   serial_body<N, ADJ>(mp.d[d], (int)blockIdx.x - mp.begin[d], mp.begin[d + 1] - mp.begin[d]);
@@ -766,18 +860,14 @@ template <int N, bool INV>
 __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2* in, float2* out, int count,
                                                              float scale) {
   using F = Fft2<N>;
-  constexpr int E = F::E, D = F::D, G3 = F::G3, T = F::T;
+  constexpr int E = F::E, A = F::A, D = F::D, G3 = F::G3, T = F::T;
   extern __shared__ float4 smem_raw[];
   float2* sm = reinterpret_cast<float2*>(smem_raw);
   float2* tw = sm + F::SM_FLOAT2;
   const int tid = threadIdx.x;
   F f;
   f.init(tid);
-  for (int k = tid; k < N; k += T) {
-    double s, c;
-    sincospi(-2.0 * (double)k / (double)N, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
-  }
+  F::fill_twiddles(tw, tid, T);
   __syncthreads();
   const size_t NN = (size_t)N * N;
   for (int t = blockIdx.x; t < count; t += gridDim.x) {
@@ -786,7 +876,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2*
     float2 x[E];
     if (!INV) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) x[e] = src[(size_t)f.s1_r * N + f.s1_col(e)];
+      for (int e = 0; e < E; ++e) x[e] = src[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)];
       f.forward(x, sm, tw);
 #pragma unroll
       for (int g = 0; g < G3; ++g)
@@ -799,7 +889,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2*
         for (int e = 0; e < D; ++e) x[g * D + e] = src[(size_t)f.s3_row(g, e) * N + f.s3_c];
       f.inverse(x, sm, tw);
 #pragma unroll
-      for (int e = 0; e < E; ++e) dst[(size_t)f.s1_r * N + f.s1_col(e)] = cscale(x[e], scale);
+      for (int e = 0; e < E; ++e) dst[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = cscale(x[e], scale);
     }
     __syncthreads();
   }
@@ -807,7 +897,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2*
 
 template <int N>
 constexpr size_t fft2_smem_bytes() {
-  return sizeof(float2) * (size_t)(Fft2<N>::SM_FLOAT2 + N);
+  return sizeof(float2) * (size_t)(Fft2<N>::SM_FLOAT2 + Fft2<N>::TW_FLOAT2);
 }
 
 }  // namespace qb
