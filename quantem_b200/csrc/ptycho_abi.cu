@@ -204,16 +204,39 @@ __global__ void potential_vjp_kernel(const float* __restrict__ v, const float2* 
 // ---------------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------------
-__global__ void reduce_partials_kernel(const float2* __restrict__ parts, float2* __restrict__ out, int nparts,
-                                       int64_t count) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+// out[i] = sum_g parts[g * count + i].  Read-bound: 16 lanes of partials per output element
+// (each a strided, fixed-order sum) keep enough loads in flight when count is only a few
+// thousand elements, then a fixed-order sum over the lanes in shared memory.  One thread
+// per element walking all the partials took 16 us for 148 x 64^2 and 34 us for
+// 148 x 4 x 128^2.
+constexpr int kPartLanes = 16;
+constexpr int kPartCols = 32;
+__global__ void __launch_bounds__(kPartLanes* kPartCols)
+    reduce_partials_kernel(const float2* __restrict__ parts, float2* __restrict__ out, int nparts, int64_t count) {
+  __shared__ float2 acc[kPartLanes][kPartCols];
+  const int tx = threadIdx.x % kPartCols, ty = threadIdx.x / kPartCols;
+  for (int64_t i0 = blockIdx.x * (int64_t)kPartCols; i0 < count; i0 += (int64_t)gridDim.x * kPartCols) {
+    const int64_t i = i0 + tx;
     float2 a = make_float2(0.f, 0.f);
-    for (int g = 0; g < nparts; ++g) {
-      const float2 v = parts[(int64_t)g * count + i];
-      a.x += v.x;
-      a.y += v.y;
+    if (i < count) {
+#pragma unroll 4
+      for (int g = ty; g < nparts; g += kPartLanes) {
+        const float2 v = parts[(int64_t)g * count + i];
+        a.x += v.x;
+        a.y += v.y;
+      }
     }
-    out[i] = a;
+    acc[ty][tx] = a;
+    __syncthreads();
+    if (ty == 0 && i < count) {
+#pragma unroll
+      for (int k = 1; k < kPartLanes; ++k) {
+        a.x += acc[k][tx].x;
+        a.y += acc[k][tx].y;
+      }
+      out[i] = a;
+    }
+    __syncthreads();
   }
 }
 
@@ -687,7 +710,7 @@ int ptycho_fft2(const void* in, void* out, int count, int n, int inverse, float 
 int ptycho_reduce_partials(const void* parts, void* out, int nparts, int64_t count, void* stream) {
   if (!parts || !out || nparts < 1 || count < 0) return fail(PTYCHO_ERR_INVALID, "reduce_partials: bad arguments");
   if (count == 0) return PTYCHO_OK;
-  reduce_partials_kernel<<<grid_for(count, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  reduce_partials_kernel<<<grid_for(count, kPartCols), kPartLanes * kPartCols, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const float2*>(parts), static_cast<float2*>(out), nparts, count);
   return check_launch("reduce_partials_kernel");
 }
