@@ -198,8 +198,8 @@ int ptycho_obj_blur(const void* in, void* out, void* tmp, int S, int Ho, int Wo,
 
 /* Butterworth filter (object_models.py:481-520): per slice, mean removed, ifft2(fft2(x)
  * env), mean added back (the real part for a real potential, is_real = 1); env: float32
- * (Ho, Wo) envelope on the fftfreq grid.  The 2-D transform is a direct DFT along each
- * axis (object sides <= 6144).  tmp: complex64 2 * S * Ho * Wo; means: complex64 2 * S.
+ * (Ho, Wo) envelope on the fftfreq grid.  The 2-D transform runs along lines of any length
+ * (object sides <= 6144).  tmp: complex64 2 * S * Ho * Wo; means: complex64 2 * S.
  * The filter is self-adjoint: the VJP is P g - mean(P g) + mean(g) per slice. */
 int ptycho_obj_butterworth(const void* in, void* out, int S, int Ho, int Wo, int is_real, const float* env, void* tmp,
                            void* means, void* stream);

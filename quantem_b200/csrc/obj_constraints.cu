@@ -17,6 +17,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "line_fft.cuh"
 #include "ptycho_b200.h"
 
 int qb_record_error(int code, const char* msg);
@@ -470,132 +471,151 @@ int grid_for(int64_t n);
 
 // ---------------------------------------------------------------- Butterworth filter
 // object_models.py:481-520: per slice, mean removed, ifft2(fft2(x) env), mean added back.
-// The 2-D transform is a direct DFT along the rows, a transpose, a direct DFT along the
-// (former) columns and a transpose back: O(H W (H + W)) per slice, exact for any object
-// size (no object-sized FFT is built on this path); the twiddles come from a per-line
-// table of w^j, j < n, indexed by (k c) mod n.
+// The mean is the DC term, so the filter is ifft2(fft2(x - c) env') + c with env' = env but 1
+// at DC, for any constant c; its VJP (P g - mean(P g) + mean(g)) is the same filter.  c is a
+// sampled mean (256 values of the slice): it only keeps the transform's rounding relative to
+// the variation of x instead of its offset.
+//
+// Three passes of line transforms of any length (line_fft.cuh): rows forward, columns forward
+// + envelope + columns inverse in one pass, rows inverse.  Each pass reads and writes the
+// object once (17 MB at 8 x 510 x 516, L2-resident); bound by the shared-memory traffic of
+// the stages.  At 8 x 510 x 516 (factors 17 and 43 among the radices) the filter took 3.4 ms as
+// four direct n^2 line transforms with transposes, mean and envelope passes in between.
+constexpr int kLineThreads = 512;
 
-// per-slice mean of a complex (or real, REAL) plane, one block per slice
+// c of a slice: the mean of 256 values at equal strides (fixed-order sums, every thread)
 template <bool REAL>
-__global__ void plane_mean_kernel(const float* __restrict__ in, int64_t hw, float2* __restrict__ means) {
-  __shared__ double red[32];
-  const int s = blockIdx.x;
-  double re = 0.0, im = 0.0;
-  for (int64_t p = threadIdx.x; p < hw; p += blockDim.x) {
-    if (REAL) {
-      re += (double)in[(int64_t)s * hw + p];
-    } else {
-      const float2 v = reinterpret_cast<const float2*>(in)[(int64_t)s * hw + p];
-      re += (double)v.x;
-      im += (double)v.y;
-    }
+__device__ float2 sampled_mean(const float* in, int64_t hw, float2* red) {
+  const int cnt = hw < 256 ? (int)hw : 256;
+  float2 v = make_float2(0.f, 0.f);
+  if ((int)threadIdx.x < cnt) {
+    const int64_t i = (int64_t)threadIdx.x * (hw / cnt);
+    v = REAL ? make_float2(in[i], 0.f) : reinterpret_cast<const float2*>(in)[i];
   }
-  const double tr = block_sum_d(re, red);
-  const double ti = block_sum_d(im, red);
-  if (threadIdx.x == 0) means[s] = make_float2((float)(tr / (double)hw), (float)(ti / (double)hw));
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  __syncthreads();  // red is free
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float2 t = make_float2(0.f, 0.f);
+  for (int w = 0; w < 8; ++w) t = make_float2(t.x + red[w].x, t.y + red[w].y);
+  const float inv = 1.0f / (float)cnt;
+  return make_float2(t.x * inv, t.y * inv);
 }
 
-// out (complex) = in - mean of its slice
-template <bool REAL>
-__global__ void center_kernel(const float* __restrict__ in, int64_t hw, int64_t n, const float2* __restrict__ means,
-                              float2* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 m = means[i / hw];
-    const float2 v = REAL ? make_float2(in[i], 0.f) : reinterpret_cast<const float2*>(in)[i];
-    out[i] = make_float2(v.x - m.x, v.y - m.y);
-  }
-}
-
-// DFT of every line of length n (lines contiguous): out[l, k] = scale sum_c x[l, c] w^(+-k c)
-template <bool INV>
-__global__ void dft_lines_kernel(const float2* __restrict__ in, float2* __restrict__ out, int n, float scale) {
+// Rows: a = row transforms of (in - c) (INV = false; c kept in base), or out = inverse row
+// transforms of a, plus c (INV = true).
+template <bool REAL, bool INV>
+__global__ void __launch_bounds__(kLineThreads)
+    butter_rows_kernel(const float* __restrict__ in, float2* __restrict__ a, float* __restrict__ out,
+                       float2* __restrict__ base, const qb::LinePlan p, int S, int H, int lg, int LP) {
   extern __shared__ float2 sh[];
-  float2* x = sh;
-  float2* tw = sh + n;
-  const int64_t line = blockIdx.x;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    x[j] = in[line * n + j];
-    double sn, cs;
-    sincospi((INV ? 2.0 : -2.0) * (double)j / (double)n, &sn, &cs);
-    tw[j] = make_float2((float)cs, (float)sn);
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    float ar = 0.f, ai = 0.f;
-    int idx = 0;
-    for (int c = 0; c < n; ++c) {
-      const float2 v = x[c], w = tw[idx];
-      ar = fmaf(v.x, w.x, fmaf(-v.y, w.y, ar));
-      ai = fmaf(v.x, w.y, fmaf(v.y, w.x, ai));
-      idx += k;
-      if (idx >= n) idx -= n;
+  __shared__ float2 red[kLineThreads / 32];
+  const int n = p.n, L = 1 << lg;
+  float2 *x = sh, *y = sh + n * LP, *tw = y + n * LP;
+  qb::line_twiddles(tw, n);
+  const int per = (H + L - 1) / L;  // line groups per slice
+  const int64_t hw = (int64_t)H * n;
+  for (int g = blockIdx.x; g < S * per; g += gridDim.x) {
+    const int s = g / per, r0 = (g - s * per) * L, nl = min(L, H - r0);
+    float2 c;
+    if (INV) {
+      c = base[s];
+    } else {
+      c = sampled_mean<REAL>(in + s * hw * (REAL ? 1 : 2), hw, red);
+      if (r0 == 0 && threadIdx.x == 0) base[s] = c;
     }
-    out[line * n + k] = make_float2(ar * scale, ai * scale);
+    const int64_t off = s * hw + (int64_t)r0 * n;
+    for (int l = 0; l < L; ++l)
+      for (int e = threadIdx.x; e < n; e += kLineThreads) {
+        float2 v = make_float2(0.f, 0.f);
+        if (l < nl) {
+          const int64_t i = off + (int64_t)l * n + e;
+          if (INV) {
+            v = a[i];
+          } else {
+            v = REAL ? make_float2(in[i], 0.f) : reinterpret_cast<const float2*>(in)[i];
+            v = make_float2(v.x - c.x, v.y - c.y);
+          }
+        }
+        x[e * LP + l] = v;
+      }
+    __syncthreads();
+    const float2* r = qb::line_dft<INV>(x, y, tw, p, lg, LP);
+    for (int l = 0; l < nl; ++l)
+      for (int e = threadIdx.x; e < n; e += kLineThreads) {
+        const int64_t i = off + (int64_t)l * n + e;
+        const float2 v = r[e * LP + l];
+        if (!INV)
+          a[i] = v;
+        else if (REAL)
+          out[i] = v.x + c.x;
+        else
+          reinterpret_cast<float2*>(out)[i] = make_float2(v.x + c.x, v.y + c.y);
+      }
+    __syncthreads();
   }
 }
 
-// (S, H, W) -> (S, W, H), 32 x 32 tiles through shared memory
-__global__ void transpose_c_kernel(const float2* __restrict__ in, float2* __restrict__ out, int H, int W) {
-  __shared__ float2 t[32][33];
-  const int64_t s = blockIdx.z;
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-    const int r = r0 + dy, c = c0 + threadIdx.x;
-    if (r < H && c < W) t[dy][threadIdx.x] = in[(s * H + r) * W + c];
-  }
-  __syncthreads();
-  for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-    const int c = c0 + dy, r = r0 + threadIdx.x;
-    if (r < H && c < W) out[(s * W + c) * H + r] = t[threadIdx.x][dy];
+// Columns of the row spectra, in place: forward, times the envelope (1 at DC) and the
+// normalisation, inverse.
+__global__ void __launch_bounds__(kLineThreads)
+    butter_cols_kernel(float2* __restrict__ a, const float* __restrict__ env, const qb::LinePlan p, int S, int W,
+                       int lg, int LP) {
+  extern __shared__ float2 sh[];
+  const int n = p.n, L = 1 << lg;
+  float2 *x = sh, *y = sh + n * LP, *tw = y + n * LP;
+  qb::line_twiddles(tw, n);
+  const int per = (W + L - 1) / L;
+  const float scale = (float)(1.0 / ((double)n * (double)W));
+  for (int g = blockIdx.x; g < S * per; g += gridDim.x) {
+    const int s = g / per, c0 = (g - s * per) * L;
+    float2* as = a + (int64_t)s * n * W + c0;
+    for (int t = threadIdx.x; t < n << lg; t += kLineThreads) {
+      const int l = t & (L - 1), e = t >> lg;
+      x[e * LP + l] = c0 + l < W ? as[(int64_t)e * W + l] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    float2* r = qb::line_dft<false>(x, y, tw, p, lg, LP);
+    for (int t = threadIdx.x; t < n << lg; t += kLineThreads) {
+      const int l = t & (L - 1), e = t >> lg;
+      if (c0 + l >= W) continue;
+      const float w = (e == 0 && c0 + l == 0 ? 1.0f : env[(int64_t)e * W + c0 + l]) * scale;
+      float2& v = r[e * LP + l];
+      v = make_float2(v.x * w, v.y * w);
+    }
+    __syncthreads();
+    const float2* o = qb::line_dft<true>(r, r == x ? y : x, tw, p, lg, LP);
+    for (int t = threadIdx.x; t < n << lg; t += kLineThreads) {
+      const int l = t & (L - 1), e = t >> lg;
+      if (c0 + l < W) as[(int64_t)e * W + l] = o[e * LP + l];
+    }
+    __syncthreads();
   }
 }
 
-// x (S, W, H) transposed spectrum *= env[kh, kw]
-__global__ void env_mul_t_kernel(float2* __restrict__ x, const float* __restrict__ env, int H, int W, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i % ((int64_t)H * W);
-    const int kw = (int)(p / H), kh = (int)(p % H);
-    const float e = env[(int64_t)kh * W + kw];
-    x[i] = make_float2(x[i].x * e, x[i].y * e);
-  }
-}
-
-// out = y + add[slice] - sub[slice] (the real part for REAL): forward y + mean(x), VJP
-// y - mean(y) + mean(g)
+// out = ifft2(env' fft2(in - c)) + c of S planes H x W; a: S H W complex scratch, base: S
 template <bool REAL>
-__global__ void butter_finish_kernel(const float2* __restrict__ y, int64_t hw, int64_t n,
-                                     const float2* __restrict__ add, const float2* __restrict__ sub,
-                                     float* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = i / hw;
-    float2 v = y[i];
-    v.x += add[s].x - (sub ? sub[s].x : 0.f);
-    v.y += add[s].y - (sub ? sub[s].y : 0.f);
-    if (REAL)
-      out[i] = v.x;
-    else
-      reinterpret_cast<float2*>(out)[i] = v;
-  }
-}
-
-// y (in a) = ifft2(env fft2(a)) of (S, H, W) complex planes; b: scratch of the same size
-int butter_core(float2* a, float2* b, int S, int H, int W, const float* env, cudaStream_t st) {
-  const size_t smw = sizeof(float2) * 2 * (size_t)W, smh = sizeof(float2) * 2 * (size_t)H;
-  cudaFuncSetAttribute(dft_lines_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(smw > smh ? smw : smh));
-  cudaFuncSetAttribute(dft_lines_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(smw > smh ? smw : smh));
-  const dim3 tb(32, 8);
-  const dim3 tg_hw((W + 31) / 32, (H + 31) / 32, S), tg_wh((H + 31) / 32, (W + 31) / 32, S);
-  const int64_t n = (int64_t)S * H * W;
-  dft_lines_kernel<false><<<S * H, kThreads, smw, st>>>(a, b, W, 1.0f);       // along W
-  transpose_c_kernel<<<tg_hw, tb, 0, st>>>(b, a, H, W);                     // (S, W, H)
-  dft_lines_kernel<false><<<S * W, kThreads, smh, st>>>(a, b, H, 1.0f);       // along H
-  env_mul_t_kernel<<<grid_for(n), kThreads, 0, st>>>(b, env, H, W, n);
-  dft_lines_kernel<true><<<S * W, kThreads, smh, st>>>(b, a, H, 1.0f / (float)H);
-  transpose_c_kernel<<<tg_wh, tb, 0, st>>>(a, b, W, H);                     // (S, H, W)
-  dft_lines_kernel<true><<<S * H, kThreads, smw, st>>>(b, a, W, 1.0f / (float)W);
-  return check("butterworth dft");
+int butterworth(const float* in, float* out, int S, int H, int W, const float* env, float2* a, float2* base,
+                cudaStream_t st) {
+  const qb::LinePlan pr = qb::line_plan(W), pc = qb::line_plan(H);
+  const int lr = qb::line_log2(W), lc = qb::line_log2(H);
+  const size_t sr = qb::line_smem(W, lr), sc = qb::line_smem(H, lc);
+  cudaFuncSetAttribute(butter_rows_kernel<REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
+  cudaFuncSetAttribute(butter_rows_kernel<REAL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
+  cudaFuncSetAttribute(butter_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc);
+  // two blocks per SM, evened out over the rounds
+  auto grid = [](int64_t groups) {
+    const int64_t rounds = (groups + kBlocks - 1) / kBlocks;
+    return (int)((groups + rounds - 1) / rounds);
+  };
+  const int gr = grid((int64_t)S * ((H + (1 << lr) - 1) >> lr)), gc = grid((int64_t)S * ((W + (1 << lc) - 1) >> lc));
+  butter_rows_kernel<REAL, false><<<gr, kLineThreads, sr, st>>>(in, a, nullptr, base, pr, S, H, lr, qb::line_pitch(lr));
+  butter_cols_kernel<<<gc, kLineThreads, sc, st>>>(a, env, pc, S, W, lc, qb::line_pitch(lc));
+  butter_rows_kernel<REAL, true><<<gr, kLineThreads, sr, st>>>(nullptr, a, out, base, pr, S, H, lr, qb::line_pitch(lr));
+  return check("butterworth");
 }
 
 int check(const char* what) {
@@ -738,25 +758,12 @@ int ptycho_obj_butterworth(const void* in, void* out, int S, int Ho, int Wo, int
     return qb_record_error(PTYCHO_ERR_INVALID, "obj_butterworth: bad arguments (object sides <= 6144)");
   if (tmp == in || tmp == out) return qb_record_error(PTYCHO_ERR_INVALID, "obj_butterworth: tmp aliases in or out");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t hw = (int64_t)Ho * Wo, n = (int64_t)S * hw;
   float2* a = static_cast<float2*>(tmp);
-  float2* b = a + n;
-  float2* mu = static_cast<float2*>(means);
+  float2* base = static_cast<float2*>(means);
   const float* x = static_cast<const float*>(in);
-  if (is_real) {
-    plane_mean_kernel<true><<<S, kThreads, 0, st>>>(x, hw, mu);
-    center_kernel<true><<<grid_for(n), kThreads, 0, st>>>(x, hw, n, mu, a);
-  } else {
-    plane_mean_kernel<false><<<S, kThreads, 0, st>>>(x, hw, mu);
-    center_kernel<false><<<grid_for(n), kThreads, 0, st>>>(x, hw, n, mu, a);
-  }
-  int rc = butter_core(a, b, S, Ho, Wo, env, st);
-  if (rc) return rc;
-  if (is_real)
-    butter_finish_kernel<true><<<grid_for(n), kThreads, 0, st>>>(a, hw, n, mu, nullptr, static_cast<float*>(out));
-  else
-    butter_finish_kernel<false><<<grid_for(n), kThreads, 0, st>>>(a, hw, n, mu, nullptr, static_cast<float*>(out));
-  return check("butter_finish_kernel");
+  float* o = static_cast<float*>(out);
+  return is_real ? butterworth<true>(x, o, S, Ho, Wo, env, a, base, st)
+                 : butterworth<false>(x, o, S, Ho, Wo, env, a, base, st);
 }
 
 int ptycho_obj_butterworth_vjp(const void* grad_out, void* grad_in, int S, int Ho, int Wo, int is_real,
@@ -766,29 +773,12 @@ int ptycho_obj_butterworth_vjp(const void* grad_out, void* grad_in, int S, int H
   if (tmp == grad_out || tmp == grad_in)
     return qb_record_error(PTYCHO_ERR_INVALID, "obj_butterworth_vjp: tmp aliases a gradient");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t hw = (int64_t)Ho * Wo, n = (int64_t)S * hw;
   float2* a = static_cast<float2*>(tmp);
-  float2* b = a + n;
-  float2* mg = static_cast<float2*>(means);  // mean of g
-  float2* my = mg + S;                      // mean of P g (zero while g is copied into a)
-  const float* g = static_cast<const float*>(grad_out);
-  if (cudaMemsetAsync(my, 0, sizeof(float2) * (size_t)S, st) != cudaSuccess)
-    return qb_record_error(PTYCHO_ERR_CUDA, "obj_butterworth_vjp: memset");
-  if (is_real) {
-    plane_mean_kernel<true><<<S, kThreads, 0, st>>>(g, hw, mg);
-    center_kernel<true><<<grid_for(n), kThreads, 0, st>>>(g, hw, n, my, a);  // my zeroed below first
-  } else {
-    plane_mean_kernel<false><<<S, kThreads, 0, st>>>(g, hw, mg);
-    center_kernel<false><<<grid_for(n), kThreads, 0, st>>>(g, hw, n, my, a);
-  }
-  int rc = butter_core(a, b, S, Ho, Wo, env, st);
-  if (rc) return rc;
-  plane_mean_kernel<false><<<S, kThreads, 0, st>>>(reinterpret_cast<const float*>(a), hw, my);
-  if (is_real)
-    butter_finish_kernel<true><<<grid_for(n), kThreads, 0, st>>>(a, hw, n, mg, my, static_cast<float*>(grad_in));
-  else
-    butter_finish_kernel<false><<<grid_for(n), kThreads, 0, st>>>(a, hw, n, mg, my, static_cast<float*>(grad_in));
-  return check("butter_finish_kernel");
+  float2* base = static_cast<float2*>(means);
+  const float* x = static_cast<const float*>(grad_out);
+  float* o = static_cast<float*>(grad_in);
+  return is_real ? butterworth<true>(x, o, S, Ho, Wo, env, a, base, st)
+                 : butterworth<false>(x, o, S, Ho, Wo, env, a, base, st);
 }
 
 int ptycho_obj_soft_loss(const void* obj, int S, int Ho, int Wo, int kind, float tv_weight_z, float tv_weight_xy,
