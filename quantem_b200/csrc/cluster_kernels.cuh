@@ -129,13 +129,13 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) cluster_batch_kernel(const Batc
         if (p.out_waves) {
           float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
+          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)] = x[e];
         }
         gather_mul<N, false>(f, x, slice, p.Wo, rowmap, colmap, cin);
         if (s == S - 1 && p.out_exit) {
           float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
+          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)] = x[e];
         }
       } else {
         const float sc = first_bwd ? inv_n : inv_n2;  // adjoint of the orthonormal FFT, or of a propagation
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) cluster_batch_kernel(const Batc
 #pragma unroll
           for (int j = 0; j < 8; ++j) ps[j] = wv[(e0 + j) * T + tid];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) sm[f.s1_row((e0 + j) / A) * PITCH + f.s1_col((e0 + j) % A)] = cmulc(x[e0 + j], ps[j]);
+          for (int j = 0; j < 8; ++j) sm[f.s1_row((e0 + j) / A) * PITCH + f.s1_col((e0 + j) / A, (e0 + j) % A)] = cmulc(x[e0 + j], ps[j]);
         }
         cluster.sync();  // every mode's contribution tile is in place
         float2* grow_s = p.grad_obj + (size_t)s * HoWo;

@@ -37,9 +37,12 @@
 // was 5-15 % slower on single-slice and forward-only launches, its code no longer fitting
 // the instruction caches (no-instruction stalls 1.4 per issue against 0.3).
 //
-// Supported N: 64 (A=16,B=4,C=4,D=16, 256 threads) and 128 (A=16,B=8,C=4,D=32,
-// 512 threads); 96 is a specialisation at the end of this file (192 threads,
-// mixed radix 3 x 2^k).
+// At 96^2, A = 8 and two CTAs of 192 threads (168 registers, 48 of them pairs of the wave)
+// replaced a 48 x 2 / 24 x 4 factorisation with one CTA of 255 registers, whose six warps left
+// the SM idle: 1000 positions of 4 slices and 2 modes 1849 -> 1214 us, forward 737 -> 583 us.
+//
+// Supported N: 64 (A=16,B=4,C=4,D=16, 256 threads), 96 (A=8,B=12,C=4,D=24, 192 threads of
+// 48 registers, mixed radix 3 x 2^k, two CTAs per SM) and 128 (A=16,B=8,C=4,D=32, 512 threads).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -186,233 +189,6 @@ __device__ __forceinline__ void dft_reg(float2 (&x)[LEN]) {
 }
 
 // ---------------------------------------------------------------------------
-// 2-D engine
-// ---------------------------------------------------------------------------
-template <int N> struct FftCfg;
-template <> struct FftCfg<64> { static constexpr int A = 16, B = 4, C = 4, D = 16, CTAS = 3; };
-template <> struct FftCfg<128> { static constexpr int A = 16, B = 8, C = 4, D = 32, CTAS = 1; };
-
-template <int N>
-struct Fft2 {
-  static constexpr int A = FftCfg<N>::A, B = FftCfg<N>::B, C = FftCfg<N>::C, D = FftCfg<N>::D;
-  static constexpr int E = B * C;        // complex registers per thread
-  static constexpr int T = N * N / E;    // threads per CTA
-  static constexpr int CTAS = FftCfg<N>::CTAS;  // resident CTAs per SM of the batch kernels
-  static constexpr int G1 = E / A;       // S1 groups per thread
-  static constexpr int G3 = E / D;       // S3 groups per thread
-  static constexpr int PITCH = N + 1;    // row pitch of a plain N x N tile kept in this buffer
-  static constexpr int PP = B * C + 1;   // pitch of a class's A x (B C) transpose
-  static constexpr int CS = A * PP;      // class stride: its transpose, or its C rows of N
-  static constexpr int SM_FLOAT2 = D * CS;
-  static_assert(A * B == N && C * D == N, "bad factorisation");
-  static_assert(G3 * D == E && G1 * A == E, "stage sizes must match");
-  static_assert(CS >= C * N && SM_FLOAT2 >= N * PITCH, "buffer too small");
-  static_assert(D * A == T && 32 % A == 0 && A % B == 0, "a warp owns whole classes");
-
-  // stage coordinates of this thread
-  int s1_r0, s1_cB;      // S1: row of group 0, column residue
-  int s2_rD, s2_kA;      // S2 (s2_rD: the class this thread works on in S1 and S2)
-  int s3_c, s3_kC0;      // S3: column, first kC (group g adds 4*g)
-  int pv_w, pv_r;        // class-private transpose: S1 side, S2 side
-  int mn_3;              // main exchange, S3 side (the S2 side starts at pv_w)
-
-  __device__ __forceinline__ void init(int tid) {
-    const int lane = tid & 31, w = tid >> 5;
-    const int cl = tid & (A - 1);  // thread within its class (A threads)
-    s2_rD = tid / A;
-    s2_kA = cl;
-    s1_cB = cl & (B - 1);
-    s1_r0 = s2_rD + D * (cl / B);
-    constexpr int CW = N / 32;  // warps per 32-column strip
-    s3_c = lane + 32 * (w % CW);
-    s3_kC0 = w / CW;
-    pv_w = s2_rD * CS + cl;
-    pv_r = s2_rD * CS + PP * cl;
-    mn_3 = s3_kC0 * N + s3_c;
-  }
-  __device__ __forceinline__ int s3_kC(int g) const { return s3_kC0 + (T / 32 / (N / 32)) * g; }
-  // natural (row, col) of S1 register (g, e) = x[g A + e]
-  __device__ __forceinline__ int s1_row(int g) const { return s1_r0 + D * (A / B) * g; }
-  __device__ __forceinline__ int s1_col(int e) const { return s1_cB + B * e; }
-  // frequency row of S3 register (g, e)
-  __device__ __forceinline__ int s3_row(int g, int e) const { return s3_kC(g) + C * e; }
-
-  // ---- class-private transpose between S1 and S2 (one warp, __syncwarp only) ----
-  // element (kA, line l = B rC + cB) of the class at kA PP + l; group g holds lines cl + A g
-  __device__ __forceinline__ void write_s1(float2* sm, const float2 (&x)[E]) const {
-#pragma unroll
-    for (int g = 0; g < G1; ++g)
-#pragma unroll
-      for (int e = 0; e < A; ++e) sm[pv_w + PP * e + A * g] = x[g * A + e];
-  }
-  __device__ __forceinline__ void read_s1(const float2* sm, float2 (&x)[E]) const {
-#pragma unroll
-    for (int g = 0; g < G1; ++g)
-#pragma unroll
-      for (int e = 0; e < A; ++e) x[g * A + e] = sm[pv_w + PP * e + A * g];
-  }
-  // S2 input layout (cB, rC)
-  __device__ __forceinline__ void read_s2_in(const float2* sm, float2 (&x)[E]) const {
-#pragma unroll
-    for (int cB = 0; cB < B; ++cB)
-#pragma unroll
-      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = sm[pv_r + B * rC + cB];
-  }
-  __device__ __forceinline__ void write_s2_in(float2* sm, const float2 (&x)[E]) const {
-#pragma unroll
-    for (int cB = 0; cB < B; ++cB)
-#pragma unroll
-      for (int rC = 0; rC < C; ++rC) sm[pv_r + B * rC + cB] = x[cB * C + rC];
-  }
-  // ---- main exchange between S2 and S3: element (rD, kC, column) at rD CS + kC N + column ----
-  // S2 output layout (kB, kC): column kA + A kB
-  __device__ __forceinline__ void write_s2_out(float2* sm, const float2 (&x)[E]) const {
-#pragma unroll
-    for (int kB = 0; kB < B; ++kB)
-#pragma unroll
-      for (int kC = 0; kC < C; ++kC) sm[pv_w + N * kC + A * kB] = x[kB * C + kC];
-  }
-  __device__ __forceinline__ void read_s2_out(const float2* sm, float2 (&x)[E]) const {
-#pragma unroll
-    for (int kB = 0; kB < B; ++kB)
-#pragma unroll
-      for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = sm[pv_w + N * kC + A * kB];
-  }
-  // S3 layout (g, e): rD = e, kC = kC_g, column s3_c
-  __device__ __forceinline__ void read_s3(const float2* sm, float2 (&x)[E]) const {
-#pragma unroll
-    for (int g = 0; g < G3; ++g)
-#pragma unroll
-      for (int e = 0; e < D; ++e) x[g * D + e] = sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g];
-  }
-  __device__ __forceinline__ void write_s3(float2* sm, const float2 (&x)[E]) const {
-#pragma unroll
-    for (int g = 0; g < G3; ++g)
-#pragma unroll
-      for (int e = 0; e < D; ++e) sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g] = x[g * D + e];
-  }
-
-  // ---- register stages ----
-  // G transforms of L consecutive registers each
-  template <int L, int G, bool INV, int K>
-  __device__ __forceinline__ void groups(float2 (&x)[E]) const {
-    if constexpr (K < G) {
-      dft_reg<L, INV, 1, K * L>(x);
-      groups<L, G, INV, K + 1>(x);
-    }
-  }
-  template <bool INV>
-  __device__ __forceinline__ void s1(float2 (&x)[E]) const {
-    groups<A, G1, INV, 0>(x);
-  }
-
-  template <bool INV>
-  __device__ __forceinline__ void s3(float2 (&x)[E]) const {
-    groups<D, G3, INV, 0>(x);
-  }
-
-  // S2 twiddles in the order the warps read them: w_N^(cB kA) at (cB - 1) A + kA (a
-  // class's lanes on consecutive words), then w_N^(rD kC) at TWC + (kC - 1) D + rD (one word
-  // per class).
-  static constexpr int TWC = (B - 1) * A;
-  static constexpr int TW_FLOAT2 = TWC + (C - 1) * D;
-  static __device__ __forceinline__ void fill_twiddles(float2* tw, int tid, int nthreads) {
-    for (int k = tid; k < TW_FLOAT2; k += nthreads) {
-      const int e = k < TWC ? (k / A + 1) * (k % A) : ((k - TWC) / D + 1) * ((k - TWC) % D);
-      double s, c;
-      sincospi(-2.0 * (double)e / (double)N, &s, &c);
-      tw[k] = make_float2((float)c, (float)s);
-    }
-  }
-  // S2 forward: x holds (cB, rC) on entry, (kB, kC) on exit.
-  __device__ __forceinline__ void s2_fwd(float2 (&x)[E], const float2* tw) const {
-#pragma unroll
-    for (int cB = 1; cB < B; ++cB) {
-      const float2 w = tw[(cB - 1) * A + s2_kA];
-#pragma unroll
-      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmul(x[cB * C + rC], w) : cmul(x[cB * C + rC], w);
-    }
-    s2_core<false>(x);
-#pragma unroll
-    for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
-#pragma unroll
-      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmul(x[kB * C + kC], w) : cmul(x[kB * C + kC], w);
-    }
-  }
-  // S2 inverse: (kB, kC) on entry, (cB, rC) on exit.
-  __device__ __forceinline__ void s2_inv(float2 (&x)[E], const float2* tw) const {
-#pragma unroll
-    for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
-#pragma unroll
-      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmulc(x[kB * C + kC], w) : cmulc(x[kB * C + kC], w);
-    }
-    s2_core<true>(x);
-#pragma unroll
-    for (int cB = 1; cB < B; ++cB) {
-      const float2 w = tw[(cB - 1) * A + s2_kA];
-#pragma unroll
-      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmulc(x[cB * C + rC], w) : cmulc(x[cB * C + rC], w);
-    }
-  }
-  // B-point DFT along index 0 (stride C) and C-point DFT along index 1 (stride 1).
-  template <bool INV>
-  __device__ __forceinline__ void s2_core(float2 (&x)[E]) const {
-    s2_bdft<INV, 0>(x);
-    s2_cdft<INV, 0>(x);
-  }
-  template <bool INV, int RC>
-  __device__ __forceinline__ void s2_bdft(float2 (&x)[E]) const {
-    if constexpr (RC < C) {
-      dft_reg<B, INV, C, RC>(x);
-      s2_bdft<INV, RC + 1>(x);
-    }
-  }
-  template <bool INV, int KB>
-  __device__ __forceinline__ void s2_cdft(float2 (&x)[E]) const {
-    if constexpr (KB < B) {
-      dft_reg<C, INV, 1, KB * C>(x);
-      s2_cdft<INV, KB + 1>(x);
-    }
-  }
-
-  // ---- whole transforms between layouts ----
-  // One CTA barrier each.  Between two barriers either every class is owned by its warp
-  // (S2 side: main exchange, private transpose, S1) or every (kC, column) pair by its
-  // thread (S3 side reads and writes the same elements), so no barrier is needed before
-  // a write.  A caller that leaves the S2 side (after inverse) without forward, or enters
-  // it (forward) without inverse, puts a __syncthreads between.
-  // Forward: registers in S1 layout -> registers in S3 layout (unnormalised).
-  __device__ __forceinline__ void forward(float2 (&x)[E], float2* sm, const float2* tw) const {
-    s1<false>(x);
-    __syncwarp();  // the warp's reads of the inverse's transpose are complete
-    write_s1(sm, x);
-    __syncwarp();
-    read_s2_in(sm, x);
-    s2_fwd(x, tw);
-    __syncwarp();
-    write_s2_out(sm, x);
-    __syncthreads();
-    read_s3(sm, x);
-    s3<false>(x);
-  }
-  // Inverse: registers in S3 layout -> registers in S1 layout (unnormalised).
-  __device__ __forceinline__ void inverse(float2 (&x)[E], float2* sm, const float2* tw) const {
-    s3<true>(x);
-    write_s3(sm, x);
-    __syncthreads();
-    read_s2_out(sm, x);
-    s2_inv(x, tw);
-    __syncwarp();
-    write_s2_in(sm, x);
-    __syncwarp();
-    read_s1(sm, x);
-    s1<true>(x);
-  }
-};
-
-// ---------------------------------------------------------------------------
 // mixed radix (N = 3 * 2^k) for 96 x 96 windows
 // ---------------------------------------------------------------------------
 // cos(2*pi*m/96) for m = 0..24 (first quadrant), IEEE double rounded to float.
@@ -508,177 +284,236 @@ __device__ __forceinline__ void dft_reg_n(float2 (&x)[LEN]) {
   }
 }
 
-// 96 x 96 engine: T = 192 threads (6 warps), E = 48 complex registers each.
-//   columns c = cB + 2*cA (A = 48, B = 2), rows r = rD + 4*rC (C = 24, D = 4)
-//   S1: 48-point DFT over cA for fixed (r, cB)               -> kA
-//   S2: twiddle w96^(cB*kA); 2-point over cB; 24-point over rC; twiddle w96^(rD*kC)
-//   S3: 4-point DFT over rD for 12 (kC, column) groups        -> kD
-// Exchange layouts (float2 index): stage 1<->2 element (r, cB, kA) at r + 100 kA + 4800 cB,
-// stage 2<->3 element (row, col) at 104 row + col; both verified to give two wavefronts per
-// warp access with the lane maps of init().
-template <>
-struct Fft2<96> {
-  static constexpr int N = 96, A = 48, B = 2, C = 24, D = 4;
-  static constexpr int T = 192;
-  static constexpr int E = 48;
-  static constexpr int G1 = 1;
-  static constexpr int CTAS = 1;
-  static constexpr int G3 = 12;
-  static constexpr int SM_FLOAT2 = 9976;
-  static constexpr int TW_FLOAT2 = N;
-  static __device__ __forceinline__ void fill_twiddles(float2* tw, int tid, int nthreads) {
-    for (int k = tid; k < N; k += nthreads) {
-      double s, c;
-      sincospi(-2.0 * (double)k / (double)N, &s, &c);
-      tw[k] = make_float2((float)c, (float)s);
-    }
-  }
+// ---------------------------------------------------------------------------
+// 2-D engine
+// ---------------------------------------------------------------------------
+template <int N> struct FftCfg;
+// LB: consecutive columns of a warp's real-space access
+template <> struct FftCfg<64> { static constexpr int A = 16, B = 4, C = 4, D = 16, LB = 4, CTAS = 3; };
+template <> struct FftCfg<96> { static constexpr int A = 8, B = 12, C = 4, D = 24, LB = 4, CTAS = 2; };
+template <> struct FftCfg<128> { static constexpr int A = 16, B = 8, C = 4, D = 32, LB = 8, CTAS = 1; };
 
-  int s1_r, s1_cB;
-  int s2_rD, s2_kA;
-  int s3_c, s3_kC0;
+template <int N>
+struct Fft2 {
+  static constexpr int A = FftCfg<N>::A, B = FftCfg<N>::B, C = FftCfg<N>::C, D = FftCfg<N>::D;
+  static constexpr int E = B * C;        // complex registers per thread
+  static constexpr int T = N * N / E;    // threads per CTA
+  static constexpr int CTAS = FftCfg<N>::CTAS;  // resident CTAs per SM of the batch kernels
+  static constexpr int G1 = E / A;       // S1 groups per thread
+  static constexpr int LB = FftCfg<N>::LB, LR = A / LB;  // columns x rows of a class's lanes in S1
+  static constexpr int GB = B / LB;      // S1 column groups
+  static constexpr int G3 = E / D;       // S3 groups per thread
+  static constexpr int PITCH = N + 1;    // row pitch of a plain N x N tile kept in this buffer
+  static constexpr int PP = B * C + 1;   // pitch of a class's A x (B C) transpose
+  static constexpr int CS = A * PP;      // class stride: its transpose, or its C rows of N
+  static constexpr int SM_FLOAT2 = D * CS;
+  static_assert(A * B == N && C * D == N, "bad factorisation");
+  static_assert(G3 * D == E && G1 * A == E, "stage sizes must match");
+  static_assert(CS >= C * N && SM_FLOAT2 >= N * PITCH, "buffer too small");
+  static_assert(D * A == T && 32 % A == 0 && LB * LR == A && GB * LB == B && G1 % GB == 0,
+                "a warp owns whole classes");
+
+  // stage coordinates of this thread
+  int s1_r0, s1_cB;      // S1: row and column residue of group 0
+  int s2_rD, s2_kA;      // S2 (s2_rD: the class this thread works on in S1 and S2)
+  int s3_c, s3_kC0;      // S3: column, first kC (group g adds 4*g)
+  int pv_w, pv_r;        // class-private transpose: S1 side, S2 side
+  int mn_2, mn_3;        // main exchange: S2 side, S3 side
 
   __device__ __forceinline__ void init(int tid) {
     const int lane = tid & 31, w = tid >> 5;
-    s1_r = (lane & 15) + 16 * w;
-    s1_cB = lane >> 4;
-    s2_rD = lane & 3;
-    s2_kA = (lane >> 2) + 8 * w;
-    s3_c = lane + 32 * (w % 3);
-    s3_kC0 = w / 3;
+    const int cl = tid & (A - 1);  // thread within its class (A threads)
+    s2_rD = tid / A;
+    s2_kA = cl;
+    s1_cB = cl % LB;
+    s1_r0 = s2_rD + D * (cl / LB);
+    constexpr int CW = N / 32;  // warps per 32-column strip
+    s3_c = lane + 32 * (w % CW);
+    s3_kC0 = w / CW;
+    pv_w = s2_rD * CS + (cl / LB) * B + cl % LB;
+    pv_r = s2_rD * CS + PP * cl;
+    mn_2 = s2_rD * CS + cl;
+    mn_3 = s3_kC0 * N + s3_c;
   }
-  __device__ __forceinline__ int s3_kC(int g) const { return s3_kC0 + 2 * g; }
-  __device__ __forceinline__ int s1_row(int) const { return s1_r; }
-  __device__ __forceinline__ int s1_col(int e) const { return s1_cB + B * e; }
+  __device__ __forceinline__ int s3_kC(int g) const { return s3_kC0 + (T / 32 / (N / 32)) * g; }
+  // natural (row, col) of S1 register (g, e) = x[g A + e]
+  __device__ __forceinline__ int s1_row(int g) const { return s1_r0 + D * LR * (g / GB); }
+  __device__ __forceinline__ int s1_col(int g, int e) const { return s1_cB + LB * (g % GB) + B * e; }
+  // the class's line of group g, from the line of group 0
+  static __device__ __forceinline__ constexpr int line(int g) { return LB * (g % GB) + B * LR * (g / GB); }
+  // frequency row of S3 register (g, e)
   __device__ __forceinline__ int s3_row(int g, int e) const { return s3_kC(g) + C * e; }
 
+  // ---- class-private transpose between S1 and S2 (one warp, __syncwarp only) ----
+  // element (kA, line l = B rC + cB) of the class at kA PP + l
   __device__ __forceinline__ void write_s1(float2* sm, const float2 (&x)[E]) const {
-    float2* w = sm + s1_r + 4800 * s1_cB;
 #pragma unroll
-    for (int e = 0; e < A; ++e) w[100 * e] = x[e];
+    for (int g = 0; g < G1; ++g)
+#pragma unroll
+      for (int e = 0; e < A; ++e) sm[pv_w + PP * e + line(g)] = x[g * A + e];
   }
   __device__ __forceinline__ void read_s1(const float2* sm, float2 (&x)[E]) const {
-    const float2* r = sm + s1_r + 4800 * s1_cB;
 #pragma unroll
-    for (int e = 0; e < A; ++e) x[e] = r[100 * e];
+    for (int g = 0; g < G1; ++g)
+#pragma unroll
+      for (int e = 0; e < A; ++e) x[g * A + e] = sm[pv_w + PP * e + line(g)];
   }
-  // S2 input layout (cB, rC): element (rD + 4 rC, cB, kA)
+  // S2 input layout (cB, rC)
   __device__ __forceinline__ void read_s2_in(const float2* sm, float2 (&x)[E]) const {
-    const float2* r = sm + s2_rD + 100 * s2_kA;
 #pragma unroll
     for (int cB = 0; cB < B; ++cB)
 #pragma unroll
-      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = r[4 * rC + 4800 * cB];
+      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = sm[pv_r + B * rC + cB];
   }
   __device__ __forceinline__ void write_s2_in(float2* sm, const float2 (&x)[E]) const {
-    float2* w = sm + s2_rD + 100 * s2_kA;
 #pragma unroll
     for (int cB = 0; cB < B; ++cB)
 #pragma unroll
-      for (int rC = 0; rC < C; ++rC) w[4 * rC + 4800 * cB] = x[cB * C + rC];
+      for (int rC = 0; rC < C; ++rC) sm[pv_r + B * rC + cB] = x[cB * C + rC];
   }
-  // S2 output layout (kB, kC): element (row rD + 4 kC, col kA + 48 kB)
+  // ---- main exchange between S2 and S3: element (rD, kC, column) at rD CS + kC N + column ----
+  // S2 output layout (kB, kC): column kA + A kB
   __device__ __forceinline__ void write_s2_out(float2* sm, const float2 (&x)[E]) const {
-    float2* w = sm + 104 * s2_rD + s2_kA;
 #pragma unroll
     for (int kB = 0; kB < B; ++kB)
 #pragma unroll
-      for (int kC = 0; kC < C; ++kC) w[416 * kC + 48 * kB] = x[kB * C + kC];
+      for (int kC = 0; kC < C; ++kC) sm[mn_2 + N * kC + A * kB] = x[kB * C + kC];
   }
   __device__ __forceinline__ void read_s2_out(const float2* sm, float2 (&x)[E]) const {
-    const float2* r = sm + 104 * s2_rD + s2_kA;
 #pragma unroll
     for (int kB = 0; kB < B; ++kB)
 #pragma unroll
-      for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = r[416 * kC + 48 * kB];
+      for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = sm[mn_2 + N * kC + A * kB];
   }
-  // S3 layout (g, e): element (row e + 4 kC_g, col)
+  // S3 layout (g, e): rD = e, kC = kC_g, column s3_c
   __device__ __forceinline__ void read_s3(const float2* sm, float2 (&x)[E]) const {
-    const float2* r = sm + 104 * 4 * s3_kC0 + s3_c;
 #pragma unroll
     for (int g = 0; g < G3; ++g)
 #pragma unroll
-      for (int e = 0; e < D; ++e) x[g * D + e] = r[104 * (e + 8 * g)];
+      for (int e = 0; e < D; ++e) x[g * D + e] = sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g];
   }
   __device__ __forceinline__ void write_s3(float2* sm, const float2 (&x)[E]) const {
-    float2* w = sm + 104 * 4 * s3_kC0 + s3_c;
 #pragma unroll
     for (int g = 0; g < G3; ++g)
 #pragma unroll
-      for (int e = 0; e < D; ++e) w[104 * (e + 8 * g)] = x[g * D + e];
+      for (int e = 0; e < D; ++e) sm[mn_3 + CS * e + (T / 32 / (N / 32)) * N * g] = x[g * D + e];
   }
 
-  template <bool INV>
-  __device__ __forceinline__ void s1(float2 (&x)[E]) const { dft_reg_n<A, INV, 1, 0>(x); }
-  template <bool INV, int G>
-  __device__ __forceinline__ void s3_groups(float2 (&x)[E]) const {
-    if constexpr (G < G3) {
-      dft_reg<D, INV, 1, G * D>(x);
-      s3_groups<INV, G + 1>(x);
+  // ---- register stages ----
+  // G transforms of L consecutive registers each
+  template <int L, int G, bool INV, int K>
+  __device__ __forceinline__ void groups(float2 (&x)[E]) const {
+    if constexpr (K < G) {
+      dft_reg_n<L, INV, 1, K * L>(x);
+      groups<L, G, INV, K + 1>(x);
     }
   }
   template <bool INV>
-  __device__ __forceinline__ void s3(float2 (&x)[E]) const { s3_groups<INV, 0>(x); }
+  __device__ __forceinline__ void s1(float2 (&x)[E]) const {
+    groups<A, G1, INV, 0>(x);
+  }
 
   template <bool INV>
-  __device__ __forceinline__ void s2_core(float2 (&x)[E]) const {
-#pragma unroll
-    for (int rC = 0; rC < C; ++rC) {  // 2-point DFT over cB
-      const float2 a = x[rC], b = x[C + rC];
-      x[rC] = cadd(a, b);
-      x[C + rC] = csub(a, b);
-    }
-    dft_reg_n<C, INV, 1, 0>(x);
-    dft_reg_n<C, INV, 1, C>(x);
+  __device__ __forceinline__ void s3(float2 (&x)[E]) const {
+    groups<D, G3, INV, 0>(x);
   }
+
+  // S2 twiddles in the order the warps read them: w_N^(cB kA) at (cB - 1) A + kA (a
+  // class's lanes on consecutive words), then w_N^(rD kC) at TWC + (kC - 1) D + rD (one word
+  // per class).
+  static constexpr int TWC = (B - 1) * A;
+  static constexpr int TW_FLOAT2 = TWC + (C - 1) * D;
+  static __device__ __forceinline__ void fill_twiddles(float2* tw, int tid, int nthreads) {
+    for (int k = tid; k < TW_FLOAT2; k += nthreads) {
+      const int e = k < TWC ? (k / A + 1) * (k % A) : ((k - TWC) / D + 1) * ((k - TWC) % D);
+      double s, c;
+      sincospi(-2.0 * (double)e / (double)N, &s, &c);
+      tw[k] = make_float2((float)c, (float)s);
+    }
+  }
+  // S2 forward: x holds (cB, rC) on entry, (kB, kC) on exit.
   __device__ __forceinline__ void s2_fwd(float2 (&x)[E], const float2* tw) const {
-    const float2 w1 = tw[s2_kA];  // w96^(1 * kA)
 #pragma unroll
-    for (int rC = 0; rC < C; ++rC) x[C + rC] = cmul(x[C + rC], w1);
+    for (int cB = 1; cB < B; ++cB) {
+      const float2 w = tw[(cB - 1) * A + s2_kA];
+#pragma unroll
+      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmul(x[cB * C + rC], w) : cmul(x[cB * C + rC], w);
+    }
     s2_core<false>(x);
 #pragma unroll
     for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[s2_rD * kC];  // rD * kC <= 69 < 96
+      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
 #pragma unroll
-      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = cmul(x[kB * C + kC], w);
+      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmul(x[kB * C + kC], w) : cmul(x[kB * C + kC], w);
     }
   }
+  // S2 inverse: (kB, kC) on entry, (cB, rC) on exit.
   __device__ __forceinline__ void s2_inv(float2 (&x)[E], const float2* tw) const {
 #pragma unroll
     for (int kC = 1; kC < C; ++kC) {
-      const float2 w = tw[s2_rD * kC];
+      const float2 w = tw[TWC + (kC - 1) * D + s2_rD];
 #pragma unroll
-      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = cmulc(x[kB * C + kC], w);
+      for (int kB = 0; kB < B; ++kB) x[kB * C + kC] = QB_F32X2_S2 ? pcmulc(x[kB * C + kC], w) : cmulc(x[kB * C + kC], w);
     }
     s2_core<true>(x);
-    const float2 w1 = tw[s2_kA];
 #pragma unroll
-    for (int rC = 0; rC < C; ++rC) x[C + rC] = cmulc(x[C + rC], w1);
+    for (int cB = 1; cB < B; ++cB) {
+      const float2 w = tw[(cB - 1) * A + s2_kA];
+#pragma unroll
+      for (int rC = 0; rC < C; ++rC) x[cB * C + rC] = QB_F32X2_S2 ? pcmulc(x[cB * C + rC], w) : cmulc(x[cB * C + rC], w);
+    }
+  }
+  // B-point DFT along index 0 (stride C) and C-point DFT along index 1 (stride 1).
+  template <bool INV>
+  __device__ __forceinline__ void s2_core(float2 (&x)[E]) const {
+    s2_bdft<INV, 0>(x);
+    s2_cdft<INV, 0>(x);
+  }
+  template <bool INV, int RC>
+  __device__ __forceinline__ void s2_bdft(float2 (&x)[E]) const {
+    if constexpr (RC < C) {
+      dft_reg_n<B, INV, C, RC>(x);
+      s2_bdft<INV, RC + 1>(x);
+    }
+  }
+  template <bool INV, int KB>
+  __device__ __forceinline__ void s2_cdft(float2 (&x)[E]) const {
+    if constexpr (KB < B) {
+      dft_reg_n<C, INV, 1, KB * C>(x);
+      s2_cdft<INV, KB + 1>(x);
+    }
   }
 
+  // ---- whole transforms between layouts ----
+  // One CTA barrier each.  Between two barriers either every class is owned by its warp
+  // (S2 side: main exchange, private transpose, S1) or every (kC, column) pair by its
+  // thread (S3 side reads and writes the same elements), so no barrier is needed before
+  // a write.  A caller that leaves the S2 side (after inverse) without forward, or enters
+  // it (forward) without inverse, puts a __syncthreads between.
+  // Forward: registers in S1 layout -> registers in S3 layout (unnormalised).
   __device__ __forceinline__ void forward(float2 (&x)[E], float2* sm, const float2* tw) const {
     s1<false>(x);
-    __syncthreads();
+    __syncwarp();  // the warp's reads of the inverse's transpose are complete
     write_s1(sm, x);
-    __syncthreads();
+    __syncwarp();
     read_s2_in(sm, x);
     s2_fwd(x, tw);
-    __syncthreads();
+    __syncwarp();
     write_s2_out(sm, x);
     __syncthreads();
     read_s3(sm, x);
     s3<false>(x);
   }
+  // Inverse: registers in S3 layout -> registers in S1 layout (unnormalised).
   __device__ __forceinline__ void inverse(float2 (&x)[E], float2* sm, const float2* tw) const {
     s3<true>(x);
-    __syncthreads();
     write_s3(sm, x);
     __syncthreads();
     read_s2_out(sm, x);
     s2_inv(x, tw);
-    __syncthreads();
+    __syncwarp();
     write_s2_in(sm, x);
-    __syncthreads();
+    __syncwarp();
     read_s1(sm, x);
     s1<true>(x);
   }

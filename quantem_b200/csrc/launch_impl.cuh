@@ -44,6 +44,7 @@ inline BatchParams to_params(const ptycho_batch_args* a) {
   p.grad_descan = a->grad_descan;
   p.grad_prop = a->grad_prop;
   p.sep_shared = 0;
+  p.tile_out = 0;
   return p;
 }
 
@@ -59,8 +60,9 @@ int carveout(size_t smem) {
   return pc < 100 ? (int)pc : 100;
 }
 template <int N>
-BatchParams batch_params(const ptycho_batch_args* a, bool tile = true) {
+BatchParams batch_params(const ptycho_batch_args* a, bool tile = true, bool tile_out = false) {
   BatchParams p = to_params(a);
+  p.tile_out = tile_out;
   p.sep_shared = sep_in_smem<N>(tile, a->S);
   return p;
 }
@@ -87,8 +89,9 @@ void launch_ext(const BatchParams& p, int grid, size_t smem, cudaStream_t st) {
 // 256 KB is L1.
 template <int N>
 int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const BatchParams p = batch_params<N>(a, !adj);
-  const size_t smem = batch_smem<N>(a, !adj);
+  const bool tile = !adj && !a->out_intensity;  // the output array serves as the tile
+  const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
+  const size_t smem = batch_smem<N>(a, tile);
   if (adj) {
     cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -104,8 +107,9 @@ int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
 // the instances with the analytic update or with extensions
 template <int N>
 int launch_special(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const BatchParams p = batch_params<N>(a, !adj);
-  const size_t smem = batch_smem<N>(a, !adj);
+  const bool tile = !adj && !a->out_intensity;  // the output array serves as the tile
+  const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
+  const size_t smem = batch_smem<N>(a, tile);
   if (!a->analytic) {
     if (adj)
       launch_ext<N, true>(p, a->grid, smem, st);

@@ -66,6 +66,7 @@ struct BatchParams {
   float* grad_positions;      // optional (B, 2) dL/d(position), serial autograd adjoint only
   const float* descan;        // optional (npos, 2) descan shifts [px] applied to the exit wave
   float* grad_descan;         // optional (B, 2) dL/d(descan), serial autograd adjoint only
+  int tile_out;               // forward kernel: out_intensity serves as the mode-sum tile (none in shared memory)
   int sep_shared;             // the separable factors fit in shared memory (else read through L1)
   float* grad_prop;           // optional (S-1, 2) propagator sensitivities, serial autograd adjoint only
 };
@@ -149,7 +150,7 @@ __device__ __forceinline__ void load_pairs(const float2* src, int tid, float2 (&
 }
 
 // Shared-memory bytes of the batch kernels: exchange buffer, twiddles, shift ramps and
-// wrap maps; the intensity tile of the forward kernel (the adjoint kernel keeps its
+// wrap maps; the intensity tile of the forward kernel when no output holds it (the adjoint kernel keeps its
 // intensity / dL/dI tile in its global scratch slot, L2-resident, 64 KB per CTA at 128^2:
 // the shared memory it would take is left to the L1 cache); and the separable propagator
 // factors when they are kept here.
@@ -159,8 +160,10 @@ constexpr size_t batch_smem_bytes(bool tile, bool sep, int S) {
          (tile ? sizeof(float) * (size_t)N * N : 0) +
          (sep ? sizeof(float2) * (size_t)2 * N * (size_t)(S > 1 ? S - 1 : 0) : 0);
 }
-// Resident CTAs per SM of the batch kernels; the instances with extensions (EXT, AN) take
-// one less, since they spill at 128 registers.
+// Resident CTAs per SM of the batch kernels.  The instances with extensions (EXT, AN) take
+// one less: at the plain kernels' register counts they spill (96^2 with position gradients:
+// 1.5 KB at 168 registers, 937 against 927 us per 701 positions at 255; 64^2: 516 us with two
+// CTAs of 128 registers, 545 with three of 80, per 1000 positions).
 template <int N>
 constexpr int batch_ctas(bool ext) {
   return ext && Fft2<N>::CTAS > 1 ? Fft2<N>::CTAS - 1 : Fft2<N>::CTAS;
@@ -279,11 +282,11 @@ __device__ __forceinline__ void apply_prop(const Fft2<N>& f, float2 (&x)[Fft2<N>
   }
 }
 
-// Offset of S1 column register e from the window's centre column c0 when the window
+// Offset of S1 column register (g, e) from the window's centre column c0 when the window
 // does not wrap around the object's columns: compile-time apart from the thread's cB.
 template <int N>
-__device__ __forceinline__ constexpr int inside_off(int e) {
-  return Fft2<N>::B * e - (e >= Fft2<N>::A / 2 ? N : 0);
+__device__ __forceinline__ constexpr int inside_off(int g, int e) {
+  return Fft2<N>::LB * (g % Fft2<N>::GB) + Fft2<N>::B * e - (e >= Fft2<N>::A / 2 ? N : 0);
 }
 
 // x (S1 layout) *= o (CONJ: conj(o)) for the object slice, rows through rowmap, columns
@@ -304,7 +307,7 @@ __device__ __forceinline__ void gather_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>
       for (int e0 = 0; e0 < A; e0 += BT) {
         float2 ob[BT];
 #pragma unroll
-        for (int j = 0; j < BT; ++j) ob[j] = ld_obj(row + inside_off<N>(e0 + j), pol);
+        for (int j = 0; j < BT; ++j) ob[j] = ld_obj(row + inside_off<N>(g, e0 + j), pol);
 #pragma unroll
         for (int j = 0; j < BT; ++j) {
           const int i = g * A + e0 + j;
@@ -320,7 +323,7 @@ __device__ __forceinline__ void gather_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>
       for (int e0 = 0; e0 < A; e0 += 2) {
         float2 ob[2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) ob[j] = ld_obj(row + colmap[f.s1_col(e0 + j)], pol);
+        for (int j = 0; j < 2; ++j) ob[j] = ld_obj(row + colmap[f.s1_col(g, e0 + j)], pol);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int i = g * A + e0 + j;
@@ -344,7 +347,7 @@ __device__ __forceinline__ void descan_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>
 #pragma unroll
     for (int e = 0; e < A; ++e) {
       float sn, cs;
-      sincospif(-2.0f * (ar + (float)fsigned(f.s1_col(e), N) * dc) / (float)N, &sn, &cs);
+      sincospif(-2.0f * (ar + (float)fsigned(f.s1_col(g, e), N) * dc) / (float)N, &sn, &cs);
       const int i = g * A + e;
       x[i] = CONJ ? cmulc(x[i], make_float2(cs, sn)) : cmul(x[i], make_float2(cs, sn));
     }
@@ -373,6 +376,12 @@ __device__ __forceinline__ void accumulate_probe_grad(const Fft2<N>& f, const fl
     }
 }
 
+// Index of frequency (kr, kc) in the detector (centred) layout.
+template <int N>
+__device__ __forceinline__ int detector_index(int kr, int kc) {
+  return (kr >= N / 2 ? kr - N / 2 : kr + N / 2) * N + (kc >= N / 2 ? kc - N / 2 : kc + N / 2);
+}
+
 // Body of the serial batch kernel for one dataset: CTA `cta` of the `ncta` CTAs
 // that work on this dataset's positions.
 // EXT: the optional extensions (descan shifts, position / descan / propagator gradients)
@@ -391,7 +400,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   float2* colf = rowf + N;
   // intensity / dL/dI tile: shared memory (forward-only) or the CTA's scratch slot (ADJ)
   float* inten_sm = reinterpret_cast<float*>(colf + N);
-  int* rowmap = reinterpret_cast<int*>(ADJ ? reinterpret_cast<float*>(colf + N) : inten_sm + N * N);
+  int* rowmap = reinterpret_cast<int*>(ADJ || p.tile_out ? inten_sm : inten_sm + N * N);
   int* colmap = rowmap + N;
   // separable propagators K_s[kr][kc] = Kr_s[kr] * Kc_s[kc] (probe_models.py:376-427
   // builds exp(-i pi lambda dz (kr^2 + kc^2)) times per-axis tilt ramps)
@@ -444,12 +453,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
     nfred[tid >> 5] = 0;
   }
 
-  // each CTA takes a contiguous block of the batch: positions processed at the same
-  // time are far apart in the batch order, so raster-ordered batches do not pile
-  // the object-gradient atomics of neighbouring windows onto the same addresses
-  const int bchunk = (p.B + ncta - 1) / ncta;
-  const int bend = min(p.B, (cta + 1) * bchunk);
-  for (int b = cta * bchunk; b < bend; ++b) {
+  // each CTA takes a contiguous block of the batch (evenly sized, so that CTAs sharing an SM
+  // get the same work): positions processed at the same time are far apart in the batch
+  // order, so raster-ordered batches do not pile the object-gradient atomics of
+  // neighbouring windows onto the same addresses
+  const int bend = (int)((int64_t)p.B * (cta + 1) / ncta);
+  for (int b = (int)((int64_t)p.B * cta / ncta); b < bend; ++b) {
     const int64_t gi64 = p.batch_idx[b];
     if (gi64 < 0 || gi64 >= p.npos) {  // invalid index: skip the position and report it
       if (tid == 0) status_add_invalid(p.status, 1);
@@ -537,14 +546,14 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         if (p.out_waves) {
           float2* ow = p.out_waves + (((size_t)s * P + m) * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
+          for (int e = 0; e < E; ++e) ow[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)] = x[e];
         }
         gather_mul<N, false>(f, x, slice, p.Wo, rowmap, colmap, cin);
         if (EXT && s == S - 1 && p.descan) descan_mul<N, false>(f, x, __ldg(p.descan + 2 * (size_t)gi), __ldg(p.descan + 2 * (size_t)gi + 1));
         if (s == S - 1 && p.out_exit) {
           float2* oe = p.out_exit + ((size_t)m * p.B + b) * NN;
 #pragma unroll
-          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = x[e];
+          for (int e = 0; e < E; ++e) oe[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)] = x[e];
         }
       } else {
         const float sc = first_bwd ? inv_n : inv_n2;  // adjoint of the orthonormal FFT, or of a propagation
@@ -569,27 +578,27 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
             ps[j + 1] = make_float2(v.z, v.w);
           }
 #pragma unroll
-          for (int j = 0; j < BT; ++j) ob[j] = ld_obj(orow + column(e0 + j), pol);
+          for (int j = 0; j < BT; ++j) ob[j] = ld_obj(orow + column(g, e0 + j), pol);
 #pragma unroll
           for (int j = 0; j < BT; ++j) {
             const float2 gx = cscale(x[i0 + j], sc);
-            atomicAdd(grow + column(e0 + j), cmulc(gx, ps[j]));  // conj(psi) * g
+            atomicAdd(grow + column(g, e0 + j), cmulc(gx, ps[j]));  // conj(psi) * g
             x[i0 + j] = cmulc(gx, ob[j]);                        // conj(o) * g
           }
           if (AN) {  // sum_patches(|psi|^2) of this slice and mode (object_models.py:701-703)
             float* nrow = p.an_norm + ((size_t)s * P + m) * HoWo + (size_t)rowmap[f.s1_row(g)] * p.Wo;
 #pragma unroll
-            for (int j = 0; j < BT; ++j) atomicAdd(nrow + column(e0 + j), cabs2(ps[j]));
+            for (int j = 0; j < BT; ++j) atomicAdd(nrow + column(g, e0 + j), cabs2(ps[j]));
           }
         };
         if (cin >= 0) {
 #pragma unroll
           for (int i = 0; i < E; i += 8)
-            scatter(std::integral_constant<int, 8>(), i, [&](int e) { return cin + inside_off<N>(e); });
+            scatter(std::integral_constant<int, 8>(), i, [&](int g, int e) { return cin + inside_off<N>(g, e); });
         } else {  // wrapping windows are few: small batches, so that this path costs no registers
 #pragma unroll
           for (int i = 0; i < E; i += 2)
-            scatter(std::integral_constant<int, 2>(), i, [&](int e) { return colmap[f.s1_col(e)]; });
+            scatter(std::integral_constant<int, 2>(), i, [&](int g, int e) { return colmap[f.s1_col(g, e)]; });
         }
         if (EXT && first_bwd && p.grad_descan) {
           // x = dL/dw of the last slice's incident wave w, so conj(x) w = conj(dL/dE) E for the
@@ -600,8 +609,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
             const float4 v = reinterpret_cast<const float4*>(wv)[(e >> 1) * T + tid];
             const float im0 = x[e].x * v.y - x[e].y * v.x;
             const float im1 = x[e + 1].x * v.w - x[e + 1].y * v.z;
-            gc = fmaf((float)fsigned(f.s1_col(e % A), N), im0, gc);
-            gc = fmaf((float)fsigned(f.s1_col(e % A + 1), N), im1, gc);
+            gc = fmaf((float)fsigned(f.s1_col(e / A, e % A), N), im0, gc);
+            gc = fmaf((float)fsigned(f.s1_col(e / A, e % A + 1), N), im1, gc);
             gr = fmaf((float)fsigned(f.s1_row(e / A), N), im0 + im1, gr);
           }
           for (int o = 16; o > 0; o >>= 1) {
@@ -635,9 +644,9 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
             float2* pg = pgrad + (size_t)m * NN + (size_t)f.s1_row(e0 / A) * N;
             float2 old[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) old[j] = pg[f.s1_col(e0 % A + j)];
+            for (int j = 0; j < 8; ++j) old[j] = pg[f.s1_col(e0 / A, e0 % A + j)];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) pg[f.s1_col(e0 % A + j)] = cadd(old[j], x[e0 + j]);
+            for (int j = 0; j < 8; ++j) pg[f.s1_col(e0 / A, e0 % A + j)] = cadd(old[j], x[e0 + j]);
           }
           if (m > 0) {
             --m;
@@ -665,10 +674,21 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
           float2* fw = slot + (size_t)(P * S + m) * NN;
           store_pairs<E, T>(fw, tid, x);
         }
+        if (!ADJ && p.tile_out) {
+          float* oi = p.out_intensity + (size_t)b * NN;
 #pragma unroll
-        for (int e = 0; e < E; e += 2) {
-          const float2 old = m == 0 ? make_float2(0.f, 0.f) : inten2[(e >> 1) * T + tid];
-          inten2[(e >> 1) * T + tid] = make_float2(old.x + cabs2(x[e]), old.y + cabs2(x[e + 1]));
+          for (int g = 0; g < G3; ++g)
+#pragma unroll
+            for (int e = 0; e < D; ++e) {
+              float* o = oi + detector_index<N>(f.s3_row(g, e), f.s3_c);
+              *o = (m == 0 ? 0.f : *o) + cabs2(x[g * D + e]);
+            }
+        } else {
+#pragma unroll
+          for (int e = 0; e < E; e += 2) {
+            const float2 old = m == 0 ? make_float2(0.f, 0.f) : inten2[(e >> 1) * T + tid];
+            inten2[(e >> 1) * T + tid] = make_float2(old.x + cabs2(x[e]), old.y + cabs2(x[e + 1]));
+          }
         }
         if (ADJ && AN) {  // sum_p |Psi_p + 1e-9|^2 (ptychography_base.py:958)
           float2* t2 = reinterpret_cast<float2*>(tile2);
@@ -694,10 +714,9 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
           for (int g = 0; g < G3; ++g)
 #pragma unroll
             for (int e = 0; e < D; ++e) {
-              const int kr = f.s3_row(g, e), kc = f.s3_c;
-              const int di = ((kr + N / 2) % N) * N + ((kc + N / 2) % N);
+              const int di = detector_index<N>(f.s3_row(g, e), f.s3_c);
               const int li = 2 * (((g * D + e) >> 1) * T + tid) + ((g * D + e) & 1);
-              const float I = inten[li];
+              const float I = !ADJ && p.tile_out ? p.out_intensity[(size_t)b * NN + di] : inten[li];
               if (!isfinite(I)) ++nonfinite;
               float dldi;
               const float tv = __ldcs(tg + di);  // targets stream through L2 once per iteration
@@ -713,8 +732,8 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
                   tile2[li] = 0.f;
                 }
               }
-              inten[li] = dldi;
-              if (p.out_intensity) p.out_intensity[(size_t)b * NN + di] = I;
+              if (ADJ) inten[li] = dldi;
+              if (p.out_intensity && !(!ADJ && p.tile_out)) p.out_intensity[(size_t)b * NN + di] = I;
             }
           for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
           const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
@@ -876,7 +895,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2*
     float2 x[E];
     if (!INV) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) x[e] = src[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)];
+      for (int e = 0; e < E; ++e) x[e] = src[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)];
       f.forward(x, sm, tw);
 #pragma unroll
       for (int g = 0; g < G3; ++g)
@@ -889,7 +908,7 @@ __global__ void __launch_bounds__(Fft2<N>::T, 1) fft2_batch_kernel(const float2*
         for (int e = 0; e < D; ++e) x[g * D + e] = src[(size_t)f.s3_row(g, e) * N + f.s3_c];
       f.inverse(x, sm, tw);
 #pragma unroll
-      for (int e = 0; e < E; ++e) dst[(size_t)f.s1_row(e / A) * N + f.s1_col(e % A)] = cscale(x[e], scale);
+      for (int e = 0; e < E; ++e) dst[(size_t)f.s1_row(e / A) * N + f.s1_col(e / A, e % A)] = cscale(x[e], scale);
     }
     __syncthreads();
   }

@@ -62,16 +62,15 @@ def _window_groups(problems):
 
 def default_grids(problems, total=None):
     """CTAs per dataset proportional to its transform count (at least one); each
-    probe-window group (a launch of its own) splits the whole SM count."""
-    total = total or ops.sm_count(problems[0].obj.device)
-    groups = _window_groups(problems)
-    if len(groups) > 1:
-        out = [0] * len(problems)
-        for idx in groups:
-            for i, g in zip(idx, _split(([problems[i] for i in idx]), total)):
-                out[i] = g
-        return out
-    return _split(problems, total)
+    probe-window group (a launch of its own) splits ``total`` CTAs (default: as many as the
+    device holds at once for that window)."""
+    out = [0] * len(problems)
+    for idx in _window_groups(problems):
+        sub = [problems[i] for i in idx]
+        t = total or ops.resident_ctas(int(sub[0].probe.shape[-1]), sub[0].obj.device)
+        for i, g in zip(idx, _split(sub, t)):
+            out[i] = g
+    return out
 
 
 def _split(problems, total):
@@ -273,15 +272,16 @@ class MultiIteration:
 def autotune_grids(problems, total=None, trials=2, cache={}):
     """Pick the CTA partition of a multi-dataset launch by timing candidates.
 
-    Candidates: the cost-proportional split of the SM count, the same with one
-    extra wave of CTAs, and splits that move CTAs towards the datasets with
+    Candidates: the cost-proportional split of the resident CTAs, of one and two CTAs per
+    SM (``total`` and twice it, when given), and splits that move CTAs towards the datasets with
     the highest cost per CTA.  Each is timed (CUDA events) on the forward +
     adjoint launch; the fastest is cached per problem signature."""
     key = tuple(p.signature() for p in problems)
     if key in cache:
         return cache[key]
     sms = total or ops.sm_count(problems[0].obj.device)
-    cands = [default_grids(problems, sms), default_grids(problems, 2 * sms)]
+    cands = ([] if total else [default_grids(problems)]) + [default_grids(problems, sms),
+                                                            default_grids(problems, 2 * sms)]
     base = np.array(cands[0])
     cost = np.array([p.cost() for p in problems])
     for shift in (1, 2):

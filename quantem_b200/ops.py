@@ -71,6 +71,19 @@ def sm_count(device: torch.device | None = None) -> int:
     return _SM_COUNT[dev]
 
 
+def resident_ctas(n: int, device: torch.device | None = None) -> int:
+    """CTAs of the plain batch kernels that one device holds at once for a window of ``n``
+    pixels: the number a persistent launch splits its positions over (several per SM for the
+    small windows)."""
+    a = _lib.BatchArgs()
+    a.n, a.S, a.P, a.B, a.variant = int(n), 1, 1, 2 ** 30, _lib.VARIANTS["serial"]
+    grid = ctypes.c_int(0)
+    with torch.cuda.device(device if device is not None else torch.cuda.current_device()):
+        _lib.check(_lib.lib().ptycho_batch_plan(ctypes.byref(a), 1, None, ctypes.byref(grid), None, None, None),
+                   "batch_plan")
+    return grid.value
+
+
 def reduce_blocks() -> int:
     return int(_lib.lib().ptycho_reduce_blocks())
 
