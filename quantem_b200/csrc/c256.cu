@@ -53,7 +53,8 @@ int qb_max_clusters_256(bool adj) {
 }
 
 int qb_launch_c256(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const qb::BatchParams p = qb::to_params(a);
+  qb::BatchParams p = qb::to_params(a);
+  p.sep_shared = (reinterpret_cast<uintptr_t>(a->prop_r) & 15) == 0;  // row factors read two at a time
   cudaLaunchAttribute attr[1];
   cudaError_t e;
   if (adj) {

@@ -80,19 +80,22 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
       for (int i = 0; i < E; ++i) pgrad[(size_t)m * NN + (size_t)f.b_kr(i) * N + kc] = make_float2(0.f, 0.f);
   }
   cl.sync();  // every CTA of the cluster runs before any distributed-shared-memory access
-  double loss_acc = 0.0;
-  int nonfinite = 0;
+  // loss and non-finite counts live in shared memory between positions (warp w owns entry w)
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = 0.0;
+    nfred[tid >> 5] = 0;
+  }
 
   // each cluster takes a contiguous block of the batch (concurrent positions far apart)
-  const int bchunk = (p.B + ncl - 1) / ncl;
-  const int bend = min(p.B, (cid + 1) * bchunk);
-  for (int b = cid * bchunk; b < bend; ++b) {
-    const int64_t gi = p.batch_idx[b];
-    if (gi < 0 || gi >= p.npos) {  // the whole cluster skips the position (same b)
+  const int bend = (int)((int64_t)p.B * (cid + 1) / ncl);
+  for (int b = (int)((int64_t)p.B * cid / ncl); b < bend; ++b) {
+    const int64_t gi64 = p.batch_idx[b];
+    if (gi64 < 0 || gi64 >= p.npos) {  // the whole cluster skips the position (same b)
       if (tid == 0 && q == 0) status_add_invalid(p.status, 1);
       continue;
     }
-    const float py = p.positions[2 * gi], px = p.positions[2 * gi + 1];
+    const int gi = (int)gi64;
+    const float py = p.positions[2 * (size_t)gi], px = p.positions[2 * (size_t)gi + 1];
     const float ry = rintf(py), rx = rintf(px);
     const float fy = py - ry, fx = px - rx;
     const int r0 = wrap_index((int)ry, p.Ho), c0 = wrap_index((int)rx, p.Wo);
@@ -112,7 +115,10 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
       }
     }
     __syncthreads();
-    const int orow = rowmap[f.a_row()];
+    // first column of this thread when the window lies inside the object's columns, else -1
+    const int cin = (c0 >= N / 2 && c0 + N / 2 <= p.Wo) ? c0 + f.tl : -1;
+    auto inside = [&](int e) { return cin + 8 * e - (e >= E / 2 ? N : 0); };
+    auto wrapped = [&](int e) { return colmap[f.a_col(e)]; };
 
     float2 x[E];
     auto load_probe = [&](int mm) {
@@ -133,10 +139,25 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
     auto apply_prop = [&](int s, bool conj) {
       if (p.prop_r) {
         const float2 kcf = __ldg(p.prop_c + (size_t)s * N + kc);
+        const float2* kr = p.prop_r + (size_t)s * N + 4 * f.tl;  // rows 4 tl + a + 32 kB
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-          const float2 k = cmul(__ldg(p.prop_r + (size_t)s * N + f.b_kr(i)), kcf);
-          x[i] = conj ? cmulc(x[i], k) : cmul(x[i], k);
+        for (int kB = 0; kB < 8; ++kB) {
+          float2 v[4];
+          if (p.sep_shared) {  // 16-byte aligned factors
+            const float4 lo = __ldg(reinterpret_cast<const float4*>(kr + 32 * kB));
+            const float4 hi = __ldg(reinterpret_cast<const float4*>(kr + 32 * kB + 2));
+            v[0] = make_float2(lo.x, lo.y), v[1] = make_float2(lo.z, lo.w);
+            v[2] = make_float2(hi.x, hi.y), v[3] = make_float2(hi.z, hi.w);
+          } else {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) v[a] = __ldg(kr + 32 * kB + a);
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const float2 k = cmul(v[a], kcf);
+            float2& y = x[a * 8 + kB];
+            y = conj ? cmulc(y, k) : cmul(y, k);
+          }
         }
       } else {
         const float2* pr = p.prop + (size_t)s * NN;
@@ -147,17 +168,47 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
         }
       }
     };
-    auto gather_mul = [&](int s) {
-      const float2* orow_ptr = p.obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
+    // x *= object row, batches of loads in flight
+    auto gather = [&](auto batch, const float2* row, auto column) {
+      constexpr int BT = decltype(batch)::value;
+      const uint64_t pol = evict_last_policy();
 #pragma unroll
-      for (int e0 = 0; e0 < E; e0 += 8) {
-        float2 ob[8];
+      for (int e0 = 0; e0 < E; e0 += BT) {
+        float2 ob[BT];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ob[j] = __ldg(orow_ptr + colmap[f.a_col(e0 + j)]);
+        for (int j = 0; j < BT; ++j) ob[j] = ld_obj(row + column(e0 + j), pol);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[e0 + j] = cmul(x[e0 + j], ob[j]);
+        for (int j = 0; j < BT; ++j) x[e0 + j] = cmul(x[e0 + j], ob[j]);
       }
     };
+    // gradient contribution conj(psi) g scattered, x = conj(o) g
+    auto scatter = [&](auto batch, int s, const float2* wv, float sc, auto column) {
+      constexpr int BT = decltype(batch)::value;
+      const uint64_t pol = evict_last_policy();
+      const size_t ro = (size_t)s * HoWo + (size_t)rowmap[f.a_row()] * p.Wo;
+      const float2* row = p.obj + ro;
+      float2* grow = p.grad_obj + ro;
+#pragma unroll
+      for (int e0 = 0; e0 < E; e0 += BT) {
+        float2 ps[BT], ob[BT];
+#pragma unroll
+        for (int j = 0; j < BT; j += 2) {
+          const float4 v = ld_stream4(reinterpret_cast<const float4*>(wv) + ((e0 + j) >> 1) * T + tid);
+          ps[j] = make_float2(v.x, v.y);
+          ps[j + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int j = 0; j < BT; ++j) ob[j] = ld_obj(row + column(e0 + j), pol);
+#pragma unroll
+        for (int j = 0; j < BT; ++j) {
+          const float2 g = cscale(x[e0 + j], sc);
+          atomicAdd(grow + column(e0 + j), cmulc(g, ps[j]));
+          x[e0 + j] = cmulc(g, ob[j]);
+        }
+      }
+    };
+    using Wide = std::integral_constant<int, 8>;
+    using Narrow = std::integral_constant<int, 2>;  // wrapping windows are few
 
     int m = 0, s = 0;
     bool bwd = false, first_bwd = false, rec = false;
@@ -195,34 +246,18 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
             continue;
           }
         }
-        gather_mul(rec ? srec : s);
+        const float2* row = p.obj + (size_t)(rec ? srec : s) * HoWo + (size_t)rowmap[f.a_row()] * p.Wo;
+        if (cin >= 0)
+          gather(Wide(), row, inside);
+        else
+          gather(Narrow(), row, wrapped);
       } else {
         const float sc = first_bwd ? inv_n : inv_n2;
         const float2* wv = ck == 0 ? wave_slot(m, s) : seg_slot(s - seg_lo);
-        const float2* orow_ptr = p.obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
-        float2* grow = p.grad_obj + (size_t)s * HoWo + (size_t)orow * p.Wo;
-#pragma unroll
-        for (int e0 = 0; e0 < E; e0 += 4) {
-          float2 ps[4], ob[4];
-          int col[4];
-#pragma unroll
-          for (int j = 0; j < 4; j += 2) {
-            const float4 v = reinterpret_cast<const float4*>(wv)[((e0 + j) >> 1) * T + tid];
-            ps[j] = make_float2(v.x, v.y);
-            ps[j + 1] = make_float2(v.z, v.w);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            col[j] = colmap[f.a_col(e0 + j)];
-            ob[j] = __ldg(orow_ptr + col[j]);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 g = cscale(x[e0 + j], sc);
-            atomicAdd(grow + col[j], cmulc(g, ps[j]));
-            x[e0 + j] = cmulc(g, ob[j]);
-          }
-        }
+        if (cin >= 0)
+          scatter(Wide(), s, wv, sc, inside);
+        else
+          scatter(Narrow(), s, wv, sc, wrapped);
       }
       f.forward(x, sm, tw, cl);
       // ---------------- Fourier space (layout B) ----------------
@@ -257,6 +292,8 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
           const float* tg = p.targets + (size_t)gi * NN + dbase;
           const float* mk = p.mask + dbase;
           float* oi = p.out_intensity ? p.out_intensity + (size_t)b * NN + dbase : nullptr;
+          double loss_acc = 0.0;
+          int nonfinite = 0;
 #pragma unroll
           for (int i = 0; i < E; ++i) {
             const int doff = ((i >> 3) + 32 * (((i & 7) + 4) & 7)) * N;
@@ -266,6 +303,12 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
             loss_elem<N>(p, I, __ldg(tg + doff), __ldg(mk + doff), loss_acc, dldi);
             inten[i * T + tid] = dldi;
             if (oi) oi[doff] = I;
+          }
+          for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
+          const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
+          if ((tid & 31) == 0) {
+            red[tid >> 5] += loss_acc;
+            nfred[tid >> 5] += nf_warp;
           }
         }
         if (!ADJ) break;
@@ -312,13 +355,7 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
     }
   }
 
-  for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
   // one status update per CTA: per-thread updates of a shared word contend and can drop counts
-  const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
-  if ((tid & 31) == 0) {
-    red[tid >> 5] = loss_acc;
-    nfred[tid >> 5] = nf_warp;
-  }
   __syncthreads();
   if (tid == 0) {
     int nf = 0;

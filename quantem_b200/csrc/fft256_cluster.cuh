@@ -15,9 +15,12 @@
 // and column transforms the slabs are redistributed across the cluster: every
 // thread stores its values straight into the owning CTA's shared memory
 // (distributed shared memory), bracketed by cluster barriers.  A 2-D FFT thus
-// costs two local exchanges and one cluster exchange.  All shared-memory
-// accesses (local and remote) use XOR-swizzled indices chosen so that each warp
-// access splits into the minimum two 128-byte wavefronts.
+// costs two local exchanges and one cluster exchange.
+//
+// A line's eight threads sit in one warp, and the four lines of a warp own one region of
+// the buffer in all three layouts (line-local exchange, column slab, row slab), so the
+// local exchanges need __syncwarp only; the CTA-wide and cluster-wide ordering is the two
+// cluster barriers of the slab exchange.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -33,7 +36,8 @@ struct Fft256C {
   static constexpr int T = 512;
   static constexpr int E = 32;
   static constexpr int LINES = 64;
-  static constexpr int SM_FLOAT2 = 17536;  // >= the largest of the three layouts below (63*274 + 271)
+  static constexpr int GS = 1056;           // region of a warp's four lines
+  static constexpr int SM_FLOAT2 = 16 * GS;
   // twiddle table: tw[t*33 + k1] = w256^(t*k1), t < 8, k1 < 32 (row padding 33 keeps the
   // eight t rows on distinct banks)
   static constexpr int TW_FLOAT2 = 8 * 33;
@@ -55,18 +59,20 @@ struct Fft256C {
     line = tid >> 3;
     tl = tid & 7;
   }
-  // Buffer layouts (float2 index).  Padding is additive, so every access is a
-  // per-thread base plus a compile-time offset (one address register per loop);
-  // the paddings were chosen by exhaustive search so that each warp access of
-  // every exchange touches each of the 16 float2 bank pairs at most twice.
-  //   line-local exchange, element (k1, t) of line ln:  ln*264 + 33*(k1/4) + 8*(k1%4) + t
-  //   column slab, element (kc_local, r):               kcl*260 + 2*(kcl/4) + r
-  //   row slab spectrum, element (r_local, kc):         rl*274 + kc + kc/16
-  // (row lengths cover each padded row: 262 < 264, 256 < 260, 271 < 274)
-  static constexpr int LP = 264, BP = 260, AP = 274;
-  __device__ __forceinline__ int lx(int ln, int k1, int t) const { return ln * LP + 33 * (k1 >> 2) + 8 * (k1 & 3) + t; }
-  __device__ __forceinline__ int bx(int kcl, int r) const { return kcl * BP + 2 * (kcl >> 2) + r; }
-  __device__ __forceinline__ int ax(int rl, int kc) const { return rl * AP + kc + (kc >> 4); }
+  // Buffer layouts (float2 index), G = line / 4 the warp, i = line % 4.  Every address is a
+  // per-thread base plus a compile-time offset, and every local access takes two wavefronts.
+  //   line-local exchange, element (k1, t):      G GS + 264 i + 33*(k1/4) + 8*(k1%4) + t
+  //   column slab, element (kc = line, r):       G GS + 260 i + r
+  //   row slab spectrum, element (r = line, kc): G GS + 256 i + 4*(kc/4) + pos
+  // A remote store of a warp writes 4 consecutive elements to each of 8 lines; the slabs keep
+  // those four in one 32-byte sector (8 sectors per store; padded layouts that were only
+  // bank-conflict-free took 13, and the queue of remote stores is the kernel's longest stall).
+  // In the row slab the four elements of a sector are rotated by pos = (kc + 2 (kc / 16 % 2) +
+  // line % 2) % 4 so that the reads, at stride 4, still spread over the banks.
+  static constexpr int LP = 264, BP = 260, AP = 256;
+  __device__ __forceinline__ int local_base() const { return (line >> 2) * GS + (line & 3) * LP; }
+  __device__ __forceinline__ int col_base() const { return (line >> 2) * GS + (line & 3) * BP; }
+  __device__ __forceinline__ int row_base() const { return (line >> 2) * GS + (line & 3) * AP; }
 
   // coordinates
   __device__ __forceinline__ int a_row() const { return 64 * q + line; }     // layout A row
@@ -87,6 +93,8 @@ struct Fft256C {
   // order every CTA's last reads of its own buffer before the peers' remote
   // stores, so each thread arrives right after those reads and waits just before
   // its own remote stores; the register work in between hides the barrier.
+  // (A CTA fence and a relaxed arrive instead of the release: 14.2 against 13.0 ms per 64
+  // positions of 16 slices and 6 modes.)
   static __device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
@@ -105,15 +113,15 @@ struct Fft256C {
 #pragma unroll
       for (int k1 = 1; k1 < 32; ++k1) x[k1] = INV ? cmulc(x[k1], twr[k1]) : cmul(x[k1], twr[k1]);
     }
-    __syncthreads();
+    __syncwarp();  // the warp's reads of its region are complete
     {
-      float2* w = sm + line * LP + tl;  // + lx offset of (k1, 0)
+      float2* w = sm + local_base() + tl;  // + offset of (k1, 0)
 #pragma unroll
       for (int k1 = 0; k1 < 32; ++k1) w[33 * (k1 >> 2) + 8 * (k1 & 3)] = x[k1];
     }
-    __syncthreads();
+    __syncwarp();
     {
-      const float2* r = sm + line * LP + 33 * tl;  // group g = tl: k1 = 4g + a
+      const float2* r = sm + local_base() + 33 * tl;  // group g = tl: k1 = 4g + a
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -127,17 +135,17 @@ struct Fft256C {
   template <bool INV, bool ARRIVE = false>
   __device__ __forceinline__ void line_bwd(float2 (&x)[E], float2* sm, const float2* tw) const {
     dft8_groups<INV, 0>(x);
-    __syncthreads();
+    __syncwarp();  // the warp's reads of its region are complete
     {
-      float2* w = sm + line * LP + 33 * tl;
+      float2* w = sm + local_base() + 33 * tl;
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int t = 0; t < 8; ++t) w[8 * a + t] = x[a * 8 + t];
     }
-    __syncthreads();
+    __syncwarp();
     {
-      const float2* r = sm + line * LP + tl;
+      const float2* r = sm + local_base() + tl;
 #pragma unroll
       for (int k1 = 0; k1 < 32; ++k1) x[k1] = r[33 * (k1 >> 2) + 8 * (k1 & 3)];
     }
@@ -167,18 +175,18 @@ struct Fft256C {
   // (the caller arrived on the cluster barrier after its last read of sm)
   __device__ __forceinline__ void a_to_b(float2 (&x)[E], float2* sm, cg::cluster_group& cl) const {
     cluster_wait();  // every CTA of the cluster is done reading its buffer
-    // bx(4tl + a + 32x, 64q + line) = [1042 tl + 64q + line] + 260a + 8336x
-    const float2* mine = sm + 1042 * tl + 64 * q + line;
+    // spectral column 4 tl + a + 32 x: warp region tl + 8 x, line a
+    const float2* mine = sm + GS * tl + 64 * q + line;
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       const uint32_t dst = peer_addr(mine, (uint32_t)d);
 #pragma unroll
       for (int xb = 0; xb < 2; ++xb)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) st_peer(dst + 8u * (uint32_t)(260 * a + 8336 * xb), x[a * 8 + 2 * d + xb]);
+        for (int a = 0; a < 4; ++a) st_peer(dst + 8u * (uint32_t)(BP * a + 8 * GS * xb), x[a * 8 + 2 * d + xb]);
     }
     cl.sync();
-    const float2* r = sm + BP * line + 2 * (line >> 2) + tl;
+    const float2* r = sm + col_base() + tl;
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = r[8 * e];
   }
@@ -186,21 +194,25 @@ struct Fft256C {
   //   -> A (row spectrum distribution of row a_row())
   __device__ __forceinline__ void b_to_a(float2 (&x)[E], float2* sm, cg::cluster_group& cl) const {
     cluster_wait();  // arrived after the caller's last read of sm
-    // ax(tl + 8j, 64q + line) = [274 tl + 68q + line + line/16] + 2192 j
-    const float2* mine = sm + AP * tl + 68 * q + line + (line >> 4);
+    // row tl + 8 j: warp region tl / 4 + 2 j, line tl % 4; kc = 64 q + line
+    const int pos = ((line & 3) + 2 * ((line >> 4) & 1) + (tl & 1)) & 3;
+    const float2* mine = sm + GS * (tl >> 2) + AP * (tl & 3) + 64 * q + (line & ~3) + pos;
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       const uint32_t dst = peer_addr(mine, (uint32_t)d);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) st_peer(dst + 8u * (uint32_t)(8 * AP * j), x[8 * d + j]);
+      for (int j = 0; j < 8; ++j) st_peer(dst + 8u * (uint32_t)(2 * GS * j), x[8 * d + j]);
     }
     cl.sync();
-    // ax(line, 4tl + a + 32kB) = [274 line + 4tl + tl/4] + a + 34kB
-    const float2* r = sm + AP * line + 4 * tl + (tl >> 2);
+    // kc = 4 tl + a + 32 kB
+    const float2* r = sm + row_base() + 4 * tl;
+    const int rot = 2 * (tl >> 2) + (line & 1);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a) {
+      const float2* ra = r + ((a + rot) & 3);
 #pragma unroll
-      for (int kB = 0; kB < 8; ++kB) x[a * 8 + kB] = r[a + 34 * kB];
+      for (int kB = 0; kB < 8; ++kB) x[a * 8 + kB] = ra[32 * kB];
+    }
   }
 
   // ---- whole 2-D transforms (unnormalised) ----
