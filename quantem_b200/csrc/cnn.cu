@@ -560,7 +560,13 @@ int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, in
   if (int rc = encode_fn()) return rc;
   const int kb_per = (nkb + splits - 1) / splits;
   splits = (nkb + kb_per - 1) / kb_per;  // every split gets >= 1 k-block
-  const int BN = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  // The widest tile (fewest re-reads of A) that still gives every SM one; the deep layers of a
+  // network (16 to 256 rows) take narrow tiles: at 16 rows x 1024 columns x 9216 one CTA per 128
+  // columns streamed the weights through 8 SMs.  A column's products and sums do not depend on
+  // the tile width.
+  const int tiles_m = (M + BM - 1) / BM;
+  int BN = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  while (BN > 16 && tiles_m * ((N + BN - 1) / BN) * splits < 148) BN /= 2;
   CUtensorMap ta, tb;
   if (int rc = make_map(&ta, A, M, K, lda, BM)) return rc;
   if (int rc = make_map(&tb, B, N, K, ldb, BN)) return rc;
@@ -571,6 +577,7 @@ int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, in
   }
   Epilogue epi{C, bias, ldc, flags, act};
   switch (BN) {
+    case 16: return launch_gemm<16>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
     case 32: return launch_gemm<32>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
     case 64: return launch_gemm<64>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
     default: return launch_gemm<128>(ta, tb, M, N, K, splits, kb_per, epi, status, st);

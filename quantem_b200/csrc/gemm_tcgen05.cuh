@@ -8,8 +8,9 @@
 // One CTA of 128 threads computes a 128 x BN tile:
 //   * warp 0, one lane: TMA producer.  Each k-block (64 bf16 = one 128-byte
 //     swizzle row) of A (128 x 64) and B (BN x 64) is copied by
-//     cp.async.bulk.tensor into a 4-stage ring with the 128-byte swizzle; an
-//     mbarrier per stage counts the transaction bytes.
+//     cp.async.bulk.tensor into a ring of 6-9 stages (about 190 KB) with the 128-byte
+//     swizzle; an mbarrier per stage counts the transaction bytes.  The ring's depth
+//     hides the copies' latency, which bounds the many products with few tiles.
 //   * warp 1, one lane: MMA issuer.  tcgen05.mma.cta_group::1.kind::f16 with
 //     M = 128, N = BN, K = 16 (four per k-block), BF16 operands read from shared
 //     memory through matrix descriptors, FP32 accumulator in tensor memory
@@ -37,7 +38,6 @@ namespace gemm {
 
 constexpr int BM = 128;
 constexpr int BK = 64;  // bf16 per 128-byte swizzle row
-constexpr int STAGES = 4;
 constexpr int THREADS = 128;
 constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s bound on any single wait
 
@@ -58,6 +58,8 @@ struct Smem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = BN >= 128 ? 6 : (BN == 64 ? 8 : 9);
+  static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;  // the smallest allocation
   static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
   static constexpr int BYTES = BAR_OFF + 256 + 1024;  // barriers + 1 KB alignment slack
 };
@@ -149,8 +151,9 @@ template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                         int N, int K, int kb_per_split, Epilogue epi, int* status) {
-  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "BN: TMEM allocation is a power of two >= 32");
+  static_assert(BN == 16 || BN == 32 || BN == 64 || BN == 128, "BN: a multiple of 16");
   using L = Smem<BN>;
+  constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
-                 "r"(BN)
+                 "r"(L::TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -278,7 +281,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS)
+                 : "memory");
   }
 }
 
