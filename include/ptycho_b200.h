@@ -396,6 +396,50 @@ enum {
 int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K,
                      const float* bias, int flags, int splits, int* status, void* stream);
 
+/* As ptycho_gemm_bf16 without a bias, with B stored as K rows of N values (ldb >= N) and A as
+ * M rows of K values (a_mn = 0) or K rows of M values (a_mn = 1, lda >= M): the products of a
+ * layer's input and weight gradients without transposed copies. */
+int ptycho_gemm_bf16_mn(const void* A, int lda, int a_mn, const void* B, int ldb, void* C, int ldc, int M, int N,
+                        int K, int flags, int splits, int* status, void* stream);
+
+/* ---- whole layers: the launches of one layer of the network, queued by one call ----
+ *
+ * Conv2dBlock layer (blocks.py:53-140): r (FP32, R x co) = act(conv3x3(x) + bias); with out
+ * (BF16, R x co, leading dimension ldo) also out = batch_norm(r) (gamma NULL: bf16(r)).
+ * col: BF16 scratch R x 9 C.  w: BF16 (co, 9 C).  R = B H W; statistics as in
+ * ptycho_cnn_bn_forward. */
+int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, const void* w, int co,
+                            const float* bias, int act, const float* gamma, const float* beta, float* run_mean,
+                            float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
+                            void* col, float* r, void* out, int ldo, void* stream);
+
+/* Gradients of the layer from dy (FP32, R x co, w.r.t. the batch norm's output): dw (added to,
+ * FP32 (co, 9 C)), db, dgamma, dbeta (written) and, if given, dx (FP32 R x C, written or added
+ * to).  dz: BF16 scratch R x ldz (ldz >= co, a multiple of 8); col: BF16 scratch R x 9 C;
+ * dcol: FP32 scratch R x 9 C (with dx). */
+int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, int B, int H, int W, int C,
+                             const void* w, const float* r, int co, const float* gamma, const float* mean,
+                             const float* rstd, int training, int act, float* dw, float* db, float* dgamma,
+                             float* dbeta, void* dz, int ldz, void* col, float* dcol, float* dx, int lddx,
+                             int dx_accumulate, void* stream);
+
+/* Upsample2dBlock (blocks.py:143-205) of y (BF16, B H W x ci): t (BF16, 4 B H W x ci) the
+ * transposed convolution, r (FP32, 4 B H W x co) its 1x1 convolution, out = batch_norm(r).
+ * colT: FP32 scratch B H W x 9 ci.  wt: BF16 (9 ci, ci), w1: BF16 (co, ci). */
+int ptycho_cnn_up_forward(const void* y, int ldy, int B, int H, int W, int ci, int co, const void* wt, const float* bt,
+                          const void* w1, const float* b1, const float* gamma, const float* beta, float* run_mean,
+                          float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
+                          float* colT, void* t, float* r, void* out, int ldo, void* stream);
+
+/* Gradients of the block from dup (FP32, 4 B H W x co): dwt, dw1 added to, dbt, db1, dgamma,
+ * dbeta and dy (FP32 B H W x ci) written.  dz: BF16 scratch 4 B H W x ldz; dt: FP32 scratch
+ * 4 B H W x ci; dcolT: BF16 scratch B H W x 9 ci; work as in ptycho_cnn_colsum. */
+int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, const void* t, const float* r, int B,
+                           int H, int W, int ci, int co, const void* wt, const void* w1, const float* gamma,
+                           const float* mean, const float* rstd, int training, float* dwt, float* dbt, float* dw1,
+                           float* db1, float* dgamma, float* dbeta, void* dz, int ldz, float* dt, void* dcolT,
+                           double* work, int64_t work_elems, float* dy, void* stream);
+
 /* col[r][(ky*3+kx)*C + c] = x[b, (y+ky-1) mod H, (x+kx-1) mod W, c] (BF16): the
  * circular-padded 3x3 patches of nn.Conv2d(padding=1, padding_mode="circular"). */
 int ptycho_cnn_im2col3x3(const void* x, int B, int H, int W, int C, int ldx, void* col, int ldcol, void* stream);

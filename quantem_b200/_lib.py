@@ -53,6 +53,11 @@ EXPORTED = (
     "ptycho_fp32_fma_probe",
     "ptycho_forward_loss_noalloc",
     "ptycho_gemm_bf16",
+    "ptycho_gemm_bf16_mn",
+    "ptycho_cnn_conv_forward",
+    "ptycho_cnn_conv_backward",
+    "ptycho_cnn_up_forward",
+    "ptycho_cnn_up_backward",
     "ptycho_cnn_im2col3x3",
     "ptycho_cnn_col2im3x3",
     "ptycho_cnn_convT_gather",
@@ -152,6 +157,14 @@ def _declare(lib):
         "ptycho_analytic_obj_finalize": (_int, [_vp, _vp, _vp, _int, _int, _i64, _vp, _vp]),
         "ptycho_analytic_probe_finalize": (_int, [_vp, _i64, _vp, _flt, _vp]),
         "ptycho_forward_loss_noalloc": (_int, [ctypes.POINTER(BatchArgs), _vp, _vp]),
+        "ptycho_cnn_conv_forward": (_int, [_vp] + [_int] * 5 + [_vp, _int, _vp, _int] + [_vp] * 4 +
+                                    [_flt, _flt, _int] + [_vp] * 5 + [_int, _vp]),
+        "ptycho_cnn_conv_backward": (_int, [_vp, _int, _vp] + [_int] * 5 + [_vp, _vp, _int] + [_vp] * 3 +
+                                     [_int, _int] + [_vp] * 5 + [_int] + [_vp] * 3 + [_int, _int, _vp]),
+        "ptycho_cnn_up_forward": (_int, [_vp] + [_int] * 6 + [_vp] * 8 + [_flt, _flt, _int] + [_vp] * 6 + [_int, _vp]),
+        "ptycho_cnn_up_backward": (_int, [_vp, _int, _vp, _int, _vp, _vp] + [_int] * 5 + [_vp] * 5 + [_int] +
+                                   [_vp] * 7 + [_int, _vp, _vp, _vp, _i64, _vp, _vp]),
+        "ptycho_gemm_bf16_mn": (_int, [_vp, _int, _int, _vp, _int, _vp, _int, _int, _int, _int, _int, _int, _vp, _vp]),
         "ptycho_gemm_bf16": (_int, [_vp, _int, _vp, _int, _vp, _int, _int, _int, _int, _vp, _int, _int, _vp, _vp]),
         "ptycho_cnn_im2col3x3": (_int, [_vp, _int, _int, _int, _int, _int, _vp, _int, _vp]),
         "ptycho_cnn_col2im3x3": (_int, [_vp, _int, _int, _int, _int, _int, _vp, _int, _int, _vp]),

@@ -108,6 +108,7 @@ class CNN2d(torch.nn.Module):
         # when a dict, each pass records every layer's inputs / outputs / gradients
         # (used by the per-layer parity tests)
         self.trace = None
+        self._arena_bytes = {}  # (B, H, W) -> bytes of one pass's buffers
         self._build()
         self._init_params(seed)
 
@@ -353,55 +354,116 @@ class CNN2d(torch.nn.Module):
     __call__ = forward
 
 
+class _Buf:
+    """A (R, C) matrix with leading dimension ``ld`` inside a byte arena."""
+
+    __slots__ = ("ptr", "R", "C", "ld", "dtype", "base", "off")
+
+    def __init__(self, base, off, R, C, ld, dtype):
+        self.base, self.off, self.R, self.C, self.ld, self.dtype = base, off, R, C, ld, dtype
+        self.ptr = base.data_ptr() + off
+
+    def cols(self, c0: int, n: int) -> "_Buf":
+        """Columns [c0, c0 + n) (a channel slice of a wider buffer)."""
+        return _Buf(self.base, self.off + c0 * self.dtype.itemsize, self.R, n, self.ld, self.dtype)
+
+    def tensor(self) -> torch.Tensor:
+        size = self.dtype.itemsize
+        n = (self.R - 1) * self.ld + self.C
+        return self.base[self.off: self.off + n * size].view(self.dtype).as_strided((self.R, self.C), (self.ld, 1))
+
+
+class _Arena:
+    """Bump allocation of one pass's buffers from a few tensors of the caching allocator."""
+
+    def __init__(self, device, first: int):
+        self.device, self.block = device, max(int(first), 1 << 20)
+        self.blocks, self.base, self.used, self.total = [], None, 0, 0
+
+    def buf(self, R, C, dtype, ld=None) -> _Buf:
+        ld = C if ld is None else ld
+        n = (R * ld * dtype.itemsize + 255) // 256 * 256
+        if self.base is None or self.used + n > self.base.numel():
+            self.base = torch.empty(max(n, self.block), dtype=torch.uint8, device=self.device)
+            self.blocks.append(self.base)
+            self.used, self.block = 0, 1 << 24
+        b = _Buf(self.base, self.used, R, C, ld, dtype)
+        self.used += n
+        self.total += n
+        return b
+
+
+_F32, _BF16 = torch.float32, torch.bfloat16
+
+
 class _Run:
-    """One forward pass: buffers and saved tensors for its backward."""
+    """One forward pass: buffers and saved matrices for its backward.  Every layer is one
+    library call that queues its launches."""
 
     def __init__(self, net: CNN2d, B: int, H: int, W: int, training: bool):
         self.net, self.B, self.H, self.W, self.training = net, B, H, W, training
-        dev = net.device
-        maxc = max(2 * net.start_filters * 2 ** net.num_layers, net.cin_pad, 64)
-        self.work = torch.empty(2 * 592 * maxc, dtype=torch.float64, device=dev)
-        self.dev = dev
+        self.dev = net.device
+        self.lib = kk._lib.lib()
         self.saved = {}
+        self.key = (B, H, W)
+        self.arena = _Arena(self.dev, net._arena_bytes.get(self.key, 1 << 22))
 
     def empty(self, *shape, dtype=torch.float32):
         return torch.empty(*shape, dtype=dtype, device=self.dev)
 
+    def call(self, name, *args):
+        kk._lib.check(getattr(self.lib, name)(*args), name)
+
+    def _bind(self):
+        """Stream and parameter addresses of this pass (forward or backward)."""
+        self.st = torch.cuda.current_stream(self.dev).cuda_stream
+        self.pf, self.p16 = self.net.flat.data_ptr(), self.net.flat16.data_ptr()
+
+    def _f(self, seg) -> int:
+        return self.pf + 4 * seg.off
+
+    def _h(self, seg) -> int:
+        return self.p16 + 2 * seg.off
+
+    def _bn_args(self, bn, mean, rstd):
+        """gamma, beta, running statistics, momentum, eps, training, mean, rstd."""
+        if bn is None:
+            return (None, None, None, None, 0.0, 0.0, 0, None, None)
+        gseg, bseg, pref = bn
+        rm, rv = self.net.running[pref]
+        return (self._f(gseg), self._f(bseg), rm.data_ptr(), rv.data_ptr(), self.net.momentum, self.net.eps,
+                int(self.training), mean.ptr, rstd.ptr)
+
+    def _stats(self, bn, co):
+        if bn is None:
+            return None, None
+        return self.arena.buf(1, co, _F32), self.arena.buf(1, co, _F32)
+
     # --- conv3x3 + bias + activation (+ BN) -> bf16 into `out` ------------------
-    def conv_fwd(self, key, layer, x16, B, H, W, out16, act=None, final=False):
+    def conv_fwd(self, key, layer, x, B, H, W, out, act=None, final=False):
         net = self.net
-        R = B * H * W
-        co = layer["co"]
-        col = self.empty(R, 9 * layer["ci_store"], dtype=torch.bfloat16)
-        kk.im2col3x3(x16, B, H, W, col)
-        w16 = net.view(layer["w"], net.flat16)
-        r = self.empty(R, co if not final else co)
-        kk.gemm(col, w16, r, bias=net.view(layer["b"]), act=net._act if act is None else act)
-        del col
-        tr = self.net.trace
+        R, co, C = B * H * W, layer["co"], layer["ci_store"]
+        r = self.arena.buf(R, co, _F32)
+        bn = None if final else layer["bn"]
+        mean, rstd = self._stats(bn, co)
+        self.call("ptycho_cnn_conv_forward", x.ptr, x.ld, B, H, W, C, self._h(layer["w"]), co, self._f(layer["b"]),
+                  int(net._act if act is None else act), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
+                  r.ptr, None if final else out.ptr, 0 if final else out.ld, self.st)
+        tr = net.trace
         seed = self._next_dropout_seed()
         if final:
             # the activation's output r stays for the backward; the dropped copy is the output
-            y = r if seed is None else kk.dropout(r.clone(), net.dropout, seed)
-            self.saved[key] = (x16, r, None, None, seed)
+            y = r.tensor() if seed is None else kk.dropout(r.tensor().clone(), net.dropout, seed)
+            self.saved[key] = (x, r, None, None, seed)
             if tr is not None:
-                tr[("fwd",) + key] = dict(x=x16.clone(), r=r.clone())
+                tr[("fwd",) + key] = dict(x=x.tensor().clone(), r=r.tensor().clone())
             return y
-        if layer["bn"] is not None:
-            gseg, bseg, pref = layer["bn"]
-            mean, rstd = self.empty(co), self.empty(co)
-            rm, rv = net.running[pref]
-            kk.bn_forward(r, net.view(gseg), net.view(bseg), rm, rv, net.momentum, net.eps, self.training, mean,
-                          rstd, self.work, out16)
-        else:
-            mean = rstd = None
-            kk.bn_forward(r, None, None, None, None, 0.0, 0.0, False, None, None, self.work, out16)
         if seed is not None:
-            kk.dropout(out16, net.dropout, seed)
-        self.saved[key] = (x16, r, mean, rstd, seed)
+            kk.dropout(out.tensor(), net.dropout, seed)
+        self.saved[key] = (x, r, mean, rstd, seed)
         if tr is not None:
-            tr[("fwd",) + key] = dict(x=x16.clone(), r=r.clone(), y=out16.clone())
-        return out16
+            tr[("fwd",) + key] = dict(x=x.tensor().clone(), r=r.tensor().clone(), y=out.tensor().clone())
+        return out
 
     def _next_dropout_seed(self):
         """A fresh mask seed per layer and pass in training mode with dropout, else None."""
@@ -411,22 +473,19 @@ class _Run:
         net._dropout_calls += 1
         return (net._dropout_seed * 0x9E3779B1 + net._dropout_calls) & 0xFFFFFFFFFFFF
 
-    def block_fwd(self, prefix, layers, x16, B, H, W, out16_last):
-        y = x16
+    def block_fwd(self, prefix, layers, x, B, H, W, out_last):
+        y = x
         for j, layer in enumerate(layers):
-            out = out16_last if j == len(layers) - 1 else self.empty(B * H * W, layer["co"], dtype=torch.bfloat16)
+            out = out_last if j == len(layers) - 1 else self.arena.buf(B * H * W, layer["co"], _BF16)
             y = self.conv_fwd((prefix, j), layer, y, B, H, W, out)
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        net = self.net
-        B, H, W = self.B, self.H, self.W
-        L = net.num_layers
-        if x.dim() == 2:  # channels-last BF16 rows given directly
-            x16 = x
-        else:
-            x16 = self._to_rows(x)
-        return self._forward_rows(x16)
+        # channels-last BF16 rows, given directly or converted from NCHW FP32
+        self.x16 = x if x.dim() == 2 else self._to_rows(x)
+        if self.x16.stride(1) != 1 or self.x16.stride(0) < self.x16.shape[1] or not self.x16.is_cuda:
+            raise ValueError("x must be a 2-D CUDA view contiguous along its last dimension")
+        return self._forward_rows()
 
     def _to_rows(self, x: torch.Tensor) -> torch.Tensor:
         net = self.net
@@ -444,136 +503,152 @@ class _Run:
             x16.view(B, H * W, net.cin_pad)[..., : net.in_channels].copy_(tmp)
         return x16
 
-    def _forward_rows(self, x16: torch.Tensor) -> torch.Tensor:
+    def _levels(self):
+        """(rows, layer) of every 3x3 convolution and (input rows, up block) of every upsampling."""
+        net, n, L = self.net, self.B * self.H * self.W, self.net.num_layers
+        convs = [(n >> 2 * l, layer) for l in range(L) for layer in net.down[l]]
+        convs += [(n >> 2 * L, layer) for layer in net.bottleneck] + [(n, net.final)]
+        ups = []
+        for u, up in enumerate(net.up):
+            l = L - 1 - u
+            convs += [(n >> 2 * l, layer) for layer in up["block"]]
+            ups.append((n >> 2 * (l + 1), up))
+        return convs, ups
+
+    def _forward_rows(self) -> torch.Tensor:
         net = self.net
         B, H, W = self.B, self.H, self.W
         L = net.num_layers
+        self._bind()
+        convs, ups = self._levels()
+        # im2col rows (BF16) or the transposed convolution's products (FP32), one layer at a time
+        self.scratch = self.empty(max([R * 9 * la["ci_store"] * 2 for R, la in convs] +
+                                      [R * 9 * up["ci"] * 4 for R, up in ups]), dtype=torch.uint8)
         self.cat = []
         self.pool_arg = []
-        y = x16
+        x16 = self.x16
+        y = _Buf.__new__(_Buf)
+        y.base, y.off, y.R, y.C, y.ld, y.dtype = None, 0, x16.shape[0], x16.shape[1], x16.stride(0), _BF16
+        y.ptr = x16.data_ptr()
+        if net.trace is not None:
+            flat = x16.as_strided((x16.shape[0] * x16.stride(0),), (1,)) if x16.is_contiguous() else None
+            y.base = (flat if flat is not None else x16.contiguous().view(-1)).view(torch.uint8)
+            y.ld = x16.stride(0) if flat is not None else x16.shape[1]
+            y.ptr = y.base.data_ptr()
         for l in range(L):
             h, w = H >> l, W >> l
             co = net.down[l][-1]["co"]
             R = B * h * w
             if net.use_skip_connections:
-                cat = self.empty(R, 2 * co, dtype=torch.bfloat16)
-                skip = cat[:, co:]
+                cat = self.arena.buf(R, 2 * co, _BF16)
+                skip = cat.cols(co, co)
             else:
                 cat = None
-                skip = self.empty(R, co, dtype=torch.bfloat16)
+                skip = self.arena.buf(R, co, _BF16)
             self.cat.append(cat)
             self.block_fwd(("down", l), net.down[l], y, B, h, w, skip)
-            pooled = self.empty(R // 4, co, dtype=torch.bfloat16)
-            arg = self.empty(R // 4, co, dtype=torch.uint8)
-            kk.maxpool2(skip, B, h, w, pooled, arg)
-            self.pool_arg.append((skip, arg))
+            pooled = self.arena.buf(R // 4, co, _BF16)
+            arg = self.arena.buf(R // 4, co, torch.uint8)
+            self.call("ptycho_cnn_maxpool2", skip.ptr, skip.ld, B, h, w, co, pooled.ptr, pooled.ld, arg.ptr, self.st)
+            self.pool_arg.append(arg)
             y = pooled
         h, w = H >> L, W >> L
         cb = net.bottleneck[-1]["co"]
-        yb = self.empty(B * h * w, cb, dtype=torch.bfloat16)
+        yb = self.arena.buf(B * h * w, cb, _BF16)
         y = self.block_fwd(("bott",), net.bottleneck, y, B, h, w, yb)
         for u, up in enumerate(net.up):
             l = L - 1 - u
             hin, win = H >> (l + 1), W >> (l + 1)
             h, w = H >> l, W >> l
             ci, co = up["ci"], up["co"]
-            Rin, R = B * hin * win, B * h * w
-            colT = self.empty(Rin, 9 * ci)
-            kk.gemm(y, net.view(up["wt"], net.flat16), colT)
-            t16 = self.empty(R, ci, dtype=torch.bfloat16)
-            kk.convT_gather(colT, B, hin, win, ci, net.view(up["bt"]), t16)
-            del colT
-            r = self.empty(R, co)
-            kk.gemm(t16, net.view(up["w1"], net.flat16), r, bias=net.view(up["b1"]))
+            R = B * h * w
+            t, r = self.arena.buf(R, ci, _BF16), self.arena.buf(R, co, _F32)
             cat = self.cat[l]
-            dst = cat[:, :co] if cat is not None else self.empty(R, co, dtype=torch.bfloat16)
-            if net._use_batchnorm:
-                gseg, bseg, pref = up["bn"]
-                mean, rstd = self.empty(co), self.empty(co)
-                rm, rv = net.running[pref]
-                kk.bn_forward(r, net.view(gseg), net.view(bseg), rm, rv, net.momentum, net.eps, self.training, mean,
-                              rstd, self.work, dst)
-            else:
-                mean = rstd = None
-                kk.bn_forward(r, None, None, None, None, 0.0, 0.0, False, None, None, self.work, dst)
-            self.saved[("upT", u)] = (y, t16, r, mean, rstd, hin, win)
+            dst = cat.cols(0, co) if cat is not None else self.arena.buf(R, co, _BF16)
+            bn = up["bn"] if net._use_batchnorm else None
+            mean, rstd = self._stats(bn, co)
+            self.call("ptycho_cnn_up_forward", y.ptr, y.ld, B, hin, win, ci, co, self._h(up["wt"]), self._f(up["bt"]),
+                      self._h(up["w1"]), self._f(up["b1"]), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
+                      t.ptr, r.ptr, dst.ptr, dst.ld, self.st)
+            self.saved[("upT", u)] = (y, t, r, mean, rstd, hin, win)
             if net.trace is not None:
-                net.trace[("upfwd", u)] = dict(x=y.clone(), t=t16.clone(), r=r.clone(), y=dst.clone())
+                net.trace[("upfwd", u)] = dict(x=y.tensor().clone(), t=t.tensor().clone(), r=r.tensor().clone(),
+                                               y=dst.tensor().clone())
             src = cat if cat is not None else dst
-            out = self.empty(R, up["block"][-1]["co"], dtype=torch.bfloat16)
+            out = self.arena.buf(R, up["block"][-1]["co"], _BF16)
             y = self.block_fwd(("upc", u), up["block"], src, B, h, w, out)
-        fin = net.final
-        r = self.conv_fwd(("final",), fin, y, B, H, W, None, act=net._final_act, final=True)
+        r = self.conv_fwd(("final",), net.final, y, B, H, W, None, act=net._final_act, final=True)
+        del self.scratch
+        if len(net._arena_bytes) > 16:
+            net._arena_bytes.clear()
+        net._arena_bytes[self.key] = self.arena.total
         out = self.empty(B, net.out_channels, H * W)
         kk.transpose(r.view(B, H * W, net.out_channels), out)
         return out.view(B, net.out_channels, H, W)
 
     # ------------------------------------------------------------------ backward
-    def conv_bwd(self, key, layer, dy, B, H, W, grad, dx_out=None, dx_accumulate=False, act=None):
-        """dy: FP32 gradient w.r.t. the layer output (after BN).  Accumulates the
-        weight / bias / BN gradients into `grad` and writes dx (FP32) if asked."""
+    def conv_bwd(self, key, layer, dy, B, H, W, dx_out=None, dx_accumulate=False, act=None):
+        """dy: FP32 gradient w.r.t. the layer output (after BN).  Writes the weight / bias /
+        BN gradients into the flat gradient and dx (FP32) if asked."""
         net = self.net
-        x16, r, mean, rstd, seed = self.saved.pop(key)
+        x, r, mean, rstd, seed = self.saved.pop(key)
         if seed is not None:  # the forward's dropout mask on the incoming gradient
             dy = kk.dropout(dy.contiguous().clone(), net.dropout, seed)
         tr = net.trace
         if tr is not None:
             tr[("bwd",) + key] = dict(dy=dy.clone())
-        R = B * H * W
-        co, ci_store = layer["co"], layer["ci_store"]
+        R, co, C = B * H * W, layer["co"], layer["ci_store"]
+        bn = layer["bn"]
+        g = self.pg
+        sc = self.scratch.data_ptr()
         ldz = _up8(co)
-        dz32 = self.empty(R, ldz)[:, :co]
-        dz16 = self.empty(R, ldz, dtype=torch.bfloat16)[:, :co]
-        act = net._act if act is None else act
-        if layer["bn"] is not None:
-            gseg, bseg, _ = layer["bn"]
-            kk.bn_backward(dy, r, net.view(gseg), mean, rstd, self.training, act, net.view(gseg, grad),
-                           net.view(bseg, grad), self.work, dz32=dz32, dz16=dz16)
-        else:
-            kk.bn_backward(dy, r, None, None, None, self.training, act, None, None, self.work, dz32=dz32, dz16=dz16)
-        kk.colsum(dz32, net.view(layer["b"], grad), self.work)
-        del dz32
-        # weight gradient: dW[co][9ci] = dz^T @ col
-        col = self.empty(R, 9 * ci_store, dtype=torch.bfloat16)
-        kk.im2col3x3(x16, B, H, W, col)
-        colT = self.empty(9 * ci_store, _up8(R), dtype=torch.bfloat16)[:, :R]
-        kk.transpose(col, colT)
-        del col
-        dzT = self.empty(co, _up8(R), dtype=torch.bfloat16)[:, :R]
-        kk.transpose(dz16, dzT)
-        gw = net.view(layer["w"], grad)
-        _gemm_acc(dzT, colT, gw, self)
-        del colT, dzT
-        if dx_out is not None:
-            # dx = col2im(dz @ W): W^T operand (9ci x co)
-            wT = self.empty(9 * ci_store, ldz, dtype=torch.bfloat16)[:, :co]
-            kk.transpose(net.view(layer["w"], net.flat16), wT)
-            dcol = self.empty(R, 9 * ci_store)
-            kk.gemm(dz16, wT, dcol)
-            kk.col2im3x3(dcol, B, H, W, ci_store, dx_out, accumulate=dx_accumulate)
-            if tr is not None:
-                tr[("bwd",) + key]["dx"] = dx_out.clone()
+        col = sc + self._align(R * ldz * 2)
+        dcol = col + self._align(R * 9 * C * 2)
+        self.call("ptycho_cnn_conv_backward", dy.data_ptr(), dy.stride(0), x.ptr, x.ld, B, H, W, C,
+                  self._h(layer["w"]), r.ptr, co, *((self._f(bn[0]), mean.ptr, rstd.ptr) if bn is not None else
+                                                    (None, None, None)),
+                  int(self.training), int(net._act if act is None else act), g + 4 * layer["w"].off,
+                  g + 4 * layer["b"].off, *((g + 4 * bn[0].off, g + 4 * bn[1].off) if bn is not None else (None, None)),
+                  sc, ldz, col, dcol, None if dx_out is None else dx_out.data_ptr(),
+                  0 if dx_out is None else dx_out.stride(0), int(dx_accumulate), self.st)
+        if tr is not None and dx_out is not None:
+            tr[("bwd",) + key]["dx"] = dx_out.clone()
 
-    def block_bwd(self, prefix, layers, dy, B, H, W, grad, dx_out, dx_accumulate=False):
+    @staticmethod
+    def _align(n: int) -> int:
+        return (n + 255) // 256 * 256
+
+    def block_bwd(self, prefix, layers, dy, B, H, W, dx_out, dx_accumulate=False):
         g = dy
         for j in range(len(layers) - 1, -1, -1):
             layer = layers[j]
             if j > 0:
                 dx = self.empty(B * H * W, layer["ci_store"])
-                self.conv_bwd((prefix, j), layer, g, B, H, W, grad, dx)
+                self.conv_bwd((prefix, j), layer, g, B, H, W, dx)
                 g = dx
             else:
-                self.conv_bwd((prefix, 0), layer, g, B, H, W, grad, dx_out, dx_accumulate)
+                self.conv_bwd((prefix, 0), layer, g, B, H, W, dx_out, dx_accumulate)
 
     def backward(self, dout: torch.Tensor, grad: torch.Tensor, need_dx: bool):
         net = self.net
         B, H, W = self.B, self.H, self.W
         L = net.num_layers
         R0 = B * H * W
+        self._bind()
+        self.pg = grad.data_ptr()
+        convs, ups = self._levels()
+        first = net.down[0][0]
+        a = self._align
+        self.scratch = self.empty(max(
+            [a(R * _up8(la["co"]) * 2) + a(R * 9 * la["ci_store"] * 2) +
+             (0 if la is first and not need_dx else R * 9 * la["ci_store"] * 4) for R, la in convs] +
+            [a(4 * R * _up8(up["co"]) * 2) + a(4 * R * up["ci"] * 4) + R * 9 * up["ci"] * 2 for R, up in ups]),
+            dtype=torch.uint8)
+        work = self.empty(2 * 592 * max([up["ci"] for up in net.up], default=1), dtype=torch.float64)
         dfin = self.empty(R0, net.out_channels)
         kk.transpose(dout.reshape(B, net.out_channels, H * W), dfin.view(B, H * W, net.out_channels))
         dy = self.empty(R0, net.final["ci_store"])
-        self.conv_bwd(("final",), net.final, dfin, B, H, W, grad, dy, act=net._final_act)
+        self.conv_bwd(("final",), net.final, dfin, B, H, W, dy, act=net._final_act)
         dcat = [None] * L
         # decoder, last level first
         for u in range(L - 1, -1, -1):
@@ -584,91 +659,53 @@ class _Run:
             R = B * h * w
             cin_block = up["block"][0]["ci_store"]
             dsrc = self.empty(R, cin_block)
-            self.block_bwd(("upc", u), up["block"], dy, B, h, w, grad, dsrc)
+            self.block_bwd(("upc", u), up["block"], dy, B, h, w, dsrc)
             dcat[l] = dsrc
             dup = dsrc[:, :co] if net.use_skip_connections else dsrc
-            yin, t16, r, mean, rstd, hin, win = self.saved.pop(("upT", u))
-            Rin = B * hin * win
+            yin, t, r, mean, rstd, hin, win = self.saved.pop(("upT", u))
+            bn = up["bn"] if net._use_batchnorm else None
             ldz = _up8(co)
-            dz32 = self.empty(R, ldz)[:, :co]
-            dz16 = self.empty(R, ldz, dtype=torch.bfloat16)[:, :co]
-            if net._use_batchnorm:
-                gseg, bseg, _ = up["bn"]
-                kk.bn_backward(dup, r, net.view(gseg), mean, rstd, self.training, False, net.view(gseg, grad),
-                               net.view(bseg, grad), self.work, dz32=dz32, dz16=dz16)
-            else:
-                kk.bn_backward(dup, r, None, None, None, self.training, False, None, None, self.work, dz32=dz32,
-                               dz16=dz16)
-            kk.colsum(dz32, net.view(up["b1"], grad), self.work)
-            # 1x1 conv: dW1 = dz^T t ; dt = dz W1
-            dzT = self.empty(co, _up8(R), dtype=torch.bfloat16)[:, :R]
-            kk.transpose(dz16, dzT)
-            tT = self.empty(ci, _up8(R), dtype=torch.bfloat16)[:, :R]
-            kk.transpose(t16, tT)
-            _gemm_acc(dzT, tT, net.view(up["w1"], grad), self)
-            del dzT, tT
-            w1T = self.empty(ci, ldz, dtype=torch.bfloat16)[:, :co]
-            kk.transpose(net.view(up["w1"], net.flat16), w1T)
-            dt = self.empty(R, ci)
-            kk.gemm(dz16, w1T, dt)
-            # transposed convolution: bias, weight and input gradients
-            kk.colsum(dt, net.view(up["bt"], grad), self.work)
-            dcolT = self.empty(Rin, 9 * ci, dtype=torch.bfloat16)
-            kk.convT_im2col(dt, B, hin, win, ci, dcolT)
-            dcolTT = self.empty(9 * ci, _up8(Rin), dtype=torch.bfloat16)[:, :Rin]
-            kk.transpose(dcolT, dcolTT)
-            yT = self.empty(ci, _up8(Rin), dtype=torch.bfloat16)[:, :Rin]
-            kk.transpose(yin, yT)
-            _gemm_acc(dcolTT, yT, net.view(up["wt"], grad), self)
-            del dcolTT, yT
-            wtT = self.empty(ci, 9 * ci, dtype=torch.bfloat16)
-            kk.transpose(net.view(up["wt"], net.flat16), wtT)
-            dy = self.empty(Rin, ci)
-            kk.gemm(dcolT, wtT, dy)
+            g, sc = self.pg, self.scratch.data_ptr()
+            dt = sc + a(R * ldz * 2)
+            dcolT = dt + a(R * ci * 4)
+            dy = self.empty(B * hin * win, ci)
+            self.call("ptycho_cnn_up_backward", dup.data_ptr(), dup.stride(0), yin.ptr, yin.ld, t.ptr, r.ptr, B, hin,
+                      win, ci, co, self._h(up["wt"]), self._h(up["w1"]),
+                      *((self._f(bn[0]), mean.ptr, rstd.ptr) if bn is not None else (None, None, None)),
+                      int(self.training), g + 4 * up["wt"].off, g + 4 * up["bt"].off, g + 4 * up["w1"].off,
+                      g + 4 * up["b1"].off,
+                      *((g + 4 * bn[0].off, g + 4 * bn[1].off) if bn is not None else (None, None)), sc, ldz, dt,
+                      dcolT, work.data_ptr(), work.numel(), dy.data_ptr(), self.st)
             if net.trace is not None:
-                net.trace[("upbwd", u)] = dict(dup=dup.clone(), dt=dt.clone(), dx=dy.clone())
+                o = dt - sc
+                net.trace[("upbwd", u)] = dict(dup=dup.clone(), dx=dy.clone(),
+                                               dt=self.scratch[o: o + R * ci * 4].view(_F32).view(R, ci).clone())
         # bottleneck
         h, w = H >> L, W >> L
         cin = net.bottleneck[0]["ci_store"]
         dpool = self.empty(B * h * w, cin)
-        self.block_bwd(("bott",), net.bottleneck, dy, B, h, w, grad, dpool)
+        self.block_bwd(("bott",), net.bottleneck, dy, B, h, w, dpool)
         # encoder, deepest first
         for l in range(L - 1, -1, -1):
             h, w = H >> l, W >> l
             R = B * h * w
             co = net.down[l][-1]["co"]
-            skip, arg = self.pool_arg[l]
-            if net.use_skip_connections:
-                dskip = dcat[l][:, co:]
-                kk.maxpool2_backward(dpool, arg, B, h, w, dskip, accumulate=True)
-            else:
-                dskip = self.empty(R, co)
-                kk.maxpool2_backward(dpool, arg, B, h, w, dskip)
+            dskip = dcat[l][:, co:] if net.use_skip_connections else self.empty(R, co)
+            self.call("ptycho_cnn_maxpool2_backward", dpool.data_ptr(), dpool.stride(0), self.pool_arg[l].ptr, B, h, w,
+                      co, dskip.data_ptr(), dskip.stride(0), int(net.use_skip_connections), self.st)
             cin = net.down[l][0]["ci_store"]
             if l > 0:
                 dpool = self.empty(R, cin)
-                self.block_bwd(("down", l), net.down[l], dskip, B, h, w, grad, dpool)
+                self.block_bwd(("down", l), net.down[l], dskip, B, h, w, dpool)
             else:
                 dx = self.empty(R, cin) if need_dx else None
-                self.block_bwd(("down", 0), net.down[0], dskip, B, h, w, grad, dx)
+                self.block_bwd(("down", 0), net.down[0], dskip, B, h, w, dx)
                 if need_dx:
                     out = self.empty(B, net.in_channels, H * W)
                     src = dx.view(B, H * W, cin)[..., : net.in_channels]
                     kk.transpose(src.contiguous(), out)
                     return out.view(B, net.in_channels, H, W)
         return None
-
-
-def _gemm_acc(A: torch.Tensor, B: torch.Tensor, out: torch.Tensor, run: _Run):
-    """out (FP32 parameter-gradient view) += A @ B.T with a long K (pixels): split-K
-    across CTAs, each adding its partial product atomically."""
-    M, K = A.shape
-    N = B.shape[0]
-    bn = 32 if N <= 32 else (64 if N <= 64 else 128)
-    tiles = ((M + 127) // 128) * ((N + bn - 1) // bn)
-    nkb = (K + 63) // 64
-    splits = max(1, min(nkb // 4, (2 * 148) // max(tiles, 1)))
-    kk.gemm(A, B, out.view(M, N), splits=splits, accumulate=True)
 
 
 class _CNNFn(torch.autograd.Function):

@@ -74,6 +74,23 @@ def gemm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, bias: torch.Tensor |
     return C
 
 
+def gemm_mn(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, a_mn: bool, splits: int = 1,
+            status: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
+    """C (op)= A @ B (``a_mn=False``: A (M, K)) or A.T @ B (``a_mn=True``: A (K, M)), with B (K, N)
+    as it is stored: BF16 operands, FP32 accumulation on the tcgen05 tensor cores, no transposed
+    copies.  ``splits`` and ``accumulate`` as in ``gemm``."""
+    if A.dtype != torch.bfloat16 or B.dtype != torch.bfloat16:
+        raise TypeError("gemm operands must be bfloat16")
+    K, M = A.shape if a_mn else A.shape[::-1]
+    K2, N = B.shape
+    if K2 != K or tuple(C.shape) != (M, N):
+        raise ValueError(f"gemm_mn shapes: A {tuple(A.shape)}, B {tuple(B.shape)}, C {tuple(C.shape)}")
+    flags = (GEMM_BF16 if C.dtype == torch.bfloat16 else 0) | (GEMM_ATOMIC if accumulate else 0)
+    _call("ptycho_gemm_bf16_mn", _p(A), _ld(A, "A"), int(a_mn), _p(B), _ld(B, "B"), _p(C), _ld(C, "C"), M, N, K,
+          flags, int(splits), _p(status), _s())
+    return C
+
+
 def im2col3x3(x: torch.Tensor, B: int, H: int, W: int, col: torch.Tensor) -> torch.Tensor:
     C = x.shape[1]
     _call("ptycho_cnn_im2col3x3", _p(x), B, H, W, C, _ld(x, "x"), _p(col), _ld(col, "col"), _s())

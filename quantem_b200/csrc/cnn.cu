@@ -16,6 +16,7 @@
 
 #include <mutex>
 
+#include "cnn_bn.cuh"
 #include "gemm_tcgen05.cuh"
 #include "ptycho_b200.h"
 
@@ -62,10 +63,10 @@ int encode_fn() {
   return g_encode ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "gemm: cuTensorMapEncodeTiled is not available");
 }
 
-// K-major bf16 matrix [rows][ld] (first k columns used) -> 2-D tensor map with
-// a box of 64 (k) x box_rows and the 128-byte swizzle.
-int make_map(CUtensorMap* map, const void* base, int rows, int k, int ld, int box_rows) {
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
+// Row-major bf16 matrix [rows][ld], `cols` used -> 2-D tensor map with a box of 64 columns x
+// box_rows and the 128-byte swizzle (K-major: rows x k; MN-major: k x rows, 64 k per box).
+int make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
   cuuint32_t box[2] = {static_cast<cuuint32_t>(qb::gemm::BK), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
@@ -75,20 +76,86 @@ int make_map(CUtensorMap* map, const void* base, int rows, int k, int ld, int bo
   return r == CUDA_SUCCESS ? PTYCHO_OK : fail(PTYCHO_ERR_INVALID, "gemm: tensor map encode failed (%d)", (int)r);
 }
 
-template <int BN>
+template <int BN, bool A_MN, bool B_MN>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int splits, int kb_per,
                 const qb::gemm::Epilogue& epi, int* status, cudaStream_t st) {
   using L = qb::gemm::Smem<BN>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(qb::gemm::gemm_bf16_tn_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                L::BYTES);
+    attr = cudaFuncSetAttribute(qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
   });
   if (attr != cudaSuccess) return fail(PTYCHO_ERR_CUDA, "gemm: smem attribute: %s", cudaGetErrorString(attr));
   dim3 grid((M + qb::gemm::BM - 1) / qb::gemm::BM, (N + BN - 1) / BN, splits);
-  qb::gemm::gemm_bf16_tn_kernel<BN><<<grid, qb::gemm::THREADS, L::BYTES, st>>>(ta, tb, M, N, K, kb_per, epi, status);
-  return check_launch("gemm_bf16_tn_kernel");
+  qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN>
+      <<<grid, qb::gemm::THREADS, L::BYTES, st>>>(ta, tb, M, N, K, kb_per, epi, status);
+  return check_launch("gemm_bf16_kernel");
+}
+
+// An operand of the product: rows of K values (K-major), or K rows of its values (mn).
+struct Operand {
+  const void* p;
+  int ld;
+  bool mn;
+};
+
+int gemm_run(const Operand& A, const Operand& B, void* C, int ldc, int M, int N, int K, const float* bias, int flags,
+             int splits, int* status, cudaStream_t st) {
+  using namespace qb::gemm;
+  if (!A.p || !B.p || !C || M < 1 || N < 1 || K < 1 || A.ld < (A.mn ? M : K) || B.ld < (B.mn ? N : K) || ldc < N)
+    return fail(PTYCHO_ERR_INVALID, "gemm: bad sizes (M=%d N=%d K=%d lda=%d ldb=%d ldc=%d)", M, N, K, A.ld, B.ld, ldc);
+  if ((A.ld & 7) || (B.ld & 7) || !al16(A.p) || !al16(B.p))
+    return fail(PTYCHO_ERR_INVALID, "gemm: A/B must be 16-byte aligned with leading dimensions a multiple of 8");
+  if (flags & ~(EPI_BF16 | EPI_RELU | EPI_ATOMIC | EPI_ACT_MASK))
+    return fail(PTYCHO_ERR_INVALID, "gemm: unknown flags %d", flags);
+  int act = (flags & EPI_ACT_MASK) >> EPI_ACT_SHIFT;
+  if (act >= qb::ACT_COUNT || ((flags & EPI_RELU) && act && act != qb::ACT_RELU))
+    return fail(PTYCHO_ERR_INVALID, "gemm: bad activation in flags %d", flags);
+  if (flags & EPI_RELU) act = qb::ACT_RELU;
+  const int nkb = (K + BK - 1) / BK;
+  if (splits < 1) splits = 1;
+  if (splits > nkb) splits = nkb;
+  const bool accumulate = (flags & EPI_ATOMIC) != 0;  // add into C as it is
+  if (splits > 1) flags |= EPI_ATOMIC;
+  if ((flags & EPI_ATOMIC) && ((flags & EPI_BF16) || act))
+    return fail(PTYCHO_ERR_INVALID, "gemm: split-K / atomic output needs FP32 output without an activation");
+  if (int rc = encode_fn()) return rc;
+  const int kb_per = (nkb + splits - 1) / splits;
+  splits = (nkb + kb_per - 1) / kb_per;  // every split gets >= 1 k-block
+  // The widest tile (fewest re-reads of A) that still gives every SM one; the deep layers of a
+  // network (16 to 256 rows) take narrow tiles: at 16 rows x 1024 columns x 9216 one CTA per 128
+  // columns streamed the weights through 8 SMs.  A column's products and sums do not depend on
+  // the tile width.  MN-major B tiles are copied in boxes of 64 columns.
+  const int tiles_m = (M + BM - 1) / BM, least = B.mn ? 64 : 16;
+  int BN = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  if (BN < least) BN = least;
+  while (BN > least && tiles_m * ((N + BN - 1) / BN) * splits < 148) BN /= 2;
+  CUtensorMap ta, tb;
+  if (int rc = A.mn ? make_map(&ta, A.p, K, M, A.ld, BK) : make_map(&ta, A.p, M, K, A.ld, BM)) return rc;
+  if (int rc = B.mn ? make_map(&tb, B.p, K, N, B.ld, BK) : make_map(&tb, B.p, N, K, B.ld, BN)) return rc;
+  if (!accumulate && splits > 1) {
+    if (cudaMemset2DAsync(C, (size_t)ldc * 4, 0, (size_t)N * 4, (size_t)M, st) != cudaSuccess)
+      return check_launch("gemm: clear split-K output");
+  }
+  const Epilogue epi{C, bias, ldc, flags, act};
+#define QB_GEMM(bn, a, b) return launch_gemm<bn, a, b>(ta, tb, M, N, K, splits, kb_per, epi, status, st)
+  if (A.mn && B.mn) {
+    if (BN == 64) QB_GEMM(64, true, true);
+    QB_GEMM(128, true, true);
+  }
+  if (B.mn) {
+    if (BN == 64) QB_GEMM(64, false, true);
+    QB_GEMM(128, false, true);
+  }
+  if (A.mn) return fail(PTYCHO_ERR_UNSUPPORTED, "gemm: an MN-major A goes with an MN-major B");
+  switch (BN) {
+    case 16: QB_GEMM(16, false, false);
+    case 32: QB_GEMM(32, false, false);
+    case 64: QB_GEMM(64, false, false);
+    default: QB_GEMM(128, false, false);
+  }
+#undef QB_GEMM
 }
 
 // ---------------------------------------------------------------------------
@@ -227,154 +294,54 @@ __global__ void transpose_kernel(const Ti* __restrict__ in, int R, int C, int ld
   }
 }
 
-// Deterministic column reductions over the rows of an FP32 matrix, in two passes:
-// per-chunk partials (double) then a fixed-order sum per column.
-//   mode 0: s0 = sum a,        s1 = sum a^2                  (batch-norm statistics)
-//   mode 1: s0 = sum a,        s1 = sum a * (b - mean) * rstd (batch-norm backward; a = dy, b = input)
-//   mode 2: s0 = sum a                                        (bias gradient)
+// Deterministic column sums over the rows of an FP32 matrix, in two passes: per-chunk
+// partials (double) then a fixed-order sum per column.
 constexpr int kColThreads = 256;
-__global__ void colsum_partial_kernel(int mode, const float* __restrict__ a, int lda, const float* __restrict__ b,
-                                      int ldb, const float* __restrict__ mean, const float* __restrict__ rstd, int R,
-                                      int C, int rows_per_chunk, double* __restrict__ part) {
-  __shared__ double red0[kColThreads], red1[kColThreads];
+__global__ void colsum_partial_kernel(const float* __restrict__ a, int lda, int R, int C, int rows_per_chunk,
+                                      double* __restrict__ part) {
+  __shared__ double red0[kColThreads];
   const int TC = C < kColThreads ? C : kColThreads;
   const int RP = kColThreads / TC;
   const int tx = threadIdx.x % TC, ty = threadIdx.x / TC;
   const int c = blockIdx.y * TC + tx;
   const int r0 = blockIdx.x * rows_per_chunk, r1 = min(R, r0 + rows_per_chunk);
-  double s0 = 0.0, s1 = 0.0;
+  double s0 = 0.0;
   if (ty < RP && c < C) {
-    const float m = (mode == 1) ? mean[c] : 0.0f, rs = (mode == 1) ? rstd[c] : 0.0f;
-    float f0 = 0.f, f1 = 0.f;
+    float f0 = 0.f;
     int cnt = 0;
     for (int r = r0 + ty; r < r1; r += RP) {
-      const float v = a[(int64_t)r * lda + c];
-      f0 += v;
-      if (mode == 0) f1 = fmaf(v, v, f1);
-      else if (mode == 1) f1 = fmaf(v, (b[(int64_t)r * ldb + c] - m) * rs, f1);
+      f0 += a[(int64_t)r * lda + c];
       if (++cnt == 64) {  // flush to double every 64 rows
         s0 += f0;
-        s1 += f1;
-        f0 = f1 = 0.f;
+        f0 = 0.f;
         cnt = 0;
       }
     }
     s0 += f0;
-    s1 += f1;
   }
   red0[threadIdx.x] = s0;
-  red1[threadIdx.x] = s1;
   __syncthreads();
   if (ty == 0 && c < C) {
-    for (int k = 1; k < RP; ++k) {
-      s0 += red0[k * TC + tx];
-      s1 += red1[k * TC + tx];
-    }
-    part[((int64_t)blockIdx.x * 2 + 0) * C + c] = s0;
-    part[((int64_t)blockIdx.x * 2 + 1) * C + c] = s1;
+    for (int k = 1; k < RP; ++k) s0 += red0[k * TC + tx];
+    part[(int64_t)blockIdx.x * C + c] = s0;
   }
 }
 
-// Finishing pass.  mode 0 (batch-norm statistics): mean, rstd = 1/sqrt(var + eps) with the
-// biased variance; running statistics updated with the unbiased one (nn.BatchNorm2d).
-// mode 1 (batch-norm backward): o0 = dbeta = sum dy, o1 = dgamma = sum dy*xhat.
-// mode 2: o0 = sum (bias gradient), written or accumulated.
-__global__ void colsum_final_kernel(int mode, const double* __restrict__ part, int nchunks, int R, int C, float eps,
-                                    float momentum, float* o0, float* o1, float* run_mean, float* run_var,
-                                    int accumulate) {
+__global__ void colsum_final_kernel(const double* __restrict__ part, int nchunks, int C, float* out, int accumulate) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  double s0 = 0.0, s1 = 0.0;
-  for (int k = 0; k < nchunks; ++k) {
-    s0 += part[((int64_t)k * 2 + 0) * C + c];
-    s1 += part[((int64_t)k * 2 + 1) * C + c];
-  }
-  if (mode == 0) {
-    const double mean = s0 / R;
-    double var = s1 / R - mean * mean;
-    if (var < 0.0) var = 0.0;
-    o0[c] = (float)mean;
-    o1[c] = (float)(1.0 / sqrt(var + (double)eps));
-    if (run_mean) {
-      const double unb = R > 1 ? var * R / (R - 1) : var;
-      run_mean[c] = (float)((1.0 - momentum) * run_mean[c] + momentum * mean);
-      run_var[c] = (float)((1.0 - momentum) * run_var[c] + momentum * unb);
-    }
-  } else if (mode == 1) {
-    if (accumulate) {
-      o0[c] += (float)s0;
-      o1[c] += (float)s1;
-    } else {
-      o0[c] = (float)s0;
-      o1[c] = (float)s1;
-    }
-  } else {
-    o0[c] = accumulate ? o0[c] + (float)s0 : (float)s0;
-  }
+  double s0 = 0.0;
+  for (int k = 0; k < nchunks; ++k) s0 += part[(int64_t)k * C + c];
+  out[c] = accumulate ? out[c] + (float)s0 : (float)s0;
 }
 
-// Eval-mode statistics: mean = running mean, rstd = 1/sqrt(running var + eps).
-__global__ void bn_eval_stats_kernel(const float* run_mean, const float* run_var, int C, float eps, float* mean,
-                                     float* rstd) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < C) {
-    mean[c] = run_mean[c];
-    rstd[c] = rsqrtf(run_var[c] + eps);
-  }
-}
-
-// y = (x - mean) * rstd * gamma + beta (or x when mean is null), bf16 out.
-__global__ void bn_apply_kernel(const float* __restrict__ x, int ldx, int R, int C, const float* __restrict__ mean,
-                                const float* __restrict__ rstd, const float* __restrict__ gamma,
-                                const float* __restrict__ beta, bf16* __restrict__ y, int ldy) {
+// y = bf16(x) (layers without batch norm)
+__global__ void to_bf16_kernel(const float* __restrict__ x, int ldx, int R, int C, bf16* __restrict__ y, int ldy) {
   const int64_t total = (int64_t)R * C;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % C);
     const int64_t r = i / C;
-    float v = x[r * ldx + c];
-    if (mean) v = (v - mean[c]) * rstd[c] * gamma[c] + beta[c];
-    y[r * ldy + c] = __float2bfloat16_rn(v);
-  }
-}
-
-// Batch-norm backward (training statistics) followed by the derivative of the activation
-// that produced its input x: dx = act'(x) * gamma * rstd * (dy - s_dy/R - xhat * s_dyxhat/R);
-// without batch norm (mean null) dx = act'(x) * dy.  act = qb::ACT_* (1 = ReLU: the mask
-// [x > 0]; 0: none).  Writes FP32 and BF16 copies.
-__global__ void bn_relu_backward_kernel(const float* __restrict__ dy, int lddy, const float* __restrict__ x, int ldx,
-                                        int R, int C, const float* __restrict__ mean, const float* __restrict__ rstd,
-                                        const float* __restrict__ gamma, const float* __restrict__ sdy,
-                                        const float* __restrict__ sdyx, int act, float* __restrict__ dz32,
-                                        bf16* __restrict__ dz16, int ldz) {
-  const int64_t total = (int64_t)R * C;
-  const float invR = 1.0f / (float)R;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t r = i / C;
-    const float xv = x[r * ldx + c];
-    float g = dy[r * lddy + c];
-    if (mean) {
-      const float xh = (xv - mean[c]) * rstd[c];
-      g = gamma[c] * rstd[c] * (g - sdy[c] * invR - xh * sdyx[c] * invR);
-    }
-    if (act) g *= qb::act_grad_from_output(act, xv);
-    if (dz32) dz32[r * ldz + c] = g;
-    if (dz16) dz16[r * ldz + c] = __float2bfloat16_rn(g);
-  }
-}
-
-// Eval-mode batch-norm backward is a per-channel scale: dx = dy * gamma * rstd (then act').
-__global__ void bn_eval_backward_kernel(const float* __restrict__ dy, int lddy, const float* __restrict__ x, int ldx,
-                                        int R, int C, const float* __restrict__ rstd, const float* __restrict__ gamma,
-                                        int act, float* __restrict__ dz32, bf16* __restrict__ dz16, int ldz) {
-  const int64_t total = (int64_t)R * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t r = i / C;
-    float g = dy[r * lddy + c] * gamma[c] * rstd[c];
-    if (act) g *= qb::act_grad_from_output(act, x[r * ldx + c]);
-    if (dz32) dz32[r * ldz + c] = g;
-    if (dz16) dz16[r * ldz + c] = __float2bfloat16_rn(g);
+    y[r * ldy + c] = __float2bfloat16_rn(x[r * ldx + c]);
   }
 }
 
@@ -482,24 +449,41 @@ __global__ void bin_features_kernel(const float* __restrict__ pat, int npos, int
 
 constexpr int kMseBlocks = 296;
 
-int colsum(int mode, const float* a, int lda, const float* b, int ldb, const float* mean, const float* rstd, int R,
-           int C, double* work, int64_t work_elems, float eps, float momentum, float* o0, float* o1, float* run_mean,
-           float* run_var, int accumulate, cudaStream_t st) {
+int work_check(int C, int64_t work_elems) {
+  if (work_elems < 2 * (int64_t)C)
+    return fail(PTYCHO_ERR_INVALID, "cnn: reduction workspace too small (%lld doubles for C=%d)",
+                (long long)work_elems, C);
+  return PTYCHO_OK;
+}
+
+int colsum(const float* a, int lda, int R, int C, double* work, int64_t work_elems, float* out, int accumulate,
+           cudaStream_t st) {
+  if (int rc = work_check(C, work_elems)) return rc;
   const int TC = C < kColThreads ? C : kColThreads;
   const int RP = kColThreads / TC;
   int chunks = (R + RP * 16 - 1) / (RP * 16);
   if (chunks > 592) chunks = 592;
   if ((int64_t)chunks * 2 * C > work_elems) chunks = (int)(work_elems / (2 * (int64_t)C));
-  if (chunks < 1) return fail(PTYCHO_ERR_INVALID, "cnn: reduction workspace too small (%lld doubles for C=%d)",
-                              (long long)work_elems, C);
   const int rpc = (R + chunks - 1) / chunks;
   chunks = (R + rpc - 1) / rpc;
   dim3 grid(chunks, (C + TC - 1) / TC);
-  colsum_partial_kernel<<<grid, kColThreads, 0, st>>>(mode, a, lda, b, ldb, mean, rstd, R, C, rpc, work);
+  colsum_partial_kernel<<<grid, kColThreads, 0, st>>>(a, lda, R, C, rpc, work);
   if (int rc = check_launch("colsum_partial_kernel")) return rc;
-  colsum_final_kernel<<<(C + 127) / 128, 128, 0, st>>>(mode, work, chunks, R, C, eps, momentum, o0, o1, run_mean,
-                                                       run_var, accumulate);
+  colsum_final_kernel<<<(C + 127) / 128, 128, 0, st>>>(work, chunks, C, out, accumulate);
   return check_launch("colsum_final_kernel");
+}
+
+int bn_forward(const qb::bn::Forward& f, int R, int C, cudaStream_t st) {
+  if (!f.gamma) {
+    to_bf16_kernel<<<blocks_for((int64_t)R * C, 256), 256, 0, st>>>(f.x, f.ldx, R, C, f.y, f.ldy);
+    return check_launch("to_bf16_kernel");
+  }
+  const cudaError_t e = qb::bn::launch(qb::bn::bn_forward_kernel, f, R, C, st);
+  return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_forward_kernel: %s", cudaGetErrorString(e));
+}
+int bn_backward(const qb::bn::Backward& b, int R, int C, cudaStream_t st) {
+  const cudaError_t e = qb::bn::launch(qb::bn::bn_backward_kernel, b, R, C, st);
+  return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_backward_kernel: %s", cudaGetErrorString(e));
 }
 
 }  // namespace
@@ -539,49 +523,14 @@ extern "C" {
 
 int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K,
                      const float* bias, int flags, int splits, int* status, void* stream) {
-  using namespace qb::gemm;
-  if (!A || !B || !C || M < 1 || N < 1 || K < 1 || lda < K || ldb < K || ldc < N)
-    return fail(PTYCHO_ERR_INVALID, "gemm: bad sizes (M=%d N=%d K=%d lda=%d ldb=%d ldc=%d)", M, N, K, lda, ldb, ldc);
-  if ((lda & 7) || (ldb & 7) || !al16(A) || !al16(B))
-    return fail(PTYCHO_ERR_INVALID, "gemm: A/B must be 16-byte aligned with leading dimensions a multiple of 8");
-  if (flags & ~(EPI_BF16 | EPI_RELU | EPI_ATOMIC | EPI_ACT_MASK))
-    return fail(PTYCHO_ERR_INVALID, "gemm: unknown flags %d", flags);
-  int act = (flags & EPI_ACT_MASK) >> EPI_ACT_SHIFT;
-  if (act >= qb::ACT_COUNT || ((flags & EPI_RELU) && act && act != qb::ACT_RELU))
-    return fail(PTYCHO_ERR_INVALID, "gemm: bad activation in flags %d", flags);
-  if (flags & EPI_RELU) act = qb::ACT_RELU;
-  const int nkb = (K + BK - 1) / BK;
-  if (splits < 1) splits = 1;
-  if (splits > nkb) splits = nkb;
-  const bool accumulate = (flags & EPI_ATOMIC) != 0;  // add into C as it is
-  if (splits > 1) flags |= EPI_ATOMIC;
-  if ((flags & EPI_ATOMIC) && ((flags & EPI_BF16) || act))
-    return fail(PTYCHO_ERR_INVALID, "gemm: split-K / atomic output needs FP32 output without an activation");
-  if (int rc = encode_fn()) return rc;
-  const int kb_per = (nkb + splits - 1) / splits;
-  splits = (nkb + kb_per - 1) / kb_per;  // every split gets >= 1 k-block
-  // The widest tile (fewest re-reads of A) that still gives every SM one; the deep layers of a
-  // network (16 to 256 rows) take narrow tiles: at 16 rows x 1024 columns x 9216 one CTA per 128
-  // columns streamed the weights through 8 SMs.  A column's products and sums do not depend on
-  // the tile width.
-  const int tiles_m = (M + BM - 1) / BM;
-  int BN = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
-  while (BN > 16 && tiles_m * ((N + BN - 1) / BN) * splits < 148) BN /= 2;
-  CUtensorMap ta, tb;
-  if (int rc = make_map(&ta, A, M, K, lda, BM)) return rc;
-  if (int rc = make_map(&tb, B, N, K, ldb, BN)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!accumulate && splits > 1) {
-    if (cudaMemset2DAsync(C, (size_t)ldc * 4, 0, (size_t)N * 4, (size_t)M, st) != cudaSuccess)
-      return check_launch("gemm: clear split-K output");
-  }
-  Epilogue epi{C, bias, ldc, flags, act};
-  switch (BN) {
-    case 16: return launch_gemm<16>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
-    case 32: return launch_gemm<32>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
-    case 64: return launch_gemm<64>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
-    default: return launch_gemm<128>(ta, tb, M, N, K, splits, kb_per, epi, status, st);
-  }
+  return gemm_run({A, lda, false}, {B, ldb, false}, C, ldc, M, N, K, bias, flags, splits, status,
+                  static_cast<cudaStream_t>(stream));
+}
+
+int ptycho_gemm_bf16_mn(const void* A, int lda, int a_mn, const void* B, int ldb, void* C, int ldc, int M, int N,
+                        int K, int flags, int splits, int* status, void* stream) {
+  return gemm_run({A, lda, a_mn != 0}, {B, ldb, true}, C, ldc, M, N, K, nullptr, flags, splits, status,
+                  static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_im2col3x3(const void* x, int B, int H, int W, int C, int ldx, void* col, int ldcol, void* stream) {
@@ -653,23 +602,15 @@ int ptycho_cnn_bn_forward(const float* x, int ldx, int R, int C, const float* ga
                           float* run_mean, float* run_var, float momentum, float eps, int training, float* mean,
                           float* rstd, double* work, int64_t work_elems, void* out, int ldo, void* stream) {
   if (!x || !out || R < 1 || C < 1 || ldx < C || ldo < C) return fail(PTYCHO_ERR_INVALID, "bn_forward: bad arguments");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool bn = gamma != nullptr;
-  if (bn) {
+  if (gamma) {
     if (!beta || !mean || !rstd || (!training && (!run_mean || !run_var)))
       return fail(PTYCHO_ERR_INVALID, "bn_forward: missing statistics buffers");
-    if (training) {
-      if (int rc = colsum(0, x, ldx, nullptr, 0, nullptr, nullptr, R, C, work, work_elems, eps, momentum, mean, rstd,
-                          run_mean, run_var, 0, st))
-        return rc;
-    } else {
-      bn_eval_stats_kernel<<<(C + 127) / 128, 128, 0, st>>>(run_mean, run_var, C, eps, mean, rstd);
-      if (int rc = check_launch("bn_eval_stats_kernel")) return rc;
-    }
+    if (training)
+      if (int rc = work_check(C, work_elems)) return rc;
   }
-  bn_apply_kernel<<<blocks_for((int64_t)R * C, 256), 256, 0, st>>>(x, ldx, R, C, bn ? mean : nullptr, rstd, gamma,
-                                                                    beta, static_cast<bf16*>(out), ldo);
-  return check_launch("bn_apply_kernel");
+  return bn_forward({x, ldx, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                     static_cast<bf16*>(out), ldo},
+                    R, C, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_bn_backward(const float* dy, int lddy, const float* x, int ldx, int R, int C, const float* gamma,
@@ -678,31 +619,19 @@ int ptycho_cnn_bn_backward(const float* dy, int lddy, const float* x, int ldx, i
   if (!dy || !x || R < 1 || C < 1 || lddy < C || ldx < C || ldz < C || (!dz32 && !dz16) || act < 0 ||
       act >= qb::ACT_COUNT)
     return fail(PTYCHO_ERR_INVALID, "bn_backward: bad arguments");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int g = blocks_for((int64_t)R * C, 256);
   if (gamma) {
     if (!mean || !rstd || !dgamma || !dbeta) return fail(PTYCHO_ERR_INVALID, "bn_backward: missing buffers");
-    if (int rc = colsum(1, dy, lddy, x, ldx, mean, rstd, R, C, work, work_elems, 0.f, 0.f, dbeta, dgamma, nullptr,
-                        nullptr, 0, st))
-      return rc;
-    if (training)
-      bn_relu_backward_kernel<<<g, 256, 0, st>>>(dy, lddy, x, ldx, R, C, mean, rstd, gamma, dbeta, dgamma, act, dz32,
-                                                 static_cast<bf16*>(dz16), ldz);
-    else
-      bn_eval_backward_kernel<<<g, 256, 0, st>>>(dy, lddy, x, ldx, R, C, rstd, gamma, act, dz32,
-                                                 static_cast<bf16*>(dz16), ldz);
-  } else {
-    bn_relu_backward_kernel<<<g, 256, 0, st>>>(dy, lddy, x, ldx, R, C, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                               act, dz32, static_cast<bf16*>(dz16), ldz);
+    if (int rc = work_check(C, work_elems)) return rc;
   }
-  return check_launch("bn_backward");
+  return bn_backward({dy, lddy, x, ldx, gamma, mean, rstd, training, act, dgamma, dbeta, nullptr, dz32,
+                      static_cast<bf16*>(dz16), ldz},
+                     R, C, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_colsum(const float* a, int lda, int R, int C, float* out, int accumulate, double* work,
                       int64_t work_elems, void* stream) {
   if (!a || !out || R < 1 || C < 1 || lda < C) return fail(PTYCHO_ERR_INVALID, "colsum: bad arguments");
-  return colsum(2, a, lda, nullptr, 0, nullptr, nullptr, R, C, work, work_elems, 0.f, 0.f, out, nullptr, nullptr,
-                nullptr, accumulate, static_cast<cudaStream_t>(stream));
+  return colsum(a, lda, R, C, work, work_elems, out, accumulate, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_maxpool2(const void* in, int ldi, int B, int H, int W, int C, void* out, int ldo, void* argmax,
@@ -764,6 +693,92 @@ int ptycho_cnn_dropout(void* x, int dtype, int R, int C, int ld, float p, uint64
   else
     dropout_kernel<bf16><<<g, 256, 0, st>>>(static_cast<bf16*>(x), R, C, ld, p, scale, seed);
   return check_launch("dropout_kernel");
+}
+
+int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, const void* w, int co,
+                            const float* bias, int act, const float* gamma, const float* beta, float* run_mean,
+                            float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
+                            void* col, float* r, void* out, int ldo, void* stream) {
+  const int R = B * H * W;
+  if (int rc = ptycho_cnn_im2col3x3(x, B, H, W, C, ldx, col, 9 * C, stream)) return rc;
+  if (int rc = ptycho_gemm_bf16(col, 9 * C, w, 9 * C, r, co, R, co, 9 * C, bias, act << 8, 1, nullptr, stream))
+    return rc;
+  if (!out) return PTYCHO_OK;
+  return bn_forward({r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                     static_cast<bf16*>(out), ldo},
+                    R, co, static_cast<cudaStream_t>(stream));
+}
+
+namespace {
+// K-splits of a weight gradient (K = rows): about two CTAs per SM, at least four k-blocks each
+int wgrad_splits(int M, int N, int K) {
+  const int bn = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  const int tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), nkb = (K + 63) / 64;
+  int s = 2 * 148 / (tiles > 0 ? tiles : 1);
+  if (s > nkb / 4) s = nkb / 4;
+  return s < 1 ? 1 : s;
+}
+}  // namespace
+
+int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, int B, int H, int W, int C,
+                             const void* w, const float* r, int co, const float* gamma, const float* mean,
+                             const float* rstd, int training, int act, float* dw, float* db, float* dgamma,
+                             float* dbeta, void* dz, int ldz, void* col, float* dcol, float* dx, int lddx,
+                             int dx_accumulate, void* stream) {
+  const int R = B * H * W, K9 = 9 * C;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (int rc = bn_backward({dy, lddy, r, co, gamma, mean, rstd, training, act, dgamma, dbeta, db, nullptr,
+                            static_cast<bf16*>(dz), ldz},
+                           R, co, st))
+    return rc;
+  // weight gradient dz^T col
+  if (int rc = ptycho_cnn_im2col3x3(x, B, H, W, C, ldx, col, K9, stream)) return rc;
+  if (int rc = gemm_run({dz, ldz, true}, {col, K9, true}, dw, K9, co, K9, R, nullptr, PTYCHO_GEMM_ATOMIC,
+                        wgrad_splits(co, K9, R), nullptr, st))
+    return rc;
+  if (!dx) return PTYCHO_OK;
+  // input gradient: dz w, folded over the taps
+  if (int rc = gemm_run({dz, ldz, false}, {w, K9, true}, dcol, K9, R, K9, co, nullptr, 0, 1, nullptr, st)) return rc;
+  return ptycho_cnn_col2im3x3(dcol, K9, B, H, W, C, dx, lddx, dx_accumulate, stream);
+}
+
+int ptycho_cnn_up_forward(const void* y, int ldy, int B, int H, int W, int ci, int co, const void* wt, const float* bt,
+                          const void* w1, const float* b1, const float* gamma, const float* beta, float* run_mean,
+                          float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
+                          float* colT, void* t, float* r, void* out, int ldo, void* stream) {
+  const int Rin = B * H * W, R = 4 * Rin;
+  if (int rc = ptycho_gemm_bf16(y, ldy, wt, ci, colT, 9 * ci, Rin, 9 * ci, ci, nullptr, 0, 1, nullptr, stream))
+    return rc;
+  if (int rc = ptycho_cnn_convT_gather(colT, 9 * ci, B, H, W, ci, bt, t, ci, stream)) return rc;
+  if (int rc = ptycho_gemm_bf16(t, ci, w1, ci, r, co, R, co, ci, b1, 0, 1, nullptr, stream)) return rc;
+  return bn_forward({r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                     static_cast<bf16*>(out), ldo},
+                    R, co, static_cast<cudaStream_t>(stream));
+}
+
+int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, const void* t, const float* r, int B,
+                           int H, int W, int ci, int co, const void* wt, const void* w1, const float* gamma,
+                           const float* mean, const float* rstd, int training, float* dwt, float* dbt, float* dw1,
+                           float* db1, float* dgamma, float* dbeta, void* dz, int ldz, float* dt, void* dcolT,
+                           double* work, int64_t work_elems, float* dy, void* stream) {
+  const int Rin = B * H * W, R = 4 * Rin, C9 = 9 * ci;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (int rc = bn_backward({dup, lddup, r, co, gamma, mean, rstd, training, 0, dgamma, dbeta, db1, nullptr,
+                            static_cast<bf16*>(dz), ldz},
+                           R, co, st))
+    return rc;
+  // 1x1 convolution: dw1 = dz^T t, dt = dz w1
+  if (int rc = gemm_run({dz, ldz, true}, {t, ci, true}, dw1, ci, co, ci, R, nullptr, PTYCHO_GEMM_ATOMIC,
+                        wgrad_splits(co, ci, R), nullptr, st))
+    return rc;
+  if (int rc = gemm_run({dz, ldz, false}, {w1, ci, true}, dt, ci, R, ci, co, nullptr, 0, 1, nullptr, st)) return rc;
+  // transposed convolution: bias, weight and input gradients
+  if (int rc = colsum(dt, ci, R, ci, work, work_elems, dbt, 0, st)) return rc;
+  if (int rc = ptycho_cnn_convT_im2col(dt, ci, B, H, W, ci, dcolT, C9, stream)) return rc;
+  if (int rc = gemm_run({dcolT, C9, true}, {y, ldy, true}, dwt, ci, C9, ci, Rin, nullptr, PTYCHO_GEMM_ATOMIC,
+                        wgrad_splits(C9, ci, Rin), nullptr, st))
+    return rc;
+  return gemm_run({dcolT, C9, false}, {wt, ci, true}, dy, ci, Rin, ci, C9, nullptr, 0, 1, nullptr, st);
 }
 
 }  // extern "C"

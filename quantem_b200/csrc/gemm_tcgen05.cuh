@@ -1,9 +1,11 @@
 // BF16 x BF16 -> FP32 GEMM on the 5th-generation tensor cores (sm_100a).
 //
-//   C[M, N] (op)= A[M, K] * B[N, K]^T (+ bias[N]) (ReLU)
+//   C[M, N] (op)= A[M, K] * B[N, K]^T (+ bias[N]) (activation)
 //
-// A and B are K-major (row-major with K contiguous, leading dimensions lda/ldb in
-// elements, multiples of 8 so that every row starts on a 16-byte boundary).
+// Each operand is K-major (rows of K contiguous values) or MN-major (stored as K rows of
+// its M or N values: the transpose of what the product takes, so that the weight and input
+// gradients of a layer need no transposed copies).  Leading dimensions are multiples of 8
+// elements so that every row starts on a 16-byte boundary.
 //
 // One CTA of 128 threads computes a 128 x BN tile:
 //   * warp 0, one lane: TMA producer.  Each k-block (64 bf16 = one 128-byte
@@ -110,16 +112,24 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// Shared-memory matrix descriptor of an MN-major operand, 128-byte swizzle: k-rows of 64
+// values (128 bytes), 8-row groups 1024 bytes apart (SBO), the next 64 values one copied
+// box further (LBO).
+__device__ __forceinline__ uint64_t sdesc_mn128(const void* tile) {
+  const uint64_t addr = (smem_u32(tile) >> 4) & 0x3FFFull;
+  return addr | (uint64_t(64 * BK * 2 >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of
 // 128 bytes, 8-row core groups 1024 bytes apart (SBO), descriptor version 1.
 __device__ __forceinline__ uint64_t sdesc_k128(const void* tile) {
   const uint64_t addr = (smem_u32(tile) >> 4) & 0x3FFFull;
   return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major.
-template <int BN>
+// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, major-ness of each.
+template <int BN, bool A_MN, bool B_MN>
 __host__ __device__ constexpr uint32_t idesc_bf16() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(BN >> 3) << 17) | (uint32_t(BM >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(A_MN) << 15) | (uint32_t(B_MN) << 16) |
+         (uint32_t(BN >> 3) << 17) | (uint32_t(BM >> 4) << 24);
 }
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
@@ -147,10 +157,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <int BN>
+template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(THREADS, 1)
-    gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
+    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                         int N, int K, int kb_per_split, Epilogue epi, int* status) {
+  static_assert(!B_MN || BN % 64 == 0, "an MN-major tile is copied in boxes of 64 values");
   static_assert(BN == 16 || BN == 32 || BN == 64 || BN == 128, "BN: a multiple of 16");
   using L = Smem<BN>;
   constexpr int STAGES = L::STAGES;
@@ -201,11 +212,26 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       uint8_t* sa = smem + s * L::STAGE_BYTES;
       mbar_expect_tx(&full[s], L::STAGE_BYTES);
-      tma_load_2d(sa, &tmA, &full[s], (kb0 + i) * BK, m0);
-      tma_load_2d(sa + L::A_BYTES, &tmB, &full[s], (kb0 + i) * BK, n0);
+      const int k0 = (kb0 + i) * BK;
+      if (A_MN) {  // boxes of 64 values x 64 k
+#pragma unroll
+        for (int j = 0; j < BM; j += 64) tma_load_2d(sa + j * BK * 2, &tmA, &full[s], m0 + j, k0);
+      } else {
+        tma_load_2d(sa, &tmA, &full[s], k0, m0);
+      }
+      uint8_t* sb = sa + L::A_BYTES;
+      if (B_MN) {
+#pragma unroll
+        for (int j = 0; j < BN; j += 64) tma_load_2d(sb + j * BK * 2, &tmB, &full[s], n0 + j, k0);
+      } else {
+        tma_load_2d(sb, &tmB, &full[s], k0, n0);
+      }
     }
   } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = idesc_bf16<BN>();
+    constexpr uint32_t idesc = idesc_bf16<BN, A_MN, B_MN>();
+    // step of K = 16 in descriptor units (16 bytes): 32 bytes along the swizzled row of a K-major
+    // operand, 16 rows of 128 bytes of an MN-major one
+    constexpr uint64_t astep = A_MN ? 128 : 2, bstep = B_MN ? 128 : 2;
     for (int i = 0; i < nkb; ++i) {
       const int s = i % STAGES;
       const uint32_t ph = (i / STAGES) & 1;
@@ -215,10 +241,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       tc_fence_after();
       const uint8_t* sa = smem + s * L::STAGE_BYTES;
-      const uint64_t ad = sdesc_k128(sa), bd = sdesc_k128(sa + L::A_BYTES);
+      const uint64_t ad = A_MN ? sdesc_mn128(sa) : sdesc_k128(sa);
+      const uint64_t bd = B_MN ? sdesc_mn128(sa + L::A_BYTES) : sdesc_k128(sa + L::A_BYTES);
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k)  // +32 bytes along the swizzled row per K = 16 step
-        umma_bf16(tmem, ad + 2 * k, bd + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+      for (int k = 0; k < BK / 16; ++k)
+        umma_bf16(tmem, ad + astep * k, bd + bstep * k, idesc, (i | k) != 0 ? 1u : 0u);
       umma_commit(&empty[s]);
     }
     umma_commit(done);  // also after a failure: completes once every issued MMA has finished
