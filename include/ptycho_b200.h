@@ -413,8 +413,8 @@ int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, 
                             float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
                             void* col, float* r, void* out, int ldo, void* stream);
 
-/* Gradients of the layer from dy (FP32, R x co, w.r.t. the batch norm's output): dw (added to,
- * FP32 (co, 9 C)), db, dgamma, dbeta (written) and, if given, dx (FP32 R x C, written or added
+/* Gradients of the layer from dy (FP32, R x co, w.r.t. the batch norm's output): dw (FP32
+ * (co, 9 C), zero on entry), db, dgamma, dbeta (written) and, if given, dx (FP32 R x C, written or added
  * to).  dz: BF16 scratch R x ldz (ldz >= co, a multiple of 8); col: BF16 scratch R x 9 C;
  * dcol: FP32 scratch R x 9 C (with dx). */
 int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, int B, int H, int W, int C,
@@ -431,7 +431,7 @@ int ptycho_cnn_up_forward(const void* y, int ldy, int B, int H, int W, int ci, i
                           float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
                           float* colT, void* t, float* r, void* out, int ldo, void* stream);
 
-/* Gradients of the block from dup (FP32, 4 B H W x co): dwt, dw1 added to, dbt, db1, dgamma,
+/* Gradients of the block from dup (FP32, 4 B H W x co): dwt, dw1 (zero on entry), dbt, db1, dgamma,
  * dbeta and dy (FP32 B H W x ci) written.  dz: BF16 scratch 4 B H W x ldz; dt: FP32 scratch
  * 4 B H W x ci; dcolT: BF16 scratch B H W x 9 ci; work as in ptycho_cnn_colsum. */
 int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, const void* t, const float* r, int B,

@@ -77,7 +77,7 @@ int make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int
 }
 
 template <int BN, bool A_MN, bool B_MN>
-int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int splits, int kb_per,
+int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int splits, int kb_per, int a_rows,
                 const qb::gemm::Epilogue& epi, int* status, cudaStream_t st) {
   using L = qb::gemm::Smem<BN>;
   static std::once_flag once;
@@ -89,7 +89,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int 
   if (attr != cudaSuccess) return fail(PTYCHO_ERR_CUDA, "gemm: smem attribute: %s", cudaGetErrorString(attr));
   dim3 grid((M + qb::gemm::BM - 1) / qb::gemm::BM, (N + BN - 1) / BN, splits);
   qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN>
-      <<<grid, qb::gemm::THREADS, L::BYTES, st>>>(ta, tb, M, N, K, kb_per, epi, status);
+      <<<grid, qb::gemm::THREADS, L::BYTES, st>>>(ta, tb, M, N, K, kb_per, a_rows, epi, status);
   return check_launch("gemm_bf16_kernel");
 }
 
@@ -132,14 +132,15 @@ int gemm_run(const Operand& A, const Operand& B, void* C, int ldc, int M, int N,
   if (BN < least) BN = least;
   while (BN > least && tiles_m * ((N + BN - 1) / BN) * splits < 148) BN /= 2;
   CUtensorMap ta, tb;
-  if (int rc = A.mn ? make_map(&ta, A.p, K, M, A.ld, BK) : make_map(&ta, A.p, M, K, A.ld, BM)) return rc;
+  const int a_rows = A.mn || M >= BM ? BM : (M + 7) / 8 * 8;
+  if (int rc = A.mn ? make_map(&ta, A.p, K, M, A.ld, BK) : make_map(&ta, A.p, M, K, A.ld, a_rows)) return rc;
   if (int rc = B.mn ? make_map(&tb, B.p, K, N, B.ld, BK) : make_map(&tb, B.p, N, K, B.ld, BN)) return rc;
   if (!accumulate && splits > 1) {
     if (cudaMemset2DAsync(C, (size_t)ldc * 4, 0, (size_t)N * 4, (size_t)M, st) != cudaSuccess)
       return check_launch("gemm: clear split-K output");
   }
   const Epilogue epi{C, bias, ldc, flags, act};
-#define QB_GEMM(bn, a, b) return launch_gemm<bn, a, b>(ta, tb, M, N, K, splits, kb_per, epi, status, st)
+#define QB_GEMM(bn, a, b) return launch_gemm<bn, a, b>(ta, tb, M, N, K, splits, kb_per, a_rows, epi, status, st)
   if (A.mn && B.mn) {
     if (BN == 64) QB_GEMM(64, true, true);
     QB_GEMM(128, true, true);
@@ -710,13 +711,16 @@ int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, 
 }
 
 namespace {
-// K-splits of a weight gradient (K = rows): about two CTAs per SM, at least four k-blocks each
-int wgrad_splits(int M, int N, int K) {
+// Weight gradient dw (M x N, zero on entry) = A^T B over K rows, split over K to about two CTAs
+// per SM with at least four k-blocks each.  One split stores its result: adding the 38 MB of a
+// 1024 x 9216 gradient atomically took 94 us.
+int wgrad(const void* A, int lda, const void* B, int ldb, float* dw, int M, int N, int K, cudaStream_t st) {
   const int bn = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
   const int tiles = ((M + 127) / 128) * ((N + bn - 1) / bn), nkb = (K + 63) / 64;
   int s = 2 * 148 / (tiles > 0 ? tiles : 1);
   if (s > nkb / 4) s = nkb / 4;
-  return s < 1 ? 1 : s;
+  return gemm_run({A, lda, true}, {B, ldb, true}, dw, N, M, N, K, nullptr, s > 1 ? PTYCHO_GEMM_ATOMIC : 0, s, nullptr,
+                  st);
 }
 }  // namespace
 
@@ -733,9 +737,7 @@ int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, 
     return rc;
   // weight gradient dz^T col
   if (int rc = ptycho_cnn_im2col3x3(x, B, H, W, C, ldx, col, K9, stream)) return rc;
-  if (int rc = gemm_run({dz, ldz, true}, {col, K9, true}, dw, K9, co, K9, R, nullptr, PTYCHO_GEMM_ATOMIC,
-                        wgrad_splits(co, K9, R), nullptr, st))
-    return rc;
+  if (int rc = wgrad(dz, ldz, col, K9, dw, co, K9, R, st)) return rc;
   if (!dx) return PTYCHO_OK;
   // input gradient: dz w, folded over the taps
   if (int rc = gemm_run({dz, ldz, false}, {w, K9, true}, dcol, K9, R, K9, co, nullptr, 0, 1, nullptr, st)) return rc;
@@ -768,16 +770,12 @@ int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, 
                            R, co, st))
     return rc;
   // 1x1 convolution: dw1 = dz^T t, dt = dz w1
-  if (int rc = gemm_run({dz, ldz, true}, {t, ci, true}, dw1, ci, co, ci, R, nullptr, PTYCHO_GEMM_ATOMIC,
-                        wgrad_splits(co, ci, R), nullptr, st))
-    return rc;
+  if (int rc = wgrad(dz, ldz, t, ci, dw1, co, ci, R, st)) return rc;
   if (int rc = gemm_run({dz, ldz, false}, {w1, ci, true}, dt, ci, R, ci, co, nullptr, 0, 1, nullptr, st)) return rc;
   // transposed convolution: bias, weight and input gradients
   if (int rc = colsum(dt, ci, R, ci, work, work_elems, dbt, 0, st)) return rc;
   if (int rc = ptycho_cnn_convT_im2col(dt, ci, B, H, W, ci, dcolT, C9, stream)) return rc;
-  if (int rc = gemm_run({dcolT, C9, true}, {y, ldy, true}, dwt, ci, C9, ci, Rin, nullptr, PTYCHO_GEMM_ATOMIC,
-                        wgrad_splits(C9, ci, Rin), nullptr, st))
-    return rc;
+  if (int rc = wgrad(dcolT, C9, y, ldy, dwt, C9, ci, Rin, st)) return rc;
   return gemm_run({dcolT, C9, false}, {wt, ci, true}, dy, ci, Rin, ci, C9, nullptr, 0, 1, nullptr, st);
 }
 

@@ -77,6 +77,33 @@ __device__ __forceinline__ void cluster_sums(Sums<NV>& sm, double (&v)[NV], int 
   }
 }
 
+// One float run: v[0] += sum a, v[1] += sum a b over rows r, r + step, ... < r1, in float up to
+// 64 rows at a time.  Eight rows are loaded before they are used: a load at a time, the latency of
+// its 16 or so rows was most of the kernel.
+template <typename L>
+__device__ __forceinline__ void run_sums(int r, int r1, int step, double (&v)[2], L load) {
+  while (r < r1) {
+    float f0 = 0.f, f1 = 0.f;
+    for (int i = 0; i < 64 && r < r1; i += 8) {
+      float a[8], b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[j] = b[j] = 0.f;
+        if (r + j * step < r1) load(r + j * step, a[j], b[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * step < r1) {
+          f0 += a[j];
+          f1 = fmaf(a[j], b[j], f1);
+        }
+      r += 8 * step;
+    }
+    v[0] += f0;
+    v[1] += f1;
+  }
+}
+
 struct Forward {
   const float* x;
   int ldx;
@@ -103,21 +130,8 @@ __global__ void __launch_bounds__(kThreads) bn_forward_kernel(const Forward p, c
     if (on)
       for (int t = slot; t < rows.runs; t += nslots) {
         const int r0 = t / rows.RP * rows.rpc, r1 = min(rows.R, r0 + rows.rpc);
-        float f0 = 0.f, f1 = 0.f;
-        int cnt = 0;
-        for (int r = r0 + t % rows.RP; r < r1; r += rows.RP) {
-          const float a = p.x[(int64_t)r * p.ldx + c];
-          f0 += a;
-          f1 = fmaf(a, a, f1);
-          if (++cnt == 64) {  // flush to double every 64 rows
-            v[0] += f0;
-            v[1] += f1;
-            f0 = f1 = 0.f;
-            cnt = 0;
-          }
-        }
-        v[0] += f0;
-        v[1] += f1;
+        run_sums(r0 + t % rows.RP, r1, rows.RP, v,
+                 [&](int r, float& a, float& b) { a = b = p.x[(int64_t)r * p.ldx + c]; });
       }
     cluster_sums<2>(sm, v, CW);
     const double mean = v[0] / rows.R;
@@ -144,9 +158,16 @@ __global__ void __launch_bounds__(kThreads) bn_forward_kernel(const Forward p, c
   }
   if (on) {
     const float g = p.gamma[c], b = p.beta[c];
-#pragma unroll 4
-    for (int r = slot; r < rows.R; r += nslots)
-      p.y[(int64_t)r * p.ldy + c] = __float2bfloat16_rn((p.x[(int64_t)r * p.ldx + c] - m) * rs * g + b);
+    for (int r = slot; r < rows.R; r += 8 * nslots) {
+      float a[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * nslots < rows.R) a[j] = p.x[(int64_t)(r + j * nslots) * p.ldx + c];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * nslots < rows.R)
+          p.y[(int64_t)(r + j * nslots) * p.ldy + c] = __float2bfloat16_rn((a[j] - m) * rs * g + b);
+    }
   }
   if (p.training) cl.sync();  // no CTA leaves while a peer may still write its slots
 }
@@ -187,21 +208,10 @@ __global__ void __launch_bounds__(kThreads) bn_backward_kernel(const Backward p,
     if (on)
       for (int t = slot; t < rows.runs; t += nslots) {
         const int r0 = t / rows.RP * rows.rpc, r1 = min(rows.R, r0 + rows.rpc);
-        float f0 = 0.f, f1 = 0.f;
-        int cnt = 0;
-        for (int r = r0 + t % rows.RP; r < r1; r += rows.RP) {
-          const float a = p.dy[(int64_t)r * p.lddy + c];
-          f0 += a;
-          f1 = fmaf(a, (p.x[(int64_t)r * p.ldx + c] - m) * rs, f1);
-          if (++cnt == 64) {
-            v[0] += f0;
-            v[1] += f1;
-            f0 = f1 = 0.f;
-            cnt = 0;
-          }
-        }
-        v[0] += f0;
-        v[1] += f1;
+        run_sums(r0 + t % rows.RP, r1, rows.RP, v, [&](int r, float& a, float& b) {
+          a = p.dy[(int64_t)r * p.lddy + c];
+          b = (p.x[(int64_t)r * p.ldx + c] - m) * rs;
+        });
       }
     cluster_sums<2>(sm, v, CW);
     sdy = (float)v[0];
@@ -214,31 +224,33 @@ __global__ void __launch_bounds__(kThreads) bn_backward_kernel(const Backward p,
   const float invR = 1.0f / (float)rows.R;
   double sum[2] = {0.0, 0.0};
   if (on) {
-    float f = 0.f;
-    int cnt = 0;
-#pragma unroll 4
-    for (int r = slot; r < rows.R; r += nslots) {
-      const float xv = p.x[(int64_t)r * p.ldx + c];
-      float g = p.dy[(int64_t)r * p.lddy + c];
-      if (p.gamma) {
-        if (p.training) {
-          const float xh = (xv - m) * rs;
-          g = ga * rs * (g - sdy * invR - xh * sdx * invR);
-        } else {
-          g = g * ga * rs;
+    for (int r = slot; r < rows.R; r += 8 * nslots) {
+      float xv[8], g[8], f = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * nslots < rows.R) {
+          xv[j] = p.x[(int64_t)(r + j * nslots) * p.ldx + c];
+          g[j] = p.dy[(int64_t)(r + j * nslots) * p.lddy + c];
         }
-      }
-      if (p.act) g *= act_grad_from_output(p.act, xv);
-      if (p.dz32) p.dz32[(int64_t)r * p.ldz + c] = g;
-      if (p.dz16) p.dz16[(int64_t)r * p.ldz + c] = __float2bfloat16_rn(g);
-      f += g;
-      if (++cnt == 64) {
-        sum[0] += f;
-        f = 0.f;
-        cnt = 0;
-      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (r + j * nslots < rows.R) {
+          if (p.gamma) {
+            if (p.training) {
+              const float xh = (xv[j] - m) * rs;
+              g[j] = ga * rs * (g[j] - sdy * invR - xh * sdx * invR);
+            } else {
+              g[j] = g[j] * ga * rs;
+            }
+          }
+          if (p.act) g[j] *= act_grad_from_output(p.act, xv[j]);
+          const int64_t o = (int64_t)(r + j * nslots) * p.ldz + c;
+          if (p.dz32) p.dz32[o] = g[j];
+          if (p.dz16) p.dz16[o] = __float2bfloat16_rn(g[j]);
+          f += g[j];
+        }
+      sum[0] += f;
     }
-    sum[0] += f;
   }
   if (p.dbias) {
     if (p.gamma) cl.sync();  // every CTA has read the first sums' slots

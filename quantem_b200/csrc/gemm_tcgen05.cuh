@@ -10,9 +10,11 @@
 // One CTA of 128 threads computes a 128 x BN tile:
 //   * warp 0, one lane: TMA producer.  Each k-block (64 bf16 = one 128-byte
 //     swizzle row) of A (128 x 64) and B (BN x 64) is copied by
-//     cp.async.bulk.tensor into a ring of 6-9 stages (about 190 KB) with the 128-byte
-//     swizzle; an mbarrier per stage counts the transaction bytes.  The ring's depth
-//     hides the copies' latency, which bounds the many products with few tiles.
+//     cp.async.bulk.tensor into a ring (160 to 200 KB) with the 128-byte swizzle; an mbarrier
+//     per stage counts the transaction bytes.  A stage holds 2 k-blocks, 5 of the narrow
+//     tiles: the products of the deep layers (K up to 9216 on one CTA per 16 columns) are
+//     bound by the turn-round of a stage (44 us with one k-block per stage, 36 with two, 30
+//     with five; the MMAs themselves take 16).
 //   * warp 1, one lane: MMA issuer.  tcgen05.mma.cta_group::1.kind::f16 with
 //     M = 128, N = BN, K = 16 (four per k-block), BF16 operands read from shared
 //     memory through matrix descriptors, FP32 accumulator in tensor memory
@@ -23,7 +25,10 @@
 //     with tcgen05.ld.32x32b, applies bias / ReLU and stores FP32 or BF16, or
 //     adds FP32 atomically (split-K).
 // Out-of-range rows / columns / k of the tile are zero-filled by TMA and masked
-// in the epilogue, so M, N, K need no padding.
+// in the epilogue, so M, N, K need no padding.  A K-major A of fewer than 128 rows is copied
+// in boxes of a_rows rows (a multiple of 8): the other rows of the tile hold whatever the
+// ring held, feed only accumulator rows that are not stored, and cost the copy engine nothing
+// (it takes about 2.4 ns per 128-byte row, the bound of the deep layers' products).
 //
 // Every mbarrier wait is bounded by the global timer; on expiry the CTA records
 // a status code, still drains what it issued, frees TMEM and returns.
@@ -59,8 +64,10 @@ template <int BN>
 struct Smem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = BN >= 128 ? 6 : (BN == 64 ? 8 : 9);
+  static constexpr int KBS = BN >= 64 ? 2 : 5;  // k-blocks per stage
+  static constexpr int BLOCK_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGE_BYTES = KBS * BLOCK_BYTES;
+  static constexpr int STAGES = (BN >= 128 ? 6 : (BN == 64 ? 8 : 10)) / KBS;
   static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;  // the smallest allocation
   static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
   static constexpr int BYTES = BAR_OFF + 256 + 1024;  // barriers + 1 KB alignment slack
@@ -77,24 +84,26 @@ __device__ __forceinline__ uint64_t global_ns() {
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
+// Barriers and tiles by shared-memory address: the copy and MMA loops run in one thread each, so
+// their own instructions are on the critical path of a long K.
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}\n"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
 // Wait for the phase with the given parity to complete; false after kWaitNs.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  if (mbar_try(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  for (int i = 0; i < 64; ++i)
+    if (mbar_try(bar, parity)) return true;
   const uint64_t t0 = global_ns();
   while (true) {
     for (int i = 0; i < 64; ++i)
@@ -102,11 +111,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (global_ns() - t0 > kWaitNs) return false;
   }
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+          dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -115,14 +124,14 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // Shared-memory matrix descriptor of an MN-major operand, 128-byte swizzle: k-rows of 64
 // values (128 bytes), 8-row groups 1024 bytes apart (SBO), the next 64 values one copied
 // box further (LBO).
-__device__ __forceinline__ uint64_t sdesc_mn128(const void* tile) {
-  const uint64_t addr = (smem_u32(tile) >> 4) & 0x3FFFull;
+__device__ __forceinline__ uint64_t sdesc_mn128(uint32_t tile) {
+  const uint64_t addr = (tile >> 4) & 0x3FFFull;
   return addr | (uint64_t(64 * BK * 2 >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of
 // 128 bytes, 8-row core groups 1024 bytes apart (SBO), descriptor version 1.
-__device__ __forceinline__ uint64_t sdesc_k128(const void* tile) {
-  const uint64_t addr = (smem_u32(tile) >> 4) & 0x3FFFull;
+__device__ __forceinline__ uint64_t sdesc_k128(uint32_t tile) {
+  const uint64_t addr = (tile >> 4) & 0x3FFFull;
   return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, major-ness of each.
@@ -140,9 +149,8 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -160,7 +168,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
-                        int N, int K, int kb_per_split, Epilogue epi, int* status) {
+                        int N, int K, int kb_per_split, int a_rows, Epilogue epi, int* status) {
   static_assert(!B_MN || BN % 64 == 0, "an MN-major tile is copied in boxes of 64 values");
   static_assert(BN == 16 || BN == 32 || BN == 64 || BN == 128, "BN: a multiple of 16");
   using L = Smem<BN>;
@@ -203,28 +211,38 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % STAGES;
-      const uint32_t ph = (i / STAGES) & 1;
-      if (!mbar_wait(&empty[s], ph ^ 1)) {
+    const uint32_t bytes = (A_MN ? L::A_BYTES : a_rows * BK * 2) + L::B_BYTES;
+    uint32_t sa = smem_u32(smem), bf = smem_u32(full), be = smem_u32(empty), ph = 1;
+    int s = 0;
+    for (int i = 0, k0 = kb0 * BK; i < nkb; i += L::KBS) {
+      if (!mbar_wait(be, ph)) {
         atomicExch(fail_flag, 1);
         break;
       }
-      uint8_t* sa = smem + s * L::STAGE_BYTES;
-      mbar_expect_tx(&full[s], L::STAGE_BYTES);
-      const int k0 = (kb0 + i) * BK;
-      if (A_MN) {  // boxes of 64 values x 64 k
+      const int n = min(L::KBS, nkb - i);
+      mbar_expect_tx(bf, n * bytes);
 #pragma unroll
-        for (int j = 0; j < BM; j += 64) tma_load_2d(sa + j * BK * 2, &tmA, &full[s], m0 + j, k0);
-      } else {
-        tma_load_2d(sa, &tmA, &full[s], k0, m0);
+      for (int u = 0; u < L::KBS; ++u, k0 += BK) {
+        if (u >= n) break;
+        const uint32_t ua = sa + u * L::BLOCK_BYTES, ub = ua + L::A_BYTES;
+        if (A_MN) {  // boxes of 64 values x 64 k
+#pragma unroll
+          for (int j = 0; j < BM; j += 64) tma_load_2d(ua + j * BK * 2, &tmA, bf, m0 + j, k0);
+        } else {
+          tma_load_2d(ua, &tmA, bf, k0, m0);
+        }
+        if (B_MN) {
+#pragma unroll
+          for (int j = 0; j < BN; j += 64) tma_load_2d(ub + j * BK * 2, &tmB, bf, n0 + j, k0);
+        } else {
+          tma_load_2d(ub, &tmB, bf, k0, n0);
+        }
       }
-      uint8_t* sb = sa + L::A_BYTES;
-      if (B_MN) {
-#pragma unroll
-        for (int j = 0; j < BN; j += 64) tma_load_2d(sb + j * BK * 2, &tmB, &full[s], n0 + j, k0);
-      } else {
-        tma_load_2d(sb, &tmB, &full[s], k0, n0);
+      sa += L::STAGE_BYTES, bf += 8, be += 8;
+      if (++s == STAGES) {
+        s = 0;
+        sa -= STAGES * L::STAGE_BYTES, bf -= STAGES * 8, be -= STAGES * 8;
+        ph ^= 1;
       }
     }
   } else if (warp == 1 && lane == 0) {
@@ -232,27 +250,39 @@ __global__ void __launch_bounds__(THREADS, 1)
     // step of K = 16 in descriptor units (16 bytes): 32 bytes along the swizzled row of a K-major
     // operand, 16 rows of 128 bytes of an MN-major one
     constexpr uint64_t astep = A_MN ? 128 : 2, bstep = B_MN ? 128 : 2;
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % STAGES;
-      const uint32_t ph = (i / STAGES) & 1;
-      if (!mbar_wait(&full[s], ph)) {
+    const uint32_t s0 = smem_u32(smem);
+    const uint64_t ad0 = A_MN ? sdesc_mn128(s0) : sdesc_k128(s0);
+    const uint64_t bd0 = B_MN ? sdesc_mn128(s0 + L::A_BYTES) : sdesc_k128(s0 + L::A_BYTES);
+    uint64_t ad = ad0, bd = bd0;
+    uint32_t bf = smem_u32(full), be = smem_u32(empty), ph = 0;
+    int s = 0;
+    for (int i = 0; i < nkb; i += L::KBS) {
+      if (!mbar_wait(bf, ph)) {
         atomicExch(fail_flag, 1);
         break;
       }
       tc_fence_after();
-      const uint8_t* sa = smem + s * L::STAGE_BYTES;
-      const uint64_t ad = A_MN ? sdesc_mn128(sa) : sdesc_k128(sa);
-      const uint64_t bd = B_MN ? sdesc_mn128(sa + L::A_BYTES) : sdesc_k128(sa + L::A_BYTES);
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k)
-        umma_bf16(tmem, ad + astep * k, bd + bstep * k, idesc, (i | k) != 0 ? 1u : 0u);
-      umma_commit(&empty[s]);
+      for (int u = 0; u < L::KBS; ++u) {
+        if (i + u >= nkb) break;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma_bf16(tmem, ad + u * (L::BLOCK_BYTES / 16) + astep * k, bd + u * (L::BLOCK_BYTES / 16) + bstep * k, idesc,
+                    (i | u | k) != 0 ? 1u : 0u);
+      }
+      umma_commit(be);
+      ad += L::STAGE_BYTES / 16, bd += L::STAGE_BYTES / 16, bf += 8, be += 8;
+      if (++s == STAGES) {
+        s = 0;
+        ad = ad0, bd = bd0, bf -= STAGES * 8, be -= STAGES * 8;
+        ph ^= 1;
+      }
     }
-    umma_commit(done);  // also after a failure: completes once every issued MMA has finished
+    umma_commit(smem_u32(done));  // also after a failure: completes once every issued MMA has finished
   }
   __syncwarp();
 
-  const bool ok = mbar_wait(done, 0);
+  const bool ok = mbar_wait(smem_u32(done), 0);
   tc_fence_after();
   if (!ok) atomicExch(fail_flag, 1);
   __syncthreads();
