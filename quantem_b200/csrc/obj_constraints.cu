@@ -304,6 +304,54 @@ __global__ void blur_pass_kernel(const float* __restrict__ in, float* __restrict
   }
 }
 
+// Both passes in one: a 32 x 32 tile and its halo of R = ntaps / 2 <= kBlurHalo elements in
+// shared memory, along the rows first, then along the columns, with the same sums as the two
+// passes.  Bound by reading and writing the object once (17 MB each way at 8 x 510 x 516 complex
+// values); the two passes, each output walking its taps through the L1 cache, took 84 us for 7
+// taps.  Longer kernels take the two passes: their tile would be mostly halo.
+constexpr int kBlurTile = 32, kBlurHalo = 16;
+template <int K>
+__global__ void __launch_bounds__(kThreads) blur_tile_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                             int Ho, int Wo, const float* __restrict__ taps,
+                                                             int ntaps) {
+  extern __shared__ float bsh[];
+  __shared__ float st[2 * kBlurHalo + 1];
+  const int R = ntaps / 2, side = kBlurTile + 2 * R, pitch = side * K;
+  float *tile = bsh, *mid = bsh + side * pitch;  // side x side, then 32 x side
+  for (int t = threadIdx.x; t < ntaps; t += kThreads) st[t] = taps[t];
+  const int64_t rowlen = (int64_t)Wo * K;
+  const float* src = in + (int64_t)blockIdx.z * Ho * rowlen;
+  float* dst = out + (int64_t)blockIdx.z * Ho * rowlen;
+  const int r0 = blockIdx.y * kBlurTile, c0 = blockIdx.x * kBlurTile;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kThreads / 32;
+  for (int i = w; i < side; i += nw) {
+    const int r = r0 + i - R;
+    for (int j = lane; j < pitch; j += 32) {
+      const int64_t ck = (int64_t)(c0 - R) * K + j;
+      tile[i * pitch + j] = r >= 0 && r < Ho && ck >= 0 && ck < rowlen ? src[r * rowlen + ck] : 0.f;
+    }
+  }
+  __syncthreads();
+  // out-of-range elements are 0 in the tile: a sum over all taps adds exact zeros
+  for (int i = w; i < kBlurTile; i += nw)
+    for (int j = lane; j < pitch; j += 32) {
+      float acc = 0.f;
+      for (int t = 0; t < ntaps; ++t) acc = fmaf(st[t], tile[(i + t) * pitch + j], acc);
+      mid[i * pitch + j] = acc;
+    }
+  __syncthreads();
+  for (int i = w; i < kBlurTile; i += nw) {
+    if (r0 + i >= Ho) break;
+    for (int j = lane; j < kBlurTile * K; j += 32) {
+      const int64_t ck = (int64_t)c0 * K + j;
+      if (ck >= rowlen) break;
+      float acc = 0.f;
+      for (int t = 0; t < ntaps; ++t) acc = fmaf(st[t], mid[i * pitch + j + t * K], acc);
+      dst[(r0 + i) * rowlen + ck] = acc;
+    }
+  }
+}
+
 // ------------------------------------------------------------- identical slices
 __global__ void slice_mean_kernel(const float* __restrict__ in, float* __restrict__ out, int S, int64_t plane) {
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < plane; p += (int64_t)gridDim.x * blockDim.x) {
@@ -371,11 +419,20 @@ __global__ void surface_sign_kernel(const float* __restrict__ obj, int S, int64_
   }
 }
 
+// A block marches a 32 x 8 tile through the slices: the phase and amplitude of the tile and its
+// one-element halo are evaluated once per slice into shared memory (two slices alternate), the
+// slice before stays in registers.  Bound by atan2 and hypot (1.33 per element and slice); one
+// evaluation per stencil point (7) took 95 us at 8 x 510 x 516.
+constexpr int kSoftX = 32, kSoftY = 8;
 template <int KIND>
-__global__ void soft_loss_kernel(const float* __restrict__ obj, int S, int Ho, int Wo, float wz, float wxy,
-                                 float wsurf, float* __restrict__ grad, double* work) {
+__global__ void __launch_bounds__(kThreads) soft_loss_kernel(const float* __restrict__ obj, int S, int Ho, int Wo,
+                                                             float wz, float wxy, float wsurf,
+                                                             float* __restrict__ grad, double* work) {
+  static_assert(kThreads == kSoftX * kSoftY, "one thread per tile element");
+  constexpr int PX = kSoftX + 2, PY = kSoftY + 2;
   __shared__ double red[32];
-  const int64_t hw = (int64_t)Ho * Wo, n = (int64_t)S * hw;
+  __shared__ float2 val[2][PY][PX];  // (phase or potential, amplitude)
+  const int64_t hw = (int64_t)Ho * Wo;
   const bool surf = wsurf > 0.f && S >= 3;
   float m0 = 0.f, m1 = 0.f, sg0 = 0.f, sg1 = 0.f;
   if (surf && KIND != 2) {
@@ -395,66 +452,94 @@ __global__ void soft_loss_kernel(const float* __restrict__ obj, int S, int Ho, i
   const float c1 = nd && wxy > 0.f ? wxy / (nd * (float)((int64_t)S * (Ho - 1) * Wo)) : 0.f;
   const float c2 = nd && wxy > 0.f ? wxy / (nd * (float)((int64_t)S * Ho * (Wo - 1))) : 0.f;
   const bool amp_terms = KIND == 0;
+  const int tx = threadIdx.x % kSoftX, ty = threadIdx.x / kSoftX;
+  const int tiles_x = (Wo + kSoftX - 1) / kSoftX, tiles = tiles_x * ((Ho + kSoftY - 1) / kSoftY);
   double lacc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(i / hw);
-    const int64_t p = i % hw;
-    const int r = (int)(p / Wo), c = (int)(p % Wo);
-    float ph, amp;
-    values_at<KIND>(obj, i, ph, amp);
-    float gph = 0.f, gamp = 0.f;
-    // one stencil step per weighted dimension: the loss term of the diff to the next element,
-    // the gradient from the diffs on both sides
-    auto tv_dim = [&](float cw, bool has_lo, int64_t lo, bool has_hi, int64_t hi) {
-      if (cw == 0.f) return;
-      float q, qa;
-      if (has_hi) {
-        values_at<KIND>(obj, hi, q, qa);
-        const float d = q - ph;
-        lacc += (double)(cw * fabsf(d));
-        gph -= cw * sgnf(d);
-        if (amp_terms) {
-          const float da = qa - amp;
-          lacc += (double)(cw * fabsf(da));
-          gamp -= cw * sgnf(da);
-        }
-      }
-      if (has_lo) {
-        values_at<KIND>(obj, lo, q, qa);
-        gph += cw * sgnf(ph - q);
-        if (amp_terms) gamp += cw * sgnf(amp - qa);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int rb = tile / tiles_x * kSoftY, cb = tile % tiles_x * kSoftX;
+    const int r = rb + ty, c = cb + tx;
+    const bool on = r < Ho && c < Wo;
+    auto fill = [&](int s) {
+      float2(*v)[PX] = val[s & 1];
+      for (int i = threadIdx.x; i < PY * PX; i += kThreads) {
+        const int y = i / PX, x = i % PX, rr = rb + y - 1, cc = cb + x - 1;
+        if (rr < 0 || rr >= Ho || cc < 0 || cc >= Wo) continue;
+        if ((y == 0 || y == PY - 1) && (x == 0 || x == PX - 1)) continue;  // corners are not read
+        float ph, amp;
+        values_at<KIND>(obj, s * hw + (int64_t)rr * Wo + cc, ph, amp);
+        v[y][x] = make_float2(ph, amp);
       }
     };
-    tv_dim(c0, s > 0, i - hw, s < S - 1, i + hw);
-    tv_dim(c1, r > 0, i - Wo, r < Ho - 1, i + Wo);
-    tv_dim(c2, c > 0, i - 1, c < Wo - 1, i + 1);
-    if (surf && (s == 0 || s == S - 1)) {
-      const float inv = 1.0f / (float)hw;
-      if (KIND == 2) {
-        lacc += (double)(wsurf * fabsf(ph) * inv);
-        gph += wsurf * sgnf(ph) * inv;
-      } else {
-        const float m = s == 0 ? m0 : m1, sgm = s == 0 ? sg0 : sg1;
-        const float u = fabsf(ph) - m;
-        lacc += (double)(wsurf * fabsf(u) * inv);
-        gph += wsurf * (sgnf(u) - sgm) * inv * sgnf(ph);
-        if (amp_terms) {
-          lacc += (double)(wsurf * (1.0f - amp) * inv);
-          gamp -= wsurf * inv;
+    __syncthreads();  // the last tile's values are read
+    fill(0);
+    float2 before = make_float2(0.f, 0.f);
+    for (int s = 0; s < S; ++s) {
+      __syncthreads();  // slice s is in place and slice s - 1 no longer read
+      if (s + 1 < S) fill(s + 1);
+      const float2(*v)[PX] = val[s & 1];
+      const float2 here = v[ty + 1][tx + 1];
+      float2 after = here;
+      // the own element of the next slice: this thread may not have filled it
+      if (s + 1 < S) {
+        __syncthreads();
+        after = val[(s + 1) & 1][ty + 1][tx + 1];
+      }
+      if (on) {
+        const int64_t i = s * hw + (int64_t)r * Wo + c;
+        const float ph = here.x, amp = here.y;
+        float gph = 0.f, gamp = 0.f;
+        // one stencil step per weighted dimension: the loss term of the diff to the next element,
+        // the gradient from the diffs on both sides
+        auto tv_dim = [&](float cw, bool has_lo, float2 lo, bool has_hi, float2 hi) {
+          if (cw == 0.f) return;
+          if (has_hi) {
+            const float d = hi.x - ph;
+            lacc += (double)(cw * fabsf(d));
+            gph -= cw * sgnf(d);
+            if (amp_terms) {
+              const float da = hi.y - amp;
+              lacc += (double)(cw * fabsf(da));
+              gamp -= cw * sgnf(da);
+            }
+          }
+          if (has_lo) {
+            gph += cw * sgnf(ph - lo.x);
+            if (amp_terms) gamp += cw * sgnf(amp - lo.y);
+          }
+        };
+        tv_dim(c0, s > 0, before, s < S - 1, after);
+        tv_dim(c1, r > 0, v[ty][tx + 1], r < Ho - 1, v[ty + 2][tx + 1]);
+        tv_dim(c2, c > 0, v[ty + 1][tx], c < Wo - 1, v[ty + 1][tx + 2]);
+        if (surf && (s == 0 || s == S - 1)) {
+          const float inv = 1.0f / (float)hw;
+          if (KIND == 2) {
+            lacc += (double)(wsurf * fabsf(ph) * inv);
+            gph += wsurf * sgnf(ph) * inv;
+          } else {
+            const float m = s == 0 ? m0 : m1, sgm = s == 0 ? sg0 : sg1;
+            const float u = fabsf(ph) - m;
+            lacc += (double)(wsurf * fabsf(u) * inv);
+            gph += wsurf * (sgnf(u) - sgm) * inv * sgnf(ph);
+            if (amp_terms) {
+              lacc += (double)(wsurf * (1.0f - amp) * inv);
+              gamp -= wsurf * inv;
+            }
+          }
+        }
+        if (KIND == 2) {
+          grad[i] = gph;
+        } else {
+          const float2 o = reinterpret_cast<const float2*>(obj)[i];
+          float2 gz = make_float2(0.f, 0.f);
+          if (amp != 0.f) {  // G = g_amp z / |z| + i g_phase z / |z|^2 (zero at a zero pixel)
+            const float inv = 1.0f / amp;
+            gz.x = gamp * o.x * inv - gph * o.y * inv * inv;
+            gz.y = gamp * o.y * inv + gph * o.x * inv * inv;
+          }
+          reinterpret_cast<float2*>(grad)[i] = gz;
         }
       }
-    }
-    if (KIND == 2) {
-      grad[i] = gph;
-    } else {
-      const float2 o = reinterpret_cast<const float2*>(obj)[i];
-      float2 gz = make_float2(0.f, 0.f);
-      if (amp != 0.f) {  // G = g_amp z / |z| + i g_phase z / |z|^2 (zero at a zero pixel)
-        const float inv = 1.0f / amp;
-        gz.x = gamp * o.x * inv - gph * o.y * inv * inv;
-        gz.y = gamp * o.y * inv + gph * o.x * inv * inv;
-      }
-      reinterpret_cast<float2*>(grad)[i] = gz;
+      before = here;
     }
   }
   const double t = block_sum_d(lacc, red);
@@ -737,6 +822,22 @@ int ptycho_obj_blur(const void* in, void* out, void* tmp, int S, int Ho, int Wo,
   if (tmp == in || tmp == out) return qb_record_error(PTYCHO_ERR_INVALID, "obj_blur: tmp aliases in or out");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int K = is_complex ? 2 : 1;
+  if (ntaps / 2 <= kBlurHalo && S <= 65535 && in != out) {
+    const int side = kBlurTile + ntaps - 1;
+    const size_t smem = sizeof(float) * (size_t)(side + kBlurTile) * side * K;
+    const dim3 grid((Wo + kBlurTile - 1) / kBlurTile, (Ho + kBlurTile - 1) / kBlurTile, S);
+    if (grid.y <= 65535) {
+      if (is_complex) {
+        cudaFuncSetAttribute(blur_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        blur_tile_kernel<2><<<grid, kThreads, smem, st>>>(static_cast<const float*>(in), static_cast<float*>(out), Ho,
+                                                          Wo, taps, ntaps);
+      } else {
+        blur_tile_kernel<1><<<grid, kThreads, smem, st>>>(static_cast<const float*>(in), static_cast<float*>(out), Ho,
+                                                          Wo, taps, ntaps);
+      }
+      return check("blur_tile_kernel");
+    }
+  }
   blur_pass_kernel<0><<<4 * kBlocks, kThreads, 0, st>>>(static_cast<const float*>(in), static_cast<float*>(tmp), S, Ho,
                                                         Wo, K, taps, ntaps);
   blur_pass_kernel<1><<<4 * kBlocks, kThreads, 0, st>>>(static_cast<const float*>(tmp), static_cast<float*>(out), S,
