@@ -593,7 +593,7 @@ __device__ float2 sampled_mean(const float* in, int64_t hw, float2* red) {
 // Rows: a = row transforms of (in - c) (INV = false; c kept in base), or out = inverse row
 // transforms of a, plus c (INV = true).
 template <bool REAL, bool INV>
-__global__ void __launch_bounds__(kLineThreads)
+__global__ void __launch_bounds__(kLineThreads, 2)
     butter_rows_kernel(const float* __restrict__ in, float2* __restrict__ a, float* __restrict__ out,
                        float2* __restrict__ base, const qb::LinePlan p, int S, int H, int lg, int LP) {
   extern __shared__ float2 sh[];
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kLineThreads)
 
 // Columns of the row spectra, in place: forward, times the envelope (1 at DC) and the
 // normalisation, inverse.
-__global__ void __launch_bounds__(kLineThreads)
+__global__ void __launch_bounds__(kLineThreads, 2)
     butter_cols_kernel(float2* __restrict__ a, const float* __restrict__ env, const qb::LinePlan p, int S, int W,
                        int lg, int LP) {
   extern __shared__ float2 sh[];
