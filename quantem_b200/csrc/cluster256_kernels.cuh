@@ -294,8 +294,8 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
           float* oi = p.out_intensity ? p.out_intensity + (size_t)b * NN + dbase : nullptr;
           double loss_acc = 0.0;
           int nonfinite = 0;
-#pragma unroll
-          for (int i = 0; i < E; ++i) {
+#pragma unroll 4
+          for (int i = 0; i < E; ++i) {  // rolled: the code of the transforms stays in the instruction caches
             const int doff = ((i >> 3) + 32 * (((i & 7) + 4) & 7)) * N;
             const float I = inten[i * T + tid];
             if (!isfinite(I)) ++nonfinite;

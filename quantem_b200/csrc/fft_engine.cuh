@@ -385,6 +385,7 @@ struct Fft2 {
 #pragma unroll
       for (int kC = 0; kC < C; ++kC) x[kB * C + kC] = sm[mn_2 + N * kC + A * kB];
   }
+  __device__ __forceinline__ int s3_slot(int g, int e) const { return mn_3 + CS * e + (T / 32 / (N / 32)) * N * g; }
   // S3 layout (g, e): rD = e, kC = kC_g, column s3_c
   __device__ __forceinline__ void read_s3(const float2* sm, float2 (&x)[E]) const {
 #pragma unroll

@@ -358,7 +358,7 @@ __device__ __forceinline__ void descan_mul(const Fft2<N>& f, float2 (&x)[Fft2<N>
 // Fourier-space probe-gradient partial (S3 layout): pg += conj(ramp) * x, batched RMW.
 template <int N>
 __device__ __forceinline__ void accumulate_probe_grad(const Fft2<N>& f, const float2 (&x)[Fft2<N>::E], float2* pg,
-                                                      const float2* rowf, const float2* colf) {
+                                                      const float2* rowf, const float2* colf, bool first = false) {
   constexpr int D = Fft2<N>::D, G3 = Fft2<N>::G3;
   constexpr int BT = D < 8 ? D : 8;  // batch of read-modify-writes within one D-point group
   static_assert(D % BT == 0, "batch must divide the group");
@@ -368,7 +368,8 @@ __device__ __forceinline__ void accumulate_probe_grad(const Fft2<N>& f, const fl
     for (int e0 = 0; e0 < D; e0 += BT) {
       float2 old[BT];
 #pragma unroll
-      for (int j = 0; j < BT; ++j) old[j] = pg[(size_t)f.s3_row(g, e0 + j) * N + f.s3_c];
+      for (int j = 0; j < BT; ++j)
+        old[j] = first ? make_float2(0.f, 0.f) : pg[(size_t)f.s3_row(g, e0 + j) * N + f.s3_c];
 #pragma unroll
       for (int j = 0; j < BT; ++j) {
         const int kr = f.s3_row(g, e0 + j), kc = f.s3_c;
@@ -439,14 +440,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   // (e / 2) * T + tid, half e % 2.
   float2* inten2 = reinterpret_cast<float2*>(inten);
   float2* pgrad = ADJ ? p.probe_grad_part + (size_t)cta * (size_t)P * NN : nullptr;
-  if (ADJ) {
-    for (int m = 0; m < P; ++m)
-#pragma unroll
-      for (int g = 0; g < G3; ++g)
-#pragma unroll
-        for (int e = 0; e < D; ++e)
-          pgrad[(size_t)m * NN + (size_t)f.s3_row(g, e) * N + f.s3_c] = make_float2(0.f, 0.f);
-  }
+  bool first_position = true;  // its probe gradient is written, the others' are added
   // loss and non-finite counts live in shared memory between positions (warp w owns
   // entry w), so the transforms do not carry them in registers
   if ((tid & 31) == 0) {
@@ -645,7 +639,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
             float2* pg = pgrad + (size_t)m * NN + (size_t)f.s1_row(e0 / A) * N;
             float2 old[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) old[j] = pg[f.s1_col(e0 / A, e0 % A + j)];
+            for (int j = 0; j < 8; ++j) old[j] = first_position ? make_float2(0.f, 0.f) : pg[f.s1_col(e0 / A, e0 % A + j)];
 #pragma unroll
             for (int j = 0; j < 8; ++j) pg[f.s1_col(e0 / A, e0 % A + j)] = cadd(old[j], x[e0 + j]);
           }
@@ -671,11 +665,16 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         }
 #pragma unroll
         for (int e = 0; e < E; ++e) x[e] = cscale(x[e], inv_n);  // orthonormal detector FFT
-        if (ADJ) {
+        // The last mode's far field goes straight through the loss and seeds the reverse chain
+        // (which runs the last mode first): it is neither stored in scratch nor summed into the
+        // tile.  The analytic update stores every mode's.
+        const bool last = !AN && m == P - 1;
+        if (ADJ && !last) {
           float2* fw = slot + (size_t)(P * S + m) * NN;
           store_pairs<E, T>(fw, tid, x);
         }
-        if (!ADJ && p.tile_out) {
+        if (last) {
+        } else if (!ADJ && p.tile_out) {
           float* oi = p.out_intensity + (size_t)b * NN;
 #pragma unroll
           for (int g = 0; g < G3; ++g)
@@ -706,36 +705,46 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
           load_probe(m);
           continue;
         }
-        // loss over the mode-summed intensity (each thread owns its S3 slots)
+        // Loss over the mode-summed intensity (each thread owns its S3 slots).  The last mode's
+        // far field waits in this thread's elements of the exchange buffer, so that the loop
+        // needs neither the wave's registers nor full unrolling: with 16 to 48 copies of the five
+        // losses in it, the code of the transforms did not stay in the instruction caches (six
+        // single-mode datasets: 15.2 -> 12.8 ms with the far field's round trip gone too).  The
+        // other per-mode steps lose as rolled loops (24.2 -> 24.9 ms per 4096-position launch):
+        // they are chains of loads.
         {
           const float* tg = p.targets + (size_t)gi * NN;
           double loss_acc = 0.0;
           int nonfinite = 0;
-#pragma unroll
-          for (int g = 0; g < G3; ++g)
-#pragma unroll
-            for (int e = 0; e < D; ++e) {
-              const int di = detector_index<N>(f.s3_row(g, e), f.s3_c);
-              const int li = 2 * (((g * D + e) >> 1) * T + tid) + ((g * D + e) & 1);
-              const float I = !ADJ && p.tile_out ? p.out_intensity[(size_t)b * NN + di] : inten[li];
-              if (!isfinite(I)) ++nonfinite;
-              float dldi;
-              const float tv = __ldcs(tg + di);  // targets stream through L2 once per iteration
-              loss_elem<N>(p, I, tv, __ldg(p.mask + di), loss_acc, dldi);
-              if (ADJ && AN) {
-                // factor f and additive fix of the Fourier projection seed
-                if (P == 1) {
-                  dldi = I > 0.f ? tv / sqrtf(I) : 0.f;   // t exp(i angle(Psi)) = Psi t / |Psi|
-                  tile2[li] = I > 0.f ? 0.f : tv;        // angle(0) = 0
-                } else {
-                  const float A = sqrtf(tile2[li]);
-                  dldi = A > 0.f ? tv / A : 0.f;         // zero estimate -> infinity -> factor 0
-                  tile2[li] = 0.f;
-                }
+          if (!AN) f.write_s3(sm, x);
+#pragma unroll 4
+          for (int i = 0; i < E; ++i) {
+            const int g = i / D, e = i % D;
+            const int di = detector_index<N>(f.s3_row(g, e), f.s3_c);
+            const int li = 2 * ((i >> 1) * T + tid) + (i & 1);
+            float2* xs = sm + f.s3_slot(g, e);
+            const float tv = __ldcs(tg + di);  // targets stream through L2 once per iteration
+            float I = 0.f;
+            if (AN || P > 1) I = !ADJ && p.tile_out ? p.out_intensity[(size_t)b * NN + di] : inten[li];
+            if (!AN) I += cabs2(*xs);
+            if (!isfinite(I)) ++nonfinite;
+            float dldi;
+            loss_elem<N>(p, I, tv, __ldg(p.mask + di), loss_acc, dldi);
+            if (ADJ && AN) {
+              // factor f and additive fix of the Fourier projection seed
+              if (P == 1) {
+                dldi = I > 0.f ? tv / sqrtf(I) : 0.f;   // t exp(i angle(Psi)) = Psi t / |Psi|
+                tile2[li] = I > 0.f ? 0.f : tv;        // angle(0) = 0
+              } else {
+                const float est = sqrtf(tile2[li]);
+                dldi = est > 0.f ? tv / est : 0.f;     // zero estimate -> infinity -> factor 0
+                tile2[li] = 0.f;
               }
-              if (ADJ) inten[li] = dldi;
-              if (p.out_intensity && !(!ADJ && p.tile_out)) p.out_intensity[(size_t)b * NN + di] = I;
             }
+            if (ADJ && (AN || P > 1)) inten[li] = dldi;
+            if (ADJ && !AN) *xs = make_float2(xs->x * 2.0f * dldi, xs->y * 2.0f * dldi);  // seed of the last mode
+            if (p.out_intensity) p.out_intensity[(size_t)b * NN + di] = I;
+          }
           for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
           const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
           if ((tid & 31) == 0) {
@@ -746,9 +755,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         if (!ADJ) break;
         bwd = true;
         first_bwd = true;
-        m = P - 1;  // last mode first: its far field and deepest waves are the most recent in L2
+        m = P - 1;  // last mode first: its far field is at hand, its deepest waves are recent in L2
         s = S - 1;
-        load_far_seed(m);
+        if (AN)
+          load_far_seed(m);
+        else
+          f.read_s3(sm, x);
         continue;
       }
       first_bwd = false;
@@ -785,7 +797,7 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         --s;
         continue;
       }
-      accumulate_probe_grad<N>(f, x, pgrad + (size_t)m * NN, rowf, colf);
+      accumulate_probe_grad<N>(f, x, pgrad + (size_t)m * NN, rowf, colf, first_position);
       if (EXT && p.grad_positions) {
         // positions enter through the probe shift Y = probe_hat * ramp(frac) only; x = N^2 dL/dY
         // here, so dL/dfrac = (2 pi / N^2) sum_k fftfreq(k) Im(conj(x_k) Y_k), summed over the modes
@@ -834,6 +846,12 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
       }
       break;
     }
+    first_position = false;
+  }
+  if (ADJ && first_position) {  // no (valid) position: the partials are zero
+    for (int m = 0; m < P; ++m)
+#pragma unroll
+      for (int e = 0; e < E; ++e) pgrad[(size_t)m * NN + (size_t)e * T + tid] = make_float2(0.f, 0.f);
   }
 
   // ------------------------------ loss reduction ------------------------------
