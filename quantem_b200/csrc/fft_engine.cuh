@@ -28,7 +28,7 @@
 // wavefronts per 256 bytes, the minimum for 8-byte words.
 //
 // The load/store unit's data pipe is the busiest unit of the batch kernels (58 % at 128^2
-// against 47 % of the FP32 pipe and 37 % of the issue slots), so the factorisation is
+// against 50 % of the FP32 pipe and 38 % of the issue slots), so the factorisation is
 // chosen for the real-space accesses: B = 8 puts 8 consecutive columns x 4 rows in a warp
 // access of the object (B = 4: 4 columns x 8 rows took 3.7 L1 wavefronts per gather and
 // 4.6 per gradient scatter, B = 8 takes 1.7 and 2.3: 28.5 -> 26.4 ms per 4096-position

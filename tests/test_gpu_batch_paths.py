@@ -86,3 +86,24 @@ def test_many_ctas_match_one_position_at_a_time(n, B):
     assert abs(loss - l2) < 1e-6 * abs(l2)
     assert rel(go, go2.cpu().numpy()) < 4e-7 * max(4.0, B ** 0.5)
     assert rel(gp, gp2.cpu().numpy()) < 4e-7 * max(4.0, B ** 0.5)
+
+
+@pytest.mark.parametrize("n,P", [(64, 1), (64, 3), (96, 2), (128, 1), (128, 2)])
+def test_blocks_without_a_valid_first_position(n, P):
+    """Three blocks of two positions: the second has only invalid indices (its probe-gradient
+    partial must still be zero, whatever the workspace held), the third starts with one (its
+    second position is then the one that writes the partial).  Against the valid positions alone,
+    one by one: sums of three float32 terms, as above."""
+    obj, probe, prop, pos, targets = _problem(n, 2, P, 6, n + 20, n + 23, seed=P)
+    mask = torch.ones((n, n), device="cuda")
+    torch.full((1 << 26,), float("nan"), device="cuda")  # what a fresh workspace may hold
+    idx = torch.tensor([0, 1, 6, -1, 7, 5], device="cuda")
+    loss, go, gp = ops.batch_forward_adjoint(obj, probe, prop, pos, idx, targets, mask, 6, 100.0, grid=3)
+    assert ops.read_status(obj.device)["invalid_indices"] == 3
+    l2, go2, gp2 = 0.0, 0, 0
+    for b in (0, 1, 5):
+        l, g, q = ops.batch_forward_adjoint(obj, probe, prop, pos, idx.new_tensor([b]), targets, mask, 6, 100.0)
+        l2, go2, gp2 = l2 + float(l) / 6, go2 + g.to(torch.complex128) / 6, gp2 + q.to(torch.complex128) / 6
+    assert abs(float(loss) - l2) < 1e-6 * abs(l2)
+    assert rel(go.cpu().numpy(), go2.cpu().numpy()) < 1.6e-6
+    assert rel(gp.cpu().numpy(), gp2.cpu().numpy()) < 1.6e-6
