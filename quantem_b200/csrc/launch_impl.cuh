@@ -67,6 +67,14 @@ BatchParams batch_params(const ptycho_batch_args* a, bool tile = true, bool tile
   return p;
 }
 
+// Dynamic shared memory that a batch kernel may be launched with: one bound for all of its calls,
+// whatever the call at hand takes.  The attribute belongs to the device, so a bound of each call's
+// own size could be lowered by another host thread before the launch.
+template <typename K>
+bool allow_smem(K kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) == cudaSuccess;
+}
+
 // the serial kernel with its optional extensions compiled in (descan, position / descan /
 // propagator gradients)
 inline bool wants_ext(const ptycho_batch_args* a) {
@@ -74,13 +82,13 @@ inline bool wants_ext(const ptycho_batch_args* a) {
 }
 
 template <int N, bool ADJ>
-void launch_ext(const BatchParams& p, int grid, size_t smem, cudaStream_t st) {
-  cudaFuncSetAttribute(fused_batch_kernel<N, ADJ, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+int launch_ext(const BatchParams& p, int grid, size_t smem, cudaStream_t st) {
+  if (!allow_smem(fused_batch_kernel<N, ADJ, false, true>)) return PTYCHO_ERR_CUDA;
   if (ADJ)
     cudaFuncSetAttribute(fused_batch_kernel<N, ADJ, false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          carveout<N>(smem));
   fused_batch_kernel<N, ADJ, false, true><<<grid, Fft2<N>::T, smem, st>>>(p);
+  return PTYCHO_OK;
 }
 
 // One CTA per position, modes in sequence.  The attributes are per device; setting them on
@@ -93,12 +101,12 @@ int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
   const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
   const size_t smem = batch_smem<N>(a, tile);
   if (adj) {
-    cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!allow_smem(fused_batch_kernel<N, true>)) return PTYCHO_ERR_CUDA;
     cudaFuncSetAttribute(fused_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          carveout<N>(smem));
     fused_batch_kernel<N, true><<<a->grid, Fft2<N>::T, smem, st>>>(p);
   } else {
-    cudaFuncSetAttribute(fused_batch_kernel<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!allow_smem(fused_batch_kernel<N, false>)) return PTYCHO_ERR_CUDA;
     fused_batch_kernel<N, false><<<a->grid, Fft2<N>::T, smem, st>>>(p);
   }
   return cudaPeekAtLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
@@ -111,12 +119,10 @@ int launch_special(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
   const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
   const size_t smem = batch_smem<N>(a, tile);
   if (!a->analytic) {
-    if (adj)
-      launch_ext<N, true>(p, a->grid, smem, st);
-    else
-      launch_ext<N, false>(p, a->grid, smem, st);
+    const int rc = adj ? launch_ext<N, true>(p, a->grid, smem, st) : launch_ext<N, false>(p, a->grid, smem, st);
+    if (rc) return rc;
   } else {
-    cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!allow_smem(fused_batch_kernel<N, true, true>)) return PTYCHO_ERR_CUDA;
     cudaFuncSetAttribute(fused_batch_kernel<N, true, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          carveout<N>(smem));
     fused_batch_kernel<N, true, true><<<a->grid, Fft2<N>::T, smem, st>>>(p);
@@ -144,7 +150,7 @@ int launch_multi(const ptycho_batch_args* sets, int nsets, cudaStream_t st) {
     const size_t sd = batch_smem<N>(&sets[d], false);
     if (sd > smem) smem = sd;
   }
-  cudaFuncSetAttribute(multi_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (!allow_smem(multi_batch_kernel<N, true>)) return PTYCHO_ERR_CUDA;
   cudaFuncSetAttribute(multi_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                        carveout<N>(smem));
   multi_batch_kernel<N, true><<<mp.begin[nsets], Fft2<N>::T, smem, st>>>(mp);
@@ -174,15 +180,13 @@ int max_clusters(const ptycho_batch_args* a, bool adj) {
   int n = 0;
   cudaError_t e;
   if (adj) {
-    cudaFuncSetAttribute(cluster_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)batch_smem<N>(a));
+    e = allow_smem(cluster_batch_kernel<N, true>) ? cudaSuccess : cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = cluster_config<N, true>(a, a->P, nullptr, attr);
-    e = cudaOccupancyMaxActiveClusters(&n, cluster_batch_kernel<N, true>, &cfg);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, cluster_batch_kernel<N, true>, &cfg);
   } else {
-    cudaFuncSetAttribute(cluster_batch_kernel<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)batch_smem<N>(a));
+    e = allow_smem(cluster_batch_kernel<N, false>) ? cudaSuccess : cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = cluster_config<N, false>(a, a->P, nullptr, attr);
-    e = cudaOccupancyMaxActiveClusters(&n, cluster_batch_kernel<N, false>, &cfg);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, cluster_batch_kernel<N, false>, &cfg);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -197,15 +201,13 @@ int launch_cluster(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
   cudaError_t e;
   if (adj) {
-    cudaFuncSetAttribute(cluster_batch_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)batch_smem<N>(a));
+    if (!allow_smem(cluster_batch_kernel<N, true>)) return PTYCHO_ERR_CUDA;
     cudaFuncSetAttribute(cluster_batch_kernel<N, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)((batch_smem<N>(a) + 1024) * 100 / (228 * 1024) + 1));
     cudaLaunchConfig_t cfg = cluster_config<N, true>(a, a->grid, st, attr);
     e = cudaLaunchKernelEx(&cfg, cluster_batch_kernel<N, true>, p);
   } else {
-    cudaFuncSetAttribute(cluster_batch_kernel<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)batch_smem<N>(a));
+    if (!allow_smem(cluster_batch_kernel<N, false>)) return PTYCHO_ERR_CUDA;
     cudaLaunchConfig_t cfg = cluster_config<N, false>(a, a->grid, st, attr);
     e = cudaLaunchKernelEx(&cfg, cluster_batch_kernel<N, false>, p);
   }

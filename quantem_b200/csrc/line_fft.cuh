@@ -194,11 +194,12 @@ __device__ float2* line_dft(float2* x, float2* y, const float2* tw, const LinePl
 // per SM, or once where that leaves fewer than four lines.
 inline int line_pitch(int lg) { return lg > 0 ? (1 << lg) + 1 : 1; }
 inline size_t line_smem(int n, int lg) { return sizeof(float2) * ((size_t)2 * n * line_pitch(lg) + n); }
+constexpr size_t kLineSmem = 225 * 1024;  // of one block: the longest line (6144) takes 144 KB
 inline int line_log2(int n) {
   for (int lg = 3; lg >= 2; --lg)
     if (line_smem(n, lg) <= 112 * 1024) return lg;
   for (int lg = 3; lg > 0; --lg)
-    if (line_smem(n, lg) <= 225 * 1024) return lg;
+    if (line_smem(n, lg) <= kLineSmem) return lg;
   return 0;
 }
 

@@ -310,6 +310,8 @@ __global__ void blur_pass_kernel(const float* __restrict__ in, float* __restrict
 // values); the two passes, each output walking its taps through the L1 cache, took 84 us for 7
 // taps.  Longer kernels take the two passes: their tile would be mostly halo.
 constexpr int kBlurTile = 32, kBlurHalo = 16;
+// dynamic shared memory with the longest taps, complex values
+constexpr size_t kBlurSmem = sizeof(float) * 2 * (2 * kBlurTile + 2 * kBlurHalo) * (kBlurTile + 2 * kBlurHalo);
 template <int K>
 __global__ void __launch_bounds__(kThreads) blur_tile_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                              int Ho, int Wo, const float* __restrict__ taps,
@@ -554,6 +556,16 @@ __global__ void loss_from_partials_kernel(const double* __restrict__ part, float
 int check(const char* what);
 int grid_for(int64_t n);
 
+// Dynamic shared memory that a kernel may be launched with: one bound for all of its calls.  The
+// attribute belongs to the device, so a bound of each call's own size could be lowered by another
+// host thread before the launch.
+template <typename K>
+int allow_smem(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess
+             ? PTYCHO_OK
+             : check("shared memory bound");
+}
+
 // ---------------------------------------------------------------- Butterworth filter
 // object_models.py:481-520: per slice, mean removed, ifft2(fft2(x) env), mean added back.
 // The mean is the DC term, so the filter is ifft2(fft2(x - c) env') + c with env' = env but 1
@@ -694,9 +706,9 @@ int butterworth(const float* in, float* out, int S, int H, int W, const float* e
   const qb::LinePlan pr = qb::line_plan(W), pc = qb::line_plan(H);
   const int lr = qb::line_log2(W), lc = qb::line_log2(H);
   const size_t sr = qb::line_smem(W, lr), sc = qb::line_smem(H, lc);
-  cudaFuncSetAttribute(butter_rows_kernel<REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
-  cudaFuncSetAttribute(butter_rows_kernel<REAL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
-  cudaFuncSetAttribute(butter_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc);
+  if (int rc = allow_smem(butter_rows_kernel<REAL, false>, qb::kLineSmem)) return rc;
+  if (int rc = allow_smem(butter_rows_kernel<REAL, true>, qb::kLineSmem)) return rc;
+  if (int rc = allow_smem(butter_cols_kernel, qb::kLineSmem)) return rc;
   // two blocks per SM, evened out over the rounds
   auto grid = [](int64_t groups) {
     const int64_t rounds = (groups + kBlocks - 1) / kBlocks;
@@ -834,7 +846,7 @@ int ptycho_obj_blur(const void* in, void* out, void* tmp, int S, int Ho, int Wo,
     const dim3 grid((Wo + kBlurTile - 1) / kBlurTile, (Ho + kBlurTile - 1) / kBlurTile, S);
     if (grid.y <= 65535) {
       if (is_complex) {
-        cudaFuncSetAttribute(blur_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (int rc = allow_smem(blur_tile_kernel<2>, kBlurSmem)) return rc;
         blur_tile_kernel<2><<<grid, kThreads, smem, st>>>(static_cast<const float*>(in), static_cast<float*>(out), Ho,
                                                           Wo, taps, ntaps);
       } else {

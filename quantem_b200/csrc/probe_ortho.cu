@@ -334,10 +334,12 @@ cudaError_t launch_cluster(K kernel, int ctas, size_t smem, cudaStream_t st, A..
 }
 
 // 16 CTAs (a non-portable cluster size) if the device can hold such a cluster with this much
-// shared memory, else 8.
+// shared memory, else 8.  The kernel's shared-memory bound is the same in every call: it belongs
+// to the device, and host threads that each set their own call's size would lower it between
+// another's set and launch.
 template <typename K>
 bool fits_cluster(K kernel, int ctas, size_t smem) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) != cudaSuccess ||
       cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return false;
