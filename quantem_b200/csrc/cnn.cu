@@ -474,7 +474,23 @@ int colsum(const float* a, int lda, int R, int C, double* work, int64_t work_ele
   return check_launch("colsum_final_kernel");
 }
 
+int bn_check(const qb::bn::Forward& f, int R, int C) {
+  if (!f.x || !f.y || R < 1 || C < 1 || f.ldx < C || f.ldy < C)
+    return fail(PTYCHO_ERR_INVALID, "bn_forward: bad arguments");
+  if (f.gamma && (!f.beta || !f.mean || !f.rstd || !f.run_mean != !f.run_var || (!f.training && !f.run_mean)))
+    return fail(PTYCHO_ERR_INVALID, "bn_forward: missing statistics buffers");
+  return PTYCHO_OK;
+}
+int bn_check(const qb::bn::Backward& b, int R, int C) {
+  if (!b.dy || !b.x || R < 1 || C < 1 || b.lddy < C || b.ldx < C || b.ldz < C || (!b.dz32 && !b.dz16) || b.act < 0 ||
+      b.act >= qb::ACT_COUNT)
+    return fail(PTYCHO_ERR_INVALID, "bn_backward: bad arguments");
+  if (b.gamma && (!b.mean || !b.rstd || !b.dgamma || !b.dbeta))
+    return fail(PTYCHO_ERR_INVALID, "bn_backward: missing buffers");
+  return PTYCHO_OK;
+}
 int bn_forward(const qb::bn::Forward& f, int R, int C, cudaStream_t st) {
+  if (int rc = bn_check(f, R, C)) return rc;
   if (!f.gamma) {
     to_bf16_kernel<<<blocks_for((int64_t)R * C, 256), 256, 0, st>>>(f.x, f.ldx, R, C, f.y, f.ldy);
     return check_launch("to_bf16_kernel");
@@ -483,6 +499,7 @@ int bn_forward(const qb::bn::Forward& f, int R, int C, cudaStream_t st) {
   return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_forward_kernel: %s", cudaGetErrorString(e));
 }
 int bn_backward(const qb::bn::Backward& b, int R, int C, cudaStream_t st) {
+  if (int rc = bn_check(b, R, C)) return rc;
   const cudaError_t e = qb::bn::launch(qb::bn::bn_backward_kernel, b, R, C, st);
   return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_backward_kernel: %s", cudaGetErrorString(e));
 }
@@ -602,31 +619,23 @@ int ptycho_cnn_transpose(const void* in, int in_dtype, int R, int C, int ldi, in
 int ptycho_cnn_bn_forward(const float* x, int ldx, int R, int C, const float* gamma, const float* beta,
                           float* run_mean, float* run_var, float momentum, float eps, int training, float* mean,
                           float* rstd, double* work, int64_t work_elems, void* out, int ldo, void* stream) {
-  if (!x || !out || R < 1 || C < 1 || ldx < C || ldo < C) return fail(PTYCHO_ERR_INVALID, "bn_forward: bad arguments");
-  if (gamma) {
-    if (!beta || !mean || !rstd || (!training && (!run_mean || !run_var)))
-      return fail(PTYCHO_ERR_INVALID, "bn_forward: missing statistics buffers");
-    if (training)
-      if (int rc = work_check(C, work_elems)) return rc;
-  }
-  return bn_forward({x, ldx, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
-                     static_cast<bf16*>(out), ldo},
-                    R, C, static_cast<cudaStream_t>(stream));
+  const qb::bn::Forward f{x, ldx, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                          static_cast<bf16*>(out), ldo};
+  if (int rc = bn_check(f, R, C)) return rc;
+  if (gamma && training)
+    if (int rc = work_check(C, work_elems)) return rc;
+  return bn_forward(f, R, C, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_bn_backward(const float* dy, int lddy, const float* x, int ldx, int R, int C, const float* gamma,
                            const float* mean, const float* rstd, int training, int act, float* dgamma, float* dbeta,
                            double* work, int64_t work_elems, float* dz32, void* dz16, int ldz, void* stream) {
-  if (!dy || !x || R < 1 || C < 1 || lddy < C || ldx < C || ldz < C || (!dz32 && !dz16) || act < 0 ||
-      act >= qb::ACT_COUNT)
-    return fail(PTYCHO_ERR_INVALID, "bn_backward: bad arguments");
-  if (gamma) {
-    if (!mean || !rstd || !dgamma || !dbeta) return fail(PTYCHO_ERR_INVALID, "bn_backward: missing buffers");
+  const qb::bn::Backward b{dy, lddy, x, ldx, gamma, mean, rstd, training, act, dgamma, dbeta, nullptr, dz32,
+                           static_cast<bf16*>(dz16), ldz};
+  if (int rc = bn_check(b, R, C)) return rc;
+  if (gamma)
     if (int rc = work_check(C, work_elems)) return rc;
-  }
-  return bn_backward({dy, lddy, x, ldx, gamma, mean, rstd, training, act, dgamma, dbeta, nullptr, dz32,
-                      static_cast<bf16*>(dz16), ldz},
-                     R, C, static_cast<cudaStream_t>(stream));
+  return bn_backward(b, R, C, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_colsum(const float* a, int lda, int R, int C, float* out, int accumulate, double* work,
@@ -696,18 +705,43 @@ int ptycho_cnn_dropout(void* x, int dtype, int R, int C, int ld, float p, uint64
   return check_launch("dropout_kernel");
 }
 
+}  // extern "C"
+
+namespace {
+// Arguments of a whole-layer call, all of them checked before its first launch: rows of
+// B H W `up` pixels (a patch matrix of more than 2^30 rows fits no device), channel counts and
+// leading dimensions that the copies of 16 bytes can take, and the pointers that are not optional.
+constexpr int64_t kMaxRows = 1 << 30;
+int layer_check(const char* what, int B, int H, int W, int up, int c, int co) {
+  if (B < 1 || H < 1 || W < 1 || c < 8 || (c & 7) || co < 1 || c > (1 << 27) || co > (1 << 27) ||
+      (int64_t)B * H > kMaxRows || (int64_t)B * H * W > kMaxRows / up)
+    return fail(PTYCHO_ERR_INVALID, "%s: bad sizes (B=%d H=%d W=%d, channels %d -> %d)", what, B, H, W, c, co);
+  return PTYCHO_OK;
+}
+// the pointers of an operand that is copied 16 bytes at a time, and its leading dimension (0: packed)
+bool operand(const void* p, int ld = 0, int cols = 0) { return p && al16(p) && !(ld & 7) && ld >= cols; }
+int bad_args(const char* what) { return fail(PTYCHO_ERR_INVALID, "%s: bad arguments", what); }
+}  // namespace
+
+extern "C" {
+
 int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, const void* w, int co,
                             const float* bias, int act, const float* gamma, const float* beta, float* run_mean,
                             float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
                             void* col, float* r, void* out, int ldo, void* stream) {
+  if (int rc = layer_check("conv_forward", B, H, W, 1, C, co)) return rc;
   const int R = B * H * W;
+  const qb::bn::Forward f{r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                          static_cast<bf16*>(out), ldo};
+  if (!operand(x, ldx, C) || !operand(w) || !operand(col) || !r || act < 0 || act >= qb::ACT_COUNT)
+    return bad_args("conv_forward");
+  if (out)
+    if (int rc = bn_check(f, R, co)) return rc;
   if (int rc = ptycho_cnn_im2col3x3(x, B, H, W, C, ldx, col, 9 * C, stream)) return rc;
   if (int rc = ptycho_gemm_bf16(col, 9 * C, w, 9 * C, r, co, R, co, 9 * C, bias, act << 8, 1, nullptr, stream))
     return rc;
   if (!out) return PTYCHO_OK;
-  return bn_forward({r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
-                     static_cast<bf16*>(out), ldo},
-                    R, co, static_cast<cudaStream_t>(stream));
+  return bn_forward(f, R, co, static_cast<cudaStream_t>(stream));
 }
 
 namespace {
@@ -729,8 +763,12 @@ int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, 
                              const float* rstd, int training, int act, float* dw, float* db, float* dgamma,
                              float* dbeta, void* dz, int ldz, void* col, float* dcol, float* dx, int lddx,
                              int dx_accumulate, void* stream) {
+  if (int rc = layer_check("conv_backward", B, H, W, 1, C, co)) return rc;
   const int R = B * H * W, K9 = 9 * C;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!operand(x, ldx, C) || !operand(dz, ldz, co) || !operand(col) || !dw ||
+      (dx && (!operand(w) || !operand(dcol) || !al16(dx) || (lddx & 3) || lddx < C)))
+    return bad_args("conv_backward");
   if (int rc = bn_backward({dy, lddy, r, co, gamma, mean, rstd, training, act, dgamma, dbeta, db, nullptr,
                             static_cast<bf16*>(dz), ldz},
                            R, co, st))
@@ -748,14 +786,17 @@ int ptycho_cnn_up_forward(const void* y, int ldy, int B, int H, int W, int ci, i
                           const void* w1, const float* b1, const float* gamma, const float* beta, float* run_mean,
                           float* run_var, float momentum, float eps, int training, float* mean, float* rstd,
                           float* colT, void* t, float* r, void* out, int ldo, void* stream) {
+  if (int rc = layer_check("up_forward", B, H, W, 4, ci, co)) return rc;
   const int Rin = B * H * W, R = 4 * Rin;
+  const qb::bn::Forward f{r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
+                          static_cast<bf16*>(out), ldo};
+  if (!operand(y, ldy, ci) || !operand(wt) || !operand(w1) || !operand(t) || !colT) return bad_args("up_forward");
+  if (int rc = bn_check(f, R, co)) return rc;
   if (int rc = ptycho_gemm_bf16(y, ldy, wt, ci, colT, 9 * ci, Rin, 9 * ci, ci, nullptr, 0, 1, nullptr, stream))
     return rc;
   if (int rc = ptycho_cnn_convT_gather(colT, 9 * ci, B, H, W, ci, bt, t, ci, stream)) return rc;
   if (int rc = ptycho_gemm_bf16(t, ci, w1, ci, r, co, R, co, ci, b1, 0, 1, nullptr, stream)) return rc;
-  return bn_forward({r, co, gamma, beta, run_mean, run_var, mean, rstd, momentum, eps, training,
-                     static_cast<bf16*>(out), ldo},
-                    R, co, static_cast<cudaStream_t>(stream));
+  return bn_forward(f, R, co, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, const void* t, const float* r, int B,
@@ -763,8 +804,13 @@ int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, 
                            const float* mean, const float* rstd, int training, float* dwt, float* dbt, float* dw1,
                            float* db1, float* dgamma, float* dbeta, void* dz, int ldz, float* dt, void* dcolT,
                            double* work, int64_t work_elems, float* dy, void* stream) {
+  if (int rc = layer_check("up_backward", B, H, W, 4, ci, co)) return rc;
   const int Rin = B * H * W, R = 4 * Rin, C9 = 9 * ci;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!operand(y, ldy, ci) || !operand(t) || !operand(wt) || !operand(w1) || !operand(dz, ldz, co) || !operand(dcolT) ||
+      !dt || !dwt || !dbt || !dw1 || !dy || !work)
+    return bad_args("up_backward");
+  if (int rc = work_check(ci, work_elems)) return rc;
   if (int rc = bn_backward({dup, lddup, r, co, gamma, mean, rstd, training, 0, dgamma, dbeta, db1, nullptr,
                             static_cast<bf16*>(dz), ldz},
                            R, co, st))
