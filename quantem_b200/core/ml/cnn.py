@@ -637,7 +637,7 @@ class _Run:
         self._bind()
         self.pg = grad.data_ptr()
         convs, ups = self._levels()
-        first = net.down[0][0]
+        first = net.down[0][0] if L else None  # the layer whose input gradient may not be wanted
         a = self._align
         self.scratch = self.empty(max(
             [a(R * _up8(la["co"]) * 2) + a(R * 9 * la["ci_store"] * 2) +
