@@ -586,13 +586,10 @@ constexpr int kLineThreads = 512;
 // is within about a sixteenth of the slice's deviation from its mean whatever its structure.
 template <bool REAL>
 __device__ float2 sampled_mean(const float* in, int H, int W, float2* red) {
-  const int64_t hw = (int64_t)H * W;
-  const int cnt = hw < 256 ? (int)hw : 256;
   const unsigned k = threadIdx.x;
   float2 v = make_float2(0.f, 0.f);
-  if ((int)k < cnt) {
-    const int64_t i =
-        hw <= 256 ? (int64_t)k : (int64_t)((int64_t)k * H >> 8) * W + (int)__umulhi(k * 2654435769u, (unsigned)W);
+  if (k < 256) {
+    const unsigned i = (k * H >> 8) * W + (((k * 40503 & 0xffff) * W) >> 16);  // sides <= 6144; 40503 / 2^16 = 0.618
     v = REAL ? make_float2(in[i], 0.f) : reinterpret_cast<const float2*>(in)[i];
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -604,7 +601,7 @@ __device__ float2 sampled_mean(const float* in, int H, int W, float2* red) {
   __syncthreads();
   float2 t = make_float2(0.f, 0.f);
   for (int w = 0; w < 8; ++w) t = make_float2(t.x + red[w].x, t.y + red[w].y);
-  const float inv = 1.0f / (float)cnt;
+  const float inv = 1.0f / 256.0f;
   return make_float2(t.x * inv, t.y * inv);
 }
 
