@@ -416,7 +416,8 @@ int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, 
 /* Gradients of the layer from dy (FP32, R x co, w.r.t. the batch norm's output): dw (FP32
  * (co, 9 C), zero on entry), db, dgamma, dbeta (written) and, if given, dx (FP32 R x C, written or added
  * to).  dz: BF16 scratch R x ldz (ldz >= co, a multiple of 8); col: BF16 scratch R x 9 C;
- * dcol: FP32 scratch R x 9 C (with dx). */
+ * dcol: FP32 scratch R x 9 C (with dx); it may share its memory with col, which is used up when
+ * it is written. */
 int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, int B, int H, int W, int C,
                              const void* w, const float* r, int co, const float* gamma, const float* mean,
                              const float* rstd, int training, int act, float* dw, float* db, float* dgamma,

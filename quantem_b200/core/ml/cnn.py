@@ -108,7 +108,7 @@ class CNN2d(torch.nn.Module):
         # when a dict, each pass records every layer's inputs / outputs / gradients
         # (used by the per-layer parity tests)
         self.trace = None
-        self._arena_bytes = {}  # (B, H, W) -> bytes of one pass's buffers
+        self._arena_bytes = {}  # (B, H, W) -> bytes of the buffers of one pass without a backward
         self._build()
         self._init_params(seed)
 
@@ -341,7 +341,7 @@ class CNN2d(torch.nn.Module):
             f = 2 ** self.num_layers
             if H % f or W % f:
                 raise ValueError(f"H and W must be divisible by 2**num_layers = {f}")
-            return _CNNFn.apply(x, self.flat, self, (B, H, W))
+            return _CNNFn.apply(x, self.flat, self, (B, H, W), torch.is_grad_enabled())
         if x.dim() != 4 or x.shape[1] != self.in_channels:
             raise ValueError(f"expected (B, {self.in_channels}, H, W), got {tuple(x.shape)}")
         if not x.is_cuda:
@@ -349,7 +349,7 @@ class CNN2d(torch.nn.Module):
         f = 2 ** self.num_layers
         if x.shape[2] % f or x.shape[3] % f:
             raise ValueError(f"H and W must be divisible by 2**num_layers = {f}")
-        return _CNNFn.apply(x.float().contiguous(), self.flat, self, None)
+        return _CNNFn.apply(x.float().contiguous(), self.flat, self, None, torch.is_grad_enabled())
 
     __call__ = forward
 
@@ -374,23 +374,36 @@ class _Buf:
 
 
 class _Arena:
-    """Bump allocation of one pass's buffers from a few tensors of the caching allocator."""
+    """Buffers of one pass out of a few tensors of the caching allocator.
 
-    def __init__(self, device, first: int):
-        self.device, self.block = device, max(int(first), 1 << 20)
+    A pass that a backward follows takes one tensor per call (what one layer's backward needs): it goes
+    back to the allocator when the backward has passed the layer and drops its last buffer.  A pass
+    without a backward takes its buffers one after the other from large tensors, ``first`` bytes and
+    then 16 MB each, which live as long as the pass."""
+
+    def __init__(self, device, first: int, keep: bool):
+        self.device, self.keep, self.block = device, keep, max(int(first), 1 << 20)
         self.blocks, self.base, self.used, self.total = [], None, 0, 0
 
-    def buf(self, R, C, dtype, ld=None) -> _Buf:
-        ld = C if ld is None else ld
-        n = (R * ld * dtype.itemsize + 255) // 256 * 256
-        if self.base is None or self.used + n > self.base.numel():
-            self.base = torch.empty(max(n, self.block), dtype=torch.uint8, device=self.device)
-            self.blocks.append(self.base)
-            self.used, self.block = 0, 1 << 24
-        b = _Buf(self.base, self.used, R, C, ld, dtype)
-        self.used += n
-        self.total += n
-        return b
+    def bufs(self, *shapes) -> list:
+        """A buffer per (R, C, dtype)."""
+        sizes = [(R * C * dtype.itemsize + 255) // 256 * 256 for R, C, dtype in shapes]
+        n = sum(sizes)
+        if self.keep:
+            base, off = torch.empty(n, dtype=torch.uint8, device=self.device), 0
+        else:
+            if self.base is None or self.used + n > self.base.numel():
+                self.base = torch.empty(max(n, self.block), dtype=torch.uint8, device=self.device)
+                self.blocks.append(self.base)
+                self.used, self.block = 0, 1 << 24
+            base, off = self.base, self.used
+            self.used += n
+            self.total += n
+        out = []
+        for (R, C, dtype), size in zip(shapes, sizes):
+            out.append(_Buf(base, off, R, C, C, dtype))
+            off += size
+        return out
 
 
 _F32, _BF16 = torch.float32, torch.bfloat16
@@ -400,13 +413,15 @@ class _Run:
     """One forward pass: buffers and saved matrices for its backward.  Every layer is one
     library call that queues its launches."""
 
-    def __init__(self, net: CNN2d, B: int, H: int, W: int, training: bool):
+    def __init__(self, net: CNN2d, B: int, H: int, W: int, training: bool, keep: bool):
+        """``keep``: a backward follows."""
+        self.keep = keep
         self.net, self.B, self.H, self.W, self.training = net, B, H, W, training
         self.dev = net.device
         self.lib = kk._lib.lib()
         self.saved = {}
         self.key = (B, H, W)
-        self.arena = _Arena(self.dev, net._arena_bytes.get(self.key, 1 << 22))
+        self.arena = _Arena(self.dev, net._arena_bytes.get(self.key, 1 << 22), keep)
 
     def empty(self, *shape, dtype=torch.float32):
         return torch.empty(*shape, dtype=dtype, device=self.dev)
@@ -434,18 +449,21 @@ class _Run:
         return (self._f(gseg), self._f(bseg), rm.data_ptr(), rv.data_ptr(), self.net.momentum, self.net.eps,
                 int(self.training), mean.ptr, rstd.ptr)
 
-    def _stats(self, bn, co):
+    def _act_bufs(self, bn, R, co, *more):
+        """A layer's activation, its batch-norm statistics (None without) and ``more`` buffers."""
         if bn is None:
-            return None, None
-        return self.arena.buf(1, co, _F32), self.arena.buf(1, co, _F32)
+            r, *more = self.arena.bufs((R, co, _F32), *more)
+            return r, None, None, *more
+        return self.arena.bufs((R, co, _F32), (1, co, _F32), (1, co, _F32), *more)
 
     # --- conv3x3 + bias + activation (+ BN) -> bf16 into `out` ------------------
     def conv_fwd(self, key, layer, x, B, H, W, out, act=None, final=False):
         net = self.net
         R, co, C = B * H * W, layer["co"], layer["ci_store"]
-        r = self.arena.buf(R, co, _F32)
         bn = None if final else layer["bn"]
-        mean, rstd = self._stats(bn, co)
+        r, mean, rstd = self._act_bufs(bn, R, co)
+        if out is None and not final:  # the next layer's input
+            out, = self.arena.bufs((R, co, _BF16))
         self.call("ptycho_cnn_conv_forward", x.ptr, x.ld, B, H, W, C, self._h(layer["w"]), co, self._f(layer["b"]),
                   int(net._act if act is None else act), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
                   r.ptr, None if final else out.ptr, 0 if final else out.ld, self.st)
@@ -473,11 +491,10 @@ class _Run:
         net._dropout_calls += 1
         return (net._dropout_seed * 0x9E3779B1 + net._dropout_calls) & 0xFFFFFFFFFFFF
 
-    def block_fwd(self, prefix, layers, x, B, H, W, out_last):
+    def block_fwd(self, prefix, layers, x, B, H, W, out_last=None):
         y = x
         for j, layer in enumerate(layers):
-            out = out_last if j == len(layers) - 1 else self.arena.buf(B * H * W, layer["co"], _BF16)
-            y = self.conv_fwd((prefix, j), layer, y, B, H, W, out)
+            y = self.conv_fwd((prefix, j), layer, y, B, H, W, out_last if j == len(layers) - 1 else None)
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
@@ -524,7 +541,7 @@ class _Run:
         # im2col rows (BF16) or the transposed convolution's products (FP32), one layer at a time
         self.scratch = self.empty(max([R * 9 * la["ci_store"] * 2 for R, la in convs] +
                                       [R * 9 * up["ci"] * 4 for R, up in ups]), dtype=torch.uint8)
-        self.cat = []
+        cats = []
         self.pool_arg = []
         x16 = self.x16
         y = _Buf.__new__(_Buf)
@@ -540,33 +557,28 @@ class _Run:
             co = net.down[l][-1]["co"]
             R = B * h * w
             if net.use_skip_connections:
-                cat = self.arena.buf(R, 2 * co, _BF16)
+                cat, = self.arena.bufs((R, 2 * co, _BF16))
                 skip = cat.cols(co, co)
             else:
                 cat = None
-                skip = self.arena.buf(R, co, _BF16)
-            self.cat.append(cat)
+                skip, = self.arena.bufs((R, co, _BF16))
+            cats.append(cat)
             self.block_fwd(("down", l), net.down[l], y, B, h, w, skip)
-            pooled = self.arena.buf(R // 4, co, _BF16)
-            arg = self.arena.buf(R // 4, co, torch.uint8)
+            pooled, arg = self.arena.bufs((R // 4, co, _BF16), (R // 4, co, torch.uint8))
             self.call("ptycho_cnn_maxpool2", skip.ptr, skip.ld, B, h, w, co, pooled.ptr, pooled.ld, arg.ptr, self.st)
             self.pool_arg.append(arg)
             y = pooled
-        h, w = H >> L, W >> L
-        cb = net.bottleneck[-1]["co"]
-        yb = self.arena.buf(B * h * w, cb, _BF16)
-        y = self.block_fwd(("bott",), net.bottleneck, y, B, h, w, yb)
+        y = self.block_fwd(("bott",), net.bottleneck, y, B, H >> L, W >> L)
         for u, up in enumerate(net.up):
             l = L - 1 - u
             hin, win = H >> (l + 1), W >> (l + 1)
             h, w = H >> l, W >> l
             ci, co = up["ci"], up["co"]
             R = B * h * w
-            t, r = self.arena.buf(R, ci, _BF16), self.arena.buf(R, co, _F32)
-            cat = self.cat[l]
-            dst = cat.cols(0, co) if cat is not None else self.arena.buf(R, co, _BF16)
+            cat = cats[l]
             bn = up["bn"] if net._use_batchnorm else None
-            mean, rstd = self._stats(bn, co)
+            r, mean, rstd, t = self._act_bufs(bn, R, co, (R, ci, _BF16))
+            dst = cat.cols(0, co) if cat is not None else self.arena.bufs((R, co, _BF16))[0]
             self.call("ptycho_cnn_up_forward", y.ptr, y.ld, B, hin, win, ci, co, self._h(up["wt"]), self._f(up["bt"]),
                       self._h(up["w1"]), self._f(up["b1"]), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
                       t.ptr, r.ptr, dst.ptr, dst.ld, self.st)
@@ -575,13 +587,13 @@ class _Run:
                 net.trace[("upfwd", u)] = dict(x=y.tensor().clone(), t=t.tensor().clone(), r=r.tensor().clone(),
                                                y=dst.tensor().clone())
             src = cat if cat is not None else dst
-            out = self.arena.buf(R, up["block"][-1]["co"], _BF16)
-            y = self.block_fwd(("upc", u), up["block"], src, B, h, w, out)
+            y = self.block_fwd(("upc", u), up["block"], src, B, h, w)
         r = self.conv_fwd(("final",), net.final, y, B, H, W, None, act=net._final_act, final=True)
         del self.scratch
-        if len(net._arena_bytes) > 16:
-            net._arena_bytes.clear()
-        net._arena_bytes[self.key] = self.arena.total
+        if not self.keep:
+            if len(net._arena_bytes) > 16:
+                net._arena_bytes.clear()
+            net._arena_bytes[self.key] = self.arena.total
         out = self.empty(B, net.out_channels, H * W)
         kk.transpose(r.view(B, H * W, net.out_channels), out)
         return out.view(B, net.out_channels, H, W)
@@ -600,16 +612,18 @@ class _Run:
         R, co, C = B * H * W, layer["co"], layer["ci_store"]
         bn = layer["bn"]
         g = self.pg
-        sc = self.scratch.data_ptr()
         ldz = _up8(co)
-        col = sc + self._align(R * ldz * 2)
-        dcol = col + self._align(R * 9 * C * 2)
+        nz = self._align(R * ldz * 2)
+        # dz, then the patches; the patches' gradient takes their place
+        scratch = self.empty(nz + R * 9 * C * (2 if dx_out is None else 4), dtype=torch.uint8)
+        sc = scratch.data_ptr()
+        col = sc + nz
         self.call("ptycho_cnn_conv_backward", dy.data_ptr(), dy.stride(0), x.ptr, x.ld, B, H, W, C,
                   self._h(layer["w"]), r.ptr, co, *((self._f(bn[0]), mean.ptr, rstd.ptr) if bn is not None else
                                                     (None, None, None)),
                   int(self.training), int(net._act if act is None else act), g + 4 * layer["w"].off,
                   g + 4 * layer["b"].off, *((g + 4 * bn[0].off, g + 4 * bn[1].off) if bn is not None else (None, None)),
-                  sc, ldz, col, dcol, None if dx_out is None else dx_out.data_ptr(),
+                  sc, ldz, col, col, None if dx_out is None else dx_out.data_ptr(),
                   0 if dx_out is None else dx_out.stride(0), int(dx_accumulate), self.st)
         if tr is not None and dx_out is not None:
             tr[("bwd",) + key]["dx"] = dx_out.clone()
@@ -636,14 +650,6 @@ class _Run:
         R0 = B * H * W
         self._bind()
         self.pg = grad.data_ptr()
-        convs, ups = self._levels()
-        first = net.down[0][0] if L else None  # the layer whose input gradient may not be wanted
-        a = self._align
-        self.scratch = self.empty(max(
-            [a(R * _up8(la["co"]) * 2) + a(R * 9 * la["ci_store"] * 2) +
-             (0 if la is first and not need_dx else R * 9 * la["ci_store"] * 4) for R, la in convs] +
-            [a(4 * R * _up8(up["co"]) * 2) + a(4 * R * up["ci"] * 4) + R * 9 * up["ci"] * 2 for R, up in ups]),
-            dtype=torch.uint8)
         work = self.empty(2 * 592 * max([up["ci"] for up in net.up], default=1), dtype=torch.float64)
         dfin = self.empty(R0, net.out_channels)
         kk.transpose(dout.reshape(B, net.out_channels, H * W), dfin.view(B, H * W, net.out_channels))
@@ -665,8 +671,11 @@ class _Run:
             yin, t, r, mean, rstd, hin, win = self.saved.pop(("upT", u))
             bn = up["bn"] if net._use_batchnorm else None
             ldz = _up8(co)
-            g, sc = self.pg, self.scratch.data_ptr()
-            dt = sc + a(R * ldz * 2)
+            g, a = self.pg, self._align
+            o = a(R * ldz * 2)
+            scratch = self.empty(o + a(R * ci * 4) + R // 4 * 9 * ci * 2, dtype=torch.uint8)
+            sc = scratch.data_ptr()
+            dt = sc + o
             dcolT = dt + a(R * ci * 4)
             dy = self.empty(B * hin * win, ci)
             self.call("ptycho_cnn_up_backward", dup.data_ptr(), dup.stride(0), yin.ptr, yin.ld, t.ptr, r.ptr, B, hin,
@@ -677,9 +686,9 @@ class _Run:
                       *((g + 4 * bn[0].off, g + 4 * bn[1].off) if bn is not None else (None, None)), sc, ldz, dt,
                       dcolT, work.data_ptr(), work.numel(), dy.data_ptr(), self.st)
             if net.trace is not None:
-                o = dt - sc
                 net.trace[("upbwd", u)] = dict(dup=dup.clone(), dx=dy.clone(),
-                                               dt=self.scratch[o: o + R * ci * 4].view(_F32).view(R, ci).clone())
+                                               dt=scratch[o: o + R * ci * 4].view(_F32).view(R, ci).clone())
+            del scratch, yin, t, r, mean, rstd
         # bottleneck
         h, w = H >> L, W >> L
         cin = net.bottleneck[0]["ci_store"]
@@ -691,7 +700,7 @@ class _Run:
             R = B * h * w
             co = net.down[l][-1]["co"]
             dskip = dcat[l][:, co:] if net.use_skip_connections else self.empty(R, co)
-            self.call("ptycho_cnn_maxpool2_backward", dpool.data_ptr(), dpool.stride(0), self.pool_arg[l].ptr, B, h, w,
+            self.call("ptycho_cnn_maxpool2_backward", dpool.data_ptr(), dpool.stride(0), self.pool_arg.pop().ptr, B, h, w,
                       co, dskip.data_ptr(), dskip.stride(0), int(net.use_skip_connections), self.st)
             cin = net.down[l][0]["ci_store"]
             if l > 0:
@@ -710,10 +719,10 @@ class _Run:
 
 class _CNNFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, flat, net, rows):
+    def forward(ctx, x, flat, net, rows, grad_mode):
         B, H, W = rows if rows is not None else (x.shape[0], x.shape[2], x.shape[3])
         net.sync_weights()
-        run = _Run(net, B, H, W, net.training)
+        run = _Run(net, B, H, W, net.training, keep=grad_mode and any(ctx.needs_input_grad))
         y = run.forward(x)
         if net.training:
             net.num_batches_tracked += 1
@@ -727,7 +736,7 @@ class _CNNFn(torch.autograd.Function):
         ctx.run = None
         grad = torch.zeros_like(run.net.flat.data)
         dx = run.backward(dy.float().resolve_neg().contiguous(), grad, ctx.needs_x)
-        return dx, grad, None, None
+        return dx, grad, None, None, None
 
 
 def mse_loss(pred: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
@@ -899,7 +908,7 @@ class ComplexCNN2d(torch.nn.Module):
         xr = torch.cat([x.real, x.imag], dim=1).float().contiguous()
         w = self._real_flat()
         self.real.flat.data.copy_(w.detach())
-        y = _CNNFn.apply(xr, w, self.real, None)
+        y = _CNNFn.apply(xr, w, self.real, None, torch.is_grad_enabled())
         C = self.out_channels
         return torch.complex(y[:, :C], y[:, C:])
 
