@@ -402,6 +402,9 @@ int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, in
 int ptycho_gemm_bf16_mn(const void* A, int lda, int a_mn, const void* B, int ldb, void* C, int ldc, int M, int N,
                         int K, int flags, int splits, int* status, void* stream);
 
+/* How a product is launched: columns of a tile, CTAs in all, and CTAs that share an SM. */
+int ptycho_gemm_plan(int M, int N, int K, int splits, int a_mn, int b_mn, int* tile_n, int64_t* ctas, int* ctas_per_sm);
+
 /* ---- whole layers: the launches of one layer of the network, queued by one call ----
  *
  * Conv2dBlock layer (blocks.py:53-140): r (FP32, R x co) = act(conv3x3(x) + bias); with out

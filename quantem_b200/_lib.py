@@ -54,6 +54,7 @@ EXPORTED = (
     "ptycho_forward_loss_noalloc",
     "ptycho_gemm_bf16",
     "ptycho_gemm_bf16_mn",
+    "ptycho_gemm_plan",
     "ptycho_cnn_conv_forward",
     "ptycho_cnn_conv_backward",
     "ptycho_cnn_up_forward",
@@ -164,6 +165,7 @@ def _declare(lib):
         "ptycho_cnn_up_forward": (_int, [_vp] + [_int] * 6 + [_vp] * 8 + [_flt, _flt, _int] + [_vp] * 6 + [_int, _vp]),
         "ptycho_cnn_up_backward": (_int, [_vp, _int, _vp, _int, _vp, _vp] + [_int] * 5 + [_vp] * 5 + [_int] +
                                    [_vp] * 7 + [_int, _vp, _vp, _vp, _i64, _vp, _vp]),
+        "ptycho_gemm_plan": (_int, [_int] * 6 + [_vp] * 3),
         "ptycho_gemm_bf16_mn": (_int, [_vp, _int, _int, _vp, _int, _vp, _int, _int, _int, _int, _int, _int, _vp, _vp]),
         "ptycho_gemm_bf16": (_int, [_vp, _int, _vp, _int, _vp, _int, _int, _int, _int, _vp, _int, _int, _vp, _vp]),
         "ptycho_cnn_im2col3x3": (_int, [_vp, _int, _int, _int, _int, _int, _vp, _int, _vp]),

@@ -39,6 +39,7 @@ int check_launch(const char* what) {
   if (e != cudaSuccess) return fail(PTYCHO_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   return PTYCHO_OK;
 }
+constexpr int kSms = 148;
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 int blocks_for(int64_t n, int threads, int cap = 148 * 16) {
   int64_t b = (n + threads - 1) / threads;
@@ -76,19 +77,19 @@ int make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int
   return r == CUDA_SUCCESS ? PTYCHO_OK : fail(PTYCHO_ERR_INVALID, "gemm: tensor map encode failed (%d)", (int)r);
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool DEEP>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int splits, int kb_per, int a_rows,
                 const qb::gemm::Epilogue& epi, int* status, cudaStream_t st) {
-  using L = qb::gemm::Smem<BN>;
+  using L = qb::gemm::Smem<BN, DEEP>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN>,
+    attr = cudaFuncSetAttribute(qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN, DEEP>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
   });
   if (attr != cudaSuccess) return fail(PTYCHO_ERR_CUDA, "gemm: smem attribute: %s", cudaGetErrorString(attr));
   dim3 grid((M + qb::gemm::BM - 1) / qb::gemm::BM, (N + BN - 1) / BN, splits);
-  qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN>
+  qb::gemm::gemm_bf16_kernel<BN, A_MN, B_MN, DEEP>
       <<<grid, qb::gemm::THREADS, L::BYTES, st>>>(ta, tb, M, N, K, kb_per, a_rows, epi, status);
   return check_launch("gemm_bf16_kernel");
 }
@@ -99,6 +100,40 @@ struct Operand {
   int ld;
   bool mn;
 };
+
+// Tile width and ring of a product of M x N, `splits` parts of K and a_rows rows of A per tile.
+//
+// A CTA's time goes with the rows that its copies bring per k-block, a_rows + BN, and the tiles are
+// worked off in rounds of one per SM: the width with the fewest rounds x (a_rows + BN), the widest of
+// equals.  16384 x 32 x 9216: 58 us as 128 CTAs of 32 columns, 98 as 256 of 16 in two rounds;
+// 16 x 1024 x 9216: 29 us at 16 columns, 46 at 128.  In several rounds two CTAs share an SM (widths 32
+// and 64 with a ring of four k-blocks), so that one's epilogue runs beside the other's copies: 65536 x
+// 32 x 288 takes 19 us, 31 with the deep ring; 20000 x 32 x 288 (157 CTAs) 12.5 against 17.  In one round
+// the deep ring is the faster: 18944 x 32 x 2304 (148 CTAs) 17 us against 19.  16 columns only in one
+// round: 262144 x 16 x 144 took 66 us with them, 40 with 32 columns.
+// A column's products and sums do not depend on the tile width.  MN-major B tiles are copied in boxes of
+// 64 columns.
+struct Tile {
+  int bn;
+  int64_t ctas;
+  bool deep;
+};
+Tile tile_of(int M, int N, int splits, int a_rows, bool b_mn) {
+  const int64_t tiles_m = (M + qb::gemm::BM - 1) / qb::gemm::BM * (int64_t)splits;
+  const int least = b_mn ? 64 : 16;
+  int widest = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+  if (widest < least) widest = least;
+  Tile t{0, 0, true};
+  int64_t best = 0;
+  for (int w = widest; w >= least; w /= 2) {
+    const int64_t n = tiles_m * ((N + w - 1) / w), cost = (n + kSms - 1) / kSms * (a_rows + w);
+    if (w == 16 && n > kSms) break;
+    if (t.bn == 0 || cost < best) t = {w, n, true}, best = cost;
+  }
+  t.deep = b_mn || t.bn == 16 || t.bn == 128 || t.ctas <= kSms;
+  return t;
+}
+int rows_of_a(int M, bool a_mn) { return a_mn || M >= qb::gemm::BM ? qb::gemm::BM : (M + 7) / 8 * 8; }
 
 int gemm_run(const Operand& A, const Operand& B, void* C, int ldc, int M, int N, int K, const float* bias, int flags,
              int splits, int* status, cudaStream_t st) {
@@ -123,16 +158,10 @@ int gemm_run(const Operand& A, const Operand& B, void* C, int ldc, int M, int N,
   if (int rc = encode_fn()) return rc;
   const int kb_per = (nkb + splits - 1) / splits;
   splits = (nkb + kb_per - 1) / kb_per;  // every split gets >= 1 k-block
-  // The widest tile (fewest re-reads of A) that still gives every SM one; the deep layers of a
-  // network (16 to 256 rows) take narrow tiles: at 16 rows x 1024 columns x 9216 one CTA per 128
-  // columns streamed the weights through 8 SMs.  A column's products and sums do not depend on
-  // the tile width.  MN-major B tiles are copied in boxes of 64 columns.
-  const int tiles_m = (M + BM - 1) / BM, least = B.mn ? 64 : 16;
-  int BN = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
-  if (BN < least) BN = least;
-  while (BN > least && tiles_m * ((N + BN - 1) / BN) * splits < 148) BN /= 2;
+  const int a_rows = rows_of_a(M, A.mn);
+  const Tile t = tile_of(M, N, splits, a_rows, B.mn);
+  const int BN = t.bn;
   CUtensorMap ta, tb;
-  const int a_rows = A.mn || M >= BM ? BM : (M + 7) / 8 * 8;
   if (int rc = A.mn ? make_map(&ta, A.p, K, M, A.ld, BK) : make_map(&ta, A.p, M, K, A.ld, a_rows)) return rc;
   if (int rc = B.mn ? make_map(&tb, B.p, K, N, B.ld, BK) : make_map(&tb, B.p, N, K, B.ld, BN)) return rc;
   if (!accumulate && splits > 1) {
@@ -140,21 +169,26 @@ int gemm_run(const Operand& A, const Operand& B, void* C, int ldc, int M, int N,
       return check_launch("gemm: clear split-K output");
   }
   const Epilogue epi{C, bias, ldc, flags, act};
-#define QB_GEMM(bn, a, b) return launch_gemm<bn, a, b>(ta, tb, M, N, K, splits, kb_per, a_rows, epi, status, st)
+#define QB_GEMM(bn, a, b, deep) \
+  return launch_gemm<bn, a, b, deep>(ta, tb, M, N, K, splits, kb_per, a_rows, epi, status, st)
   if (A.mn && B.mn) {
-    if (BN == 64) QB_GEMM(64, true, true);
-    QB_GEMM(128, true, true);
+    if (BN == 64) QB_GEMM(64, true, true, true);
+    QB_GEMM(128, true, true, true);
   }
   if (B.mn) {
-    if (BN == 64) QB_GEMM(64, false, true);
-    QB_GEMM(128, false, true);
+    if (BN == 64) QB_GEMM(64, false, true, true);
+    QB_GEMM(128, false, true, true);
   }
   if (A.mn) return fail(PTYCHO_ERR_UNSUPPORTED, "gemm: an MN-major A goes with an MN-major B");
+  if (!t.deep) {
+    if (BN == 32) QB_GEMM(32, false, false, false);
+    QB_GEMM(64, false, false, false);
+  }
   switch (BN) {
-    case 16: QB_GEMM(16, false, false);
-    case 32: QB_GEMM(32, false, false);
-    case 64: QB_GEMM(64, false, false);
-    default: QB_GEMM(128, false, false);
+    case 16: QB_GEMM(16, false, false, true);
+    case 32: QB_GEMM(32, false, false, true);
+    case 64: QB_GEMM(64, false, false, true);
+    default: QB_GEMM(128, false, false, true);
   }
 #undef QB_GEMM
 }
@@ -543,6 +577,18 @@ int ptycho_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, in
                      const float* bias, int flags, int splits, int* status, void* stream) {
   return gemm_run({A, lda, false}, {B, ldb, false}, C, ldc, M, N, K, bias, flags, splits, status,
                   static_cast<cudaStream_t>(stream));
+}
+
+int ptycho_gemm_plan(int M, int N, int K, int splits, int a_mn, int b_mn, int* tile_n, int64_t* ctas, int* ctas_per_sm) {
+  if (M < 1 || N < 1 || K < 1 || (a_mn && !b_mn)) return fail(PTYCHO_ERR_INVALID, "gemm_plan: bad arguments");
+  const int nkb = (K + qb::gemm::BK - 1) / qb::gemm::BK;
+  splits = splits < 1 ? 1 : (splits > nkb ? nkb : splits);
+  const int kb_per = (nkb + splits - 1) / splits;
+  const Tile t = tile_of(M, N, (nkb + kb_per - 1) / kb_per, rows_of_a(M, a_mn != 0), b_mn != 0);
+  if (tile_n) *tile_n = t.bn;
+  if (ctas) *ctas = t.ctas;
+  if (ctas_per_sm) *ctas_per_sm = t.deep ? 1 : 2;
+  return PTYCHO_OK;
 }
 
 int ptycho_gemm_bf16_mn(const void* A, int lda, int a_mn, const void* B, int ldb, void* C, int ldc, int M, int N,

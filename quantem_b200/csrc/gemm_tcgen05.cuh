@@ -10,11 +10,12 @@
 // One CTA of 128 threads computes a 128 x BN tile:
 //   * warp 0, one lane: TMA producer.  Each k-block (64 bf16 = one 128-byte
 //     swizzle row) of A (128 x 64) and B (BN x 64) is copied by
-//     cp.async.bulk.tensor into a ring (160 to 200 KB) with the 128-byte swizzle; an mbarrier
-//     per stage counts the transaction bytes.  A stage holds 2 k-blocks, 5 of the narrow
-//     tiles: the products of the deep layers (K up to 9216 on one CTA per 16 columns) are
-//     bound by the turn-round of a stage (44 us with one k-block per stage, 36 with two, 30
-//     with five; the MMAs themselves take 16).
+//     cp.async.bulk.tensor into a ring with the 128-byte swizzle; an mbarrier per stage counts
+//     the transaction bytes.  The deep ring (180 to 200 KB) has stages of 2 k-blocks, 5 for the
+//     narrow tiles: the products of the deep layers (4 to 256 rows, K up to 9216 in one walk of 144
+//     k-blocks per CTA) are bound by the turn-round of a stage (16 x 1024 x 9216: 44 us with one
+//     k-block per stage, 36 with two, 29 with five; the MMAs themselves take 16).  The short
+//     ring (four stages of one k-block, 80 or 96 KB) lets two CTAs share an SM.
 //   * warp 1, one lane: MMA issuer.  tcgen05.mma.cta_group::1.kind::f16 with
 //     M = 128, N = BN, K = 16 (four per k-block), BF16 operands read from shared
 //     memory through matrix descriptors, FP32 accumulator in tensor memory
@@ -27,8 +28,8 @@
 // Out-of-range rows / columns / k of the tile are zero-filled by TMA and masked
 // in the epilogue, so M, N, K need no padding.  A K-major A of fewer than 128 rows is copied
 // in boxes of a_rows rows (a multiple of 8): the other rows of the tile hold whatever the
-// ring held, feed only accumulator rows that are not stored, and cost the copy engine nothing
-// (it takes about 2.4 ns per 128-byte row, the bound of the deep layers' products).
+// ring held, and feed only accumulator rows that are not stored.  4 x 1024 x 9216 takes 29 us so, 54
+// with boxes of 128 rows; from 16 rows on the two are equal.
 //
 // Every mbarrier wait is bounded by the global timer; on expiry the CTA records
 // a status code, still drains what it issued, frees TMEM and returns.
@@ -60,14 +61,15 @@ struct Epilogue {
   int act;  // qb::ACT_* applied to acc + bias
 };
 
-template <int BN>
+// DEEP: the ring fills an SM's shared memory; else two CTAs share an SM.
+template <int BN, bool DEEP>
 struct Smem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int KBS = BN >= 64 ? 2 : 5;  // k-blocks per stage
+  static constexpr int KBS = !DEEP ? 1 : (BN >= 64 ? 2 : 5);  // k-blocks per stage
   static constexpr int BLOCK_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGE_BYTES = KBS * BLOCK_BYTES;
-  static constexpr int STAGES = (BN >= 128 ? 6 : (BN == 64 ? 8 : 10)) / KBS;
+  static constexpr int STAGES = !DEEP ? 4 : (BN >= 128 ? 6 : (BN == 64 ? 8 : 10)) / KBS;
   static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;  // the smallest allocation
   static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
   static constexpr int BYTES = BAR_OFF + 256 + 1024;  // barriers + 1 KB alignment slack
@@ -165,13 +167,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool DEEP>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                         int N, int K, int kb_per_split, int a_rows, Epilogue epi, int* status) {
   static_assert(!B_MN || BN % 64 == 0, "an MN-major tile is copied in boxes of 64 values");
   static_assert(BN == 16 || BN == 32 || BN == 64 || BN == 128, "BN: a multiple of 16");
-  using L = Smem<BN>;
+  using L = Smem<BN, DEEP>;
   constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
