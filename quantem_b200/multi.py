@@ -6,7 +6,7 @@ positions, measured amplitudes).  Datasets that share a probe window run in one
 ``ptycho_forward_adjoint_multi`` launch whose CTAs are partitioned between them
 (datasets with 96 x 96 and 128 x 128 windows: one launch per window size);
 the partition comes from ``autotune_grids`` (timed candidates, cached per
-problem signature).  ``GraphedMultiIteration`` captures one full iteration of all
+problem signature and device).  ``GraphedMultiIteration`` captures one full iteration of all
 datasets (probe orthogonalisation and its autograd backward, hard constraint,
 the multi launch, reductions, constraint VJPs, Adam with device-side step
 counts) in a CUDA graph and replays it.
@@ -275,8 +275,10 @@ def autotune_grids(problems, total=None, trials=2, cache={}):
     Candidates: the cost-proportional split of the resident CTAs, of one and two CTAs per
     SM (``total`` and twice it, when given), and splits that move CTAs towards the datasets with
     the highest cost per CTA.  Each is timed (CUDA events) on the forward +
-    adjoint launch; the fastest is cached per problem signature."""
-    key = tuple(p.signature() for p in problems)
+    adjoint launch; the fastest is cached for these problems' sizes and kinds of propagators (factors
+    or whole arrays: other kernel paths), ``total`` and the device."""
+    key = (tuple(p.signature() + (isinstance(p.prop, (tuple, list)),) for p in problems), total,
+           str(problems[0].obj.device))
     if key in cache:
         return cache[key]
     sms = total or ops.sm_count(problems[0].obj.device)
