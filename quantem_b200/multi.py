@@ -47,6 +47,11 @@ class Problem:
         P, n, _ = self.probe.shape
         return (n, S, P, Ho, Wo, int(self.batch_idx.numel()))
 
+    def slots(self):
+        """Complex scratch values of one CTA: waves, far fields and the intensity tile."""
+        n, S, P, _, _, _ = self.signature()
+        return (P * S + P + 1) * n * n
+
     def cost(self):
         n, S, P, _, _, B = self.signature()
         return float(B) * P * (4 * S + 2)  # transforms per position: P(2S + 1) forward + P(2S + 1) adjoint
@@ -63,12 +68,15 @@ def _window_groups(problems):
 def default_grids(problems, total=None):
     """CTAs per dataset proportional to its transform count (at least one); each
     probe-window group (a launch of its own) splits ``total`` CTAs (default: as many as the
-    device holds at once for that window)."""
+    device holds at once for that window, or one per SM where their scratch would not fit)."""
     out = [0] * len(problems)
     for idx in _window_groups(problems):
         sub = [problems[i] for i in idx]
-        t = total or ops.resident_ctas(int(sub[0].probe.shape[-1]), sub[0].obj.device)
-        for i, g in zip(idx, _split(sub, t)):
+        dev = sub[0].obj.device
+        grids = _split(sub, total or ops.resident_ctas(int(sub[0].probe.shape[-1]), dev))
+        if not total and sum(g * p.slots() for g, p in zip(grids, sub)) * 8 > ops.free_bytes(dev):
+            grids = _split(sub, ops.sm_count(dev))
+        for i, g in zip(idx, grids):
             out[i] = g
     return out
 

@@ -84,6 +84,12 @@ def resident_ctas(n: int, device: torch.device | None = None) -> int:
     return grid.value
 
 
+def free_bytes(device) -> int:
+    """Device memory that new tensors can take: free, or kept by the allocator for reuse."""
+    return (torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device)
+            - torch.cuda.memory_allocated(device))
+
+
 def reduce_blocks() -> int:
     return int(_lib.lib().ptycho_reduce_blocks())
 
@@ -385,7 +391,17 @@ def plan_and_bind(a, device, adjoint: bool, grid=None):
         nn = a.n * a.n
         slots = a.P * a.S + a.P + 1 + (a.P * (a.S - 1) if a.grad_prop else 0)
         se.value, pe.value = grid_v * slots * nn, grid_v * a.P * nn
-    ws = workspace(device).ensure(se.value if adjoint else 0, pe.value if adjoint else 0, grid_v)
+    ws = workspace(device)
+    if not adjoint:
+        ws.ensure(0, 0, grid_v)
+    else:
+        try:
+            ws.ensure(se.value, pe.value, grid_v)
+        except torch.OutOfMemoryError:
+            sms = sm_count(torch.device(device))
+            if grid is not None or v.value != _lib.VARIANTS["serial"] or grid_v <= sms:
+                raise
+            return plan_and_bind(a, device, adjoint, grid=sms)  # one CTA per SM holds less scratch
     a.grid = grid_v
     a.scratch = ws.scratch.data_ptr() if adjoint else None
     a.probe_grad_part = ws.partials.data_ptr() if adjoint else None

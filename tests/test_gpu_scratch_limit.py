@@ -1,0 +1,48 @@
+"""Small windows run several CTAs per SM; where the scratch of so many does not fit on the device the
+launch takes one per SM, which is what earlier memory plans were made for."""
+import pytest
+import torch
+
+from quantem_b200 import ops
+from tests.conftest import rel
+from tests.test_gpu_batch_paths import _problem
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [64, 96])
+def test_less_memory_than_the_resident_ctas_take(cuda_device, monkeypatch, n):
+    B = 2 * ops.resident_ctas(n)
+    sms = ops.sm_count()
+    obj, probe, prop, pos, targets = _problem(n, 2, 2, B, n + 20, n + 25)
+    idx, mask = torch.arange(B, device="cuda"), torch.ones((n, n), device="cuda")
+
+    def run():
+        return ops.batch_forward_adjoint(obj, probe, prop, pos, idx, targets, mask, B, 100.0)
+
+    want = run()
+    limit = sms * (2 * 2 + 2 + 1) * n * n  # the scratch of one CTA per SM
+    ensure, grids = ops.Workspace.ensure, []
+
+    def small(self, scratch_elems, partial_elems, grid):
+        if scratch_elems > limit:
+            raise torch.OutOfMemoryError("no memory")
+        grids.append(grid)
+        return ensure(self, scratch_elems, partial_elems, grid)
+
+    monkeypatch.setattr(ops.Workspace, "ensure", small)
+    got = run()
+    assert grids == [sms]
+    assert abs(float(got[0]) - float(want[0])) < 1e-6 * abs(float(want[0]))
+    for a, b in zip(got[1:], want[1:]):  # sums of the same terms in another order
+        assert rel(a.cpu().numpy(), b.cpu().numpy()) < 4e-7 * B ** 0.5
+
+
+def test_partition_of_several_datasets(cuda_device, monkeypatch):
+    from quantem_b200 import multi
+    from tests.test_gpu_multi import _problems
+
+    probs = _problems(cuda_device, [(20, 3, 2), (22, 2, 2)])
+    assert sum(multi.default_grids(probs)) == ops.resident_ctas(64)
+    monkeypatch.setattr(ops, "free_bytes", lambda device: 0)
+    assert sum(multi.default_grids(probs)) == ops.sm_count()
