@@ -88,7 +88,8 @@ typedef struct ptycho_batch_args {
                                 (those positions are skipped); each field saturates at its
                                 maximum instead of carrying into the next */
   const void* prop_r;        /* optional complex64 (S-1, N): separable propagator factors, */
-  const void* prop_c;        /*   K_s[kr][kc] = prop_r[s][kr] * prop_c[s][kc] (kept in shared memory) */
+  const void* prop_c;        /*   K_s[kr][kc] = prop_r[s][kr] * prop_c[s][kc]; up to 176, 73, 15
+                              *   slices at N = 64, 96, 128 */
   int n, S, P, B, Ho, Wo, npos, grid;
   int loss_type;             /* PTYCHO_LOSS_* */
   float loss_scale;          /* npos_total / (B * mean_intensity) */
@@ -199,7 +200,7 @@ int ptycho_obj_blur(const void* in, void* out, void* tmp, int S, int Ho, int Wo,
 /* Butterworth filter (object_models.py:481-520): per slice, mean removed, ifft2(fft2(x)
  * env), mean added back (the real part for a real potential, is_real = 1); env: float32
  * (Ho, Wo) envelope on the fftfreq grid.  The 2-D transform runs along lines of any length
- * (object sides <= 6144).  tmp: complex64 2 * S * Ho * Wo; means: complex64 2 * S.
+ * (object sides <= 6144).  tmp: complex64 S * Ho * Wo; means: complex64 S.
  * The filter is self-adjoint: the VJP is P g - mean(P g) + mean(g) per slice. */
 int ptycho_obj_butterworth(const void* in, void* out, int S, int Ho, int Wo, int is_real, const float* env, void* tmp,
                            void* means, void* stream);
@@ -471,7 +472,7 @@ int ptycho_cnn_transpose(const void* in, int in_dtype, int R, int C, int ldi, in
  * statistics (biased variance for normalisation, running statistics updated with
  * the unbiased one and `momentum`), else running statistics.  gamma == NULL skips
  * the normalisation (plain BF16 conversion).  Writes the used mean / rstd.
- * `work` holds >= 2 * C doubles (more gives more parallel partial sums). */
+ * `work` is not used any more; work_elems >= 2 * C is still required (training). */
 int ptycho_cnn_bn_forward(const float* x, int ldx, int R, int C, const float* gamma, const float* beta,
                           float* run_mean, float* run_var, float momentum, float eps, int training, float* mean,
                           float* rstd, double* work, int64_t work_elems, void* out, int ldo, void* stream);

@@ -493,11 +493,9 @@ int validate_batch(const ptycho_batch_args* a, bool adj) {
     return fail(PTYCHO_ERR_INVALID, "propagators are NULL with S > 1");
   if ((a->prop_r == nullptr) != (a->prop_c == nullptr))
     return fail(PTYCHO_ERR_INVALID, "prop_r and prop_c must be given together");
-  if (a->prop_r && a->n != 256) {  // n = 256 reads the factors through the L1 cache
-    if (qb::sep_limit_bytes(a->n, a->S) > qb::kMaxSmem)
-      return fail(PTYCHO_ERR_UNSUPPORTED, "separable propagators of %d slices do not fit in shared memory; pass prop",
-                  a->S);
-  }
+  if (a->prop_r && a->S > qb::sep_max_slices(a->n))
+    return fail(PTYCHO_ERR_UNSUPPORTED, "separable propagators are taken for up to %d slices at n=%d (S=%d); pass prop",
+                qb::sep_max_slices(a->n), a->n, a->S);
   if (adj && (!a->grad_obj || !a->probe_grad_part || !a->scratch))
     return fail(PTYCHO_ERR_INVALID, "adjoint buffers are NULL");
   const void* ptrs[] = {a->obj, a->probe_hat, a->prop, a->grad_obj, a->probe_grad_part, a->scratch, a->out_exit,

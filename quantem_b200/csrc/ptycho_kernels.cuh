@@ -182,14 +182,10 @@ template <int N>
 constexpr bool sep_in_smem(bool tile, int S) {
   return batch_smem_bytes<N>(tile, true, S) <= max_smem<N>(Fft2<N>::CTAS);
 }
-// Slices accepted with separable propagators: the bound of the interface (a tile of
-// N (N + 1) complex values, 3 N more, the intensity tile, the maps and the factors of
-// every slice within one SM), whatever a kernel keeps in shared memory itself.
-constexpr size_t sep_limit_bytes(int n, int S) {
-  return sizeof(float2) * ((n == 96 ? (size_t)9976 : (size_t)n * (n + 1)) + 3 * (size_t)n) +
-         sizeof(float) * (size_t)n * n + sizeof(int) * 2 * (size_t)n +
-         sizeof(float2) * 2 * (size_t)n * (size_t)(S > 1 ? S - 1 : 0);
-}
+// Slices accepted with separable propagators, a bound of the interface: what one SM's shared memory
+// holds beside a wave, its intensity tile and its maps, although the kernels read factors that do not fit
+// beside their own buffers through the L1 cache.  No bound at 256^2.
+constexpr int sep_max_slices(int n) { return n == 64 ? 176 : (n == 96 ? 73 : (n == 128 ? 15 : 1 << 30)); }
 
 template <int N>
 __device__ __forceinline__ void loss_elem(const BatchParams& p, float I, float t, float m,
