@@ -338,6 +338,7 @@ def check_status(device=None) -> dict:
 
 
 def default_grid(B: int, device=None) -> int:
+    """One CTA per SM, at most one per position: an explicit grid with the smallest scratch."""
     return max(1, min(B, sm_count(device)))
 
 
@@ -885,8 +886,8 @@ def _butter(x: torch.Tensor, env: torch.Tensor, vjp: bool) -> torch.Tensor:
     x = dense(x)
     S, Ho, Wo = (int(d) for d in x.shape)
     out = torch.empty_like(x)
-    tmp = torch.empty((2, S, Ho, Wo), dtype=torch.complex64, device=x.device)
-    means = torch.empty((2, S), dtype=torch.complex64, device=x.device)
+    tmp = torch.empty((S, Ho, Wo), dtype=torch.complex64, device=x.device)
+    means = torch.empty(S, dtype=torch.complex64, device=x.device)
     fn = _lib.lib().ptycho_obj_butterworth_vjp if vjp else _lib.lib().ptycho_obj_butterworth
     _lib.check(fn(_p(x), _p(out), S, Ho, Wo, int(not x.is_complex()), _p(env), _p(tmp), _p(means), _stream()),
                "obj_butterworth" + ("_vjp" if vjp else ""))
