@@ -472,7 +472,8 @@ int ptycho_cnn_transpose(const void* in, int in_dtype, int R, int C, int ldi, in
  * statistics (biased variance for normalisation, running statistics updated with
  * the unbiased one and `momentum`), else running statistics.  gamma == NULL skips
  * the normalisation (plain BF16 conversion).  Writes the used mean / rstd.
- * `work` is not used any more; work_elems >= 2 * C is still required (training). */
+ * `work` holds >= 2 * C doubles (training); with 1184 * C of them many rows are summed over
+ * all SMs. */
 int ptycho_cnn_bn_forward(const float* x, int ldx, int R, int C, const float* gamma, const float* beta,
                           float* run_mean, float* run_var, float momentum, float eps, int training, float* mean,
                           float* rstd, double* work, int64_t work_elems, void* out, int ldo, void* stream);

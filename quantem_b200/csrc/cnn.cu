@@ -523,18 +523,27 @@ int bn_check(const qb::bn::Backward& b, int R, int C) {
     return fail(PTYCHO_ERR_INVALID, "bn_backward: missing buffers");
   return PTYCHO_OK;
 }
-int bn_forward(const qb::bn::Forward& f, int R, int C, cudaStream_t st) {
+// work: scratch for the partial sums of many rows (may be NULL or too small: the cluster launch runs)
+bool bn_wide(int R, int C, bool forward, bool sums, const double* work, int64_t work_elems) {
+  return qb::bn::wide(R, forward && sums) && (!sums || (work && (reinterpret_cast<uintptr_t>(work) & 7) == 0 &&
+                                          work_elems >= qb::bn::wide_elems(R, C)));
+}
+int bn_forward(const qb::bn::Forward& f, int R, int C, double* work, int64_t work_elems, cudaStream_t st) {
   if (int rc = bn_check(f, R, C)) return rc;
   if (!f.gamma) {
     to_bf16_kernel<<<blocks_for((int64_t)R * C, 256), 256, 0, st>>>(f.x, f.ldx, R, C, f.y, f.ldy);
     return check_launch("to_bf16_kernel");
   }
-  const cudaError_t e = qb::bn::launch(qb::bn::bn_forward_kernel, f, R, C, st);
+  const cudaError_t e = bn_wide(R, C, true, f.training, work, work_elems)
+                            ? qb::bn::launch_wide(f, R, C, work, st)
+                            : qb::bn::launch(qb::bn::bn_forward_kernel, f, R, C, st);
   return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_forward_kernel: %s", cudaGetErrorString(e));
 }
-int bn_backward(const qb::bn::Backward& b, int R, int C, cudaStream_t st) {
+int bn_backward(const qb::bn::Backward& b, int R, int C, double* work, int64_t work_elems, cudaStream_t st) {
   if (int rc = bn_check(b, R, C)) return rc;
-  const cudaError_t e = qb::bn::launch(qb::bn::bn_backward_kernel, b, R, C, st);
+  const cudaError_t e = bn_wide(R, C, false, b.gamma || b.dbias, work, work_elems)
+                            ? qb::bn::launch_wide(b, R, C, work, st)
+                            : qb::bn::launch(qb::bn::bn_backward_kernel, b, R, C, st);
   return e == cudaSuccess ? PTYCHO_OK : fail(PTYCHO_ERR_CUDA, "bn_backward_kernel: %s", cudaGetErrorString(e));
 }
 
@@ -670,7 +679,7 @@ int ptycho_cnn_bn_forward(const float* x, int ldx, int R, int C, const float* ga
   if (int rc = bn_check(f, R, C)) return rc;
   if (gamma && training)
     if (int rc = work_check(C, work_elems)) return rc;
-  return bn_forward(f, R, C, static_cast<cudaStream_t>(stream));
+  return bn_forward(f, R, C, work, work_elems, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_bn_backward(const float* dy, int lddy, const float* x, int ldx, int R, int C, const float* gamma,
@@ -681,7 +690,7 @@ int ptycho_cnn_bn_backward(const float* dy, int lddy, const float* x, int ldx, i
   if (int rc = bn_check(b, R, C)) return rc;
   if (gamma)
     if (int rc = work_check(C, work_elems)) return rc;
-  return bn_backward(b, R, C, static_cast<cudaStream_t>(stream));
+  return bn_backward(b, R, C, work, work_elems, static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_colsum(const float* a, int lda, int R, int C, float* out, int accumulate, double* work,
@@ -787,7 +796,8 @@ int ptycho_cnn_conv_forward(const void* x, int ldx, int B, int H, int W, int C, 
   if (int rc = ptycho_gemm_bf16(col, 9 * C, w, 9 * C, r, co, R, co, 9 * C, bias, act << 8, 1, nullptr, stream))
     return rc;
   if (!out) return PTYCHO_OK;
-  return bn_forward(f, R, co, static_cast<cudaStream_t>(stream));
+  // the patches are used up: their memory takes the partial sums
+  return bn_forward(f, R, co, static_cast<double*>(col), (int64_t)R * 9 * C / 4, static_cast<cudaStream_t>(stream));
 }
 
 namespace {
@@ -817,7 +827,7 @@ int ptycho_cnn_conv_backward(const float* dy, int lddy, const void* x, int ldx, 
     return bad_args("conv_backward");
   if (int rc = bn_backward({dy, lddy, r, co, gamma, mean, rstd, training, act, dgamma, dbeta, db, nullptr,
                             static_cast<bf16*>(dz), ldz},
-                           R, co, st))
+                           R, co, static_cast<double*>(col), (int64_t)R * K9 / 4, st))
     return rc;
   // weight gradient dz^T col
   if (int rc = ptycho_cnn_im2col3x3(x, B, H, W, C, ldx, col, K9, stream)) return rc;
@@ -842,7 +852,9 @@ int ptycho_cnn_up_forward(const void* y, int ldy, int B, int H, int W, int ci, i
     return rc;
   if (int rc = ptycho_cnn_convT_gather(colT, 9 * ci, B, H, W, ci, bt, t, ci, stream)) return rc;
   if (int rc = ptycho_gemm_bf16(t, ci, w1, ci, r, co, R, co, ci, b1, 0, 1, nullptr, stream)) return rc;
-  return bn_forward(f, R, co, static_cast<cudaStream_t>(stream));
+  // the transposed convolution's products are used up
+  return bn_forward(f, R, co, reinterpret_cast<double*>(colT), (int64_t)Rin * 9 * ci / 2,
+                    static_cast<cudaStream_t>(stream));
 }
 
 int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, const void* t, const float* r, int B,
@@ -859,7 +871,7 @@ int ptycho_cnn_up_backward(const float* dup, int lddup, const void* y, int ldy, 
   if (int rc = work_check(ci, work_elems)) return rc;
   if (int rc = bn_backward({dup, lddup, r, co, gamma, mean, rstd, training, 0, dgamma, dbeta, db1, nullptr,
                             static_cast<bf16*>(dz), ldz},
-                           R, co, st))
+                           R, co, work, work_elems, st))
     return rc;
   // 1x1 convolution: dw1 = dz^T t, dt = dz w1
   if (int rc = wgrad(dz, ldz, t, ci, dw1, co, ci, R, st)) return rc;

@@ -9,6 +9,9 @@
 // to 592 partials and separate elementwise and bias-gradient passes, the batch norms of one
 // training step of the 5-level network took 229 launches and 1.3 ms.
 //
+// Many rows take separate launches over all SMs instead (below): a cluster per sector of channels leaves
+// most of the device idle then.
+//
 // The float runs are those of a fixed partition of the rows (BnRows), whatever the cluster: the
 // statistics feed BF16 roundings, so they keep their values from one launch shape to the next.
 #pragma once
@@ -186,6 +189,36 @@ struct Backward {
   int ldz;
 };
 
+// Up to eight rows r, r + step, ... < end of dz for channel c; returns their sum.
+__device__ __forceinline__ float dz_rows(const Backward& p, int r, int step, int end, int c, float m, float rs, float ga,
+                                         float sdy, float sdx, float invR) {
+  float xv[8], g[8], f = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (r + j * step < end) {
+      xv[j] = p.x[(int64_t)(r + j * step) * p.ldx + c];
+      g[j] = p.dy[(int64_t)(r + j * step) * p.lddy + c];
+    }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (r + j * step < end) {
+      if (p.gamma) {
+        if (p.training) {
+          const float xh = (xv[j] - m) * rs;
+          g[j] = ga * rs * (g[j] - sdy * invR - xh * sdx * invR);
+        } else {
+          g[j] = g[j] * ga * rs;
+        }
+      }
+      if (p.act) g[j] *= act_grad_from_output(p.act, xv[j]);
+      const int64_t o = (int64_t)(r + j * step) * p.ldz + c;
+      if (p.dz32) p.dz32[o] = g[j];
+      if (p.dz16) p.dz16[o] = __float2bfloat16_rn(g[j]);
+      f += g[j];
+    }
+  return f;
+}
+
 // dz = act'(x) gamma rstd (dy - s_dy / R - xhat s_dyxhat / R) (training statistics),
 // act'(x) dy gamma rstd (running statistics), act'(x) dy (no batch norm).
 __global__ void __launch_bounds__(kThreads) bn_backward_kernel(const Backward p, const BnRows rows, int CW) {
@@ -223,41 +256,160 @@ __global__ void __launch_bounds__(kThreads) bn_backward_kernel(const Backward p,
   }
   const float invR = 1.0f / (float)rows.R;
   double sum[2] = {0.0, 0.0};
-  if (on) {
-    for (int r = slot; r < rows.R; r += 8 * nslots) {
-      float xv[8], g[8], f = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (r + j * nslots < rows.R) {
-          xv[j] = p.x[(int64_t)(r + j * nslots) * p.ldx + c];
-          g[j] = p.dy[(int64_t)(r + j * nslots) * p.lddy + c];
-        }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (r + j * nslots < rows.R) {
-          if (p.gamma) {
-            if (p.training) {
-              const float xh = (xv[j] - m) * rs;
-              g[j] = ga * rs * (g[j] - sdy * invR - xh * sdx * invR);
-            } else {
-              g[j] = g[j] * ga * rs;
-            }
-          }
-          if (p.act) g[j] *= act_grad_from_output(p.act, xv[j]);
-          const int64_t o = (int64_t)(r + j * nslots) * p.ldz + c;
-          if (p.dz32) p.dz32[o] = g[j];
-          if (p.dz16) p.dz16[o] = __float2bfloat16_rn(g[j]);
-          f += g[j];
-        }
-      sum[0] += f;
-    }
-  }
+  if (on)
+    for (int r = slot; r < rows.R; r += 8 * nslots)
+      sum[0] += dz_rows(p, r, nslots, rows.R, c, m, rs, ga, sdy, sdx, invR);
   if (p.dbias) {
     if (p.gamma) cl.sync();  // every CTA has read the first sums' slots
     cluster_sums<2>(sm, sum, CW);
     if (on && first) p.dbias[c] = (float)sum[0];
   }
   if (p.gamma || p.dbias) cl.sync();  // no CTA leaves while a peer may still write its slots
+}
+
+// ---- many rows: separate launches over all SMs ----
+// A cluster's channels are at least one 32-byte sector wide, so C / 8 clusters of 8 CTAs are all that
+// the kernels above can put to work: at 32 channels 32 CTAs, whatever the number of rows.  Here blocks
+// of 256 threads (a thread: one channel, every RP-th row of a chunk, the same float runs) write partial
+// sums, a warp per channel adds them in a fixed order, and an elementwise pass follows.
+constexpr int kWideThreads = 256;
+
+struct WideRows {
+  int c, first, step, end;  // this thread's channel and rows
+  bool on;
+  __device__ __forceinline__ WideRows(const BnRows& rows) {
+    const int tc = rows.C < kWideThreads ? rows.C : kWideThreads;
+    const int tx = threadIdx.x % tc, ty = threadIdx.x / tc, r0 = blockIdx.x * rows.rpc;
+    c = blockIdx.y * tc + tx;
+    on = ty < rows.RP && c < rows.C;
+    first = r0 + ty;
+    step = rows.RP;
+    end = min(rows.R, r0 + rows.rpc);
+  }
+};
+// Sums of v over the threads of a channel, in the first row of threads
+template <int NV>
+__device__ __forceinline__ void wide_block_sums(double (&v)[NV], const BnRows& rows) {
+  __shared__ double red[NV][kWideThreads];
+  const int tc = rows.C < kWideThreads ? rows.C : kWideThreads;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) red[i][threadIdx.x] = v[i];
+  __syncthreads();
+  if ((int)threadIdx.x < tc)
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+      for (int k = 1; k < rows.RP; ++k) v[i] += red[i][k * tc + threadIdx.x];
+}
+
+// part[(2 chunk + i) C + c]: sums of x and x^2 (forward), of dy and dy xhat (backward)
+__global__ void __launch_bounds__(kWideThreads)
+    wide_forward_sums_kernel(const Forward p, const BnRows rows, double* __restrict__ part) {
+  const WideRows w(rows);
+  double v[2] = {0.0, 0.0};
+  if (w.on)
+    run_sums(w.first, w.end, w.step, v, [&](int r, float& a, float& b) { a = b = p.x[(int64_t)r * p.ldx + w.c]; });
+  wide_block_sums<2>(v, rows);
+  if (w.on && w.first == (int)blockIdx.x * rows.rpc)
+    for (int i = 0; i < 2; ++i) part[((int64_t)blockIdx.x * 2 + i) * rows.C + w.c] = v[i];
+}
+__global__ void __launch_bounds__(kWideThreads)
+    wide_backward_sums_kernel(const Backward p, const BnRows rows, double* __restrict__ part) {
+  const WideRows w(rows);
+  double v[2] = {0.0, 0.0};
+  if (w.on) {
+    const float m = p.mean[w.c], rs = p.rstd[w.c];
+    run_sums(w.first, w.end, w.step, v, [&](int r, float& a, float& b) {
+      a = p.dy[(int64_t)r * p.lddy + w.c];
+      b = (p.x[(int64_t)r * p.ldx + w.c] - m) * rs;
+    });
+  }
+  wide_block_sums<2>(v, rows);
+  if (w.on && w.first == (int)blockIdx.x * rows.rpc)
+    for (int i = 0; i < 2; ++i) part[((int64_t)blockIdx.x * 2 + i) * rows.C + w.c] = v[i];
+}
+// Sum of value i of every chunk for channel c, one warp
+__device__ __forceinline__ double wide_total(const double* part, int chunks, int nv, int i, int C, int c) {
+  double t = 0.0;
+  for (int k = threadIdx.x & 31; k < chunks; k += 32) t += part[((int64_t)k * nv + i) * C + c];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+__global__ void __launch_bounds__(kWideThreads)
+    wide_forward_stats_kernel(const Forward p, const BnRows rows, int chunks, const double* __restrict__ part) {
+  const int c = blockIdx.x * (kWideThreads / 32) + (threadIdx.x >> 5);
+  if (c >= rows.C) return;
+  const double s0 = wide_total(part, chunks, 2, 0, rows.C, c), s1 = wide_total(part, chunks, 2, 1, rows.C, c);
+  if (threadIdx.x & 31) return;
+  const double mean = s0 / rows.R;
+  double var = s1 / rows.R - mean * mean;
+  if (var < 0.0) var = 0.0;
+  p.mean[c] = (float)mean;
+  p.rstd[c] = (float)(1.0 / sqrt(var + (double)p.eps));
+  if (p.run_mean) {
+    const double unb = rows.R > 1 ? var * rows.R / (rows.R - 1) : var;
+    p.run_mean[c] = (float)((1.0 - p.momentum) * p.run_mean[c] + p.momentum * mean);
+    p.run_var[c] = (float)((1.0 - p.momentum) * p.run_var[c] + p.momentum * unb);
+  }
+}
+// out0[c], out1[c] = sums 0 and 1 of nv per chunk (out1 may be NULL)
+__global__ void __launch_bounds__(kWideThreads)
+    wide_totals_kernel(const double* __restrict__ part, int chunks, int nv, int C, float* out0, float* out1) {
+  const int c = blockIdx.x * (kWideThreads / 32) + (threadIdx.x >> 5);
+  if (c >= C) return;
+  const double s0 = wide_total(part, chunks, nv, 0, C, c), s1 = out1 ? wide_total(part, chunks, nv, 1, C, c) : 0.0;
+  if (threadIdx.x & 31) return;
+  out0[c] = (float)s0;
+  if (out1) out1[c] = (float)s1;
+}
+__global__ void __launch_bounds__(kWideThreads) wide_forward_kernel(const Forward p, const BnRows rows) {
+  const WideRows w(rows);
+  if (!w.on) return;
+  float m, rs;
+  if (p.training) {
+    m = p.mean[w.c];
+    rs = p.rstd[w.c];
+  } else {
+    m = p.run_mean[w.c];
+    rs = rsqrtf(p.run_var[w.c] + p.eps);
+    if (w.first == 0) {
+      p.mean[w.c] = m;
+      p.rstd[w.c] = rs;
+    }
+  }
+  const float g = p.gamma[w.c], b = p.beta[w.c];
+  for (int r = w.first; r < w.end; r += 8 * w.step) {
+    float a[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (r + j * w.step < w.end) a[j] = p.x[(int64_t)(r + j * w.step) * p.ldx + w.c];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (r + j * w.step < w.end)
+        p.y[(int64_t)(r + j * w.step) * p.ldy + w.c] = __float2bfloat16_rn((a[j] - m) * rs * g + b);
+  }
+}
+// dz; part[chunk C + c]: its sums (with dbias)
+__global__ void __launch_bounds__(kWideThreads)
+    wide_backward_kernel(const Backward p, const BnRows rows, double* __restrict__ part) {
+  const WideRows w(rows);
+  double sum[1] = {0.0};
+  if (w.on) {
+    float m = 0.f, rs = 0.f, ga = 0.f, sdy = 0.f, sdx = 0.f;
+    if (p.gamma) {
+      m = p.mean[w.c];
+      rs = p.rstd[w.c];
+      ga = p.gamma[w.c];
+      sdy = p.dbeta[w.c];
+      sdx = p.dgamma[w.c];
+    }
+    const float invR = 1.0f / (float)rows.R;
+    for (int r = w.first; r < w.end; r += 8 * w.step)
+      sum[0] += dz_rows(p, r, w.step, w.end, w.c, m, rs, ga, sdy, sdx, invR);
+  }
+  if (p.dbias) {
+    wide_block_sums<1>(sum, rows);
+    if (w.on && w.first == (int)blockIdx.x * rows.rpc) part[(int64_t)blockIdx.x * rows.C + w.c] = sum[0];
+  }
 }
 
 // Channels per warp and CTAs per cluster: enough rows per CTA to keep its warps busy, and
@@ -285,6 +437,43 @@ cudaError_t launch(void (*kernel)(P, BnRows, int), const P& p, int R, int C, cud
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, p, BnRows(R, C), s.cw);
+}
+
+// Where the launches over all SMs replace the cluster launch: from 32768 rows in the forward with batch
+// statistics (three launches; device times at 32 channels: 8192 rows 9.4 us against 7.2, 16384 rows 9.2
+// against 9.9, 32768 rows 10.6 against 15.4, 262144 rows 27 against 87; at 128 channels 16384 rows
+// 16.6 against 15.2, 32768 rows 21.6 against 25.8), from 16384 rows in the other passes (backward at 32
+// channels: 8192 rows 11.7 us against 10.6, 16384 rows 11.9 against 16.6, 262144 rows 43 against 260;
+// running statistics, 16384 rows: 3.3 against 5.5).
+inline bool wide(int R, bool batch_stats_forward) { return R >= (batch_stats_forward ? 32768 : 16384); }
+
+// Partial sums (doubles) of the wide launches
+inline int64_t wide_elems(int R, int C) {
+  const BnRows rows(R, C);
+  return (int64_t)2 * (rows.runs / rows.RP) * C;
+}
+inline cudaError_t launch_wide(const Forward& p, int R, int C, double* part, cudaStream_t st) {
+  const BnRows rows(R, C);
+  const int chunks = rows.runs / rows.RP, tiles = (C + kWideThreads - 1) / kWideThreads;
+  const dim3 grid(chunks, tiles);
+  if (p.training) {
+    wide_forward_sums_kernel<<<grid, kWideThreads, 0, st>>>(p, rows, part);
+    wide_forward_stats_kernel<<<(C + 7) / 8, kWideThreads, 0, st>>>(p, rows, chunks, part);
+  }
+  wide_forward_kernel<<<grid, kWideThreads, 0, st>>>(p, rows);
+  return cudaGetLastError();
+}
+inline cudaError_t launch_wide(const Backward& p, int R, int C, double* part, cudaStream_t st) {
+  const BnRows rows(R, C);
+  const int chunks = rows.runs / rows.RP, tiles = (C + kWideThreads - 1) / kWideThreads;
+  const dim3 grid(chunks, tiles);
+  if (p.gamma) {
+    wide_backward_sums_kernel<<<grid, kWideThreads, 0, st>>>(p, rows, part);
+    wide_totals_kernel<<<(C + 7) / 8, kWideThreads, 0, st>>>(part, chunks, 2, C, p.dbeta, p.dgamma);
+  }
+  wide_backward_kernel<<<grid, kWideThreads, 0, st>>>(p, rows, part);
+  if (p.dbias) wide_totals_kernel<<<(C + 7) / 8, kWideThreads, 0, st>>>(part, chunks, 1, C, p.dbias, nullptr);
+  return cudaGetLastError();
 }
 
 }  // namespace bn
