@@ -421,131 +421,190 @@ __global__ void surface_sign_kernel(const float* __restrict__ obj, int S, int64_
   }
 }
 
-// A block marches a 32 x 8 tile through the slices: the phase and amplitude of the tile and its
-// one-element halo are evaluated once per slice into shared memory (two slices alternate), the
-// slice before stays in registers.  Bound by atan2 and hypot (1.33 per element and slice); one
-// evaluation per stencil point (7) took 95 us at 8 x 510 x 516.
-constexpr int kSoftX = 32, kSoftY = 8;
+// Weights and surface terms of one launch (object_models.py:398-411): z with wz (3-D arrays, S > 1),
+// rows and columns with wxy; each term w mean|diff| divided by the number of weighted dimensions.
+struct SoftTerms {
+  float c0, c1, c2, wsurf, inv_hw, m0, m1, sg0, sg1;
+  bool surf;
+};
 template <int KIND>
-__global__ void __launch_bounds__(kThreads) soft_loss_kernel(const float* __restrict__ obj, int S, int Ho, int Wo,
-                                                             float wz, float wxy, float wsurf,
-                                                             float* __restrict__ grad, double* work) {
+__device__ SoftTerms soft_terms(int S, int Ho, int Wo, float wz, float wxy, float wsurf, const double* work) {
+  const int64_t hw = (int64_t)Ho * Wo;
+  SoftTerms t = {0.f, 0.f, 0.f, wsurf, 1.0f / (float)hw, 0.f, 0.f, 0.f, 0.f, wsurf > 0.f && S >= 3};
+  if (t.surf && KIND != 2) {
+    t.m0 = (float)(partials_sum(work + kBlocks, kBlocks) / (double)hw);
+    __syncthreads();
+    t.m1 = (float)(partials_sum(work + 2 * kBlocks, kBlocks) / (double)hw);
+    __syncthreads();
+    t.sg0 = (float)(partials_sum(work + 3 * kBlocks, kBlocks) / (double)hw);
+    __syncthreads();
+    t.sg1 = (float)(partials_sum(work + 4 * kBlocks, kBlocks) / (double)hw);
+  }
+  const float w0 = S > 1 ? wz : 0.f;
+  const int nd = (w0 > 0.f) + 2 * (wxy > 0.f);
+  if (nd && w0 > 0.f) t.c0 = w0 / (nd * (float)((int64_t)(S - 1) * hw));
+  if (nd && wxy > 0.f) {
+    t.c1 = wxy / (nd * (float)((int64_t)S * (Ho - 1) * Wo));
+    t.c2 = wxy / (nd * (float)((int64_t)S * Ho * (Wo - 1)));
+  }
+  return t;
+}
+// Loss terms (into lacc) and gradient of element i of slice s.  tv(dim) yields each weighted dimension's
+// neighbours: per dimension the loss term of the diff to the next element, the gradient from the diffs on
+// both sides.
+template <int KIND, typename TV>
+__device__ __forceinline__ void soft_element(const float* obj, float* grad, int64_t i, int s, int S, const SoftTerms& t,
+                                             float2 here, double& lacc, TV tv) {
+  constexpr bool amp_terms = KIND == 0;
+  const float ph = here.x, amp = here.y;
+  float gph = 0.f, gamp = 0.f;
+  auto dim = [&](float cw, bool has_lo, auto lo, bool has_hi, auto hi) {
+    if (cw == 0.f) return;
+    if (has_hi) {
+      const float2 q = hi();
+      const float d = q.x - ph;
+      lacc += (double)(cw * fabsf(d));
+      gph -= cw * sgnf(d);
+      if (amp_terms) {
+        const float da = q.y - amp;
+        lacc += (double)(cw * fabsf(da));
+        gamp -= cw * sgnf(da);
+      }
+    }
+    if (has_lo) {
+      const float2 q = lo();
+      gph += cw * sgnf(ph - q.x);
+      if (amp_terms) gamp += cw * sgnf(amp - q.y);
+    }
+  };
+  tv(dim);
+  if (t.surf && (s == 0 || s == S - 1)) {
+    if (KIND == 2) {
+      lacc += (double)(t.wsurf * fabsf(ph) * t.inv_hw);
+      gph += t.wsurf * sgnf(ph) * t.inv_hw;
+    } else {
+      const float m = s == 0 ? t.m0 : t.m1, sgm = s == 0 ? t.sg0 : t.sg1;
+      const float u = fabsf(ph) - m;
+      lacc += (double)(t.wsurf * fabsf(u) * t.inv_hw);
+      gph += t.wsurf * (sgnf(u) - sgm) * t.inv_hw * sgnf(ph);
+      if (amp_terms) {
+        lacc += (double)(t.wsurf * (1.0f - amp) * t.inv_hw);
+        gamp -= t.wsurf * t.inv_hw;
+      }
+    }
+  }
+  if (KIND == 2) {
+    grad[i] = gph;
+  } else {
+    const float2 o = reinterpret_cast<const float2*>(obj)[i];
+    float2 gz = make_float2(0.f, 0.f);
+    if (amp != 0.f) {  // G = g_amp z / |z| + i g_phase z / |z|^2 (zero at a zero pixel)
+      const float inv = 1.0f / amp;
+      gz.x = gamp * o.x * inv - gph * o.y * inv * inv;
+      gz.y = gamp * o.y * inv + gph * o.x * inv * inv;
+    }
+    reinterpret_cast<float2*>(grad)[i] = gz;
+  }
+}
+
+// One thread per element, the stencil's values read (and for complex objects evaluated, up to seven times)
+// where they are needed.
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) soft_direct_kernel(const float* __restrict__ obj, int S, int Ho, int Wo,
+                                                               float wz, float wxy, float wsurf,
+                                                               float* __restrict__ grad, double* work) {
+  __shared__ double red[32];
+  const int64_t hw = (int64_t)Ho * Wo, n = (int64_t)S * hw;
+  const SoftTerms t = soft_terms<KIND>(S, Ho, Wo, wz, wxy, wsurf, work);
+  double lacc = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int s = (int)(i / hw);
+    const int64_t p = i % hw;
+    const int r = (int)(p / Wo), c = (int)(p % Wo);
+    auto at = [&](int64_t k) {
+      return [&obj, k] {
+        float ph, amp;
+        values_at<KIND>(obj, k, ph, amp);
+        return make_float2(ph, amp);
+      };
+    };
+    soft_element<KIND>(obj, grad, i, s, S, t, at(i)(), lacc, [&](auto dim) {
+      dim(t.c0, s > 0, at(i - hw), s < S - 1, at(i + hw));
+      dim(t.c1, r > 0, at(i - Wo), r < Ho - 1, at(i + Wo));
+      dim(t.c2, c > 0, at(i - 1), c < Wo - 1, at(i + 1));
+    });
+  }
+  const double sum = block_sum_d(lacc, red);
+  if (threadIdx.x == 0) work[blockIdx.x] = sum;
+}
+
+// Complex objects of large planes: a block marches a 32 x 8 tile through `run` slices.  The phase and
+// amplitude of the tile and its one-element halo are evaluated once per slice into shared memory (two
+// slices alternate), the slice before stays in registers.  Bound by atan2 and hypot (1.33 per element and
+// slice against up to 7): 8 x 510 x 516 takes 80 us, 107 element by element.
+constexpr int kSoftX = 32, kSoftY = 8;
+inline int soft_tiles(int Ho, int Wo) { return ((Wo + kSoftX - 1) / kSoftX) * ((Ho + kSoftY - 1) / kSoftY); }
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) soft_march_kernel(const float* __restrict__ obj, int S, int Ho, int Wo,
+                                                              float wz, float wxy, float wsurf,
+                                                              float* __restrict__ grad, double* work, int run) {
   static_assert(kThreads == kSoftX * kSoftY, "one thread per tile element");
   constexpr int PX = kSoftX + 2, PY = kSoftY + 2;
   __shared__ double red[32];
-  __shared__ float2 val[2][PY][PX];  // (phase or potential, amplitude)
+  __shared__ float2 val[2][PY][PX];  // (phase, amplitude)
   const int64_t hw = (int64_t)Ho * Wo;
-  const bool surf = wsurf > 0.f && S >= 3;
-  float m0 = 0.f, m1 = 0.f, sg0 = 0.f, sg1 = 0.f;
-  if (surf && KIND != 2) {
-    m0 = (float)(partials_sum(work + kBlocks, kBlocks) / (double)hw);
-    __syncthreads();
-    m1 = (float)(partials_sum(work + 2 * kBlocks, kBlocks) / (double)hw);
-    __syncthreads();
-    sg0 = (float)(partials_sum(work + 3 * kBlocks, kBlocks) / (double)hw);
-    __syncthreads();
-    sg1 = (float)(partials_sum(work + 4 * kBlocks, kBlocks) / (double)hw);
-  }
-  // weighted dimensions (object_models.py:398-411): z with wz (3-D arrays, S > 1), rows and
-  // columns with wxy; each term w mean|diff| divided by the number of weighted dimensions
-  const float w0 = S > 1 ? wz : 0.f;
-  const int nd = (w0 > 0.f) + 2 * (wxy > 0.f);
-  const float c0 = nd && w0 > 0.f ? w0 / (nd * (float)((int64_t)(S - 1) * hw)) : 0.f;
-  const float c1 = nd && wxy > 0.f ? wxy / (nd * (float)((int64_t)S * (Ho - 1) * Wo)) : 0.f;
-  const float c2 = nd && wxy > 0.f ? wxy / (nd * (float)((int64_t)S * Ho * (Wo - 1))) : 0.f;
-  const bool amp_terms = KIND == 0;
+  const SoftTerms t = soft_terms<KIND>(S, Ho, Wo, wz, wxy, wsurf, work);
   const int tx = threadIdx.x % kSoftX, ty = threadIdx.x / kSoftX;
   const int tiles_x = (Wo + kSoftX - 1) / kSoftX, tiles = tiles_x * ((Ho + kSoftY - 1) / kSoftY);
+  const int tasks = tiles * ((S + run - 1) / run);
   double lacc = 0.0;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
+    const int tile = task % tiles, s0 = task / tiles * run, s1 = min(S, s0 + run);
     const int rb = tile / tiles_x * kSoftY, cb = tile % tiles_x * kSoftX;
     const int r = rb + ty, c = cb + tx;
     const bool on = r < Ho && c < Wo;
+    auto value = [&](int64_t k) {
+      float ph, amp;
+      values_at<KIND>(obj, k, ph, amp);
+      return make_float2(ph, amp);
+    };
     auto fill = [&](int s) {
       float2(*v)[PX] = val[s & 1];
-      for (int i = threadIdx.x; i < PY * PX; i += kThreads) {
-        const int y = i / PX, x = i % PX, rr = rb + y - 1, cc = cb + x - 1;
+      for (int k = threadIdx.x; k < PY * PX; k += kThreads) {
+        const int y = k / PX, x = k % PX, rr = rb + y - 1, cc = cb + x - 1;
         if (rr < 0 || rr >= Ho || cc < 0 || cc >= Wo) continue;
         if ((y == 0 || y == PY - 1) && (x == 0 || x == PX - 1)) continue;  // corners are not read
-        float ph, amp;
-        values_at<KIND>(obj, s * hw + (int64_t)rr * Wo + cc, ph, amp);
-        v[y][x] = make_float2(ph, amp);
+        v[y][x] = value(s * hw + (int64_t)rr * Wo + cc);
       }
     };
-    __syncthreads();  // the last tile's values are read
-    fill(0);
+    const int64_t own = (int64_t)r * Wo + c;
+    __syncthreads();  // the last task's values are read
+    fill(s0);
     float2 before = make_float2(0.f, 0.f);
-    for (int s = 0; s < S; ++s) {
+    if (on && s0 > 0) before = value((s0 - 1) * hw + own);
+    for (int s = s0; s < s1; ++s) {
       __syncthreads();  // slice s is in place and slice s - 1 no longer read
-      if (s + 1 < S) fill(s + 1);
+      if (s + 1 < s1) fill(s + 1);
       const float2(*v)[PX] = val[s & 1];
       const float2 here = v[ty + 1][tx + 1];
       float2 after = here;
-      // the own element of the next slice: this thread may not have filled it
-      if (s + 1 < S) {
+      if (s + 1 < s1) {  // the own element of the next slice: this thread may not have filled it
         __syncthreads();
         after = val[(s + 1) & 1][ty + 1][tx + 1];
+      } else if (on && s + 1 < S) {
+        after = value((s + 1) * hw + own);
       }
-      if (on) {
-        const int64_t i = s * hw + (int64_t)r * Wo + c;
-        const float ph = here.x, amp = here.y;
-        float gph = 0.f, gamp = 0.f;
-        // one stencil step per weighted dimension: the loss term of the diff to the next element,
-        // the gradient from the diffs on both sides
-        auto tv_dim = [&](float cw, bool has_lo, float2 lo, bool has_hi, float2 hi) {
-          if (cw == 0.f) return;
-          if (has_hi) {
-            const float d = hi.x - ph;
-            lacc += (double)(cw * fabsf(d));
-            gph -= cw * sgnf(d);
-            if (amp_terms) {
-              const float da = hi.y - amp;
-              lacc += (double)(cw * fabsf(da));
-              gamp -= cw * sgnf(da);
-            }
-          }
-          if (has_lo) {
-            gph += cw * sgnf(ph - lo.x);
-            if (amp_terms) gamp += cw * sgnf(amp - lo.y);
-          }
-        };
-        tv_dim(c0, s > 0, before, s < S - 1, after);
-        tv_dim(c1, r > 0, v[ty][tx + 1], r < Ho - 1, v[ty + 2][tx + 1]);
-        tv_dim(c2, c > 0, v[ty + 1][tx], c < Wo - 1, v[ty + 1][tx + 2]);
-        if (surf && (s == 0 || s == S - 1)) {
-          const float inv = 1.0f / (float)hw;
-          if (KIND == 2) {
-            lacc += (double)(wsurf * fabsf(ph) * inv);
-            gph += wsurf * sgnf(ph) * inv;
-          } else {
-            const float m = s == 0 ? m0 : m1, sgm = s == 0 ? sg0 : sg1;
-            const float u = fabsf(ph) - m;
-            lacc += (double)(wsurf * fabsf(u) * inv);
-            gph += wsurf * (sgnf(u) - sgm) * inv * sgnf(ph);
-            if (amp_terms) {
-              lacc += (double)(wsurf * (1.0f - amp) * inv);
-              gamp -= wsurf * inv;
-            }
-          }
-        }
-        if (KIND == 2) {
-          grad[i] = gph;
-        } else {
-          const float2 o = reinterpret_cast<const float2*>(obj)[i];
-          float2 gz = make_float2(0.f, 0.f);
-          if (amp != 0.f) {  // G = g_amp z / |z| + i g_phase z / |z|^2 (zero at a zero pixel)
-            const float inv = 1.0f / amp;
-            gz.x = gamp * o.x * inv - gph * o.y * inv * inv;
-            gz.y = gamp * o.y * inv + gph * o.x * inv * inv;
-          }
-          reinterpret_cast<float2*>(grad)[i] = gz;
-        }
-      }
+      if (on)
+        soft_element<KIND>(obj, grad, s * hw + own, s, S, t, here, lacc, [&](auto dim) {
+          dim(t.c0, s > 0, [&] { return before; }, s < S - 1, [&] { return after; });
+          dim(t.c1, r > 0, [&] { return v[ty][tx + 1]; }, r < Ho - 1, [&] { return v[ty + 2][tx + 1]; });
+          dim(t.c2, c > 0, [&] { return v[ty + 1][tx]; }, c < Wo - 1, [&] { return v[ty + 1][tx + 2]; });
+        });
       before = here;
     }
   }
-  const double t = block_sum_d(lacc, red);
-  if (threadIdx.x == 0) work[blockIdx.x] = t;
+  const double sum = block_sum_d(lacc, red);
+  if (threadIdx.x == 0) work[blockIdx.x] = sum;
 }
 
 __global__ void loss_from_partials_kernel(const double* __restrict__ part, float* __restrict__ out) {
@@ -897,6 +956,33 @@ int ptycho_obj_butterworth_vjp(const void* grad_out, void* grad_in, int S, int H
                  : butterworth<false>(x, o, S, Ho, Wo, env, a, base, st);
 }
 
+}  // extern "C"
+
+namespace {
+// Complex objects march where at least three quarters of the tiles' elements exist and the tiles, in runs of
+// four slices, fill the blocks; the runs are then as long as leaves four tasks per block.  Measured (march
+// against element by element, amplitude and phase): 200 x 128 x 128 115 us against 150 (345 as one run),
+// 64 x 200 x 200 100 against 127, 8 x 256 x 256 39 against 44, 1 x 510 x 516 16.5 both, 8 x 128 x 128 (128
+// tasks) 30 against 29, 1 x 3000 x 40 (62 % of the tiles) 14.5 against 12.5.  Potentials have nothing to
+// evaluate: 8 x 510 x 516 29 us element by element, 39 marching.
+template <int KIND>
+void soft_launch(const float* o, int S, int Ho, int Wo, float wz, float wxy, float wsurf, float* g, double* work,
+                 cudaStream_t st) {
+  if constexpr (KIND != 2) {
+    const int64_t tiles = soft_tiles(Ho, Wo);
+    if ((int64_t)Ho * Wo * 4 >= tiles * kThreads * 3 && tiles * ((S + 3) / 4) >= kBlocks) {
+      const int64_t parts = (4 * kBlocks + tiles - 1) / tiles;  // of the slices
+      const int run = parts * 4 >= S ? 4 : (int)((S + parts - 1) / parts);
+      soft_march_kernel<KIND><<<kBlocks, kThreads, 0, st>>>(o, S, Ho, Wo, wz, wxy, wsurf, g, work, run);
+      return;
+    }
+  }
+  soft_direct_kernel<KIND><<<kBlocks, kThreads, 0, st>>>(o, S, Ho, Wo, wz, wxy, wsurf, g, work);
+}
+}  // namespace
+
+extern "C" {
+
 int ptycho_obj_soft_loss(const void* obj, int S, int Ho, int Wo, int kind, float tv_weight_z, float tv_weight_xy,
                          float surface_zero_weight, double* work, int nwork, float* loss, void* grad, void* stream) {
   if (!obj || !work || !loss || !grad || S < 1 || Ho < 2 || Wo < 2 || kind < 0 || kind > 2 || nwork < 5 * kBlocks)
@@ -912,18 +998,15 @@ int ptycho_obj_soft_loss(const void* obj, int S, int Ho, int Wo, int kind, float
       surface_abs_phase_kernel<0><<<kBlocks, kThreads, 0, st>>>(o, S, hw, work);
       surface_sign_kernel<0><<<kBlocks, kThreads, 0, st>>>(o, S, hw, work);
     }
-    soft_loss_kernel<0><<<kBlocks, kThreads, 0, st>>>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g,
-                                                      work);
+    soft_launch<0>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g, work, st);
   } else if (kind == 1) {
     if (surf) {
       surface_abs_phase_kernel<1><<<kBlocks, kThreads, 0, st>>>(o, S, hw, work);
       surface_sign_kernel<1><<<kBlocks, kThreads, 0, st>>>(o, S, hw, work);
     }
-    soft_loss_kernel<1><<<kBlocks, kThreads, 0, st>>>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g,
-                                                      work);
+    soft_launch<1>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g, work, st);
   } else {
-    soft_loss_kernel<2><<<kBlocks, kThreads, 0, st>>>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g,
-                                                      work);
+    soft_launch<2>(o, S, Ho, Wo, tv_weight_z, tv_weight_xy, surface_zero_weight, g, work, st);
   }
   loss_from_partials_kernel<<<1, kThreads, 0, st>>>(work, loss);
   return check("soft_loss_kernel");
