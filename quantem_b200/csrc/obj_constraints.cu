@@ -308,7 +308,11 @@ __global__ void blur_pass_kernel(const float* __restrict__ in, float* __restrict
 // shared memory, along the rows first, then along the columns, with the same sums as the two
 // passes.  Bound by reading and writing the object once (17 MB each way at 8 x 510 x 516 complex
 // values); the two passes, each output walking its taps through the L1 cache, took 84 us for 7
-// taps.  Longer kernels take the two passes: their tile would be mostly halo.
+// taps.  Longer kernels take the two passes, since their tile would be mostly halo, and so do objects of
+// fewer than kBlurLeast elements, whose tiles leave SMs idle (complex, 7 and 33 taps, passes against
+// tiles: 1 x 100 x 100 5.0 / 7.6 us against 9.4 / 14.7, 1 x 400 x 400 9.6 / 19.6 against 10.1 / 18.7, 1 x 450
+// x 450 11.5 / 24.3 against 10.2 / 18.9).
+constexpr int64_t kBlurLeast = 200000;
 constexpr int kBlurTile = 32, kBlurHalo = 16;
 // dynamic shared memory with the longest taps, complex values
 constexpr size_t kBlurSmem = sizeof(float) * 2 * (2 * kBlurTile + 2 * kBlurHalo) * (kBlurTile + 2 * kBlurHalo);
@@ -896,7 +900,7 @@ int ptycho_obj_blur(const void* in, void* out, void* tmp, int S, int Ho, int Wo,
   if (tmp == in || tmp == out) return qb_record_error(PTYCHO_ERR_INVALID, "obj_blur: tmp aliases in or out");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int K = is_complex ? 2 : 1;
-  if (ntaps / 2 <= kBlurHalo && S <= 65535 && in != out) {
+  if (ntaps / 2 <= kBlurHalo && (int64_t)S * Ho * Wo >= kBlurLeast && S <= 65535 && in != out) {
     const int side = kBlurTile + ntaps - 1;
     const size_t smem = sizeof(float) * (size_t)(side + kBlurTile) * side * K;
     const dim3 grid((Wo + kBlurTile - 1) / kBlurTile, (Ho + kBlurTile - 1) / kBlurTile, S);
