@@ -204,11 +204,43 @@ __global__ void potential_vjp_kernel(const float* __restrict__ v, const float2* 
 // ---------------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------------
-// out[i] = sum_g parts[g * count + i].  Read-bound: 16 lanes of partials per output element
-// (each a strided, fixed-order sum) keep enough loads in flight when count is only a few
-// thousand elements, then a fixed-order sum over the lanes in shared memory.  One thread
-// per element walking all the partials took 16 us for 148 x 64^2 and 34 us for
-// 148 x 4 x 128^2.
+// out[i] = sum_g parts[g * count + i], in a fixed order.
+//
+// One thread per output element is bound by reading the partials when there are enough elements, and by
+// the latency of its walk over them when there are few: then 16 lanes of partials per element keep more
+// loads in flight, added up in shared memory.  Lanes up to 65536 elements with at least one partial per
+// 768 of them (thread per element against lanes: 444 x 4096 32.8 / 6.4 us, 148 x 65536 13.0 / 11.2,
+// 64 x 65536 6.2 / 6.8, 148 x 131072 36.6 / 41.1, 8 x 16384 1.9 / 2.2, 2 x 4194304 13.5 / 177).
+constexpr int kSerialThreads = 256;
+__global__ void __launch_bounds__(kSerialThreads)
+    reduce_serial_kernel(const float2* __restrict__ parts, float2* __restrict__ out, int nparts, int64_t count) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  // few partials: four elements at a time (2 x 4194304 27 -> 13.5 us; 33 x 1048576 61 -> 73)
+  for (; nparts <= 4 && i + 3 * stride < count; i += 4 * stride) {
+    float2 a[4] = {};
+    for (int g = 0; g < nparts; ++g) {
+      const float2* p = parts + (int64_t)g * count + i;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 v = p[j * stride];
+        a[j].x += v.x;
+        a[j].y += v.y;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[i + j * stride] = a[j];
+  }
+  for (; i < count; i += stride) {
+    float2 a = make_float2(0.f, 0.f);
+    for (int g = 0; g < nparts; ++g) {
+      const float2 v = parts[(int64_t)g * count + i];
+      a.x += v.x;
+      a.y += v.y;
+    }
+    out[i] = a;
+  }
+}
 constexpr int kPartLanes = 16;
 constexpr int kPartCols = 32;
 __global__ void __launch_bounds__(kPartLanes* kPartCols)
@@ -714,6 +746,11 @@ int ptycho_fft2(const void* in, void* out, int count, int n, int inverse, float 
 int ptycho_reduce_partials(const void* parts, void* out, int nparts, int64_t count, void* stream) {
   if (!parts || !out || nparts < 1 || count < 0) return fail(PTYCHO_ERR_INVALID, "reduce_partials: bad arguments");
   if (count == 0) return PTYCHO_OK;
+  if (count > 65536 || (int64_t)nparts * 768 < count) {
+    reduce_serial_kernel<<<grid_for(count, kSerialThreads), kSerialThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const float2*>(parts), static_cast<float2*>(out), nparts, count);
+    return check_launch("reduce_serial_kernel");
+  }
   reduce_partials_kernel<<<grid_for(count, kPartCols), kPartLanes * kPartCols, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const float2*>(parts), static_cast<float2*>(out), nparts, count);
   return check_launch("reduce_partials_kernel");

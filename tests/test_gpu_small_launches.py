@@ -65,3 +65,25 @@ def test_small_blur_takes_less_than_a_large_one(cuda_device):
         times.append(device_us(lambda: lib.ptycho_obj_blur(ops._p(x), ops._p(o), ops._p(tmp), 1, H, W, 1, ops._p(taps), 33,
                                                            ops._stream())))
     assert times[0] < 0.6 * times[1], times
+
+
+@pytest.mark.parametrize("nparts,count", [(1, 1), (7, 100), (444, 4096), (85, 65536), (86, 65536), (148, 65536),
+                                          (148, 65537), (21, 16384), (22, 16384), (33, 1 << 18), (2, 3000001)])
+def test_reduce_partials_any_shape(cuda_device, nparts, count):
+    """Sums of nparts float32 values: nparts 2^-24 of the absolute sum."""
+    g = torch.Generator(device="cuda").manual_seed(nparts)
+    x = torch.randn(nparts, count, dtype=torch.complex64, device="cuda", generator=g)
+    out = torch.full((count,), float("nan"), dtype=torch.complex64, device="cuda")
+    _lib.check(_lib.lib().ptycho_reduce_partials(ops._p(x), ops._p(out), nparts, count, ops._stream()), "reduce")
+    want, size = x.to(torch.complex128).sum(0), torch.view_as_real(x).abs().double().sum(0)
+    err = torch.view_as_real(out.to(torch.complex128) - want).abs()
+    assert bool((err <= nparts * 2.0 ** -24 * size).all())
+
+
+def test_large_reductions_read_their_input_once(cuda_device):
+    """Two partials of four million values: close to a copy of one (13 times a copy with the lanes)."""
+    n = 1 << 22
+    x, out = torch.randn(2, n, dtype=torch.complex64, device="cuda"), torch.empty(n, dtype=torch.complex64, device="cuda")
+    copy = device_us(lambda: out.copy_(x[0]))
+    t = device_us(lambda: _lib.lib().ptycho_reduce_partials(ops._p(x), ops._p(out), 2, n, ops._stream()))
+    assert t < 4 * copy, (t, copy)
