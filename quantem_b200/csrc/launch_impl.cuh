@@ -91,13 +91,22 @@ int launch_ext(const BatchParams& p, int grid, size_t smem, cudaStream_t st) {
   return PTYCHO_OK;
 }
 
+// Where the forward kernel sums the mode intensities.  One mode: nowhere, it goes straight through the loss.
+// Several: a tile in shared memory if it fits beside the separable factors without costing a resident
+// CTA, else the output array if there is one.
+template <int N>
+bool forward_tile(const ptycho_batch_args* a) {
+  if (a->P == 1) return false;
+  return !a->out_intensity || batch_smem_bytes<N>(true, a->prop_r != nullptr, a->S) <= max_smem<N>(Fft2<N>::CTAS);
+}
+
 // One CTA per position, modes in sequence.  The attributes are per device; setting them on
 // every launch keeps multi-device processes correct and costs far less than one launch.
 // The adjoint kernels take the smallest shared-memory carve-out that fits: the rest of the
 // 256 KB is L1.
 template <int N>
 int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const bool tile = !adj && !a->out_intensity;  // the output array serves as the tile
+  const bool tile = !adj && forward_tile<N>(a);
   const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
   const size_t smem = batch_smem<N>(a, tile);
   if (adj) {
@@ -115,7 +124,7 @@ int launch_plain(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
 // the instances with the analytic update or with extensions
 template <int N>
 int launch_special(const ptycho_batch_args* a, bool adj, cudaStream_t st) {
-  const bool tile = !adj && !a->out_intensity;  // the output array serves as the tile
+  const bool tile = !adj && forward_tile<N>(a);
   const BatchParams p = batch_params<N>(a, tile, !adj && !tile);
   const size_t smem = batch_smem<N>(a, tile);
   if (!a->analytic) {

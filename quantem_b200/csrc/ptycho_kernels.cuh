@@ -66,7 +66,8 @@ struct BatchParams {
   float* grad_positions;      // optional (B, 2) dL/d(position), serial autograd adjoint only
   const float* descan;        // optional (npos, 2) descan shifts [px] applied to the exit wave
   float* grad_descan;         // optional (B, 2) dL/d(descan), serial autograd adjoint only
-  int tile_out;               // forward kernel: out_intensity serves as the mode-sum tile (none in shared memory)
+  int tile_out;               // forward kernel: no mode-sum tile in shared memory (several modes: out_intensity
+                              // serves as the tile)
   int sep_shared;             // the separable factors fit in shared memory, else read through L1
                               // (256^2: the row factors are 16-byte aligned)
   float* grad_prop;           // optional (S-1, 2) propagator sensitivities, serial autograd adjoint only
