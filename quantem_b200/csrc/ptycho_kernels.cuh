@@ -706,41 +706,59 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
         // far field waits in this thread's elements of the exchange buffer, so that the loop
         // needs neither the wave's registers nor full unrolling: with 16 to 48 copies of the five
         // losses in it, the code of the transforms did not stay in the instruction caches (six
-        // single-mode datasets: 15.2 -> 12.8 ms with the far field's round trip gone too).  The
-        // other per-mode steps lose as rolled loops (24.2 -> 24.9 ms per 4096-position launch):
-        // they are chains of loads.
+        // single-mode datasets: 15.2 -> 12.8 ms with the far field's round trip gone too).  A trip's
+        // loads are issued before its stores, which the compiler cannot reorder: element by
+        // element each target was a DRAM latency of its own (128^2, one slice and mode, 3000
+        // positions: forward 664 -> 440 us, adjoint 988 -> 828; four per trip 480 and 859).  The
+        // instances with extensions take four, for their registers (64^2, one position: 23 us with
+        // eight, 22.3 with four).  The other per-mode steps lose as rolled loops (24.2 -> 24.9 ms
+        // per 4096-position launch): they are chains of loads.
         {
+          constexpr int TRIP = AN || EXT ? 4 : 8;
+          static_assert(E % TRIP == 0, "whole trips");
           const float* tg = p.targets + (size_t)gi * NN;
           double loss_acc = 0.0;
           int nonfinite = 0;
           if (!AN) f.write_s3(sm, x);
-#pragma unroll 4
-          for (int i = 0; i < E; ++i) {
-            const int g = i / D, e = i % D;
-            const int di = detector_index<N>(f.s3_row(g, e), f.s3_c);
-            const int li = 2 * ((i >> 1) * T + tid) + (i & 1);
-            float2* xs = sm + f.s3_slot(g, e);
-            const float tv = __ldcs(tg + di);  // targets stream through L2 once per iteration
-            float I = 0.f;
-            if (AN || P > 1) I = !ADJ && p.tile_out ? p.out_intensity[(size_t)b * NN + di] : inten[li];
-            if (!AN) I += cabs2(*xs);
-            if (!isfinite(I)) ++nonfinite;
-            float dldi;
-            loss_elem<N>(p, I, tv, __ldg(p.mask + di), loss_acc, dldi);
-            if (ADJ && AN) {
-              // factor f and additive fix of the Fourier projection seed
-              if (P == 1) {
-                dldi = I > 0.f ? tv / sqrtf(I) : 0.f;   // t exp(i angle(Psi)) = Psi t / |Psi|
-                tile2[li] = I > 0.f ? 0.f : tv;        // angle(0) = 0
-              } else {
-                const float est = sqrtf(tile2[li]);
-                dldi = est > 0.f ? tv / est : 0.f;     // zero estimate -> infinity -> factor 0
-                tile2[li] = 0.f;
-              }
+#pragma unroll 1
+          for (int i0 = 0; i0 < E; i0 += TRIP) {
+            float tv[TRIP], mk[TRIP], Is[TRIP];
+#pragma unroll
+            for (int j = 0; j < TRIP; ++j) {  // a trip's loads go out before its stores
+              const int i = i0 + j, di = detector_index<N>(f.s3_row(i / D, i % D), f.s3_c);
+              tv[j] = __ldcs(tg + di);  // targets stream through L2 once per iteration
+              mk[j] = __ldg(p.mask + di);
+              Is[j] = 0.f;
+              if (AN || P > 1)
+                Is[j] = !ADJ && p.tile_out ? p.out_intensity[(size_t)b * NN + di]
+                                           : inten[2 * ((i >> 1) * T + tid) + (i & 1)];
             }
-            if (ADJ && (AN || P > 1)) inten[li] = dldi;
-            if (ADJ && !AN) *xs = make_float2(xs->x * 2.0f * dldi, xs->y * 2.0f * dldi);  // seed of the last mode
-            if (p.out_intensity) p.out_intensity[(size_t)b * NN + di] = I;
+#pragma unroll
+            for (int j = 0; j < TRIP; ++j) {
+              const int i = i0 + j, g = i / D, e = i % D;
+              const int di = detector_index<N>(f.s3_row(g, e), f.s3_c);
+              const int li = 2 * ((i >> 1) * T + tid) + (i & 1);
+              float2* xs = sm + f.s3_slot(g, e);
+              float I = Is[j];
+              if (!AN) I += cabs2(*xs);
+              if (!isfinite(I)) ++nonfinite;
+              float dldi;
+              loss_elem<N>(p, I, tv[j], mk[j], loss_acc, dldi);
+              if (ADJ && AN) {
+                // factor f and additive fix of the Fourier projection seed
+                if (P == 1) {
+                  dldi = I > 0.f ? tv[j] / sqrtf(I) : 0.f;   // t exp(i angle(Psi)) = Psi t / |Psi|
+                  tile2[li] = I > 0.f ? 0.f : tv[j];        // angle(0) = 0
+                } else {
+                  const float est = sqrtf(tile2[li]);
+                  dldi = est > 0.f ? tv[j] / est : 0.f;     // zero estimate -> infinity -> factor 0
+                  tile2[li] = 0.f;
+                }
+              }
+              if (ADJ && (AN || P > 1)) inten[li] = dldi;
+              if (ADJ && !AN) *xs = make_float2(xs->x * 2.0f * dldi, xs->y * 2.0f * dldi);  // seed of the last mode
+              if (p.out_intensity) p.out_intensity[(size_t)b * NN + di] = I;
+            }
           }
           for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
           const int nf_warp = __reduce_add_sync(0xffffffffu, nonfinite);
