@@ -108,7 +108,7 @@ class CNN2d(torch.nn.Module):
         # when a dict, each pass records every layer's inputs / outputs / gradients
         # (used by the per-layer parity tests)
         self.trace = None
-        self._arena_bytes = {}  # (B, H, W) -> bytes of the buffers of one pass without a backward
+        self._arena_bytes = {}  # (B, H, W, keep) -> bytes of one pass's buffers that share tensors
         self._build()
         self._init_params(seed)
 
@@ -374,36 +374,30 @@ class _Buf:
 
 
 class _Arena:
-    """Buffers of one pass out of a few tensors of the caching allocator.
+    """Buffers of one pass, cut one after the other from a few tensors of the caching allocator (``first``
+    bytes, then 16 MB each) that live as long as the pass.
 
-    A pass that a backward follows takes one tensor per call (what one layer's backward needs): it goes
-    back to the allocator when the backward has passed the layer and drops its last buffer.  A pass
-    without a backward takes its buffers one after the other from large tensors, ``first`` bytes and
-    then 16 MB each, which live as long as the pass."""
+    In a pass that a backward follows, buffers of ``_OWN`` bytes and more are tensors of their own: they go
+    back to the allocator when the backward has passed their layer and drops them."""
+
+    _OWN = 1 << 20
 
     def __init__(self, device, first: int, keep: bool):
         self.device, self.keep, self.block = device, keep, max(int(first), 1 << 20)
         self.blocks, self.base, self.used, self.total = [], None, 0, 0
 
-    def bufs(self, *shapes) -> list:
-        """A buffer per (R, C, dtype)."""
-        sizes = [(R * C * dtype.itemsize + 255) // 256 * 256 for R, C, dtype in shapes]
-        n = sum(sizes)
-        if self.keep:
-            base, off = torch.empty(n, dtype=torch.uint8, device=self.device), 0
-        else:
-            if self.base is None or self.used + n > self.base.numel():
-                self.base = torch.empty(max(n, self.block), dtype=torch.uint8, device=self.device)
-                self.blocks.append(self.base)
-                self.used, self.block = 0, 1 << 24
-            base, off = self.base, self.used
-            self.used += n
-            self.total += n
-        out = []
-        for (R, C, dtype), size in zip(shapes, sizes):
-            out.append(_Buf(base, off, R, C, C, dtype))
-            off += size
-        return out
+    def buf(self, R, C, dtype) -> _Buf:
+        n = (R * C * dtype.itemsize + 255) // 256 * 256
+        if self.keep and n >= self._OWN:
+            return _Buf(torch.empty(n, dtype=torch.uint8, device=self.device), 0, R, C, C, dtype)
+        if self.base is None or self.used + n > self.base.numel():
+            self.base = torch.empty(max(n, self.block), dtype=torch.uint8, device=self.device)
+            self.blocks.append(self.base)
+            self.used, self.block = 0, 1 << 24
+        b = _Buf(self.base, self.used, R, C, C, dtype)
+        self.used += n
+        self.total += n
+        return b
 
 
 _F32, _BF16 = torch.float32, torch.bfloat16
@@ -415,12 +409,11 @@ class _Run:
 
     def __init__(self, net: CNN2d, B: int, H: int, W: int, training: bool, keep: bool):
         """``keep``: a backward follows."""
-        self.keep = keep
         self.net, self.B, self.H, self.W, self.training = net, B, H, W, training
         self.dev = net.device
         self.lib = kk._lib.lib()
         self.saved = {}
-        self.key = (B, H, W)
+        self.key = (B, H, W, keep)
         self.arena = _Arena(self.dev, net._arena_bytes.get(self.key, 1 << 22), keep)
 
     def empty(self, *shape, dtype=torch.float32):
@@ -449,21 +442,20 @@ class _Run:
         return (self._f(gseg), self._f(bseg), rm.data_ptr(), rv.data_ptr(), self.net.momentum, self.net.eps,
                 int(self.training), mean.ptr, rstd.ptr)
 
-    def _act_bufs(self, bn, R, co, *more):
-        """A layer's activation, its batch-norm statistics (None without) and ``more`` buffers."""
+    def _stats(self, bn, co):
         if bn is None:
-            r, *more = self.arena.bufs((R, co, _F32), *more)
-            return r, None, None, *more
-        return self.arena.bufs((R, co, _F32), (1, co, _F32), (1, co, _F32), *more)
+            return None, None
+        return self.arena.buf(1, co, _F32), self.arena.buf(1, co, _F32)
 
     # --- conv3x3 + bias + activation (+ BN) -> bf16 into `out` ------------------
     def conv_fwd(self, key, layer, x, B, H, W, out, act=None, final=False):
         net = self.net
         R, co, C = B * H * W, layer["co"], layer["ci_store"]
         bn = None if final else layer["bn"]
-        r, mean, rstd = self._act_bufs(bn, R, co)
+        r = self.arena.buf(R, co, _F32)
+        mean, rstd = self._stats(bn, co)
         if out is None and not final:  # the next layer's input
-            out, = self.arena.bufs((R, co, _BF16))
+            out = self.arena.buf(R, co, _BF16)
         self.call("ptycho_cnn_conv_forward", x.ptr, x.ld, B, H, W, C, self._h(layer["w"]), co, self._f(layer["b"]),
                   int(net._act if act is None else act), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
                   r.ptr, None if final else out.ptr, 0 if final else out.ld, self.st)
@@ -557,14 +549,14 @@ class _Run:
             co = net.down[l][-1]["co"]
             R = B * h * w
             if net.use_skip_connections:
-                cat, = self.arena.bufs((R, 2 * co, _BF16))
+                cat = self.arena.buf(R, 2 * co, _BF16)
                 skip = cat.cols(co, co)
             else:
                 cat = None
-                skip, = self.arena.bufs((R, co, _BF16))
+                skip = self.arena.buf(R, co, _BF16)
             cats.append(cat)
             self.block_fwd(("down", l), net.down[l], y, B, h, w, skip)
-            pooled, arg = self.arena.bufs((R // 4, co, _BF16), (R // 4, co, torch.uint8))
+            pooled, arg = self.arena.buf(R // 4, co, _BF16), self.arena.buf(R // 4, co, torch.uint8)
             self.call("ptycho_cnn_maxpool2", skip.ptr, skip.ld, B, h, w, co, pooled.ptr, pooled.ld, arg.ptr, self.st)
             self.pool_arg.append(arg)
             y = pooled
@@ -577,8 +569,9 @@ class _Run:
             R = B * h * w
             cat = cats[l]
             bn = up["bn"] if net._use_batchnorm else None
-            r, mean, rstd, t = self._act_bufs(bn, R, co, (R, ci, _BF16))
-            dst = cat.cols(0, co) if cat is not None else self.arena.bufs((R, co, _BF16))[0]
+            t, r = self.arena.buf(R, ci, _BF16), self.arena.buf(R, co, _F32)
+            mean, rstd = self._stats(bn, co)
+            dst = cat.cols(0, co) if cat is not None else self.arena.buf(R, co, _BF16)
             self.call("ptycho_cnn_up_forward", y.ptr, y.ld, B, hin, win, ci, co, self._h(up["wt"]), self._f(up["bt"]),
                       self._h(up["w1"]), self._f(up["b1"]), *self._bn_args(bn, mean, rstd), self.scratch.data_ptr(),
                       t.ptr, r.ptr, dst.ptr, dst.ld, self.st)
@@ -590,10 +583,9 @@ class _Run:
             y = self.block_fwd(("upc", u), up["block"], src, B, h, w)
         r = self.conv_fwd(("final",), net.final, y, B, H, W, None, act=net._final_act, final=True)
         del self.scratch
-        if not self.keep:
-            if len(net._arena_bytes) > 16:
-                net._arena_bytes.clear()
-            net._arena_bytes[self.key] = self.arena.total
+        if len(net._arena_bytes) > 16:
+            net._arena_bytes.clear()
+        net._arena_bytes[self.key] = self.arena.total
         out = self.empty(B, net.out_channels, H * W)
         kk.transpose(r.view(B, H * W, net.out_channels), out)
         return out.view(B, net.out_channels, H, W)
