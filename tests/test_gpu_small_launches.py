@@ -87,3 +87,20 @@ def test_large_reductions_read_their_input_once(cuda_device):
     copy = device_us(lambda: out.copy_(x[0]))
     t = device_us(lambda: _lib.lib().ptycho_reduce_partials(ops._p(x), ops._p(out), 2, n, ops._stream()))
     assert t < 4 * copy, (t, copy)
+
+
+@pytest.mark.parametrize("n,per_sm", [(64, 3), (96, 2)])
+def test_a_few_positions_more_than_blocks(cuda_device, n, per_sm):
+    """Six positions more than resident blocks cost about one position on an SM of its own, half of a full round
+    or less (0.9 of one when the six longer blocks shared two SMs)."""
+    from tests.test_gpu_batch_paths import _problem
+
+    times = []
+    for B in (ops.resident_ctas(n), ops.resident_ctas(n) + 6):
+        assert ops.resident_ctas(n) == per_sm * ops.sm_count()
+        obj, probe, prop, pos, targets = _problem(n, 16, 1, B, n + 150, n + 150)
+        idx, mask = torch.arange(B, device="cuda"), torch.ones((n, n), device="cuda")
+        ph, go, gp = ops.fft2(probe), torch.zeros_like(obj), torch.empty_like(probe)
+        times.append(device_us(lambda: ops.batch_forward_adjoint(obj, probe, prop, pos, idx, targets, mask, B, 100.0,
+                                                                 probe_hat=ph, grad_obj=go, grad_probe=gp)))
+    assert times[1] < 1.75 * times[0], times
