@@ -451,7 +451,10 @@ __device__ __forceinline__ void serial_body(const BatchParams& p, const int cta,
   // each: they sit on SMs of their own (64^2, 16 slices, 450 positions on 444 CTAs: 399 us, 612 where an even
   // spread put the six longer CTAs on two SMs)
   const int bq = p.B / ncta, brem = p.B % ncta;
-  const int b0 = cta * bq + min(cta, brem), bend = b0 + bq + (cta < brem);
+  const int b0 = cta * bq + min(cta, brem);
+  __shared__ int bend;  // not a register: the instances with extensions spill 40 to 70 bytes less
+  if (tid == 0) bend = b0 + bq + (cta < brem);
+  __syncthreads();
   for (int b = b0; b < bend; ++b) {
     const int64_t gi64 = p.batch_idx[b];
     if (gi64 < 0 || gi64 >= p.npos) {  // invalid index: skip the position and report it
