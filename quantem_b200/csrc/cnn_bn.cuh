@@ -4,8 +4,9 @@
 // A thread-block cluster owns CW channels (a warp: CW channels x 32 / CW rows) and its CTAs
 // split the rows: per-channel sums (float over runs of rows, then double), one exchange of the
 // partial sums through distributed shared memory, and the elementwise pass over the same rows.
-// The backward also sums the bias gradient.  Bound by latency and by reading the activation
-// twice (L2-resident): the layers hold 64 KB to 2 MB.  As partial sums, a serial final sum over up
+// The backward also sums the bias gradient.  Bound by its cluster barriers at few rows (64 x 512: 12.5
+// cycles per issued instruction) and by the latency of its loads at many (16384 x 32: 4.4), the
+// layers' 64 KB to 2 MB being L2-resident.  As partial sums, a serial final sum over up
 // to 592 partials and separate elementwise and bias-gradient passes, the batch norms of one
 // training step of the 5-level network took 229 launches and 1.3 ms.
 //
@@ -271,7 +272,8 @@ __global__ void __launch_bounds__(kThreads) bn_backward_kernel(const Backward p,
 // A cluster's channels are at least one 32-byte sector wide, so C / 8 clusters of 8 CTAs are all that
 // the kernels above can put to work: at 32 channels 32 CTAs, whatever the number of rows.  Here blocks
 // of 256 threads (a thread: one channel, every RP-th row of a chunk, the same float runs) write partial
-// sums, a warp per channel adds them in a fixed order, and an elementwise pass follows.
+// sums, a warp per channel adds them in a fixed order, and an elementwise pass follows.  Bound by the
+// latency of the loads of 29 warps per SM, at 31 to 43 % of the DRAM throughput (262144 x 32, cold).
 constexpr int kWideThreads = 256;
 
 struct WideRows {
@@ -412,8 +414,11 @@ __global__ void __launch_bounds__(kWideThreads)
   }
 }
 
-// Channels per warp and CTAs per cluster: enough rows per CTA to keep its warps busy, and
-// narrow tiles for the wide, shallow-channel layers (32 channels x 16384 rows).
+// Channels per warp and CTAs per cluster: narrow tiles for many rows (16384 x 32, forward / backward: 8
+// channels 14.6 / 18.7 us a call, 16 channels 16.7 / 29.9, 32 channels 26.9 / 53.5; one CTA instead of
+// eight 47.8 / 98.7), few CTAs for few rows, whose barriers cost more than they share out (16 x 1024: one to
+// four CTAs of 16 or 32 channels 12.0 / 12.6, eight of 8 channels 20.7 / 25.3).  In between the
+// shapes are equal, at the 12 us of a call.
 struct Shape {
   int cw, ctas, grid;
   Shape(int R, int C) {

@@ -27,9 +27,10 @@
 // of N spectral values share the class's region of the buffer.  Every warp access is two
 // wavefronts per 256 bytes, the minimum for 8-byte words.
 //
-// The load/store unit's data pipe is the busiest unit of the batch kernels (58 % at 128^2
-// against 50 % of the FP32 pipe and 38 % of the issue slots), so the factorisation is
-// chosen for the real-space accesses: B = 8 puts 8 consecutive columns x 4 rows in a warp
+// No unit of the batch kernels is full.  At 128^2 the load/store unit's data pipe is at 59 % of its peak,
+// the FP32 pipe at 50 %, the issue slots at 39 %; the 16 warps of an SM wait most for global loads
+// (2.2 cycles per issued instruction), then for the FP32 pipe (1.7).  The data pipe being the busiest,
+// the factorisation is chosen for the real-space accesses: B = 8 puts 8 consecutive columns x 4 rows in a warp
 // access of the object (B = 4: 4 columns x 8 rows took 3.7 L1 wavefronts per gather and
 // 4.6 per gradient scatter, B = 8 takes 1.7 and 2.3: 28.5 -> 26.4 ms per 4096-position
 // launch).  At 64^2 B = 4 keeps 16 registers per thread, half the code and three CTAs per

@@ -306,9 +306,9 @@ __global__ void blur_pass_kernel(const float* __restrict__ in, float* __restrict
 
 // Both passes in one: a 32 x 32 tile and its halo of R = ntaps / 2 <= kBlurHalo elements in
 // shared memory, along the rows first, then along the columns, with the same sums as the two
-// passes.  Bound by reading and writing the object once (17 MB each way at 8 x 510 x 516 complex
-// values); the two passes, each output walking its taps through the L1 cache, took 84 us for 7
-// taps.  Longer kernels take the two passes, since their tile would be mostly halo, and so do objects of
+// passes.  Bound by the walk over the taps: 31, 39, 58 and 105 us for 3, 7, 15 and 33 taps at 8 x 510 x 516
+// complex values, 17 MB each way; the two passes, each output walking its taps through the L1 cache,
+// take 60, 81, 122 and 202.  Longer kernels take the two passes, since their tile would be mostly halo, and so do objects of
 // fewer than kBlurLeast elements, whose tiles leave SMs idle (complex, 7 and 33 taps, passes against
 // tiles: 1 x 100 x 100 5.0 / 7.6 us against 9.4 / 14.7, 1 x 400 x 400 9.6 / 19.6 against 10.1 / 18.7, 1 x 450
 // x 450 11.5 / 24.3 against 10.2 / 18.9).
@@ -638,8 +638,10 @@ int allow_smem(K kernel, size_t bytes) {
 //
 // Three passes of line transforms of any length (line_fft.cuh): rows forward, columns forward
 // + envelope + columns inverse in one pass, rows inverse.  Each pass reads and writes the
-// object once (17 MB at 8 x 510 x 516, L2-resident); bound by the shared-memory traffic of
-// the stages.  At 8 x 510 x 516 (factors 17 and 43 among the radices) the filter took 3.4 ms as
+// object once (17 MB at 8 x 510 x 516, L2-resident), 55 to 60 us each; bound by the chain of stages: the 27
+// of 64 warps wait at the stages' barriers (3.9 cycles per issued instruction in the row passes, 1.7 in the
+// columns) and for their shared and twiddle loads (3.9 and 3.6), with 50 to 58 % of the issue slots and
+// 32 to 41 % of the load/store data pipe used.  At 8 x 510 x 516 (factors 17 and 43 among the radices) the filter took 3.4 ms as
 // four direct n^2 line transforms with transposes, mean and envelope passes in between.
 constexpr int kLineThreads = 512;
 
