@@ -86,8 +86,9 @@ def resident_ctas(n: int, device: torch.device | None = None) -> int:
 
 def free_bytes(device) -> int:
     """Device memory that new tensors can take: free, or kept by the allocator for reuse."""
-    return (torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device)
-            - torch.cuda.memory_allocated(device))
+    st = torch.cuda.memory_stats_as_nested_dict(device)  # memory_reserved() flattens all of it: 0.3 ms a call
+    kept = sum(st[k]["all"]["current"] * sign for k, sign in (("reserved_bytes", 1), ("allocated_bytes", -1)) if st)
+    return torch.cuda.mem_get_info(device)[0] + kept
 
 
 def reduce_blocks() -> int:
