@@ -511,7 +511,7 @@ int colsum(const float* a, int lda, int R, int C, double* work, int64_t work_ele
 int bn_check(const qb::bn::Forward& f, int R, int C) {
   if (!f.x || !f.y || R < 1 || C < 1 || f.ldx < C || f.ldy < C)
     return fail(PTYCHO_ERR_INVALID, "bn_forward: bad arguments");
-  if (f.gamma && (!f.beta || !f.mean || !f.rstd || !f.run_mean != !f.run_var || (!f.training && !f.run_mean)))
+  if (f.gamma && (!f.beta || !f.mean || !f.rstd || (f.run_mean && !f.run_var) || (!f.training && !f.run_mean)))
     return fail(PTYCHO_ERR_INVALID, "bn_forward: missing statistics buffers");
   return PTYCHO_OK;
 }

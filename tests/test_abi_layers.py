@@ -27,11 +27,13 @@ CALLS = {
 }
 SIZES = [dict(B=0), dict(H=0), dict(W=-1), dict(co=0), dict(B=1 << 15, H=1 << 15, W=4),
          dict(B=1 << 30, H=1 << 30, W=1 << 30)]
+# running statistics: wanted without the batch's, the variance also with the mean
+NO_STATISTICS = [dict(training=0, run_mean=None), dict(training=0, run_var=None), dict(training=1, run_var=None),
+                 dict(training=0, run_mean=None, run_var=None)]
 BAD = {
     "ptycho_cnn_conv_forward": SIZES + [dict(C=0), dict(C=12), dict(ldx=8), dict(ldo=7), dict(act=-1), dict(act=7)] + [
         {k: None} for k in ("x", "w", "col", "r", "beta", "mean", "rstd")] + [
-        {k: ODD} for k in ("x", "w", "col")] + [dict(training=t, **{k: None}) for t in (0, 1) for k in ("run_mean", "run_var")] + [
-        dict(training=0, run_mean=None, run_var=None)],
+        {k: ODD} for k in ("x", "w", "col")] + NO_STATISTICS,
     "ptycho_cnn_conv_backward": SIZES + [dict(C=0), dict(C=12), dict(lddy=7), dict(ldx=8), dict(ldz=7), dict(ldz=12),
                                          dict(lddx=15), dict(lddx=8), dict(act=-1), dict(act=7)] + [
         {k: None} for k in ("dy", "x", "w", "r", "mean", "rstd", "dw", "dgamma", "dbeta", "dz", "col", "dcol")] + [
@@ -39,8 +41,7 @@ BAD = {
     "ptycho_cnn_up_forward": SIZES + [dict(ci=0), dict(ci=12), dict(ldy=8), dict(ldo=7),
                                       dict(B=1 << 14, H=1 << 15, W=1)] + [
         {k: None} for k in ("y", "wt", "w1", "beta", "mean", "rstd", "colT", "t", "r", "out")] + [
-        {k: ODD} for k in ("y", "wt", "w1", "t")] + [dict(training=t, **{k: None}) for t in (0, 1) for k in ("run_mean", "run_var")] + [
-        dict(training=0, run_mean=None, run_var=None)],
+        {k: ODD} for k in ("y", "wt", "w1", "t")] + NO_STATISTICS,
     "ptycho_cnn_up_backward": SIZES + [dict(ci=0), dict(ci=12), dict(lddup=7), dict(ldy=8), dict(ldz=7), dict(ldz=12),
                                        dict(work_elems=31), dict(B=1 << 14, H=1 << 15, W=1)] + [
         {k: None} for k in ("dup", "y", "t", "r", "wt", "w1", "mean", "rstd", "dwt", "dbt", "dw1", "dgamma", "dbeta", "dz",

@@ -101,3 +101,17 @@ def test_many_rows_use_the_device(cuda_device):
     fwd = us(lambda: kk.bn_forward(x, ga, be, rm, rv, 0.1, 1e-5, True, mean, rstd, work, y))
     bwd = us(lambda: kk.bn_backward(dy, x, ga, mean, rstd, True, 1, dg, db, work, dz16=y))
     assert fwd < 5 * copy and bwd < 9 * copy, (copy, fwd, bwd)
+
+
+@pytest.mark.parametrize("R", [64, 40000])
+def test_running_variance_without_mean_is_ignored(cuda_device, R):
+    """Batch statistics with a running variance but no running mean: nothing is updated, as without both."""
+    x, _, ga, be, _, rv = _data(R, 24, 24, R)
+    work = torch.empty(2 * 592 * 24, device="cuda", dtype=torch.float64)
+    outs = []
+    for var in (None, rv.clone()):
+        mean, rstd = torch.empty(24, device="cuda"), torch.empty(24, device="cuda")
+        y = torch.empty(R, 24, device="cuda", dtype=torch.bfloat16)
+        kk.bn_forward(x, ga, be, None, var, 0.1, 1e-5, True, mean, rstd, work, y)
+        outs.append((mean, rstd, y))
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and torch.equal(var, rv)
