@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(512, 1) cluster256_kernel(const BatchParams p)
       }
     };
     using Wide = std::integral_constant<int, 8>;
-    using Narrow = std::integral_constant<int, 2>;  // wrapping windows are few
+    // wrapping windows: pairs, for their registers (66 positions of 4 slices and 2 modes 1465 us, 1453 unwrapped)
+    using Narrow = std::integral_constant<int, 2>;
 
     int m = 0, s = 0;
     bool bwd = false, first_bwd = false, rec = false;

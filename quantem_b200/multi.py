@@ -37,6 +37,7 @@ class Problem:
         self.batch_idx = (torch.arange(n, device=obj.device, dtype=torch.int64) if batch_idx is None
                           else batch_idx)
         self.ws = ops.Workspace(obj.device)
+        self.most_ctas = None  # where the scratch of more did not fit
 
     @property
     def num_gpts(self):
@@ -46,11 +47,6 @@ class Problem:
         S, Ho, Wo = self.obj.shape
         P, n, _ = self.probe.shape
         return (n, S, P, Ho, Wo, int(self.batch_idx.numel()))
-
-    def slots(self):
-        """Complex scratch values of one CTA: waves, far fields and the intensity tile."""
-        n, S, P, _, _, _ = self.signature()
-        return (P * S + P + 1) * n * n
 
     def cost(self):
         n, S, P, _, _, B = self.signature()
@@ -68,15 +64,12 @@ def _window_groups(problems):
 def default_grids(problems, total=None):
     """CTAs per dataset proportional to its transform count (at least one); each
     probe-window group (a launch of its own) splits ``total`` CTAs (default: as many as the
-    device holds at once for that window, or one per SM where their scratch would not fit)."""
+    device holds at once for that window)."""
     out = [0] * len(problems)
     for idx in _window_groups(problems):
         sub = [problems[i] for i in idx]
-        dev = sub[0].obj.device
-        grids = _split(sub, total or ops.resident_ctas(int(sub[0].probe.shape[-1]), dev))
-        if not total and sum(g * p.slots() for g, p in zip(grids, sub)) * 8 > ops.free_bytes(dev):
-            grids = _split(sub, ops.sm_count(dev))
-        for i, g in zip(idx, grids):
+        t = total or ops.resident_ctas(int(sub[0].probe.shape[-1]), sub[0].obj.device)
+        for i, g in zip(idx, _split(sub, t)):
             out[i] = g
     return out
 
@@ -107,11 +100,37 @@ def multi_forward_adjoint(problems, obj_cs, probe_os, grids):
     return _multi_launch(problems, obj_cs, probe_os, grids)
 
 
+def _reserve(problems, geoms, grids):
+    """The workspaces of one launch, and its partition: ``grids``, or one CTA per SM where the scratch of more
+    cannot be allocated.  The smaller partition stays with the problems: later launches do not try again,
+    so a warmed-up capture meets no failing allocation.  (Asking the driver for the free memory beforehand
+    took 0.1 to 130 ms a call on a shared host.)"""
+    grids = [min(int(g), pr.most_ctas or int(g)) for g, pr in zip(grids, problems)]
+
+    def ensure():
+        for pr, q, g in zip(problems, geoms, grids):
+            nn = q.n * q.n
+            pr.ws.ensure(g * (q.P * q.S + q.P + 1) * nn, g * q.P * nn, g)
+
+    try:
+        ensure()
+    except torch.OutOfMemoryError:
+        less = [min(a, b) for a, b in zip(grids, _split(problems, ops.sm_count(problems[0].obj.device)))]
+        if less == grids:
+            raise
+        for pr, g in zip(problems, less):
+            pr.most_ctas = g
+            pr.ws.scratch = pr.ws.partials = None
+        grids = less
+        ensure()
+    return grids
+
+
 def _multi_launch(problems, obj_cs, probe_os, grids):
     n = problems[0].probe.shape[-1]
     args = (_lib.BatchArgs * len(problems))()
     keep, outs = [], []
-    for d, (pr, oc, po, g) in enumerate(zip(problems, obj_cs, probe_os, grids)):
+    for d, (pr, oc, po) in enumerate(zip(problems, obj_cs, probe_os)):
         geom = ops._check_batch_inputs(oc, po, pr.prop, pr.positions, pr.batch_idx, pr.targets, pr.mask)
         if geom.n != n:
             raise ValueError("datasets of one multi launch need the same probe window")
@@ -121,14 +140,14 @@ def _multi_launch(problems, obj_cs, probe_os, grids):
         a = ops._batch_args(geom, oc, ph, pr.prop, pr.positions, pr.batch_idx, pr.targets, pr.mask, B, pr.loss_type,
                             ops.loss_scale_of(pr.loss_type, B, pr.num_gpts, pr.mean_intensity),
                             1.0 / pr.mean_intensity, grad_obj=gobj, variant="serial")
-        nn = geom.n * geom.n
-        pr.ws.ensure(g * (geom.P * geom.S + geom.P + 1) * nn, g * geom.P * nn, g)
-        a.grid = g
-        a.scratch, a.probe_grad_part = pr.ws.scratch.data_ptr(), pr.ws.partials.data_ptr()
-        a.loss_part, a.status = pr.ws.loss_part.data_ptr(), pr.ws.status.data_ptr()
         args[d] = a
         keep += [ph]
         outs.append((gobj, geom))
+    grids = _reserve(problems, [geom for _, geom in outs], grids)
+    for a, pr, g in zip(args, problems, grids):
+        a.grid = g
+        a.scratch, a.probe_grad_part = pr.ws.scratch.data_ptr(), pr.ws.partials.data_ptr()
+        a.loss_part, a.status = pr.ws.loss_part.data_ptr(), pr.ws.status.data_ptr()
     lib = _lib.lib()
     st = ops._stream()
     _lib.check(lib.ptycho_forward_adjoint_multi(ctypes.cast(args, ctypes.c_void_p), len(problems), st),

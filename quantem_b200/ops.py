@@ -84,13 +84,6 @@ def resident_ctas(n: int, device: torch.device | None = None) -> int:
     return grid.value
 
 
-def free_bytes(device) -> int:
-    """Device memory that new tensors can take: free, or kept by the allocator for reuse."""
-    st = torch.cuda.memory_stats_as_nested_dict(device)  # memory_reserved() flattens all of it: 0.3 ms a call
-    kept = sum(st[k]["all"]["current"] * sign for k, sign in (("reserved_bytes", 1), ("allocated_bytes", -1)) if st)
-    return torch.cuda.mem_get_info(device)[0] + kept
-
-
 def reduce_blocks() -> int:
     return int(_lib.lib().ptycho_reduce_blocks())
 
