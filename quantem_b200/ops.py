@@ -267,6 +267,7 @@ class Workspace:
         self.scratch = None
         self.partials = None
         self.loss_part = None
+        self.refused = None  # scratch elements that did not fit
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
 
     def ensure(self, scratch_elems: int, partial_elems: int, grid: int):
@@ -390,13 +391,19 @@ def plan_and_bind(a, device, adjoint: bool, grid=None):
     if not adjoint:
         ws.ensure(0, 0, grid_v)
     else:
+        # one CTA per SM holds less scratch.  What did not fit once is not tried again: a warmed-up capture
+        # meets no failing allocation
+        sms = sm_count(torch.device(device))
+        shrinks = grid is None and v.value == _lib.VARIANTS["serial"] and grid_v > sms
+        if shrinks and ws.refused is not None and se.value >= ws.refused:
+            return plan_and_bind(a, device, adjoint, grid=sms)
         try:
             ws.ensure(se.value, pe.value, grid_v)
         except torch.OutOfMemoryError:
-            sms = sm_count(torch.device(device))
-            if grid is not None or v.value != _lib.VARIANTS["serial"] or grid_v <= sms:
+            if not shrinks:
                 raise
-            return plan_and_bind(a, device, adjoint, grid=sms)  # one CTA per SM holds less scratch
+            ws.refused = se.value
+            return plan_and_bind(a, device, adjoint, grid=sms)
     a.grid = grid_v
     a.scratch = ws.scratch.data_ptr() if adjoint else None
     a.probe_grad_part = ws.partials.data_ptr() if adjoint else None
